@@ -621,13 +621,6 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     a.probe = cols_of(P);
     const bool mat = materialize_probe_estimate(ctx, B) && P.rows > 0;
     cudaStream_t main_stream = ctx->stream;
-    // the two sides' partition passes share the GPU: register-capped scatter
-    struct BesideGuard
-    {
-        phj_ctx * c;
-        ~BesideGuard() { c->p1_beside = false; }
-    } beside_guard{ctx};
-    ctx->p1_beside = mat;
     if (mat)
     {
         if (!ctx->side)
@@ -642,21 +635,7 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
             const bool split = pb > 11;
             const Cols ptmp = split ? alloc_cols_like(s, P.schema, P.rows) : ppart;
             uint32_t * poff = s.get<uint32_t>((1ull << pb) + 1);
-            // a two-stage ring leaves shared memory on each SM for the build
-            // side's kernels running beside this pass (unless pinned)
-            const uint32_t pinned_stages = ctx->p1_stages;
-            if (!pinned_stages)
-                ctx->p1_stages = 2;
-            try
-            {
-                radix_partition(ctx, s, a.probe, P.rows, {pb}, ppart, ptmp, poff, "probe_scatter");
-            }
-            catch (...)
-            {
-                ctx->p1_stages = pinned_stages;
-                throw;
-            }
-            ctx->p1_stages = pinned_stages;
+            radix_partition(ctx, s, a.probe, P.rows, {pb}, ppart, ptmp, poff, "probe_scatter");
             a.probe = ppart;
             PHJ_CUDA(cudaEventRecord(ev[6], ctx->stream));
         }
@@ -687,7 +666,11 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
         a.build = payload_cols(bpart);
         a.any_dup = 0;
         if (!ctx->aux)
-            PHJ_CUDA(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
+        {
+            int least = 0, greatest = 0; // as the main stream's
+            PHJ_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            PHJ_CUDA(cudaStreamCreateWithPriority(&ctx->aux, cudaStreamNonBlocking, greatest));
+        }
         PHJ_CUDA(cudaEventRecord(ev[7], ctx->stream));
         PHJ_CUDA(cudaStreamWaitEvent(ctx->aux, ev[7], 0));
         ctx->stream = ctx->aux;
@@ -803,12 +786,6 @@ static void run_phj_bep(phj_ctx * ctx, const phj_table & B, const phj_table & P,
     cudaStream_t main_stream = ctx->stream;
     const bool early = P.rows > 0;
     cudaEvent_t es[2] = {take_event(ctx), take_event(ctx)}; // the side pass's span
-    struct BesideGuard
-    {
-        phj_ctx * c;
-        ~BesideGuard() { c->p1_beside = false; }
-    } beside_guard{ctx};
-    ctx->p1_beside = early;
     if (early)
     {
         if (!ctx->side)
@@ -817,24 +794,18 @@ static void run_phj_bep(phj_ctx * ctx, const phj_table & B, const phj_table & P,
         PHJ_CUDA(cudaEventRecord(ready, ctx->stream));
         PHJ_CUDA(cudaStreamWaitEvent(ctx->side, ready, 0));
         ctx->stream = ctx->side;
-        const uint32_t pinned_stages = ctx->p1_stages;
         try
         {
             PHJ_CUDA(cudaEventRecord(es[0], ctx->stream));
             // the batch's first radix pass also flags the leaves its rows
-            // touch (its histogram reads every key once anyway); a two-stage
-            // ring leaves shared memory for the build side's kernels
+            // touch (its histogram reads every key once anyway)
             ctx->leaf_mark = LeafMark{touched, 64u - total_bits, (n_leaves + 31) / 32};
-            if (!pinned_stages)
-                ctx->p1_stages = 2;
             radix_partition(ctx, s, pin, std::min(batch_rows, P.rows), {pb}, ppart, ptmp, poff, "probe_scatter");
-            ctx->p1_stages = pinned_stages;
             ctx->leaf_mark = LeafMark{};
             PHJ_CUDA(cudaEventRecord(es[1], ctx->stream));
         }
         catch (...)
         {
-            ctx->p1_stages = pinned_stages;
             ctx->leaf_mark = LeafMark{};
             ctx->stream = main_stream;
             cudaStreamSynchronize(ctx->side);
@@ -855,7 +826,6 @@ static void run_phj_bep(phj_ctx * ctx, const phj_table & B, const phj_table & P,
         throw;
     }
     PHJ_CUDA(cudaEventRecord(ev[1], ctx->stream));
-    ctx->p1_beside = false;
 
     // -------- BUILD: table layout only; cells are built on first use --------
     LeafTables lt;
@@ -1640,7 +1610,11 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         ctx->num_sms = prop.multiProcessorCount;
         ctx->smem_optin = prop.sharedMemPerBlockOptin;
         ctx->l2_bytes = prop.l2CacheSize;
-        PHJ_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+        // the main stream goes first: its kernels take the SMs as the side
+        // stream's short CTAs end (probe side's first pass, see k_scatter)
+        int prio_least = 0, prio_greatest = 0;
+        PHJ_CUDA(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
+        PHJ_CUDA(cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, prio_greatest));
         cudaMemPoolProps pp{};
         pp.allocType = cudaMemAllocationTypePinned;
         pp.location.type = cudaMemLocationTypeDevice;

@@ -3,20 +3,23 @@
 // refineToLeaves :417-539).
 //
 // One physical pass splits every segment of the previous pass (rows that
-// share their top c_prev hash bits, stored contiguously) into 2^b
-// sub-buckets on the next b bits.  Three kernels per pass:
-//   k_part_hist    per 4096-row tile: shared-memory histogram of the b-bit
-//                  digit, one count per (segment, digit, tile) written
-//                  digit-major;
-//   scan_u32       device-wide exclusive scan over those counts, which yields
-//                  every tile's first output row for every digit;
-//   k_part_scatter re-reads the tile, ranks its rows by digit in shared
-//                  memory, and for each column (key first, then payloads of
-//                  1/2/4/8/16 bytes) stages the tile in digit order and writes
-//                  each digit's run contiguously -- the column-first scatter
-//                  of the reference, with the staging done in shared memory so
-//                  stores coalesce.
-// No atomics touch global memory; the output is deterministic.
+// share their top hash bits, stored contiguously; the first pass has one
+// segment, the input) into 2^b buckets on the next b bits:
+//   k_p1_hist / k_seg_hist   rows per bucket: shared-memory histograms, added
+//                  to the buckets' global counts;
+//   a scan         bucket counts -> bucket offsets (the first pass's last
+//                  histogram CTA does it; later passes use scan_u32);
+//   k_scatter      tiles of 4096 rows (one segment's each) arrive in shared
+//                  memory by bulk asynchronous copies, their rows are ranked
+//                  by digit, each tile reserves its rows' places with one
+//                  atomic per digit on the bucket's count, and every column
+//                  (key first, then payloads of 1/2/4/8/16 bytes) is written
+//                  in digit order -- the column-first scatter of the
+//                  reference, so that stores coalesce.
+// The tiles of all CTAs in flight write next to each other in every bucket
+// (one frontier a bucket, not one a bucket and CTA), and no per-tile counts
+// are written, scanned and read back.  The order of the rows inside a bucket
+// is not fixed, as in the reference.
 #include "internal.h"
 
 namespace phjg
@@ -24,10 +27,11 @@ namespace phjg
 namespace
 {
 constexpr int kNT = 512;
-constexpr int kRPT = 8;
-constexpr uint32_t kTile = kNT * kRPT; // rows per tile
 constexpr uint32_t kMaxPassBits = 11;  // shared-memory digit histogram <= 2048 bins
+constexpr uint32_t kMaxRPT = 8;        // rows per thread of a tile: 4096-row tiles
+constexpr uint32_t kMaxStages = 4;
 
+// One segment's tiles of a later pass: row0, rows, first bucket.
 struct PassGeom
 {
     const uint32_t * seg_off;  // n_segs + 1: first row of each input segment
@@ -37,261 +41,45 @@ struct PassGeom
     uint32_t b;
 };
 
-struct TileRef
-{
-    uint32_t seg, k, nt, row0, row1, tile0;
-};
-
-__device__ __forceinline__ bool locate_tile(const PassGeom & g, uint32_t t, TileRef & r)
-{
-    const uint32_t total = g.tile_pre[g.n_segs];
-    if (t >= total)
-        return false;
-    // Largest s with tile_pre[s] <= t; segments without tiles are skipped
-    // because then tile_pre[s] == tile_pre[s+1].
-    uint32_t lo = 0, hi = g.n_segs; // invariant: tile_pre[lo] <= t < tile_pre[hi]
-    while (hi - lo > 1)
-    {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (g.tile_pre[mid] <= t)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    r.seg = lo;
-    r.tile0 = g.tile_pre[lo];
-    r.k = t - r.tile0;
-    r.nt = g.tile_pre[lo + 1] - r.tile0;
-    const uint32_t s0 = g.seg_off[lo], s1 = g.seg_off[lo + 1];
-    r.row0 = s0 + r.k * kTile;
-    r.row1 = min(r.row0 + kTile, s1);
-    return true;
-}
-
-
-__global__ void __launch_bounds__(kNT) k_part_hist(const uint64_t * __restrict__ keys, PassGeom g, uint32_t * __restrict__ counts)
-{
-    extern __shared__ uint32_t bins[];
-    TileRef tr;
-    if (!locate_tile(g, blockIdx.x, tr))
-        return;
-    const uint32_t nb = 1u << g.b, mask = nb - 1;
-    for (uint32_t i = threadIdx.x; i < nb; i += kNT)
-        bins[i] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-    {
-        const uint32_t row = tr.row0 + j * kNT + threadIdx.x;
-        if (row < tr.row1)
-            atomicAdd(&bins[(uint32_t)(int_hash64(__ldcs(keys + row)) >> g.shift) & mask], 1u);
-    }
-    __syncthreads();
-    const uint64_t base = (uint64_t)tr.tile0 * nb;
-    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
-        counts[base + (uint64_t)d * tr.nt + tr.k] = bins[d];
-}
-
-// Exclusive scan of nb bins in shared memory by kNT threads.
-// Exclusive scan of the tile's digit counts by the first warp alone (the
-// caller's next barrier publishes excl).
-__device__ __forceinline__ void smem_bins_scan(const uint32_t * bins, uint32_t * excl, uint32_t nb)
-{
-    if (threadIdx.x >= 32)
-        return;
-    const uint32_t lane = threadIdx.x;
-    const uint32_t per = (nb + 31) / 32;
-    const uint32_t b0 = lane * per;
-    uint32_t local = 0;
-    for (uint32_t i = 0; i < per; ++i)
-        if (b0 + i < nb)
-            local += bins[b0 + i];
-    uint32_t x = local;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-    {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= (uint32_t)d)
-            x += y;
-    }
-    uint32_t run = x - local;
-    for (uint32_t i = 0; i < per; ++i)
-        if (b0 + i < nb)
-        {
-            excl[b0 + i] = run;
-            run += bins[b0 + i];
-        }
-}
-
-// One column of the tile: stage it in digit order in shared memory, then
-// each thread stores its kRPT staged elements to their precomputed rows.
-template <class T>
-__device__ __forceinline__ void scatter_column(const T * __restrict__ src, T * __restrict__ dst, T * stage, const uint32_t (&lp)[kRPT],
-                                               const uint32_t (&dest)[kRPT], const TileRef & tr)
-{
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-    {
-        const uint32_t row = tr.row0 + j * kNT + threadIdx.x;
-        if (row < tr.row1)
-            stage[lp[j]] = __ldcs(src + row);
-    }
-    __syncthreads();
-    const uint32_t cnt = tr.row1 - tr.row0;
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-    {
-        const uint32_t pos = j * kNT + threadIdx.x;
-        if (pos < cnt)
-            dst[dest[j]] = stage[pos];
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(kNT, 2) k_part_scatter(const __grid_constant__ Cols in, const __grid_constant__ Cols out,
-                                                         const __grid_constant__ PassGeom g, const uint32_t * __restrict__ offs, uint32_t maxw)
-{
-    extern __shared__ __align__(16) uint8_t smem[];
-    TileRef tr;
-    if (!locate_tile(g, blockIdx.x, tr))
-        return;
-    const uint32_t nb = 1u << g.b, mask = nb - 1;
-    uint8_t * stage = smem;
-    uint16_t * sorted_d = reinterpret_cast<uint16_t *>(smem + (size_t)kTile * maxw);
-    uint32_t * bins = reinterpret_cast<uint32_t *>(sorted_d + kTile);
-    uint32_t * excl = bins + nb;
-    uint32_t * gbase = excl + nb;
-
-    for (uint32_t i = threadIdx.x; i < nb; i += kNT)
-        bins[i] = 0;
-    __syncthreads();
-
-    // digit and rank within the digit (shared atomics return the rank)
-    uint64_t key[kRPT];
-    uint32_t lp[kRPT]; // digit, then position in the tile's digit order
-    uint32_t rank[kRPT];
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-    {
-        const uint32_t row = tr.row0 + j * kNT + threadIdx.x;
-        lp[j] = 0xFFFFFFFFu;
-        key[j] = 0;
-        rank[j] = 0;
-        if (row < tr.row1)
-        {
-            key[j] = __ldcs(in.keys + row);
-            lp[j] = (uint32_t)(int_hash64(key[j]) >> g.shift) & mask;
-            rank[j] = atomicAdd(&bins[lp[j]], 1u);
-        }
-    }
-    __syncthreads();
-    smem_bins_scan(bins, excl, nb);
-    const uint64_t ebase = (uint64_t)tr.tile0 * nb;
-    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
-        gbase[d] = offs[ebase + (uint64_t)d * tr.nt + tr.k];
-    __syncthreads();
-
-    uint64_t * stage64 = reinterpret_cast<uint64_t *>(stage);
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-        if (lp[j] != 0xFFFFFFFFu)
-        {
-            const uint32_t d = lp[j];
-            lp[j] = excl[d] + rank[j];
-            stage64[lp[j]] = key[j];
-            sorted_d[lp[j]] = (uint16_t)d;
-        }
-        else
-            lp[j] = 0;
-    __syncthreads();
-    // Each thread owns tile positions j*kNT + tid: their output rows.
-    const uint32_t cnt = tr.row1 - tr.row0;
-    uint32_t dest[kRPT];
-#pragma unroll
-    for (int j = 0; j < kRPT; ++j)
-    {
-        const uint32_t pos = j * kNT + threadIdx.x;
-        dest[j] = 0;
-        if (pos < cnt)
-        {
-            const uint32_t d = sorted_d[pos];
-            dest[j] = gbase[d] + (pos - excl[d]);
-            out.keys[dest[j]] = stage64[pos];
-        }
-    }
-    __syncthreads();
-
-    for (uint32_t c = 0; c < in.n; ++c)
-    {
-        switch (in.width[c])
-        {
-            case 1: scatter_column<uint8_t>((const uint8_t *)in.col[c], (uint8_t *)out.col[c], stage, lp, dest, tr); break;
-            case 2: scatter_column<uint16_t>((const uint16_t *)in.col[c], (uint16_t *)out.col[c], (uint16_t *)stage, lp, dest, tr); break;
-            case 4: scatter_column<uint32_t>((const uint32_t *)in.col[c], (uint32_t *)out.col[c], (uint32_t *)stage, lp, dest, tr); break;
-            case 8: scatter_column<uint64_t>((const uint64_t *)in.col[c], (uint64_t *)out.col[c], (uint64_t *)stage, lp, dest, tr); break;
-            default: scatter_column<uint4>((const uint4 *)in.col[c], (uint4 *)out.col[c], (uint4 *)stage, lp, dest, tr); break;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// First pass (one input segment): each CTA owns a contiguous range of whole
-// tiles, so the histogram is per CTA (digit-major, 2^b x G counts) and the
-// scatter keeps one running output cursor per digit in shared memory.  Tiles
-// arrive by bulk asynchronous copies (cp.async.bulk through the TMA engine)
-// into two shared-memory buffers: tile t+1 streams in while tile t is ranked
-// and written out, with no registers spent on prefetching.
+// Histograms
 // ---------------------------------------------------------------------------
-constexpr int kP1NT = 512;
 
-struct P1Geom
-{
-    uint64_t n;
-    uint32_t tiles_per_cta;
-    uint32_t tile_rows;
-    uint32_t shift, b;
-};
-
-// H CTAs share one scatter CTA's row range (counts are zeroed first and
-// summed with global atomics), so the histogram keeps more loads in flight
-// than the scatter's one-CTA-per-SM grid would.
+// First pass: bucket counts, then (in the CTA that finishes last) the
+// bucket offsets off[0..2^b].  `done` is zero at launch.
 // With `mark` set (PHJ/BEP probe batches) the same pass also flags the
 // leaves the rows hash to: a shared-memory bitmap per CTA (a bit is read
 // before it is set), ORed into the global bitmap at the end.
-__global__ void __launch_bounds__(kP1NT) k_p1_hist(const uint64_t * __restrict__ keys, P1Geom g, uint32_t H, uint32_t G,
-                                                   uint32_t * __restrict__ counts, LeafMark mark)
+__global__ void __launch_bounds__(kNT) k_p1_hist(const uint64_t * __restrict__ keys, uint64_t n, uint32_t shift, uint32_t b,
+                                                 uint32_t * __restrict__ counts, uint32_t * __restrict__ done, uint32_t * __restrict__ off,
+                                                 LeafMark mark)
 {
     extern __shared__ uint32_t bins[];
-    const uint32_t nb = 1u << g.b, mask = nb - 1;
+    __shared__ uint32_t ws[kNT / 32];
+    __shared__ uint32_t last;
+    const uint32_t nb = 1u << b, mask = nb - 1;
     uint32_t * bm = bins + nb;
-    for (uint32_t i = threadIdx.x; i < nb; i += kP1NT)
+    for (uint32_t i = threadIdx.x; i < nb; i += kNT)
         bins[i] = 0;
     if (mark.bits)
-        for (uint32_t i = threadIdx.x; i < mark.words; i += kP1NT)
+        for (uint32_t i = threadIdx.x; i < mark.words; i += kNT)
             bm[i] = 0;
     __syncthreads();
-    const uint32_t gi = blockIdx.x / H, q = blockIdx.x % H;
-    const uint64_t span = (uint64_t)g.tiles_per_cta * g.tile_rows;
-    const uint64_t g0 = (uint64_t)gi * span;
-    const uint64_t g1 = min(g.n, g0 + span);
-    const uint64_t part = ceil_div(span, (uint64_t)H * 8 * kP1NT) * 8 * kP1NT;
-    const uint64_t r0 = g0 + q * part;
-    const uint64_t r1 = min(g1, r0 + part);
-    for (uint64_t base = r0; base < r1; base += 8 * kP1NT)
+    for (uint64_t base = (uint64_t)blockIdx.x * 8 * kNT; base < n; base += (uint64_t)gridDim.x * 8 * kNT)
     {
         uint64_t k[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
         {
-            const uint64_t row = base + j * kP1NT + threadIdx.x;
-            k[j] = row < r1 ? __ldcs(keys + row) : 0;
+            const uint64_t row = base + j * kNT + threadIdx.x;
+            k[j] = row < n ? __ldcs(keys + row) : 0;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (base + j * kP1NT + threadIdx.x < r1)
+            if (base + j * kNT + threadIdx.x < n)
             {
                 const uint64_t h = int_hash64(k[j]);
-                atomicAdd(&bins[(uint32_t)(h >> g.shift) & mask], 1u);
+                atomicAdd(&bins[(uint32_t)(h >> shift) & mask], 1u);
                 if (mark.bits)
                 {
                     const uint32_t L = (uint32_t)(h >> mark.shift);
@@ -301,362 +89,573 @@ __global__ void __launch_bounds__(kP1NT) k_p1_hist(const uint64_t * __restrict__
             }
     }
     __syncthreads();
-    for (uint32_t d = threadIdx.x; d < nb; d += kP1NT)
+    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
         if (bins[d])
-            atomicAdd(&counts[(uint64_t)d * G + gi], bins[d]);
+            atomicAdd(&counts[d], bins[d]);
     if (mark.bits)
-        for (uint32_t w = threadIdx.x; w < mark.words; w += kP1NT)
+        for (uint32_t w = threadIdx.x; w < mark.words; w += kNT)
         {
             const uint32_t v = bm[w];
             if (v && (__ldcg(mark.bits + w) & v) != v)
                 atomicOr(mark.bits + w, v);
         }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+    constexpr uint32_t kPer = (1u << kMaxPassBits) / kNT;
+    const uint32_t per = (nb + kNT - 1) / kNT, d0 = threadIdx.x * per;
+    uint32_t v[kPer], acc = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i)
+    {
+        v[i] = i < per && d0 + i < nb ? __ldcg(counts + d0 + i) : 0u;
+        acc += v[i];
+    }
+    uint32_t total;
+    uint32_t run = block_excl_scan<kNT>(acc, ws, &total);
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i)
+        if (i < per && d0 + i < nb)
+        {
+            off[d0 + i] = run;
+            run += v[i];
+        }
+    if (threadIdx.x == 0)
+        off[nb] = total;
 }
 
-struct P1Smem
+// Later passes, one CTA: first tile of each of at most 4 * 1024 segments.
+__global__ void __launch_bounds__(1024) k_seg_tiles(const uint32_t * __restrict__ seg_off, uint32_t n_segs, uint32_t tile_rows,
+                                                    uint32_t * __restrict__ tile_pre)
+{
+    __shared__ uint32_t ws[32];
+    const uint32_t per = (n_segs + 1023) / 1024, s0 = threadIdx.x * per;
+    uint32_t v[4], acc = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+    {
+        v[i] = i < per && s0 + i < n_segs ? (seg_off[s0 + i + 1] - seg_off[s0 + i] + tile_rows - 1) / tile_rows : 0u;
+        acc += v[i];
+    }
+    uint32_t total;
+    uint32_t run = block_excl_scan<1024>(acc, ws, &total);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+        if (i < per && s0 + i < n_segs)
+        {
+            tile_pre[s0 + i] = run;
+            run += v[i];
+        }
+    if (threadIdx.x == 0)
+        tile_pre[n_segs] = total;
+}
+
+__global__ void k_tiles_per_seg(const uint32_t * __restrict__ seg_off, uint32_t n_segs, uint32_t tile_rows, uint32_t * __restrict__ nt)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < n_segs)
+        nt[s] = (seg_off[s + 1] - seg_off[s] + tile_rows - 1) / tile_rows;
+}
+
+// Later passes: each CTA counts a contiguous range of tiles, adding its
+// histogram to the segment's buckets when the segment changes, and writes
+// the tiles' descriptors {first row, rows, first bucket} for the scatter.
+template <int RPT>
+__global__ void __launch_bounds__(kNT) k_seg_hist(const uint64_t * __restrict__ keys, PassGeom g, uint32_t * __restrict__ counts,
+                                                  uint4 * __restrict__ desc)
+{
+    constexpr uint32_t kT = kNT * RPT;
+    extern __shared__ uint32_t bins[];
+    const uint32_t nb = 1u << g.b, mask = nb - 1;
+    const uint32_t n_tiles = g.tile_pre[g.n_segs];
+    const uint32_t t0 = (uint32_t)((uint64_t)n_tiles * blockIdx.x / gridDim.x), t1 = (uint32_t)((uint64_t)n_tiles * (blockIdx.x + 1) / gridDim.x);
+    if (t0 >= t1)
+        return;
+    // largest s with tile_pre[s] <= t0 (segments without tiles are skipped:
+    // tile_pre[s] == tile_pre[s + 1] there)
+    uint32_t seg = 0, hi = g.n_segs;
+    while (hi - seg > 1)
+    {
+        const uint32_t mid = (seg + hi) >> 1;
+        if (g.tile_pre[mid] <= t0)
+            seg = mid;
+        else
+            hi = mid;
+    }
+    for (uint32_t i = threadIdx.x; i < nb; i += kNT)
+        bins[i] = 0;
+    __syncthreads();
+    uint32_t seg_end = g.tile_pre[seg + 1];
+    for (uint32_t t = t0; t < t1; ++t)
+    {
+        if (t >= seg_end)
+        {
+            // the segment's histogram so far, then the next segment
+            __syncthreads();
+            for (uint32_t d = threadIdx.x; d < nb; d += kNT)
+                if (bins[d])
+                {
+                    atomicAdd(&counts[((uint64_t)seg << g.b) + d], bins[d]);
+                    bins[d] = 0;
+                }
+            __syncthreads();
+            while (t >= seg_end)
+                seg_end = g.tile_pre[++seg + 1];
+        }
+        const uint32_t row0 = g.seg_off[seg] + (t - g.tile_pre[seg]) * kT, cnt = min(kT, g.seg_off[seg + 1] - row0);
+        if (threadIdx.x == 0)
+            desc[t] = make_uint4(row0, cnt, seg << g.b, 0);
+        uint64_t k[RPT];
+#pragma unroll
+        for (int j = 0; j < RPT; ++j)
+        {
+            const uint32_t i = j * kNT + threadIdx.x;
+            k[j] = i < cnt ? keys[row0 + i] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < RPT; ++j)
+            if (j * kNT + threadIdx.x < cnt)
+                atomicAdd(&bins[(uint32_t)(int_hash64(k[j]) >> g.shift) & mask], 1u);
+    }
+    __syncthreads();
+    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
+        if (bins[d])
+            atomicAdd(&counts[((uint64_t)seg << g.b) + d], bins[d]);
+}
+
+// ---------------------------------------------------------------------------
+// Scatter
+// ---------------------------------------------------------------------------
+struct TileSmem
 {
     uint32_t buf_bytes;              // one tile of every column
     uint32_t col_off[kMaxCols + 1];  // byte offset of each payload column in a buffer (keys at 0)
 };
 
+struct ScatterGeom
+{
+    uint64_t n;               // rows (first pass)
+    const uint4 * desc;       // later passes: tile descriptors, nullptr in the first pass
+    const uint32_t * n_tiles; // later passes: number of tiles (device)
+    uint32_t shift, b;
+    uint32_t wave, tiles_per_cta; // tile k of CTA c: (c / wave) * wave * tiles_per_cta + k * wave + c % wave
+    uint32_t stages;
+    int use_tma;
+};
+
 template <class T, int RPT>
-__device__ __forceinline__ void p1_write_column(const uint8_t * buf, T * __restrict__ dst, const uint32_t (&src)[RPT], const uint32_t (&dest)[RPT],
-                                                uint32_t cnt)
+__device__ __forceinline__ void write_column(const uint8_t * buf, T * __restrict__ dst, const uint32_t (&src)[RPT], const uint32_t (&dest)[RPT],
+                                             uint32_t cnt)
 {
     const T * b = reinterpret_cast<const T *>(buf);
 #pragma unroll
     for (int j = 0; j < RPT; ++j)
-        if (j * kP1NT + threadIdx.x < cnt)
+        if (j * kNT + threadIdx.x < cnt)
             dst[dest[j]] = b[src[j]];
 }
 
-// kMinB 2 holds the kernel to 64 registers a thread (a launch bound of two
-// CTAs, though shared memory admits one): half of the register file stays
-// free, so the build side's later pass (scan, histogram, scatter) runs
-// beside the probe side's first pass instead of waiting for it to retire.
-// A pass that runs alone takes kMinB 1 (72 registers).
-template <int RPT, int kMinB>
-__global__ void __launch_bounds__(kP1NT, kMinB) k_p1_scatter(const __grid_constant__ Cols in, const __grid_constant__ Cols out, P1Geom g,
-                                                         const __grid_constant__ P1Smem sm, uint32_t stages, const uint32_t * __restrict__ offs,
-                                                         int use_tma, int * __restrict__ err)
+// Bound by DRAM when enough tiles are in flight: a tile is a chain of
+// dependent steps (rank with shared atomics, digit scan, reservation,
+// permutation, column writes) with three block barriers, during which one
+// CTA alone leaves the SM idle, so two CTAs of 512 threads share a SM (64
+// registers a thread, at most half of the shared memory each) and one's
+// copies and writes fill the other's barriers.  Measured (256M rows of 16
+// bytes, 6 bits): 5.4 TB/s, 80% of a plain copy's rate; one CTA a SM with a
+// deeper ring reached 4.0 (stalls: block barriers, then shared memory).
+template <int RPT, bool kLater>
+__global__ void __launch_bounds__(kNT, 2) k_scatter(const __grid_constant__ Cols in, const __grid_constant__ Cols out,
+                                                    const __grid_constant__ ScatterGeom g, const __grid_constant__ TileSmem sm,
+                                                    const uint32_t * __restrict__ offs, uint32_t * __restrict__ counts, int * __restrict__ err)
 {
-    constexpr uint32_t kT = kP1NT * RPT;
-    constexpr uint32_t kMaxStages = 4;
+    constexpr uint32_t kT = kNT * RPT;
+    constexpr uint32_t kWarps = kNT / 32;
+    constexpr int kRows = (1 << kMaxPassBits) / 32 / kWarps; // 32-digit rows a warp scans
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar[kMaxStages];
-    uint16_t * inv = reinterpret_cast<uint16_t *>(smem + (size_t)stages * sm.buf_bytes);
-    uint16_t * dsort = inv + kT;
     const uint32_t nb = 1u << g.b, mask = nb - 1;
-    uint32_t * bins = reinterpret_cast<uint32_t *>(dsort + kT);
+    uint32_t * perm = reinterpret_cast<uint32_t *>(smem + (size_t)g.stages * sm.buf_bytes); // tile row | digit << 12, in digit order
+    uint32_t * bins = perm + kT;
     uint32_t * excl = bins + nb;
-    // running output cursors per digit, two arrays in turn: the scan of tile
-    // t writes tile t+1's cursors while tile t's are still being read, so no
-    // barrier is needed to advance them
-    uint32_t * cur = excl + nb;
-    uint32_t * nxt = cur + nb;
+    uint32_t * delta = excl + nb; // output row of a digit's first row, less its position in the tile's digit order
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    const uint64_t n_tiles = ceil_div(g.n, kT);
-    const uint64_t t_begin = (uint64_t)blockIdx.x * g.tiles_per_cta;
-    const uint64_t t_end = min(n_tiles, t_begin + g.tiles_per_cta);
-    if (t_begin >= t_end)
+    const uint64_t n_tiles = kLater ? *g.n_tiles : ceil_div(g.n, kT);
+    const uint64_t t_first = (uint64_t)(blockIdx.x / g.wave) * g.wave * g.tiles_per_cta + blockIdx.x % g.wave;
+    if (t_first >= n_tiles)
         return;
-    for (uint32_t d = threadIdx.x; d < nb; d += kP1NT)
-    {
-        cur[d] = offs[(uint64_t)d * gridDim.x + blockIdx.x];
+    const uint32_t my_tiles = (uint32_t)min((uint64_t)g.tiles_per_cta, (n_tiles - t_first + g.wave - 1) / g.wave);
+    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
         bins[d] = 0;
-    }
     if (threadIdx.x == 0)
     {
-        for (uint32_t i = 0; i < stages; ++i)
+        for (uint32_t i = 0; i < g.stages; ++i)
             mbar_init(&bar[i], 1);
         fence_barrier_init();
     }
     __syncthreads();
 
-    // A tile is fetched by bulk copy when every column slice is a whole
-    // number of 16-byte units (always, except a short last tile).
-    auto tile_rows = [&](uint64_t t) -> uint32_t { const uint64_t r = g.n - t * kT; return r < kT ? (uint32_t)r : kT; };
-    auto tma_ok = [&](uint64_t t) -> bool {
-        if (!use_tma)
-            return false;
-        const uint32_t r = tile_rows(t);
-        if ((r * 8u) & 15u)
+    auto tile_of = [&](uint32_t k) -> uint4 {
+        const uint64_t t = t_first + (uint64_t)k * g.wave;
+        if (kLater)
+            return __ldg(g.desc + t);
+        const uint64_t r = g.n - t * kT;
+        return make_uint4((uint32_t)(t * kT), r < kT ? (uint32_t)r : kT, 0, 0);
+    };
+    // A first-pass tile is fetched by bulk copy when every column slice is a
+    // whole number of 16-byte units (always, except a short last tile); a
+    // later pass reads the library's own buffers (256-byte granules), where
+    // a slice may be widened to 16-byte units on both sides.
+    auto tma_ok = [&](const uint4 & t) -> bool {
+        if (kLater)
+            return true;
+        if (!g.use_tma || ((t.y * 8u) & 15u))
             return false;
         for (uint32_t c = 0; c < in.n; ++c)
-            if ((r * in.width[c]) & 15u)
+            if ((t.y * in.width[c]) & 15u)
                 return false;
         return true;
     };
     auto buffer = [&](uint32_t i) -> uint8_t * { return smem + (size_t)i * sm.buf_bytes; };
-    auto issue = [&](uint64_t t, uint32_t bi) {
-        const uint32_t r = tile_rows(t);
-        uint32_t bytes = r * 8u;
+    auto issue = [&](const uint4 & t, uint32_t bi) {
+        auto span = [&](uint32_t w, uint64_t & a) -> uint32_t {
+            a = ((uint64_t)t.x * w) & ~15ull;
+            return (uint32_t)((((uint64_t)(t.x + t.y) * w + 15) & ~15ull) - a);
+        };
+        uint64_t a;
+        uint32_t bytes = span(8, a);
         for (uint32_t c = 0; c < in.n; ++c)
-            bytes += r * in.width[c];
+            bytes += span(in.width[c], a);
         fence_proxy_async_smem();
         mbar_arrive_expect_tx(&bar[bi], bytes);
-        bulk_copy_g2s(buffer(bi), in.keys + t * kT, r * 8u, &bar[bi]);
+        const uint32_t kb = span(8, a);
+        bulk_copy_g2s(buffer(bi), reinterpret_cast<const uint8_t *>(in.keys) + a, kb, &bar[bi]);
         for (uint32_t c = 0; c < in.n; ++c)
-            bulk_copy_g2s(buffer(bi) + sm.col_off[c], static_cast<const uint8_t *>(in.col[c]) + t * kT * in.width[c], r * in.width[c], &bar[bi]);
+        {
+            const uint32_t cb = span(in.width[c], a);
+            bulk_copy_g2s(buffer(bi) + sm.col_off[c], static_cast<const uint8_t *>(in.col[c]) + a, cb, &bar[bi]);
+        }
     };
+    // tiles in flight ahead of the one being written: stages - 1, or the
+    // next one once this one's buffer is free
+    const uint32_t ahead = g.stages > 1 ? g.stages - 1 : 1;
     uint32_t parity = 0; // bit i: phase of bar[i] to wait for
     if (threadIdx.x == 0)
-        for (uint32_t i = 0; i + 1 < stages && t_begin + i < t_end; ++i)
-            if (tma_ok(t_begin + i))
-                issue(t_begin + i, i);
+        for (uint32_t i = 0; i < ahead && i < my_tiles; ++i)
+        {
+            const uint4 t = tile_of(i);
+            if (tma_ok(t))
+                issue(t, i);
+        }
 
     uint32_t bi = 0;
-    for (uint64_t t = t_begin; t < t_end; ++t, bi = (bi + 1 == stages) ? 0 : bi + 1)
+    for (uint32_t k = 0; k < my_tiles; ++k, bi = (bi + 1 == g.stages) ? 0 : bi + 1)
     {
-        const uint32_t cnt = tile_rows(t);
+        const uint4 tile = tile_of(k);
+        const uint32_t cnt = tile.y;
         uint8_t * buf = buffer(bi);
-        if (tma_ok(t))
+        bool ok = true;
+        if (tma_ok(tile))
         {
-            const bool ok = mbar_wait(&bar[bi], (parity >> bi) & 1u, err, 1);
-            if (!__syncthreads_and(ok))
-                break;
-            parity ^= 1u << bi;
+            ok = mbar_wait(&bar[bi], (parity >> bi) & 1u, err, 1);
         }
         else
         {
             uint64_t * bk = reinterpret_cast<uint64_t *>(buf);
-            for (uint32_t i = threadIdx.x; i < cnt; i += kP1NT)
-                bk[i] = in.keys[t * kT + i];
+            for (uint32_t i = threadIdx.x; i < cnt; i += kNT)
+                bk[i] = in.keys[tile.x + i];
             for (uint32_t c = 0; c < in.n; ++c)
-                for (uint32_t i = threadIdx.x; i < cnt; i += kP1NT)
-                    copy_elem(buf + sm.col_off[c], i, in.col[c], t * kT + i, in.width[c]);
+                for (uint32_t i = threadIdx.x; i < cnt; i += kNT)
+                    copy_elem(buf + sm.col_off[c], i, in.col[c], (uint64_t)tile.x + i, in.width[c]);
             __syncthreads();
         }
-        // keep stages-1 tiles in flight: refill the buffer the previous tile
-        // used (its readers finished at the barrier ending that iteration)
-        const uint32_t nbi = (bi + stages - 1) % stages;
-        if (threadIdx.x == 0 && t + stages - 1 < t_end && tma_ok(t + stages - 1))
-            issue(t + stages - 1, nbi);
-        // (bins were zeroed by the last tile's scan)
+        // bytes of a column before the tile's first row in its buffer
+        auto lead = [&](uint32_t w) -> uint32_t { return kLater ? (tile.x * w) & 15u : 0u; };
 
-        const uint64_t * bk = reinterpret_cast<const uint64_t *>(buf);
-        uint32_t dg[RPT], rk[RPT];
+        // digit and rank within the digit (bins are zero here)
+        const uint64_t * bk = reinterpret_cast<const uint64_t *>(buf + lead(8));
+        uint32_t dr[RPT]; // digit | rank << 11
 #pragma unroll
         for (int j = 0; j < RPT; ++j)
         {
-            const uint32_t i = j * kP1NT + threadIdx.x;
-            dg[j] = 0xFFFFu;
-            rk[j] = 0;
+            const uint32_t i = j * kNT + threadIdx.x;
+            dr[j] = 0xFFFFFFFFu;
             if (i < cnt)
             {
-                dg[j] = (uint32_t)(int_hash64(bk[i]) >> g.shift) & mask;
-                rk[j] = atomicAdd(&bins[dg[j]], 1u);
+                const uint32_t d = (uint32_t)(int_hash64(bk[i]) >> g.shift) & mask;
+                dr[j] = d | atomicAdd(&bins[d], 1u) << kMaxPassBits;
             }
         }
-        __syncthreads();
-        // exclusive scan of the digit counts by the first warp alone (one
-        // barrier instead of the block scan's three), which also advances
-        // the cursors for the next tile and zeroes the counts
-        if (threadIdx.x < 32)
+        if (!__syncthreads_and(ok))
+            break;
+        if (tma_ok(tile))
+            parity ^= 1u << bi;
+        // every thread is past the previous tile: its buffer can be refilled
+        if (g.stages > 1 && threadIdx.x == 0 && k + ahead < my_tiles)
         {
-            const uint32_t lane = threadIdx.x;
-            const uint32_t per = (nb + 31) / 32;
-            const uint32_t b0 = lane * per;
-            uint32_t local = 0;
-            for (uint32_t i = 0; i < per; ++i)
-                if (b0 + i < nb)
-                    local += bins[b0 + i];
-            uint32_t x = local;
+            const uint4 t = tile_of(k + ahead);
+            if (tma_ok(t))
+                issue(t, bi == 0 ? g.stages - 1 : bi - 1);
+        }
+
+        // each warp scans its rows of 32 digits (its prefix from the counts
+        // of all rows before) and reserves the digits' output places
+        uint32_t ex[kRows], place[kRows];
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1)
+        for (int q = 0; q < kRows; ++q)
+        {
+            const uint32_t r = warp + q * kWarps;
+            ex[q] = place[q] = 0;
+            if (r * 32 >= nb)
+                continue;
+            uint32_t before = 0;
+            for (uint32_t p = 0; p < r; ++p)
+                before += bins[p * 32 + lane];
+            const uint32_t d = r * 32 + lane;
+            const uint32_t v = d < nb ? bins[d] : 0u;
+            if (v)
+                place[q] = __ldg(offs + tile.z + d) + atomicSub(counts + tile.z + d, v) - v;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                before += __shfl_xor_sync(0xffffffffu, before, o);
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
             {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= (uint32_t)d)
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= (uint32_t)o)
                     x += y;
             }
-            uint32_t run = x - local;
-            for (uint32_t i = 0; i < per; ++i)
-                if (b0 + i < nb)
-                {
-                    const uint32_t c = bins[b0 + i];
-                    excl[b0 + i] = run;
-                    run += c;
-                    nxt[b0 + i] = cur[b0 + i] + c;
-                    bins[b0 + i] = 0;
-                }
+            ex[q] = before + x - v;
+            if (d < nb)
+                excl[d] = ex[q];
         }
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < RPT; ++j)
-            if (dg[j] != 0xFFFFu)
+            if (dr[j] != 0xFFFFFFFFu)
             {
-                const uint32_t pos = excl[dg[j]] + rk[j];
-                inv[pos] = (uint16_t)(j * kP1NT + threadIdx.x);
-                dsort[pos] = (uint16_t)dg[j];
+                const uint32_t d = dr[j] & ((1u << kMaxPassBits) - 1);
+                perm[excl[d] + (dr[j] >> kMaxPassBits)] = (j * kNT + threadIdx.x) | d << 12;
             }
+#pragma unroll
+        for (int q = 0; q < kRows; ++q)
+        {
+            const uint32_t d = (warp + q * kWarps) * 32 + lane;
+            if (d < nb)
+            {
+                delta[d] = place[q] - ex[q];
+                bins[d] = 0;
+            }
+        }
         __syncthreads();
         uint32_t src[RPT], dest[RPT];
 #pragma unroll
         for (int j = 0; j < RPT; ++j)
         {
-            const uint32_t pos = j * kP1NT + threadIdx.x;
-            src[j] = 0;
-            dest[j] = 0;
+            const uint32_t pos = j * kNT + threadIdx.x;
+            src[j] = dest[j] = 0;
             if (pos < cnt)
             {
-                const uint32_t d = dsort[pos];
-                src[j] = inv[pos];
-                dest[j] = cur[d] + (pos - excl[d]);
+                const uint32_t e = perm[pos];
+                src[j] = e & 4095u;
+                dest[j] = delta[e >> 12] + pos;
             }
         }
-        p1_write_column<uint64_t, RPT>(buf, out.keys, src, dest, cnt);
+        write_column<uint64_t, RPT>(buf + lead(8), out.keys, src, dest, cnt);
         for (uint32_t c = 0; c < in.n; ++c)
         {
-            const uint8_t * cb = buf + sm.col_off[c];
+            const uint8_t * cb = buf + sm.col_off[c] + lead(in.width[c]);
             switch (in.width[c])
             {
-                case 1: p1_write_column<uint8_t, RPT>(cb, (uint8_t *)out.col[c], src, dest, cnt); break;
-                case 2: p1_write_column<uint16_t, RPT>(cb, (uint16_t *)out.col[c], src, dest, cnt); break;
-                case 4: p1_write_column<uint32_t, RPT>(cb, (uint32_t *)out.col[c], src, dest, cnt); break;
-                case 8: p1_write_column<uint64_t, RPT>(cb, (uint64_t *)out.col[c], src, dest, cnt); break;
-                default: p1_write_column<uint4, RPT>(cb, (uint4 *)out.col[c], src, dest, cnt); break;
+                case 1: write_column<uint8_t, RPT>(cb, (uint8_t *)out.col[c], src, dest, cnt); break;
+                case 2: write_column<uint16_t, RPT>(cb, (uint16_t *)out.col[c], src, dest, cnt); break;
+                case 4: write_column<uint32_t, RPT>(cb, (uint32_t *)out.col[c], src, dest, cnt); break;
+                case 8: write_column<uint64_t, RPT>(cb, (uint64_t *)out.col[c], src, dest, cnt); break;
+                default: write_column<uint4, RPT>(cb, (uint4 *)out.col[c], src, dest, cnt); break;
             }
         }
-        // No barrier here: the next tile's first barrier (after its wait)
-        // comes before this buffer is refilled, before the counts are
-        // ranked into again and before `cur` is overwritten as the next
-        // tile's `nxt`.
-        uint32_t * t_swap = cur;
-        cur = nxt;
-        nxt = t_swap;
+        // The next tile's first barrier (after its ranking) comes before
+        // this tile's perm, excl and delta are written again; its ranking
+        // finds the counts zeroed before this tile's last barrier.  Only a
+        // single buffer must be free before it is refilled.
+        if (g.stages == 1 && k + 1 < my_tiles)
+        {
+            __syncthreads();
+            if (threadIdx.x == 0)
+            {
+                const uint4 t = tile_of(k + 1);
+                if (tma_ok(t))
+                    issue(t, 0);
+            }
+        }
     }
     // Bulk copies still in flight (only after a timeout) must land before
     // the CTA's shared memory is released.
     if (threadIdx.x == 0 && *err)
-        for (uint32_t i = 0; i < stages; ++i)
+        for (uint32_t i = 0; i < g.stages; ++i)
             (void)mbar_wait(&bar[i], (parity >> i) & 1u, err, 1);
 }
 
-__global__ void k_p1_bucket_offsets(const uint32_t * __restrict__ offs, uint32_t nb, uint32_t G, uint32_t n, uint32_t * __restrict__ out_off)
+// Tile shape of a scatter: rows per thread, ring depth, dynamic shared memory.
+struct TileShape
 {
-    const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d < nb)
-        out_off[d] = offs[(uint64_t)d * G];
-    else if (d == nb)
-        out_off[d] = n;
-}
+    uint32_t rpt = 0, stages = 0;
+    TileSmem sm{};
+    size_t smem = 0;
+};
 
-__global__ void k_tiles_per_seg(const uint32_t * __restrict__ seg_off, uint32_t n_segs, uint32_t * __restrict__ nt)
+TileShape shape_of(const Cols & c, uint32_t rpt, uint32_t stages, uint32_t b)
 {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n_segs)
-        nt[s] = (seg_off[s + 1] - seg_off[s] + kTile - 1) / kTile;
-}
-
-__global__ void k_init_single_seg(uint32_t * seg_off, uint32_t n)
-{
-    seg_off[0] = 0;
-    seg_off[1] = n;
-}
-
-// Output bucket offsets of a pass: bucket (s, d) starts at the scanned
-// offset of its first tile; a segment without tiles is empty and all its
-// buckets start where it starts.
-__global__ void k_bucket_offsets(PassGeom g, const uint32_t * __restrict__ offs, uint32_t n, uint32_t * __restrict__ out_off)
-{
-    const uint32_t nb = 1u << g.b;
-    const uint64_t nbuckets = (uint64_t)g.n_segs * nb;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > nbuckets)
-        return;
-    if (i == nbuckets)
+    TileShape s;
+    s.rpt = rpt;
+    s.stages = stages;
+    const uint32_t kT = kNT * rpt;
+    uint32_t off = kT * 8 + 16; // 16 more bytes a column: a slice widened to 16-byte units
+    for (uint32_t i = 0; i < c.n; ++i)
     {
-        out_off[i] = n;
-        return;
+        s.sm.col_off[i] = off;
+        off += (kT * c.width[i] + 31) & ~15u;
     }
-    const uint32_t s = (uint32_t)(i >> g.b), d = (uint32_t)(i & (nb - 1));
-    const uint32_t t0 = g.tile_pre[s], nt = g.tile_pre[s + 1] - t0;
-    out_off[i] = nt ? offs[(uint64_t)t0 * nb + (uint64_t)d * nt] : g.seg_off[s];
+    s.sm.buf_bytes = (off + 127) & ~127u;
+    s.smem = (size_t)stages * s.sm.buf_bytes + 4ull * kT + 3 * 4ull * (1u << b);
+    return s;
 }
-} // namespace
 
-// The first physical pass: histogram per CTA range, scan, bulk-copy fed
-// scatter with running cursors, then the bucket offsets.
-static void first_pass(phj_ctx * ctx, Scratch & s, const Cols & src, const Cols & dst, uint64_t n, uint32_t b, uint32_t * bucket_off,
-                       const char * phase)
+// The tile of the most rows (longest runs a digit) and the deepest ring of
+// at most two buffers with which two CTAs fit on a SM; one CTA a SM where
+// no tile leaves room for two.  Fewer rows a tile where the input would
+// leave SMs without one.  Options "p1_tile_rows" and "p1_stages" pin the
+// first pass's.  (32M rows of 20 bytes, 8 bits: 4096-row tiles, one buffer
+// and two CTAs a SM write a pass in 256-266 us, 5.0-5.2 TB/s; 2048-row tiles
+// in a ring of four and one CTA a SM took 496 us.)
+TileShape choose_shape(const phj_ctx * ctx, const Cols & c, uint64_t n, uint32_t b, bool first)
+{
+    const uint32_t pin_rows = first ? ctx->p1_tile_rows : 0, pin_stages = first ? ctx->p1_stages : 0;
+    const size_t most = ctx->smem_optin - 2048, half = (ctx->smem_optin + 1024) / 2 - 1024 - 64;
+    uint32_t top = kMaxRPT;
+    while (!pin_rows && top > 2 && ceil_div(n, (uint64_t)kNT * top) < (uint64_t)ctx->num_sms)
+        top /= 2;
+    TileShape best;
+    for (int pass = 0; pass < 2 && !best.rpt; ++pass)
+        for (uint32_t r = top; r >= 2 && !best.rpt; r /= 2)
+            for (uint32_t st = pin_stages ? pin_stages : 2; st >= 1; --st)
+            {
+                if ((pin_rows && (uint32_t)kNT * r != pin_rows) || (pin_stages && st != pin_stages))
+                    continue;
+                const TileShape s = shape_of(c, r, st, b);
+                if (s.smem <= (pass == 0 ? half : most))
+                {
+                    best = s;
+                    break;
+                }
+            }
+    if (!best.rpt)
+        throw Error(PHJ_ERR_UNSUPPORTED, "row too wide for the shared-memory tile of the partition pass");
+    return best;
+}
+
+uint64_t row_bytes_of(const Cols & c)
+{
+    uint64_t b = 8;
+    for (uint32_t i = 0; i < c.n; ++i)
+        b += c.width[i];
+    return b;
+}
+
+// Launches the scatter over at most `tiles` tiles.  CTAs take a few tiles
+// each and end, so that a kernel of another stream gets its turn on the
+// SMs; the tiles in flight at a time are neighbours.
+void launch_scatter(phj_ctx * ctx, const Cols & src, const Cols & dst, ScatterGeom g, const TileShape & sh, uint64_t tiles, const uint32_t * offs,
+                    uint32_t * counts, const char * phase, uint64_t n)
+{
+    g.stages = sh.stages;
+    g.wave = (uint32_t)ctx->num_sms * 2;
+    g.tiles_per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(8, tiles / g.wave / 4));
+    const uint64_t waves = ceil_div(tiles, (uint64_t)g.wave * g.tiles_per_cta);
+    const unsigned grid = (unsigned)(waves == 1 ? std::min<uint64_t>(g.wave, tiles) : waves * g.wave);
+    auto kern = g.desc ? (sh.rpt == 8 ? k_scatter<8, true> : sh.rpt == 4 ? k_scatter<4, true> : k_scatter<2, true>)
+                       : (sh.rpt == 8 ? k_scatter<8, false> : sh.rpt == 4 ? k_scatter<4, false> : k_scatter<2, false>);
+    KTimer kt(ctx, phase, n, 2 * n * row_bytes_of(src));
+    kern<<<grid, kNT, sh.smem, ctx->stream>>>(src, dst, g, sh.sm, offs, counts, ctx->d_err);
+    PHJ_LAUNCHED(ctx, "scatter");
+}
+
+// The first physical pass: bucket counts and offsets in one kernel, then the
+// scatter.
+void first_pass(phj_ctx * ctx, Scratch & s, const Cols & src, const Cols & dst, uint64_t n, uint32_t b, uint32_t * bucket_off, const char * phase)
 {
     const uint32_t nb = 1u << b;
-    uint64_t row_bytes = 8;
-    P1Smem sm{};
-    for (uint32_t c = 0; c < src.n; ++c)
-        row_bytes += src.width[c];
-    // Tile rows (4096/2048/1024) and ring depth (2-4): the pair that keeps
-    // the most bytes in flight ((stages - 1) tiles) within shared memory.
-    // (Measured: two resident CTAs of half the tile, same bytes in flight,
-    // run the 16M x 256M first passes 40% slower: the fixed per-tile work
-    // doubles per row, and the build side's pass no longer fits beside the
-    // probe side's on the SMs.)
-    int rpt = 0;
-    uint32_t stages = 0;
-    uint64_t best = 0;
-    for (int r = 8; r >= 2; r /= 2)
-        for (uint32_t st = 2; st <= 4; ++st)
-        {
-            // context options (an autotuner's choice) pin the tile or the depth
-            if ((ctx->p1_tile_rows && (uint32_t)(kP1NT * r) != ctx->p1_tile_rows) || (ctx->p1_stages && st != ctx->p1_stages))
-                continue;
-            const uint64_t kT = (uint64_t)kP1NT * r;
-            uint64_t buf = kT * 8;
-            for (uint32_t c = 0; c < src.n; ++c)
-                buf += kT * src.width[c];
-            buf = (buf + 127) & ~127ull;
-            const uint64_t need_rs = st * buf + 4 * kT + 4ull * nb * 4;
-            if (need_rs + 2048 > ctx->smem_optin)
-                continue;
-            const uint64_t inflight = (st - 1) * buf;
-            if (inflight > best)
-            {
-                best = inflight;
-                rpt = r;
-                stages = st;
-            }
-        }
-    if (rpt == 0)
-        throw Error(PHJ_ERR_UNSUPPORTED, "row too wide for the shared-memory tile of the partition pass");
-    const uint32_t kT = kP1NT * (uint32_t)rpt;
-    uint32_t off = kT * 8;
-    for (uint32_t c = 0; c < src.n; ++c)
-    {
-        sm.col_off[c] = off;
-        off += kT * src.width[c];
-    }
-    sm.buf_bytes = (off + 127) & ~127u;
-    const size_t need = (size_t)stages * sm.buf_bytes + 4ull * kT + 4ull * nb * 4;
-    int per_sm = 1;
-    auto kern = ctx->p1_beside ? (rpt == 8 ? k_p1_scatter<8, 2> : rpt == 4 ? k_p1_scatter<4, 2> : k_p1_scatter<2, 2>)
-                               : (rpt == 8 ? k_p1_scatter<8, 1> : rpt == 4 ? k_p1_scatter<4, 1> : k_p1_scatter<2, 1>);
-    PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kP1NT, need));
-    const uint64_t n_tiles = ceil_div(n, kT);
-    const uint32_t G = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, (uint64_t)ctx->num_sms * std::max(per_sm, 1)));
-    P1Geom g{n, (uint32_t)ceil_div(n_tiles, G), kT, 64u - b, b};
+    const TileShape sh = choose_shape(ctx, src, n, b, true);
     bool aligned = (reinterpret_cast<uintptr_t>(src.keys) & 15u) == 0;
     for (uint32_t c = 0; c < src.n; ++c)
         aligned = aligned && (reinterpret_cast<uintptr_t>(src.col[c]) & 15u) == 0;
-    uint32_t * counts = s.get<uint32_t>((uint64_t)nb * G + 1);
-    PHJ_CUDA(cudaMemsetAsync(counts, 0, ((uint64_t)nb * G + 1) * sizeof(uint32_t), ctx->stream));
+    uint32_t * counts = s.get<uint32_t>((uint64_t)nb + 1); // and the finished CTAs
+    PHJ_CUDA(cudaMemsetAsync(counts, 0, ((uint64_t)nb + 1) * sizeof(uint32_t), ctx->stream));
     {
-        const uint32_t H = 4;
         KTimer kt(ctx, "part_hist", n, n * 8);
         // a pending leaf mark (PHJ/BEP) rides on this pass, once
         const LeafMark mark = ctx->leaf_mark;
         ctx->leaf_mark = LeafMark{};
-        k_p1_hist<<<G * H, kP1NT, (size_t)(nb + (mark.bits ? mark.words : 0)) * sizeof(uint32_t), ctx->stream>>>(src.keys, g, H, G, counts, mark);
+        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 8 * kNT), (uint64_t)ctx->num_sms * 4));
+        k_p1_hist<<<grid, kNT, (size_t)(nb + (mark.bits ? mark.words : 0)) * sizeof(uint32_t), ctx->stream>>>(src.keys, n, 64u - b, b, counts,
+                                                                                                               counts + nb, bucket_off, mark);
         PHJ_LAUNCHED(ctx, "p1_hist");
     }
-    scan_u32(ctx, s, counts, counts, (uint64_t)nb * G);
-    {
-        KTimer kt(ctx, phase, n, 2 * n * row_bytes);
-        kern<<<G, kP1NT, need, ctx->stream>>>(src, dst, g, sm, stages, counts, aligned ? 1 : 0, ctx->d_err);
-        PHJ_LAUNCHED(ctx, "p1_scatter");
-    }
-    k_p1_bucket_offsets<<<(unsigned)ceil_div(nb + 1, 256), 256, 0, ctx->stream>>>(counts, nb, G, (uint32_t)n, bucket_off);
-    PHJ_LAUNCHED(ctx, "p1_offsets");
+    ScatterGeom g{};
+    g.n = n;
+    g.shift = 64u - b;
+    g.b = b;
+    g.use_tma = aligned ? 1 : 0;
+    launch_scatter(ctx, src, dst, g, sh, ceil_div(n, (uint64_t)kNT * sh.rpt), bucket_off, counts, phase, n);
 }
+
+// A later physical pass over n_segs segments.
+void later_pass(phj_ctx * ctx, Scratch & s, const Cols & src, const Cols & dst, uint64_t n, const uint32_t * seg_off, uint32_t n_segs,
+                uint32_t consumed, uint32_t b, uint32_t * next_off, const char * phase)
+{
+    const uint32_t nb = 1u << b;
+    const uint64_t nbuckets = (uint64_t)n_segs * nb;
+    const TileShape sh = choose_shape(ctx, src, n, b, false);
+    const uint32_t kT = kNT * sh.rpt;
+    uint32_t * tile_pre = s.get<uint32_t>((uint64_t)n_segs + 1);
+    if (n_segs <= 4096)
+    {
+        k_seg_tiles<<<1, 1024, 0, ctx->stream>>>(seg_off, n_segs, kT, tile_pre);
+        PHJ_LAUNCHED(ctx, "part_tiles");
+    }
+    else
+    {
+        uint32_t * nt = s.get<uint32_t>(n_segs);
+        k_tiles_per_seg<<<(unsigned)ceil_div(n_segs, 256), 256, 0, ctx->stream>>>(seg_off, n_segs, kT, nt);
+        PHJ_LAUNCHED(ctx, "part_tiles");
+        scan_u32(ctx, s, nt, tile_pre, n_segs);
+    }
+    const uint64_t tiles_ub = ceil_div(n, kT) + std::min<uint64_t>(n_segs, n);
+    uint32_t * counts = s.get<uint32_t>(nbuckets);
+    PHJ_CUDA(cudaMemsetAsync(counts, 0, nbuckets * sizeof(uint32_t), ctx->stream));
+    uint4 * desc = s.get<uint4>(tiles_ub);
+    const PassGeom pg{seg_off, tile_pre, n_segs, 64u - consumed - b, b};
+    {
+        KTimer kt(ctx, "part_hist", n, n * 8);
+        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles_ub, (uint64_t)ctx->num_sms * 4));
+        auto kern = sh.rpt == 8 ? k_seg_hist<8> : sh.rpt == 4 ? k_seg_hist<4> : k_seg_hist<2>;
+        kern<<<grid, kNT, nb * sizeof(uint32_t), ctx->stream>>>(src.keys, pg, counts, desc);
+        PHJ_LAUNCHED(ctx, "part_hist");
+    }
+    scan_u32(ctx, s, counts, next_off, nbuckets);
+    ScatterGeom g{};
+    g.desc = desc;
+    g.n_tiles = tile_pre + n_segs;
+    g.shift = 64u - consumed - b;
+    g.b = b;
+    launch_scatter(ctx, src, dst, g, sh, tiles_ub, next_off, counts, phase, n);
+}
+} // namespace
 
 void radix_partition(phj_ctx * ctx, Scratch & s, const Cols & in, uint64_t n, const std::vector<uint32_t> & pass_bits, const Cols & out,
                      const Cols & tmp, uint32_t * leaf_off, const char * phase)
@@ -688,64 +687,21 @@ void radix_partition(phj_ctx * ctx, Scratch & s, const Cols & in, uint64_t n, co
         PHJ_CUDA(cudaMemsetAsync(leaf_off, 0, (n_leaves + 1) * sizeof(uint32_t), ctx->stream));
         return;
     }
-    const uint32_t maxw = max_width(in) < 8 ? 8 : max_width(in);
-
-    // Segments of the first pass: the whole input.
-    uint32_t * seg_off = s.get<uint32_t>(2);
-    k_init_single_seg<<<1, 1, 0, ctx->stream>>>(seg_off, (uint32_t)n);
-    PHJ_LAUNCHED(ctx, "part_init");
-    uint32_t n_segs = 1, consumed = 0;
     const size_t np = phys.size();
+    const uint32_t * seg_off = nullptr;
+    uint32_t n_segs = 1, consumed = 0;
     Cols src = in;
     for (size_t p = 0; p < np; ++p)
     {
         const uint32_t b = phys[p];
-        const uint32_t nb = 1u << b;
         const Cols & dst = ((np - 1 - p) % 2 == 0) ? out : tmp;
-        if (n_segs == 1)
-        {
-            // first pass: contiguous tile ranges per CTA, bulk-copy fed
-            uint32_t * next_off = (p + 1 == np) ? leaf_off : s.get<uint32_t>((uint64_t)nb + 1);
+        uint32_t * next_off = (p + 1 == np) ? leaf_off : s.get<uint32_t>(((uint64_t)n_segs << b) + 1);
+        if (p == 0)
             first_pass(ctx, s, src, dst, n, b, next_off, phase);
-            seg_off = next_off;
-            n_segs = nb;
-            consumed += b;
-            src = dst;
-            continue;
-        }
-        // Tiles of each segment, then their prefix.
-        uint32_t * nt = s.get<uint32_t>(n_segs + 1);
-        k_tiles_per_seg<<<(unsigned)ceil_div(n_segs, 256), 256, 0, ctx->stream>>>(seg_off, n_segs, nt);
-        PHJ_LAUNCHED(ctx, "part_tiles");
-        uint32_t * tile_pre = s.get<uint32_t>(n_segs + 1);
-        scan_u32(ctx, s, nt, tile_pre, n_segs);
-        const uint64_t tiles_ub = ceil_div(n, kTile) + n_segs;
-        const uint64_t entries_ub = tiles_ub * nb;
-        // Entries past the real tile count stay unwritten; they only follow
-        // the real ones in the scan, so they cannot disturb real offsets.
-        uint32_t * counts = s.get<uint32_t>(entries_ub + 1);
-        const PassGeom g{seg_off, tile_pre, n_segs, 64u - consumed - b, b};
-        {
-            KTimer kt(ctx, "part_hist", n, n * 8);
-            k_part_hist<<<(unsigned)tiles_ub, kNT, nb * sizeof(uint32_t), ctx->stream>>>(src.keys, g, counts);
-            PHJ_LAUNCHED(ctx, "part_hist");
-        }
-        scan_u32(ctx, s, counts, counts, entries_ub);
-        {
-            const size_t smem = (size_t)kTile * maxw + (size_t)kTile * sizeof(uint16_t) + 3ull * nb * sizeof(uint32_t) + 32 * sizeof(uint32_t);
-            uint64_t row_bytes = 8;
-            for (uint32_t c = 0; c < in.n; ++c)
-                row_bytes += in.width[c];
-            KTimer kt(ctx, phase, n, 2 * n * row_bytes);
-            k_part_scatter<<<(unsigned)tiles_ub, kNT, smem, ctx->stream>>>(src, dst, g, counts, maxw);
-            PHJ_LAUNCHED(ctx, "part_scatter");
-        }
-        const uint64_t nbuckets = (uint64_t)n_segs * nb;
-        uint32_t * next_off = (p + 1 == np) ? leaf_off : s.get<uint32_t>(nbuckets + 1);
-        k_bucket_offsets<<<(unsigned)ceil_div(nbuckets + 1, 256), 256, 0, ctx->stream>>>(g, counts, (uint32_t)n, next_off);
-        PHJ_LAUNCHED(ctx, "part_offsets");
+        else
+            later_pass(ctx, s, src, dst, n, seg_off, n_segs, consumed, b, next_off, phase);
         seg_off = next_off;
-        n_segs = (uint32_t)nbuckets;
+        n_segs <<= b;
         consumed += b;
         src = dst;
     }
@@ -753,18 +709,10 @@ void radix_partition(phj_ctx * ctx, Scratch & s, const Cols & in, uint64_t n, co
 
 void set_partition_smem_limits(int smem_optin)
 {
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_p1_scatter<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
+    for (auto * k : {k_scatter<8, false>, k_scatter<4, false>, k_scatter<2, false>, k_scatter<8, true>, k_scatter<4, true>, k_scatter<2, true>})
+        PHJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
     PHJ_CUDA(cudaFuncSetAttribute(k_p1_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::min<size_t>(((1u << kMaxPassBits) + (1u << 20) / 32) * sizeof(uint32_t), (size_t)smem_optin - 1024)));
-    // The scatter kernel stages a 4096-row tile of the widest column (<= 16
-    // bytes) plus digit bins: up to ~96 KiB.
-    const size_t need = (size_t)kTile * 16 + (size_t)kTile * sizeof(uint16_t) + 3ull * (1u << kMaxPassBits) * sizeof(uint32_t) + 128;
-    PHJ_CUDA(cudaFuncSetAttribute(k_part_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(need, (size_t)smem_optin)));
 }
 
 } // namespace phjg
