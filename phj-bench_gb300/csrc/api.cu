@@ -288,30 +288,38 @@ phj_output * new_output(phj_ctx * ctx, const phj_schema & left, const phj_schema
     o->left = left;
     o->right = right;
     o->cap = cap;
+    // a small output is one allocation, cut into columns of 256-byte
+    // granules (a batch makes 64 at once); a large one is an allocation a
+    // column: one 1.9 GB piece did not find its place again between the
+    // run's other buffers, and the pool mapped it anew at 1.6 ms a join
+    constexpr uint64_t kSlabBytes = 160ull << 20;
+    auto room = [&](uint64_t w) { return (std::max<uint64_t>(cap * w, 1) + 255) & ~255ull; };
+    uint64_t total = room(8);
+    for (const phj_schema * sc : {&left, &right})
+        for (uint32_t c = 0; c < sc->n_payloads; ++c)
+            total += room(payload_width(sc->types[c]));
     try
     {
-        o->keys = dalloc_n<uint64_t>(ctx, cap);
-        o->bytes += cap * 8;
+        uint8_t * at = nullptr;
+        if (total <= kSlabBytes)
+            o->slab = at = static_cast<uint8_t *>(dalloc(ctx, total));
+        auto column = [&](uint64_t w) -> void * {
+            o->bytes += cap * w;
+            if (!o->slab)
+                return dalloc(ctx, room(w));
+            uint8_t * p = at;
+            at += room(w);
+            return p;
+        };
+        o->keys = static_cast<uint64_t *>(column(8));
         for (uint32_t c = 0; c < left.n_payloads; ++c)
-        {
-            o->lcol[c] = dalloc(ctx, std::max<uint64_t>(1, cap * payload_width(left.types[c])));
-            o->bytes += cap * payload_width(left.types[c]);
-        }
+            o->lcol[c] = column(payload_width(left.types[c]));
         for (uint32_t c = 0; c < right.n_payloads; ++c)
-        {
-            o->rcol[c] = dalloc(ctx, std::max<uint64_t>(1, cap * payload_width(right.types[c])));
-            o->bytes += cap * payload_width(right.types[c]);
-        }
+            o->rcol[c] = column(payload_width(right.types[c]));
     }
     catch (...)
     {
-        dfree(ctx, o->keys);
-        for (uint32_t c = 0; c < PHJ_MAX_PAYLOADS; ++c)
-        {
-            dfree(ctx, o->lcol[c]);
-            dfree(ctx, o->rcol[c]);
-        }
-        delete o;
+        free_output(ctx, o);
         throw;
     }
     return o;
@@ -321,11 +329,16 @@ void free_output(phj_ctx * ctx, phj_output * o)
 {
     if (!o)
         return;
-    dfree(ctx, o->keys);
-    for (uint32_t c = 0; c < PHJ_MAX_PAYLOADS; ++c)
+    if (o->slab)
+        dfree(ctx, o->slab);
+    else
     {
-        dfree(ctx, o->lcol[c]);
-        dfree(ctx, o->rcol[c]);
+        dfree(ctx, o->keys);
+        for (uint32_t c = 0; c < PHJ_MAX_PAYLOADS; ++c)
+        {
+            dfree(ctx, o->lcol[c]);
+            dfree(ctx, o->rcol[c]);
+        }
     }
     delete o;
 }

@@ -4,27 +4,29 @@
 // thousand to a few million build rows).  Run one at a time, each pays a
 // dozen launches, host round trips and grids too small to fill 152 SMs.
 // Here n joins share every launch:
-//   1. k_bt_hist     tiles of 4096 rows of every join's build and probe
-//                    side, found by binary search in their prefix: each
-//                    join's rows are counted per radix partition (the top
-//                    bits of intHash64, src/Hash.h:18-25; enough bits for
-//                    about 1024 build rows a partition, at most 11);
+//   1. k_bt_hist     tiles of up to 4096 rows of every join's build and
+//                    probe side, found by binary search in their prefix:
+//                    each join's rows are counted per radix partition (the
+//                    top bits of intHash64, src/Hash.h:18-25; enough bits for
+//                    about 1024 build rows a partition, at most 11), and the
+//                    tiles' descriptors are written;
 //   2. scan_u32      the counts of all joins' partitions -> offsets;
-//   3. k_bt_scatter  the same tiles: each tile reserves its rows' places in
-//                    each partition with one atomic per partition and
-//                    writes them (src/RadixPartition.cpp:316-393);
+//   3. k_bt_scatter  the partition passes' tile scatter (scatter.cuh) over
+//                    the same tiles: ranked in shared memory, one
+//                    reservation per tile and partition, written in
+//                    partition order (src/RadixPartition.cpp:316-393);
 //   4. k_bt_join     ONE persistent launch whose CTAs pop (join, partition)
 //                    work items from a device queue (one atomic counter):
 //                    the partition's build rows go into a shared-memory
-//                    JoinHashTable with its next-chain (src/HashTable.h,
-//                    src/BlockStore.h), its probe rows are looked up there,
-//                    and the matches are projected (key, build payloads,
-//                    probe payloads: src/JoinOps.h:52-196) after one
-//                    reservation of output rows per step in the join's
-//                    output.  A partition with more build rows than the
-//                    shared table holds is built and probed in pieces.
-// The chain (counter clears, the three kernels, the scans and cursor
-// copies) reads no size back to the host: the join count and the joins'
+//                    table with its next-chain (src/HashTable.h,
+//                    src/BlockStore.h), then each warp on its own takes
+//                    chunks of 128 probe rows: lookups, one reservation of
+//                    output rows a chunk in the join's output, projection
+//                    (key, build payloads, probe payloads:
+//                    src/JoinOps.h:52-196).  A partition with more build
+//                    rows than the shared table holds is built and probed
+//                    in pieces.
+// The chain (counter clears, the three kernels and the scan) reads no size back to the host: the join count and the joins'
 // prefix arrays and descriptors are uploaded in one copy into a workspace
 // the context keeps, the kernels read the count from there, and the chain
 // is captured once into a CUDA graph at the workspace's capacity and
@@ -35,20 +37,19 @@
 // Output multisets equal those of the single-join entry points; the order
 // of the rows is not fixed.
 #include "internal.h"
+#include "scatter.cuh"
 
 #include <cstring>
-#include <numeric>
 
 namespace phjg
 {
 namespace
 {
-constexpr int kTNT = 256;              // threads of the partition kernels
-constexpr uint32_t kTile = 4096;       // rows per partition tile
-constexpr int kJNT = 512;              // threads of the join kernel
+constexpr int kJNT = 256;              // threads of the join kernel
 constexpr uint32_t kPieceRows = 2048;  // build rows a shared table holds
-constexpr uint32_t kPieceCells = 4096; // its cells (load <= 1/2)
-constexpr uint32_t kNil = 0xFFFFFFFFu;
+constexpr uint32_t kPieceSlots = 4096; // its slots (load <= 1/2)
+constexpr uint32_t kEmptySlot = 0xFFFFFFFFu; // a slot: 20 hash bits << 11 | row of the piece
+constexpr uint32_t kNil = 0xFFFFu;     // end of a chain
 
 struct BatchJoin
 {
@@ -60,6 +61,7 @@ struct BatchJoin
     uint64_t build_rows, probe_rows, out_cap;
     uint32_t bits;      // radix bits
     uint32_t part_base; // index of its first partition among all joins'
+    uint32_t aligned_b, aligned_p; // every input column starts on a 16-byte boundary
 };
 
 // Index j with pre[j] <= t < pre[j+1] (pre non-decreasing, pre[0] = 0).
@@ -82,128 +84,398 @@ __device__ __forceinline__ uint32_t part_of(uint64_t key, uint32_t bits)
     return bits ? (uint32_t)(int_hash64(key) >> (64u - bits)) : 0u;
 }
 
-// Tile t of the build sides (t < tiles_b[n]) or of the probe sides.
-struct TileRef
-{
-    const BatchJoin * J;
-    bool build;
-    uint64_t r0, r1;
-};
-__device__ __forceinline__ TileRef tile_ref(const BatchJoin * d, uint32_t n, const uint64_t * tb, const uint64_t * tp, uint64_t t)
-{
-    TileRef x;
-    const uint64_t nb = tb[n];
-    x.build = t < nb;
-    const uint64_t u = x.build ? t : t - nb;
-    const uint32_t j = find_join(x.build ? tb : tp, n, u);
-    x.J = d + j;
-    x.r0 = (u - (x.build ? tb : tp)[j]) * kTile;
-    const uint64_t rows = x.build ? x.J->build_rows : x.J->probe_rows;
-    x.r1 = x.r0 + kTile < rows ? x.r0 + kTile : rows;
-    return x;
-}
+// Tile descriptors for the scatter: bit 31 of aux is the side, the rest the
+// join.
+constexpr uint32_t kProbeSide = 0x80000000u;
 
-__global__ void __launch_bounds__(kTNT) k_bt_hist(const BatchJoin * __restrict__ d, const uint32_t * __restrict__ d_n,
-                                                  const uint64_t * __restrict__ tb, const uint64_t * __restrict__ tp,
-                                                  uint32_t * __restrict__ cnt_b, uint32_t * __restrict__ cnt_p)
+// Each CTA counts a contiguous range of tiles (the build sides' tiles, then
+// the probe sides'), adding its histogram to the counts of the join's side
+// when that changes, and writes the tiles' descriptors.
+template <int RPT>
+__global__ void __launch_bounds__(kNT) k_bt_hist(const BatchJoin * __restrict__ d, const uint32_t * __restrict__ d_n,
+                                                 const uint64_t * __restrict__ tb, const uint64_t * __restrict__ tp,
+                                                 uint32_t * __restrict__ cnt_b, uint32_t * __restrict__ cnt_p, uint4 * __restrict__ desc,
+                                                 uint32_t * __restrict__ d_tiles)
 {
-    __shared__ uint32_t h[1u << 11];
+    constexpr uint32_t kT = kNT * RPT;
+    __shared__ uint32_t h[1u << kMaxPassBits];
     const uint32_t n = *d_n;
-    const uint64_t n_tiles = tb[n] + tp[n];
-    for (uint64_t t = blockIdx.x; t < n_tiles; t += gridDim.x)
+    const uint64_t nb = tb[n], n_tiles = nb + tp[n];
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *d_tiles = (uint32_t)n_tiles;
+    const uint64_t t0 = n_tiles * blockIdx.x / gridDim.x, t1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
+    for (uint32_t q = threadIdx.x; q < (1u << kMaxPassBits); q += kNT)
+        h[q] = 0;
+    __syncthreads();
+    uint64_t t = t0;
+    while (t < t1)
     {
-        const TileRef x = tile_ref(d, n, tb, tp, t);
-        const uint32_t Q = 1u << x.J->bits;
-        for (uint32_t q = threadIdx.x; q < Q; q += kTNT)
-            h[q] = 0;
+        const bool build = t < nb;
+        const uint64_t * pre = build ? tb : tp;
+        const uint64_t u0 = build ? t : t - nb;
+        const uint32_t j = find_join(pre, n, u0);
+        const BatchJoin & J = d[j];
+        const uint64_t rows = build ? J.build_rows : J.probe_rows;
+        const uint64_t * keys = build ? J.build.keys : J.probe.keys;
+        const uint32_t bits = J.bits, base = J.part_base;
+        // this side's tiles of the CTA's range
+        const uint64_t n_side = min(t1 - t, pre[j + 1] - u0);
+        for (uint64_t u = u0; u < u0 + n_side; ++u)
+        {
+            const uint64_t r0 = (u - pre[j]) * kT;
+            const uint32_t cnt = (uint32_t)min((uint64_t)kT, rows - r0);
+            if (threadIdx.x == 0)
+                desc[t + (u - u0)] = make_uint4((uint32_t)r0, cnt, base, j | (build ? 0u : kProbeSide));
+            uint64_t k[RPT];
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+            {
+                const uint32_t r = i * kNT + threadIdx.x;
+                k[i] = r < cnt ? keys[r0 + r] : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+                if (i * kNT + threadIdx.x < cnt)
+                    atomicAdd(&h[part_of(k[i], bits)], 1u);
+        }
+        t += n_side;
         __syncthreads();
-        const uint64_t * keys = x.build ? x.J->build.keys : x.J->probe.keys;
-        for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += kTNT)
-            atomicAdd(&h[part_of(keys[r], x.J->bits)], 1u);
-        __syncthreads();
-        uint32_t * cnt = (x.build ? cnt_b : cnt_p) + x.J->part_base;
-        for (uint32_t q = threadIdx.x; q < Q; q += kTNT)
+        uint32_t * cnt = (build ? cnt_b : cnt_p) + base;
+        for (uint32_t q = threadIdx.x; q < (1u << bits); q += kNT)
             if (h[q])
+            {
                 atomicAdd(cnt + q, h[q]);
+                h[q] = 0;
+            }
         __syncthreads();
     }
 }
 
-// Rows of the tile to their partitions: one reservation per partition and
-// tile on the running cursors (offsets over all joins' partitions), the
-// row's rank inside the tile's share from a shared counter.
-__global__ void __launch_bounds__(kTNT) k_bt_scatter(const BatchJoin * __restrict__ d, const uint32_t * __restrict__ d_n,
-                                                     const uint64_t * __restrict__ tb, const uint64_t * __restrict__ tp,
-                                                     const uint32_t * __restrict__ off_b, const uint32_t * __restrict__ off_p,
-                                                     uint32_t * __restrict__ cur_b, uint32_t * __restrict__ cur_p)
+// The batch's tiles for scatter_tiles: CTA c takes tiles c, c + grid, ...
+struct BatchTiles
 {
-    __shared__ uint32_t h[1u << 11];
-    __shared__ uint32_t base[1u << 11];
-    const uint32_t n = *d_n;
-    const uint64_t n_tiles = tb[n] + tp[n];
-    for (uint64_t t = blockIdx.x; t < n_tiles; t += gridDim.x)
+    const BatchJoin * d;
+    const uint4 * desc;
+    const uint32_t *off_b, *off_p;
+    uint32_t *cnt_b, *cnt_p;
+    uint32_t my_tiles;
+
+    __device__ __forceinline__ uint32_t n() const { return my_tiles; }
+    __device__ __forceinline__ ScatterTile tile(uint32_t k) const
     {
-        const TileRef x = tile_ref(d, n, tb, tp, t);
-        const uint32_t Q = 1u << x.J->bits;
-        for (uint32_t q = threadIdx.x; q < Q; q += kTNT)
-            h[q] = 0;
-        __syncthreads();
-        const Cols & src = x.build ? x.J->build : x.J->probe;
-        const Cols & dst = x.build ? x.J->bpart : x.J->ppart;
-        for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += kTNT)
-            atomicAdd(&h[part_of(src.keys[r], x.J->bits)], 1u);
-        __syncthreads();
-        // this tile's places in each partition, as rows of the join's
-        // partitioned columns
-        const uint32_t * off = (x.build ? off_b : off_p) + x.J->part_base;
-        uint32_t * cur = (x.build ? cur_b : cur_p) + x.J->part_base;
-        const uint32_t first = off[0];
-        for (uint32_t q = threadIdx.x; q < Q; q += kTNT)
-        {
-            base[q] = h[q] ? atomicAdd(cur + q, h[q]) - first : 0u;
-            h[q] = 0;
-        }
-        __syncthreads();
-        for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += kTNT)
-        {
-            const uint64_t k = src.keys[r];
-            const uint32_t q = part_of(k, x.J->bits);
-            const uint32_t pos = base[q] + atomicAdd(&h[q], 1u);
-            dst.keys[pos] = k;
-            for (uint32_t c = 0; c < src.n; ++c)
-                copy_elem(dst.col[c], pos, src.col[c], r, src.width[c]);
-        }
-        __syncthreads();
+        const uint4 x = __ldg(desc + blockIdx.x + (uint64_t)k * gridDim.x);
+        return ScatterTile{x.x, x.y, x.z, x.w};
     }
+    __device__ __forceinline__ const BatchJoin & join(const ScatterTile & t) const { return d[t.aux & ~kProbeSide]; }
+    __device__ __forceinline__ const Cols & in(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).probe : join(t).build; }
+    __device__ __forceinline__ const Cols & out(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).ppart : join(t).bpart; }
+    __device__ __forceinline__ bool widened(const ScatterTile &) const { return false; }
+    __device__ __forceinline__ bool aligned(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).aligned_p : join(t).aligned_b; }
+    __device__ __forceinline__ uint32_t shift(const ScatterTile & t) const { return join(t).bits ? 64u - join(t).bits : 0u; }
+    __device__ __forceinline__ uint32_t bits(const ScatterTile & t) const { return join(t).bits; }
+    __device__ __forceinline__ const uint32_t * offs(const ScatterTile & t) const { return t.aux & kProbeSide ? off_p : off_b; }
+    __device__ __forceinline__ uint32_t * counts(const ScatterTile & t) const { return t.aux & kProbeSide ? cnt_p : cnt_b; }
+    __device__ __forceinline__ uint32_t first(const ScatterTile & t) const { return __ldg(offs(t) + t.bucket0); }
+};
+
+// (Each thread copying its rows one by one, column by column, to scattered
+// places took 1,835 us for 64 joins of 4K-256K build rows, 77M rows in all.)
+template <int RPT>
+__global__ void __launch_bounds__(kNT, 2) k_bt_scatter(const BatchJoin * __restrict__ d, const uint4 * __restrict__ desc,
+                                                       const uint32_t * __restrict__ d_tiles, const uint32_t * __restrict__ off_b,
+                                                       const uint32_t * __restrict__ off_p, uint32_t * __restrict__ cnt_b,
+                                                       uint32_t * __restrict__ cnt_p, uint32_t stages, uint32_t buf_bytes, uint32_t nb_max,
+                                                       int * __restrict__ err)
+{
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar[kMaxStages];
+    const uint32_t n_tiles = *d_tiles;
+    const BatchTiles s{d, desc, off_b, off_p, cnt_b, cnt_p, blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u};
+    scatter_tiles<RPT>(s, smem, bar, stages, buf_bytes, nb_max, err);
+}
+
+// Four values of a payload column of at most 8 bytes, in 64-bit registers.
+__device__ __forceinline__ void load4(uint64_t (&v)[4], const void * src, uint32_t width, const uint32_t (&idx)[4], uint32_t one)
+{
+    switch (width)
+    {
+#define PHJ_LOAD4(W, T)                                                                                                                              \
+    case W:                                                                                                                                          \
+        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) v[u] = static_cast<const T *>(src)[idx[u]];                                 \
+        break;
+        PHJ_LOAD4(1, uint8_t)
+        PHJ_LOAD4(2, uint16_t)
+        PHJ_LOAD4(4, uint32_t)
+        default: PHJ_LOAD4(8, uint64_t)
+#undef PHJ_LOAD4
+    }
+}
+
+__device__ __forceinline__ void store4(const uint64_t (&v)[4], void * dst, uint32_t width, uint64_t base, const uint32_t (&rel)[4], uint32_t one)
+{
+    switch (width)
+    {
+#define PHJ_STORE4(W, T)                                                                                                                             \
+    case W:                                                                                                                                          \
+        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) __stcs(static_cast<T *>(dst) + base + rel[u], (T)v[u]);                     \
+        break;
+        PHJ_STORE4(1, uint8_t)
+        PHJ_STORE4(2, uint16_t)
+        PHJ_STORE4(4, uint32_t)
+        default: PHJ_STORE4(8, uint64_t)
+#undef PHJ_STORE4
+    }
+}
+
+// A slot's 20 hash bits, in place (its group of slots is chosen by the low
+// 12).
+__device__ __forceinline__ uint32_t slot_tag(uint64_t h)
+{
+    return (uint32_t)(h >> 1) & 0x7FFFF800u;
+}
+
+// A piece's table in shared memory.
+struct PieceTable
+{
+    const uint32_t * slots;
+    const uint64_t * keys;
+    const uint16_t * nxt;
+    uint32_t mask;
+
+    // The piece's row that heads `key`'s chain, kNil when the key is absent:
+    // groups of four slots are filled from their first slot on, so a group
+    // with an empty slot ends the search.
+    __device__ __forceinline__ uint32_t find(uint64_t key) const
+    {
+        const uint64_t h = int_hash64(key);
+        const uint32_t tag = slot_tag(h);
+        for (uint32_t pos = (uint32_t)h & mask & ~3u;; pos = (pos + 4) & mask) // some group has an empty slot
+        {
+            const uint4 s = *reinterpret_cast<const uint4 *>(slots + pos);
+            const uint32_t v[4] = {s.x, s.y, s.z, s.w};
+            // the group's last slot with the key's hash bits, without branches
+            uint32_t row = kNil;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                row = (v[i] ^ tag) < kPieceRows ? v[i] ^ tag : row;
+            if (row != kNil)
+            {
+                if (keys[row] == key)
+                    return row;
+                // other keys with the same hash bits: one by one
+                for (int i = 0; i < 4; ++i)
+                    if ((v[i] ^ tag) < kPieceRows && keys[v[i] ^ tag] == key)
+                        return v[i] ^ tag;
+            }
+            if (s.w == kEmptySlot)
+                return kNil;
+        }
+    }
+};
+
+__device__ __forceinline__ void prefetch_l2(const void * p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// The CTA's warps probe rows [p0, p1) of the partition against the piece
+// whose first build row is c0, 128 rows a warp at a time.  kDup: some key
+// of the piece has more than one row (a row's matches are its chain).
+template <bool kDup>
+__device__ __forceinline__ void probe_piece(const BatchJoin & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable & tab,
+                                            unsigned long long * __restrict__ out_cur, int * __restrict__ over)
+{
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+    for (uint32_t base = p0 + warp * 128; base < p1; base += kJNT / 32 * 128)
+    {
+        // the descriptor (in shared memory) is read where it is used: kept
+        // out of the loop its three dozen pointers would be spilled
+        asm volatile("" ::: "memory");
+        const uint64_t * pkeys = J.ppart.keys;
+        const uint64_t out_cap = J.out_cap;
+        uint64_t key[4];
+        uint32_t head[4], rel[4], total = 0, one = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const uint32_t r = base + u * 32 + lane;
+            key[u] = r < p1 ? __ldcs(pkeys + r) : 0ull;
+        }
+        {
+            // the warp's next chunk into L2, a line a lane
+            const uint32_t next = base + kJNT / 32 * 128;
+            const uint32_t rows = next < p1 ? min(128u, p1 - next) : 0u;
+            if (lane * 16 < rows)
+                prefetch_l2(pkeys + next + lane * 16);
+            for (uint32_t c = 0; c < J.ppart.n; ++c)
+                if (lane * 128 < rows * J.ppart.width[c])
+                    prefetch_l2(static_cast<const uint8_t *>(J.ppart.col[c]) + (uint64_t)next * J.ppart.width[c] + lane * 128);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            head[u] = base + u * 32 + lane < p1 ? tab.find(key[u]) : kNil;
+            if (head[u] != kNil)
+                one |= 1u << u;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if constexpr (kDup)
+            {
+                uint32_t cnt = 0;
+                for (uint32_t b = head[u]; b != kNil; b = tab.nxt[b])
+                    ++cnt;
+                uint32_t x = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= (uint32_t)o)
+                        x += y;
+                }
+                rel[u] = total + x - cnt;
+                total += __shfl_sync(0xffffffffu, x, 31);
+            }
+            else
+            {
+                const uint32_t m = __ballot_sync(0xffffffffu, one >> u & 1u);
+                rel[u] = total + __popc(m & ((1u << lane) - 1u));
+                total += __popc(m);
+            }
+        if (total == 0)
+            continue;
+        // the build payloads' columns, then the probe's; the first one's
+        // loads go out before the reservation comes back, each next one's
+        // before the last one's stores
+        const uint32_t nl = J.bpart.n, nc = nl + J.ppart.n;
+        auto load_column = [&](uint32_t c, uint64_t (&v)[4]) {
+            uint32_t idx[4];
+            const bool left = c < nl;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                idx[u] = left ? c0 + head[u] : base + u * 32 + lane;
+            const uint32_t i = left ? c : c - nl;
+            load4(v, left ? J.bpart.col[i] : J.ppart.col[i], left ? J.bpart.width[i] : J.ppart.width[i], idx, one);
+        };
+        unsigned long long o0 = 0;
+        if (lane == 0)
+        {
+            o0 = atomicAdd(out_cur, (unsigned long long)total);
+            if (o0 + total > out_cap)
+                *over = 1;
+        }
+        uint64_t v[4] = {0, 0, 0, 0};
+        if (!kDup && nc)
+            load_column(0, v);
+        o0 = __shfl_sync(0xffffffffu, o0, 0);
+        if constexpr (kDup)
+        {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                uint64_t o = o0 + rel[u];
+                for (uint32_t b = head[u]; b != kNil; b = tab.nxt[b], ++o)
+                    if (o < out_cap)
+                    {
+                        J.out_keys[o] = key[u];
+                        for (uint32_t c = 0; c < J.bpart.n; ++c)
+                            copy_elem(J.out_l[c], o, J.bpart.col[c], c0 + b, J.bpart.width[c]);
+                        for (uint32_t c = 0; c < J.ppart.n; ++c)
+                            copy_elem(J.out_r[c], o, J.ppart.col[c], base + u * 32 + lane, J.ppart.width[c]);
+                    }
+            }
+        }
+        else
+        {
+            uint64_t * out = J.out_keys + o0;
+            uint32_t fits = one;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                if (o0 + rel[u] >= out_cap)
+                    fits &= ~(1u << u);
+                if (fits >> u & 1u)
+                    __stcs(out + rel[u], key[u]);
+            }
+#pragma unroll 1
+            for (uint32_t c = 0; c < nc; ++c)
+            {
+                asm volatile("" ::: "memory");
+                const bool left = c < nl;
+                const uint32_t i = left ? c : c - nl, w = left ? J.bpart.width[i] : J.ppart.width[i];
+                void * dst = left ? J.out_l[i] : J.out_r[i];
+                uint64_t nx[4] = {0, 0, 0, 0};
+                if (c + 1 < nc)
+                    load_column(c + 1, nx);
+                if (w <= 8)
+                    store4(v, dst, w, o0, rel, fits);
+                else
+                {
+                    const uint4 * src = static_cast<const uint4 *>(left ? J.bpart.col[i] : J.ppart.col[i]);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (fits >> u & 1u)
+                            __stcs(static_cast<uint4 *>(dst) + o0 + rel[u], src[left ? c0 + head[u] : base + u * 32 + lane]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    v[u] = nx[u];
+            }
+        }
+    }
+}
+
+// (out of line, so that its registers do not weigh on the unique-key form)
+__device__ __noinline__ void probe_piece_dup(const BatchJoin & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable tab,
+                                             unsigned long long * out_cur, int * over)
+{
+    probe_piece<true>(J, p0, p1, c0, tab, out_cur, over);
 }
 
 // The persistent join: CTAs pop (join, partition) items until the queue is
 // empty.  out_cur[j] counts join j's output rows (also past its capacity,
 // where nothing is written and over[j] is set).
-__global__ void __launch_bounds__(kJNT) k_bt_join(const BatchJoin * __restrict__ d, const uint32_t * __restrict__ d_n,
-                                                  const uint64_t * __restrict__ parts,
-                                                  const uint32_t * __restrict__ off_b, const uint32_t * __restrict__ off_p,
-                                                  unsigned int * __restrict__ next_item, unsigned long long * __restrict__ out_cur,
-                                                  int * __restrict__ over)
+//
+// A piece's table is 4096 slots of 4 bytes (hash bits and row), its keys
+// and its next-chain: 36 KB, filled with 32-bit compare-and-swaps, so four
+// 256-thread CTAs share a SM.  Warps probe without block barriers: a chunk
+// is a chain of a key load, lookups, a reservation and the payload loads,
+// and 32 warps a SM keep enough chains in flight.  (512-thread CTAs in
+// steps of 512 probe rows with a block scan each, and 16-byte cells with
+// 128-bit compare-and-swaps, took 1,575 us for 64 joins of 73M probe rows
+// in all.)
+__global__ void __launch_bounds__(kJNT, 4) k_bt_join(const BatchJoin * __restrict__ d, const uint32_t * __restrict__ d_n,
+                                                     const uint64_t * __restrict__ parts,
+                                                     const uint32_t * __restrict__ off_b, const uint32_t * __restrict__ off_p,
+                                                     unsigned int * __restrict__ next_item, unsigned long long * __restrict__ out_cur,
+                                                     int * __restrict__ over, const int * __restrict__ err, int * __restrict__ err_out)
 {
-    __shared__ Cell cells[kPieceCells];
-    __shared__ uint32_t nxt[kPieceRows];
-    __shared__ uint32_t ws[kJNT / 32];
+    __shared__ __align__(16) uint32_t slots[kPieceSlots];
+    __shared__ uint64_t bkeys[kPieceRows];
+    __shared__ uint16_t nxt[kPieceRows];
+    __shared__ BatchJoin J; // the item's join
     __shared__ uint32_t s_item;
-    __shared__ unsigned long long s_out;
+    __shared__ int s_dup;
     const uint32_t n = *d_n;
     const uint64_t n_items = parts[n];
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *err_out = *err; // a copy of the scatter that gave up: read back with the row counts
     for (;;)
     {
+        __syncthreads(); // the last item's table and s_item are no longer read
         if (threadIdx.x == 0)
             s_item = atomicAdd(next_item, 1u);
         __syncthreads();
         const uint64_t item = s_item;
-        __syncthreads();
         if (item >= n_items)
             return;
         const uint32_t j = find_join(parts, n, item);
-        const BatchJoin & J = d[j];
+        static_assert(sizeof(BatchJoin) % 8 == 0 && sizeof(BatchJoin) / 8 <= kJNT, "one 8-byte word a thread");
+        if (threadIdx.x < sizeof(BatchJoin) / 8)
+            reinterpret_cast<uint64_t *>(&J)[threadIdx.x] = reinterpret_cast<const uint64_t *>(d + j)[threadIdx.x];
+        __syncthreads();
         const uint32_t g = J.part_base + (uint32_t)(item - parts[j]);
         const uint32_t b0 = off_b[g] - off_b[J.part_base], b1 = off_b[g + 1] - off_b[J.part_base];
         const uint32_t p0 = off_p[g] - off_p[J.part_base], p1 = off_p[g + 1] - off_p[J.part_base];
@@ -212,67 +484,53 @@ __global__ void __launch_bounds__(kJNT) k_bt_join(const BatchJoin * __restrict__
         // the partition's build rows, a piece at a time
         for (uint32_t c0 = b0; c0 < b1; c0 += kPieceRows)
         {
-            const uint32_t c1 = c0 + kPieceRows < b1 ? c0 + kPieceRows : b1;
-            const uint32_t cap = (uint32_t)bit_ceil64(2ull * (c1 - c0));
+            const uint32_t rows = min(kPieceRows, b1 - c0);
+            const uint32_t cap = max(4u, min(kPieceSlots, (uint32_t)bit_ceil64(3ull * rows))), mask = cap - 1;
+            if (c0 != b0)
+                __syncthreads(); // the last piece is no longer probed
+            if (threadIdx.x == 0)
+                s_dup = 0;
             for (uint32_t i = threadIdx.x; i < cap; i += kJNT)
-                reinterpret_cast<ulonglong2 *>(cells)[i] = make_ulonglong2(0ull, INVALID_REF);
+                slots[i] = kEmptySlot;
+            for (uint32_t i = threadIdx.x; i < rows; i += kJNT)
+                bkeys[i] = J.bpart.keys[c0 + i];
             __syncthreads();
-            for (uint32_t r = c0 + threadIdx.x; r < c1; r += kJNT)
+            for (uint32_t i = threadIdx.x; i < rows; i += kJNT)
             {
-                const uint64_t k = J.bpart.keys[r];
-                const uint64_t prev = table_insert<true>(cells, cap, int_hash64(k), k, make_ref(0, r));
-                nxt[r - c0] = ref_valid(prev) ? ref_row(prev) : kNil;
-            }
-            __syncthreads();
-            // its probe rows: count, reserve, project
-            for (uint32_t base = p0; base < p1; base += kJNT)
-            {
-                const uint32_t r = base + threadIdx.x;
-                uint64_t key = 0;
-                uint32_t head = kNil, cnt = 0;
-                if (r < p1)
+                const uint64_t k = bkeys[i];
+                const uint64_t h = int_hash64(k);
+                const uint32_t tag = slot_tag(h), mine = tag | i;
+                uint32_t pos = (uint32_t)h & mask & ~3u, link = kNil;
+                for (;; pos = (pos + 1) & mask) // fewer rows than slots: an empty one is found
                 {
-                    key = J.ppart.keys[r];
-                    const uint64_t h = int_hash64(key);
-                    const uint64_t mask = cap - 1;
-                    uint64_t pos = probe_start(h, cap);
-                    for (uint32_t step = 0; step < cap; ++step)
+                    uint32_t old = slots[pos];
+                    if (old == kEmptySlot)
+                        old = atomicCAS(&slots[pos], kEmptySlot, mine);
+                    if (old == kEmptySlot)
+                        break;
+                    if ((old ^ tag) < kPieceRows && bkeys[old ^ tag] == k)
                     {
-                        const Cell c = cells[pos];
-                        if (!ref_valid(c.ref))
-                            break;
-                        if (c.key == key)
+                        // the key's slot: this row becomes its head (another
+                        // row of the key may have done so meanwhile)
+                        for (;;)
                         {
-                            head = ref_row(c.ref);
-                            break;
+                            const uint32_t seen = atomicCAS(&slots[pos], old, mine);
+                            if (seen == old)
+                                break;
+                            old = seen;
                         }
-                        pos = (pos + 1) & mask;
+                        link = old ^ tag;
+                        s_dup = 1;
+                        break;
                     }
-                    for (uint32_t b = head; b != kNil; b = nxt[b - c0])
-                        ++cnt;
                 }
-                uint32_t total;
-                const uint32_t ex = block_excl_scan<kJNT>(cnt, ws, &total);
-                if (total == 0)
-                    continue;
-                if (threadIdx.x == 0)
-                    s_out = atomicAdd(out_cur + j, (unsigned long long)total);
-                __syncthreads();
-                const uint64_t o0 = s_out + ex;
-                if (threadIdx.x == 0 && s_out + total > J.out_cap)
-                    over[j] = 1;
-                uint64_t o = o0;
-                for (uint32_t b = head; b != kNil; b = nxt[b - c0], ++o)
-                    if (o < J.out_cap)
-                    {
-                        J.out_keys[o] = key;
-                        for (uint32_t c = 0; c < J.bpart.n; ++c)
-                            copy_elem(J.out_l[c], o, J.bpart.col[c], b, J.bpart.width[c]);
-                        for (uint32_t c = 0; c < J.ppart.n; ++c)
-                            copy_elem(J.out_r[c], o, J.ppart.col[c], r, J.ppart.width[c]);
-                    }
-                __syncthreads(); // s_out is reused by the next step
+                nxt[i] = (uint16_t)link;
             }
+            __syncthreads();
+            if (s_dup)
+                probe_piece_dup(J, p0, p1, c0, PieceTable{slots, bkeys, nxt, mask}, out_cur + j, over + j);
+            else
+                probe_piece<false>(J, p0, p1, c0, PieceTable{slots, bkeys, nxt, mask}, out_cur + j, over + j);
         }
     }
 }
@@ -293,19 +551,24 @@ size_t round_up(size_t x, size_t a)
 
 // The chain's workspace, kept by the context across batches at fixed
 // addresses, so that one captured graph of the chain replays for every
-// batch of at most n_cap joins and q_cap partitions in all.  Device block:
-// the upload region (join count, the three prefix arrays, the join
+// batch of at most n_cap joins, q_cap partitions and t_cap tiles in all,
+// rows of at most row_cap bytes and bits_cap radix bits a join.  Device
+// block: the upload region (join count, the three prefix arrays, the join
 // descriptors), then the per-join output counters and overflow flags
-// (adjacent: one download), then the partitions' counts, offsets and
-// cursors and the scan's carry space.  Pinned host block: the upload
-// staging at the same offsets, then the download staging.
+// (adjacent: one download), the item counter and the partitions' counts
+// (with them: one clear), the partitions' offsets, the scan's carry space
+// and the tile descriptors.  Pinned host block: the upload staging at the
+// same offsets, then the download staging.
 struct BatchGraph
 {
     uint32_t n_cap = 0;
-    uint64_t q_cap = 0;
+    uint64_t q_cap = 0, t_cap = 0;
+    uint32_t row_cap = 0, bits_cap = 0;
+    uint32_t rpt = 0, stages = 0, buf_bytes = 0; // the scatter's tile for row_cap and bits_cap
+    size_t smem = 0;
     uint8_t * dev = nullptr;
     uint8_t * host = nullptr;
-    size_t o_tb = 0, o_tp = 0, o_parts = 0, o_desc = 0, o_out = 0, o_cnt = 0, o_carry = 0, o_next = 0, bytes = 0;
+    size_t o_tb = 0, o_tp = 0, o_parts = 0, o_desc = 0, o_out = 0, o_next = 0, o_cnt = 0, o_off = 0, o_carry = 0, o_tile = 0, bytes = 0;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0; // kernel launches in one replay
 };
@@ -338,28 +601,62 @@ struct Chain
     BatchJoin * desc() const { return (BatchJoin *)(base + W->o_desc); }
     unsigned long long * out_cur() const { return (unsigned long long *)(base + W->o_out); }
     int * over() const { return (int *)(base + W->o_out + 8ull * W->n_cap); }
-    uint32_t * cnt(int k) const { return (uint32_t *)(base + W->o_cnt) + (uint64_t)k * (W->q_cap + 1); } // cnt_b, cnt_p, off_b, off_p, cur_b, cur_p
-    uint32_t * carry() const { return (uint32_t *)(base + W->o_carry); }
     unsigned int * next() const { return (unsigned int *)(base + W->o_next); }
+    uint32_t * n_tiles() const { return (uint32_t *)(base + W->o_next) + 1; }
+    uint32_t * cnt() const { return (uint32_t *)(base + W->o_cnt); } // build sides' partitions, then (from q_cap) the probe sides'
+    uint32_t * off() const { return (uint32_t *)(base + W->o_off); } // offsets over the same array
+    uint32_t * carry() const { return (uint32_t *)(base + W->o_carry); }
+    uint4 * tiles() const { return (uint4 *)(base + W->o_tile); }
 };
 
-BatchGraph & batch_workspace(phj_ctx * ctx, uint32_t n, uint64_t nq)
+// The scatter tile for rows of row_cap bytes in up to kMaxCols + 1 columns:
+// the most rows a tile with which two CTAs fit on a SM, else one CTA.
+void choose_tile(const phj_ctx * ctx, BatchGraph & W)
+{
+    const size_t most = ctx->smem_optin - 2048, half = (ctx->smem_optin + 1024) / 2 - 1024 - 64;
+    for (size_t limit : {half, most})
+        for (uint32_t r = kMaxRPT; r >= 2; r /= 2)
+            for (uint32_t st = 2; st >= 1; --st)
+            {
+                const uint32_t buf = (kNT * r * W.row_cap + 32 * (kMaxCols + 1) + 127) & ~127u;
+                const size_t need = scatter_smem(kNT * r, st, buf, W.bits_cap);
+                if (need > limit)
+                    continue;
+                W.rpt = r;
+                W.stages = st;
+                W.buf_bytes = buf;
+                W.smem = need;
+                return;
+            }
+    throw Error(PHJ_ERR_UNSUPPORTED, "row too wide for the shared-memory tile of the batched partition");
+}
+
+// The workspace for a batch of n joins, nq partitions, rows of at most
+// row_bytes and at most `bits` radix bits a join.  Tiles are counted once
+// its tile is known: the caller asks again with nt tiles.
+BatchGraph & batch_workspace(phj_ctx * ctx, uint32_t n, uint64_t nq, uint64_t nt, uint32_t row_bytes, uint32_t bits)
 {
     BatchGraph * W = ctx->batch_ws;
-    if (W && n <= W->n_cap && nq <= W->q_cap)
+    if (W && n <= W->n_cap && nq <= W->q_cap && nt <= W->t_cap && row_bytes <= W->row_cap && bits <= W->bits_cap)
         return *W;
     uint32_t n_cap = W ? W->n_cap : 16;
-    uint64_t q_cap = W ? W->q_cap : 4096;
+    uint64_t q_cap = W ? W->q_cap : 4096, t_cap = W ? W->t_cap : 4096;
+    const uint32_t row_cap = std::max(W ? W->row_cap : 20u, row_bytes), bits_cap = std::max(W ? W->bits_cap : 8u, bits);
     while (n_cap < n)
         n_cap *= 2;
     while (q_cap < nq)
         q_cap *= 2;
+    while (t_cap < nt)
+        t_cap *= 2;
     PHJ_CUDA(cudaStreamSynchronize(ctx->stream));
     free_batch_graph(ctx);
     W = new BatchGraph;
     ctx->batch_ws = W;
     W->n_cap = n_cap;
     W->q_cap = q_cap;
+    W->t_cap = t_cap;
+    W->row_cap = row_cap;
+    W->bits_cap = bits_cap;
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t o = at;
@@ -371,15 +668,20 @@ BatchGraph & batch_workspace(phj_ctx * ctx, uint32_t n, uint64_t nq)
     W->o_tp = take(8ull * (n_cap + 1));
     W->o_parts = take(8ull * (n_cap + 1));
     W->o_desc = take(sizeof(BatchJoin) * n_cap);
-    W->o_out = take(12ull * n_cap);
-    W->o_cnt = take(6 * 4ull * (q_cap + 1));
-    W->o_carry = take(4ull * std::max<uint64_t>(scan_u32_carry(q_cap), 1));
-    W->o_next = take(sizeof(unsigned int));
+    W->o_out = take(12ull * n_cap + 4);
+    W->o_next = take(2 * sizeof(unsigned int));
+    W->o_cnt = take(2 * 4ull * q_cap);
+    W->o_off = take(4ull * (2 * q_cap + 1));
+    W->o_carry = take(4ull * std::max<uint64_t>(scan_u32_carry(2 * q_cap), 1));
+    W->o_tile = take(sizeof(uint4) * t_cap);
     W->bytes = at;
     try
     {
+        choose_tile(ctx, *W);
+        for (auto * k : {k_bt_scatter<8>, k_bt_scatter<4>, k_bt_scatter<2>})
+            PHJ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin - 1024));
         PHJ_CUDA(cudaMalloc(&W->dev, W->bytes));
-        PHJ_CUDA(cudaMallocHost(&W->host, W->o_cnt));
+        PHJ_CUDA(cudaMallocHost(&W->host, W->o_next));
     }
     catch (...)
     {
@@ -389,36 +691,36 @@ BatchGraph & batch_workspace(phj_ctx * ctx, uint32_t n, uint64_t nq)
     return *W;
 }
 
-// The chain on the context's stream: counts, offsets and cursors of q_len
-// partitions (zero past the batch's own), then the three kernels.  With
-// `bytes` (rows, input bytes) each kernel is timed; without, nothing but
-// stream work is issued, so the chain can be captured.
-void enqueue_chain(phj_ctx * ctx, const Chain & c, uint64_t q_len, unsigned tgrid, unsigned jgrid, const uint64_t * bytes)
+// The chain on the context's stream: counts and offsets of q_len partitions
+// a side at stride q_cap (zero past the batch's own), then the three
+// kernels.  With `bytes` (rows, input bytes) each kernel is timed; without,
+// nothing but stream work is issued, so the chain can be captured.
+void enqueue_chain(phj_ctx * ctx, const Chain & c, unsigned tgrid, unsigned jgrid, const uint64_t * bytes)
 {
     cudaStream_t st = ctx->stream;
-    const uint64_t q_bytes = (q_len + 1) * sizeof(uint32_t);
-    uint32_t *cnt_b = c.cnt(0), *cnt_p = c.cnt(1), *off_b = c.cnt(2), *off_p = c.cnt(3), *cur_b = c.cnt(4), *cur_p = c.cnt(5);
-    PHJ_CUDA(cudaMemsetAsync(cnt_b, 0, q_bytes, st));
-    PHJ_CUDA(cudaMemsetAsync(cnt_p, 0, q_bytes, st));
-    PHJ_CUDA(cudaMemsetAsync(c.next(), 0, sizeof(unsigned int), st));
-    PHJ_CUDA(cudaMemsetAsync(c.out_cur(), 0, 12ull * c.W->n_cap, st));
+    const BatchGraph & W = *c.W;
+    uint32_t *cnt_b = c.cnt(), *cnt_p = c.cnt() + W.q_cap, *off_b = c.off(), *off_p = c.off() + W.q_cap;
+    PHJ_CUDA(cudaMemsetAsync(W.dev + W.o_out, 0, W.o_off - W.o_out, st)); // output counters, flags, item counter, counts
     {
         KTimer kt(ctx, bytes ? "batch_hist" : nullptr, bytes ? bytes[0] : 0, bytes ? bytes[0] * 8 : 0);
-        k_bt_hist<<<tgrid, kTNT, 0, st>>>(c.desc(), c.n(), c.tb(), c.tp(), cnt_b, cnt_p);
+        auto kern = W.rpt == 8 ? k_bt_hist<8> : W.rpt == 4 ? k_bt_hist<4> : k_bt_hist<2>;
+        kern<<<tgrid * 2, kNT, 0, st>>>(c.desc(), c.n(), c.tb(), c.tp(), cnt_b, cnt_p, c.tiles(), c.n_tiles());
         PHJ_LAUNCHED(ctx, "batch_hist");
     }
-    scan_u32_into(ctx, cnt_b, off_b, q_len, c.carry());
-    scan_u32_into(ctx, cnt_p, off_p, q_len, c.carry());
-    PHJ_CUDA(cudaMemcpyAsync(cur_b, off_b, q_bytes, cudaMemcpyDeviceToDevice, st));
-    PHJ_CUDA(cudaMemcpyAsync(cur_p, off_p, q_bytes, cudaMemcpyDeviceToDevice, st));
+    // (32-bit offsets of both sides in one array: only differences within a
+    // side are used, which a wrapped sum gives as well)
+    scan_u32_into(ctx, cnt_b, off_b, 2 * W.q_cap, c.carry());
     {
         KTimer kt(ctx, bytes ? "batch_scatter" : nullptr, bytes ? bytes[0] : 0, bytes ? 2 * bytes[1] : 0);
-        k_bt_scatter<<<tgrid, kTNT, 0, st>>>(c.desc(), c.n(), c.tb(), c.tp(), off_b, off_p, cur_b, cur_p);
+        auto kern = W.rpt == 8 ? k_bt_scatter<8> : W.rpt == 4 ? k_bt_scatter<4> : k_bt_scatter<2>;
+        kern<<<tgrid, kNT, W.smem, st>>>(c.desc(), c.tiles(), c.n_tiles(), off_b, off_p, cnt_b, cnt_p, W.stages, W.buf_bytes, 1u << W.bits_cap,
+                                         ctx->d_err);
         PHJ_LAUNCHED(ctx, "batch_scatter");
     }
     {
         KTimer kt(ctx, bytes ? "batch_join" : nullptr, bytes ? bytes[2] : 0, bytes ? bytes[1] : 0);
-        k_bt_join<<<jgrid, kJNT, 0, st>>>(c.desc(), c.n(), c.parts(), off_b, off_p, c.next(), c.out_cur(), c.over());
+        k_bt_join<<<jgrid, kJNT, 0, st>>>(c.desc(), c.n(), c.parts(), off_b, off_p, c.next(), c.out_cur(), c.over(), ctx->d_err,
+                                          c.over() + W.n_cap);
         PHJ_LAUNCHED(ctx, "batch_join");
     }
 }
@@ -441,7 +743,7 @@ void capture_chain(phj_ctx * ctx, BatchGraph & W)
     PHJ_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     try
     {
-        enqueue_chain(ctx, Chain{W.dev, &W}, W.q_cap, (unsigned)ctx->num_sms * 8, jgrid, nullptr);
+        enqueue_chain(ctx, Chain{W.dev, &W}, (unsigned)ctx->num_sms * 2, jgrid, nullptr);
     }
     catch (...)
     {
@@ -479,7 +781,25 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
 
     std::vector<BatchJoin> h(n);
     std::vector<uint64_t> tb(n + 1, 0), tp(n + 1, 0), parts(n + 1, 0);
-    uint64_t brows = 0, prows = 0, in_bytes = 0;
+    uint64_t brows = 0, prows = 0, in_bytes = 0, copy_bytes = 0;
+    uint32_t row_bytes = 8, most_bits = 0;
+    auto side_aligned = [](const Cols & c) {
+        uintptr_t x = reinterpret_cast<uintptr_t>(c.keys);
+        for (uint32_t i = 0; i < c.n; ++i)
+            x |= reinterpret_cast<uintptr_t>(c.col[i]);
+        return (x & 15u) == 0 ? 1u : 0u;
+    };
+    // the partitioned copies' columns, cut from one allocation
+    auto place = [&](Cols & c, const Cols & like, uint64_t rows) {
+        c = like;
+        c.keys = reinterpret_cast<uint64_t *>(copy_bytes);
+        copy_bytes += round_up(std::max<uint64_t>(rows, 1) * 8, 256);
+        for (uint32_t i = 0; i < c.n; ++i)
+        {
+            c.col[i] = reinterpret_cast<void *>(copy_bytes);
+            copy_bytes += round_up(std::max<uint64_t>(rows, 1) * c.width[i], 256);
+        }
+    };
     for (uint32_t j = 0; j < n; ++j)
     {
         const phj_table & B = *builds[j];
@@ -492,11 +812,13 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
         J.probe_rows = P.rows;
         J.bits = partition_bits(B.rows);
         J.part_base = (uint32_t)parts[j];
-        J.bpart = alloc_cols_like(s, B.schema, std::max<uint64_t>(B.rows, 1));
-        J.ppart = alloc_cols_like(s, P.schema, std::max<uint64_t>(P.rows, 1));
+        J.aligned_b = side_aligned(J.build);
+        J.aligned_p = side_aligned(J.probe);
+        place(J.bpart, J.build, B.rows);
+        place(J.ppart, J.probe, P.rows);
         parts[j + 1] = parts[j] + (1ull << J.bits);
-        tb[j + 1] = tb[j] + ceil_div(B.rows, kTile);
-        tp[j + 1] = tp[j] + ceil_div(P.rows, kTile);
+        most_bits = std::max(most_bits, J.bits);
+        row_bytes = std::max<uint32_t>(row_bytes, 8 + (uint32_t)std::max(schema_bytes(B.schema), schema_bytes(P.schema)));
         brows += B.rows;
         prows += P.rows;
         in_bytes += B.rows * (8 + schema_bytes(B.schema)) + P.rows * (8 + schema_bytes(P.schema));
@@ -504,6 +826,17 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
     if (brows >= (1ull << 32) || prows >= (1ull << 32))
         throw Error(PHJ_ERR_UNSUPPORTED, "batch: fewer than 2^32 build rows and 2^32 probe rows in all");
     const uint64_t NQ = parts[n];
+    uint8_t * copies = s.get<uint8_t>(copy_bytes);
+    auto based = [&](Cols & c) {
+        c.keys = reinterpret_cast<uint64_t *>(copies + reinterpret_cast<uintptr_t>(c.keys));
+        for (uint32_t i = 0; i < c.n; ++i)
+            c.col[i] = copies + reinterpret_cast<uintptr_t>(c.col[i]);
+    };
+    for (BatchJoin & J : h)
+    {
+        based(J.bpart);
+        based(J.ppart);
+    }
 
     // outputs at one row per probe row (exact for unique build keys)
     std::vector<phj_output *> made(n, nullptr);
@@ -524,7 +857,15 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
         std::vector<int> ov(n, 0);
         if (n)
         {
-            BatchGraph & W = batch_workspace(ctx, n, NQ);
+            // the tiles' rows follow from the workspace's tile, then the
+            // workspace has to hold that many tiles (a growth keeps the tile)
+            const uint32_t kT = kNT * batch_workspace(ctx, n, NQ, 0, row_bytes, most_bits).rpt;
+            for (uint32_t j = 0; j < n; ++j)
+            {
+                tb[j + 1] = tb[j] + ceil_div(builds[j]->rows, kT);
+                tp[j + 1] = tp[j] + ceil_div(probes[j]->rows, kT);
+            }
+            BatchGraph & W = batch_workspace(ctx, n, NQ, tb[n] + tp[n], row_bytes, most_bits);
             // one upload: join count, prefix arrays, descriptors
             uint8_t * H = W.host;
             std::memcpy(H, &n, sizeof(uint32_t));
@@ -545,16 +886,23 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
             else
             {
                 const uint64_t n_tiles = tb[n] + tp[n];
-                const unsigned tgrid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, (uint64_t)ctx->num_sms * 8));
+                const unsigned tgrid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n_tiles, (uint64_t)ctx->num_sms * 2));
                 const unsigned jgrid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(NQ, join_grid(ctx)));
                 const uint64_t bytes[3] = {brows + prows, in_bytes, prows};
-                enqueue_chain(ctx, c, NQ, tgrid, jgrid, bytes);
+                enqueue_chain(ctx, c, tgrid, jgrid, bytes);
             }
             uint8_t * D = H + W.o_out;
-            PHJ_CUDA(cudaMemcpyAsync(D, c.out_cur(), 12ull * W.n_cap, cudaMemcpyDeviceToHost, ctx->stream));
+            PHJ_CUDA(cudaMemcpyAsync(D, c.out_cur(), 12ull * W.n_cap + 4, cudaMemcpyDeviceToHost, ctx->stream));
             PHJ_CUDA(cudaStreamSynchronize(ctx->stream));
             std::memcpy(rows.data(), D, n * sizeof(unsigned long long));
             std::memcpy(ov.data(), D + 8ull * W.n_cap, n * sizeof(int));
+            int gave_up = 0;
+            std::memcpy(&gave_up, D + 12ull * W.n_cap, sizeof(int));
+            if (gave_up)
+            {
+                PHJ_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+                throw Error(PHJ_ERR_DEVICE_TIMEOUT, "a bounded device wait gave up (code " + std::to_string(gave_up) + ")");
+            }
         }
         uint64_t out_rows = 0;
         for (uint32_t j = 0; j < n; ++j)

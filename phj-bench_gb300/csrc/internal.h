@@ -145,6 +145,7 @@ struct phj_output
     uint64_t * keys = nullptr;
     void * lcol[PHJ_MAX_PAYLOADS] = {};
     void * rcol[PHJ_MAX_PAYLOADS] = {};
+    void * slab = nullptr; // a small output: the one allocation its columns are cut from
     uint64_t bytes = 0;
 };
 

@@ -21,16 +21,12 @@
 // are written, scanned and read back.  The order of the rows inside a bucket
 // is not fixed, as in the reference.
 #include "internal.h"
+#include "scatter.cuh"
 
 namespace phjg
 {
 namespace
 {
-constexpr int kNT = 512;
-constexpr uint32_t kMaxPassBits = 11;  // shared-memory digit histogram <= 2048 bins
-constexpr uint32_t kMaxRPT = 8;        // rows per thread of a tile: 4096-row tiles
-constexpr uint32_t kMaxStages = 4;
-
 // One segment's tiles of a later pass: row0, rows, first bucket.
 struct PassGeom
 {
@@ -229,14 +225,8 @@ __global__ void __launch_bounds__(kNT) k_seg_hist(const uint64_t * __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Scatter
+// Scatter (scatter.cuh)
 // ---------------------------------------------------------------------------
-struct TileSmem
-{
-    uint32_t buf_bytes;              // one tile of every column
-    uint32_t col_off[kMaxCols + 1];  // byte offset of each payload column in a buffer (keys at 0)
-};
-
 struct ScatterGeom
 {
     uint64_t n;               // rows (first pass)
@@ -244,268 +234,67 @@ struct ScatterGeom
     const uint32_t * n_tiles; // later passes: number of tiles (device)
     uint32_t shift, b;
     uint32_t wave, tiles_per_cta; // tile k of CTA c: (c / wave) * wave * tiles_per_cta + k * wave + c % wave
-    uint32_t stages;
+    uint32_t stages, buf_bytes;
     int use_tma;
 };
 
-template <class T, int RPT>
-__device__ __forceinline__ void write_column(const uint8_t * buf, T * __restrict__ dst, const uint32_t (&src)[RPT], const uint32_t (&dest)[RPT],
-                                             uint32_t cnt)
-{
-    const T * b = reinterpret_cast<const T *>(buf);
-#pragma unroll
-    for (int j = 0; j < RPT; ++j)
-        if (j * kNT + threadIdx.x < cnt)
-            dst[dest[j]] = b[src[j]];
-}
-
-// Bound by DRAM when enough tiles are in flight: a tile is a chain of
-// dependent steps (rank with shared atomics, digit scan, reservation,
-// permutation, column writes) with three block barriers, during which one
-// CTA alone leaves the SM idle, so two CTAs of 512 threads share a SM (64
-// registers a thread, at most half of the shared memory each) and one's
-// copies and writes fill the other's barriers.  Measured (256M rows of 16
-// bytes, 6 bits): 5.4 TB/s, 80% of a plain copy's rate; one CTA a SM with a
-// deeper ring reached 4.0 (stalls: block barriers, then shared memory).
+// The tiles of a pass, for scatter_tiles.
 template <int RPT, bool kLater>
-__global__ void __launch_bounds__(kNT, 2) k_scatter(const __grid_constant__ Cols in, const __grid_constant__ Cols out,
-                                                    const __grid_constant__ ScatterGeom g, const __grid_constant__ TileSmem sm,
-                                                    const uint32_t * __restrict__ offs, uint32_t * __restrict__ counts, int * __restrict__ err)
+struct PassTiles
 {
-    constexpr uint32_t kT = kNT * RPT;
-    constexpr uint32_t kWarps = kNT / 32;
-    constexpr int kRows = (1 << kMaxPassBits) / 32 / kWarps; // 32-digit rows a warp scans
-    extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bar[kMaxStages];
-    const uint32_t nb = 1u << g.b, mask = nb - 1;
-    uint32_t * perm = reinterpret_cast<uint32_t *>(smem + (size_t)g.stages * sm.buf_bytes); // tile row | digit << 12, in digit order
-    uint32_t * bins = perm + kT;
-    uint32_t * excl = bins + nb;
-    uint32_t * delta = excl + nb; // output row of a digit's first row, less its position in the tile's digit order
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Cols & cin;
+    const Cols & cout;
+    const ScatterGeom & g;
+    const uint32_t * off;
+    uint32_t * cnt;
+    uint64_t t_first;
+    uint32_t my_tiles;
 
-    const uint64_t n_tiles = kLater ? *g.n_tiles : ceil_div(g.n, kT);
-    const uint64_t t_first = (uint64_t)(blockIdx.x / g.wave) * g.wave * g.tiles_per_cta + blockIdx.x % g.wave;
-    if (t_first >= n_tiles)
-        return;
-    const uint32_t my_tiles = (uint32_t)min((uint64_t)g.tiles_per_cta, (n_tiles - t_first + g.wave - 1) / g.wave);
-    for (uint32_t d = threadIdx.x; d < nb; d += kNT)
-        bins[d] = 0;
-    if (threadIdx.x == 0)
+    __device__ __forceinline__ PassTiles(const Cols & i, const Cols & o, const ScatterGeom & geom, const uint32_t * offs, uint32_t * counts)
+        : cin(i), cout(o), g(geom), off(offs), cnt(counts)
     {
-        for (uint32_t i = 0; i < g.stages; ++i)
-            mbar_init(&bar[i], 1);
-        fence_barrier_init();
+        const uint64_t n_tiles = kLater ? *g.n_tiles : ceil_div(g.n, kNT * RPT);
+        t_first = (uint64_t)(blockIdx.x / g.wave) * g.wave * g.tiles_per_cta + blockIdx.x % g.wave;
+        my_tiles = t_first >= n_tiles ? 0u : (uint32_t)min((uint64_t)g.tiles_per_cta, (n_tiles - t_first + g.wave - 1) / g.wave);
     }
-    __syncthreads();
-
-    auto tile_of = [&](uint32_t k) -> uint4 {
+    __device__ __forceinline__ uint32_t n() const { return my_tiles; }
+    __device__ __forceinline__ ScatterTile tile(uint32_t k) const
+    {
         const uint64_t t = t_first + (uint64_t)k * g.wave;
         if (kLater)
-            return __ldg(g.desc + t);
-        const uint64_t r = g.n - t * kT;
-        return make_uint4((uint32_t)(t * kT), r < kT ? (uint32_t)r : kT, 0, 0);
-    };
-    // A first-pass tile is fetched by bulk copy when every column slice is a
-    // whole number of 16-byte units (always, except a short last tile); a
-    // later pass reads the library's own buffers (256-byte granules), where
-    // a slice may be widened to 16-byte units on both sides.
-    auto tma_ok = [&](const uint4 & t) -> bool {
-        if (kLater)
-            return true;
-        if (!g.use_tma || ((t.y * 8u) & 15u))
-            return false;
-        for (uint32_t c = 0; c < in.n; ++c)
-            if ((t.y * in.width[c]) & 15u)
-                return false;
-        return true;
-    };
-    auto buffer = [&](uint32_t i) -> uint8_t * { return smem + (size_t)i * sm.buf_bytes; };
-    auto issue = [&](const uint4 & t, uint32_t bi) {
-        auto span = [&](uint32_t w, uint64_t & a) -> uint32_t {
-            a = ((uint64_t)t.x * w) & ~15ull;
-            return (uint32_t)((((uint64_t)(t.x + t.y) * w + 15) & ~15ull) - a);
-        };
-        uint64_t a;
-        uint32_t bytes = span(8, a);
-        for (uint32_t c = 0; c < in.n; ++c)
-            bytes += span(in.width[c], a);
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&bar[bi], bytes);
-        const uint32_t kb = span(8, a);
-        bulk_copy_g2s(buffer(bi), reinterpret_cast<const uint8_t *>(in.keys) + a, kb, &bar[bi]);
-        for (uint32_t c = 0; c < in.n; ++c)
         {
-            const uint32_t cb = span(in.width[c], a);
-            bulk_copy_g2s(buffer(bi) + sm.col_off[c], static_cast<const uint8_t *>(in.col[c]) + a, cb, &bar[bi]);
+            const uint4 d = __ldg(g.desc + t);
+            return ScatterTile{d.x, d.y, d.z, 0};
         }
-    };
-    // tiles in flight ahead of the one being written: stages - 1, or the
-    // next one once this one's buffer is free
-    const uint32_t ahead = g.stages > 1 ? g.stages - 1 : 1;
-    uint32_t parity = 0; // bit i: phase of bar[i] to wait for
-    if (threadIdx.x == 0)
-        for (uint32_t i = 0; i < ahead && i < my_tiles; ++i)
-        {
-            const uint4 t = tile_of(i);
-            if (tma_ok(t))
-                issue(t, i);
-        }
-
-    uint32_t bi = 0;
-    for (uint32_t k = 0; k < my_tiles; ++k, bi = (bi + 1 == g.stages) ? 0 : bi + 1)
-    {
-        const uint4 tile = tile_of(k);
-        const uint32_t cnt = tile.y;
-        uint8_t * buf = buffer(bi);
-        bool ok = true;
-        if (tma_ok(tile))
-        {
-            ok = mbar_wait(&bar[bi], (parity >> bi) & 1u, err, 1);
-        }
-        else
-        {
-            uint64_t * bk = reinterpret_cast<uint64_t *>(buf);
-            for (uint32_t i = threadIdx.x; i < cnt; i += kNT)
-                bk[i] = in.keys[tile.x + i];
-            for (uint32_t c = 0; c < in.n; ++c)
-                for (uint32_t i = threadIdx.x; i < cnt; i += kNT)
-                    copy_elem(buf + sm.col_off[c], i, in.col[c], (uint64_t)tile.x + i, in.width[c]);
-            __syncthreads();
-        }
-        // bytes of a column before the tile's first row in its buffer
-        auto lead = [&](uint32_t w) -> uint32_t { return kLater ? (tile.x * w) & 15u : 0u; };
-
-        // digit and rank within the digit (bins are zero here)
-        const uint64_t * bk = reinterpret_cast<const uint64_t *>(buf + lead(8));
-        uint32_t dr[RPT]; // digit | rank << 11
-#pragma unroll
-        for (int j = 0; j < RPT; ++j)
-        {
-            const uint32_t i = j * kNT + threadIdx.x;
-            dr[j] = 0xFFFFFFFFu;
-            if (i < cnt)
-            {
-                const uint32_t d = (uint32_t)(int_hash64(bk[i]) >> g.shift) & mask;
-                dr[j] = d | atomicAdd(&bins[d], 1u) << kMaxPassBits;
-            }
-        }
-        if (!__syncthreads_and(ok))
-            break;
-        if (tma_ok(tile))
-            parity ^= 1u << bi;
-        // every thread is past the previous tile: its buffer can be refilled
-        if (g.stages > 1 && threadIdx.x == 0 && k + ahead < my_tiles)
-        {
-            const uint4 t = tile_of(k + ahead);
-            if (tma_ok(t))
-                issue(t, bi == 0 ? g.stages - 1 : bi - 1);
-        }
-
-        // each warp scans its rows of 32 digits (its prefix from the counts
-        // of all rows before) and reserves the digits' output places
-        uint32_t ex[kRows], place[kRows];
-#pragma unroll
-        for (int q = 0; q < kRows; ++q)
-        {
-            const uint32_t r = warp + q * kWarps;
-            ex[q] = place[q] = 0;
-            if (r * 32 >= nb)
-                continue;
-            uint32_t before = 0;
-            for (uint32_t p = 0; p < r; ++p)
-                before += bins[p * 32 + lane];
-            const uint32_t d = r * 32 + lane;
-            const uint32_t v = d < nb ? bins[d] : 0u;
-            if (v)
-                place[q] = __ldg(offs + tile.z + d) + atomicSub(counts + tile.z + d, v) - v;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                before += __shfl_xor_sync(0xffffffffu, before, o);
-            uint32_t x = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= (uint32_t)o)
-                    x += y;
-            }
-            ex[q] = before + x - v;
-            if (d < nb)
-                excl[d] = ex[q];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < RPT; ++j)
-            if (dr[j] != 0xFFFFFFFFu)
-            {
-                const uint32_t d = dr[j] & ((1u << kMaxPassBits) - 1);
-                perm[excl[d] + (dr[j] >> kMaxPassBits)] = (j * kNT + threadIdx.x) | d << 12;
-            }
-#pragma unroll
-        for (int q = 0; q < kRows; ++q)
-        {
-            const uint32_t d = (warp + q * kWarps) * 32 + lane;
-            if (d < nb)
-            {
-                delta[d] = place[q] - ex[q];
-                bins[d] = 0;
-            }
-        }
-        __syncthreads();
-        uint32_t src[RPT], dest[RPT];
-#pragma unroll
-        for (int j = 0; j < RPT; ++j)
-        {
-            const uint32_t pos = j * kNT + threadIdx.x;
-            src[j] = dest[j] = 0;
-            if (pos < cnt)
-            {
-                const uint32_t e = perm[pos];
-                src[j] = e & 4095u;
-                dest[j] = delta[e >> 12] + pos;
-            }
-        }
-        write_column<uint64_t, RPT>(buf + lead(8), out.keys, src, dest, cnt);
-        for (uint32_t c = 0; c < in.n; ++c)
-        {
-            const uint8_t * cb = buf + sm.col_off[c] + lead(in.width[c]);
-            switch (in.width[c])
-            {
-                case 1: write_column<uint8_t, RPT>(cb, (uint8_t *)out.col[c], src, dest, cnt); break;
-                case 2: write_column<uint16_t, RPT>(cb, (uint16_t *)out.col[c], src, dest, cnt); break;
-                case 4: write_column<uint32_t, RPT>(cb, (uint32_t *)out.col[c], src, dest, cnt); break;
-                case 8: write_column<uint64_t, RPT>(cb, (uint64_t *)out.col[c], src, dest, cnt); break;
-                default: write_column<uint4, RPT>(cb, (uint4 *)out.col[c], src, dest, cnt); break;
-            }
-        }
-        // The next tile's first barrier (after its ranking) comes before
-        // this tile's perm, excl and delta are written again; its ranking
-        // finds the counts zeroed before this tile's last barrier.  Only a
-        // single buffer must be free before it is refilled.
-        if (g.stages == 1 && k + 1 < my_tiles)
-        {
-            __syncthreads();
-            if (threadIdx.x == 0)
-            {
-                const uint4 t = tile_of(k + 1);
-                if (tma_ok(t))
-                    issue(t, 0);
-            }
-        }
+        const uint64_t r = g.n - t * (kNT * RPT);
+        return ScatterTile{(uint32_t)(t * (kNT * RPT)), r < kNT * RPT ? (uint32_t)r : kNT * RPT, 0, 0};
     }
-    // Bulk copies still in flight (only after a timeout) must land before
-    // the CTA's shared memory is released.
-    if (threadIdx.x == 0 && *err)
-        for (uint32_t i = 0; i < g.stages; ++i)
-            (void)mbar_wait(&bar[i], (parity >> i) & 1u, err, 1);
+    __device__ __forceinline__ const Cols & in(const ScatterTile &) const { return cin; }
+    __device__ __forceinline__ const Cols & out(const ScatterTile &) const { return cout; }
+    __device__ __forceinline__ bool widened(const ScatterTile &) const { return kLater; }
+    __device__ __forceinline__ bool aligned(const ScatterTile &) const { return g.use_tma != 0; }
+    __device__ __forceinline__ uint32_t shift(const ScatterTile &) const { return g.shift; }
+    __device__ __forceinline__ uint32_t bits(const ScatterTile &) const { return g.b; }
+    __device__ __forceinline__ const uint32_t * offs(const ScatterTile &) const { return off; }
+    __device__ __forceinline__ uint32_t * counts(const ScatterTile &) const { return cnt; }
+    __device__ __forceinline__ uint32_t first(const ScatterTile &) const { return 0; }
+};
+
+template <int RPT, bool kLater>
+__global__ void __launch_bounds__(kNT, 2) k_scatter(const __grid_constant__ Cols in, const __grid_constant__ Cols out,
+                                                    const __grid_constant__ ScatterGeom g, const uint32_t * __restrict__ offs,
+                                                    uint32_t * __restrict__ counts, int * __restrict__ err)
+{
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar[kMaxStages];
+    const PassTiles<RPT, kLater> s(in, out, g, offs, counts);
+    scatter_tiles<RPT>(s, smem, bar, g.stages, g.buf_bytes, 1u << g.b, err);
 }
 
 // Tile shape of a scatter: rows per thread, ring depth, dynamic shared memory.
 struct TileShape
 {
-    uint32_t rpt = 0, stages = 0;
-    TileSmem sm{};
+    uint32_t rpt = 0, stages = 0, buf_bytes = 0;
     size_t smem = 0;
 };
 
@@ -515,14 +304,11 @@ TileShape shape_of(const Cols & c, uint32_t rpt, uint32_t stages, uint32_t b)
     s.rpt = rpt;
     s.stages = stages;
     const uint32_t kT = kNT * rpt;
-    uint32_t off = kT * 8 + 16; // 16 more bytes a column: a slice widened to 16-byte units
+    uint32_t bytes = tile_col_bytes(kT, 8);
     for (uint32_t i = 0; i < c.n; ++i)
-    {
-        s.sm.col_off[i] = off;
-        off += (kT * c.width[i] + 31) & ~15u;
-    }
-    s.sm.buf_bytes = (off + 127) & ~127u;
-    s.smem = (size_t)stages * s.sm.buf_bytes + 4ull * kT + 3 * 4ull * (1u << b);
+        bytes += tile_col_bytes(kT, c.width[i]);
+    s.buf_bytes = (bytes + 127) & ~127u;
+    s.smem = scatter_smem(kT, stages, s.buf_bytes, b);
     return s;
 }
 
@@ -574,6 +360,7 @@ void launch_scatter(phj_ctx * ctx, const Cols & src, const Cols & dst, ScatterGe
                     uint32_t * counts, const char * phase, uint64_t n)
 {
     g.stages = sh.stages;
+    g.buf_bytes = sh.buf_bytes;
     g.wave = (uint32_t)ctx->num_sms * 2;
     g.tiles_per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(8, tiles / g.wave / 4));
     const uint64_t waves = ceil_div(tiles, (uint64_t)g.wave * g.tiles_per_cta);
@@ -581,7 +368,7 @@ void launch_scatter(phj_ctx * ctx, const Cols & src, const Cols & dst, ScatterGe
     auto kern = g.desc ? (sh.rpt == 8 ? k_scatter<8, true> : sh.rpt == 4 ? k_scatter<4, true> : k_scatter<2, true>)
                        : (sh.rpt == 8 ? k_scatter<8, false> : sh.rpt == 4 ? k_scatter<4, false> : k_scatter<2, false>);
     KTimer kt(ctx, phase, n, 2 * n * row_bytes_of(src));
-    kern<<<grid, kNT, sh.smem, ctx->stream>>>(src, dst, g, sh.sm, offs, counts, ctx->d_err);
+    kern<<<grid, kNT, sh.smem, ctx->stream>>>(src, dst, g, offs, counts, ctx->d_err);
     PHJ_LAUNCHED(ctx, "scatter");
 }
 
