@@ -155,7 +155,9 @@ void *phj_ctx_stream(phj_ctx *ctx);
 /* Integer options of a context:
  *   "probe_materialize": -1 auto (default), 0 never, 1 always -- whether the
  *        partitioned schemes write the probe side's first radix pass to
- *        memory or probe the input order directly against the leaf tables;
+ *        memory or probe the input order directly against the leaf tables, and
+ *        whether CHJ first copies the probe side into sub-table order (auto:
+ *        tables and build rows past L2);
  *   "time_kernels": 1 (default) records CUDA events around each kernel;
  *   "wait_limit_ms": bound of a device wait on another warp's work
  *        (PHJ/BEP leaf builds), 1..60000, default 1000;
@@ -274,7 +276,8 @@ phj_status phj_radix_shuffle(phj_ctx *ctx, const phj_table *input, const uint8_t
 
 /* runCHJ (src/CHJ.h:31, src/CHJ.cpp:49-152): one global device table of
  * 16-byte cells namespaced by the top 8 hash bits, 128-bit CAS inserts, then
- * an unpartitioned probe.  `threads` of the reference has no device meaning. */
+ * an unpartitioned probe (past L2, of the probe side in sub-table order:
+ * option "probe_materialize").  `threads` of the reference has no device meaning. */
 phj_status phj_run_chj(phj_ctx *ctx, const phj_table *build, const phj_table *probe, phj_output **out,
                        phj_chj_result *result);
 

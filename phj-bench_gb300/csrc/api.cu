@@ -540,18 +540,98 @@ static void debug_timeline(phj_ctx * ctx, cudaEvent_t t0)
 // ---------------------------------------------------------------------------
 // schemes
 // ---------------------------------------------------------------------------
-static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj_output ** out, phj_chj_result * res)
+// Bits of the probe side's first (and only written) radix pass in PHJ-PURE.
+// The lookup takes every row's leaf from the whole hash, so this width is a
+// performance choice, not the configuration's: buckets narrow enough that
+// one bucket's leaf tables and build payloads stay in L2 while its rows are
+// probed, and otherwise as wide as possible (fewer buckets: longer runs per
+// bucket in the scatter's tiles).  The working set is estimated before the
+// tables exist (the pass runs beside the build side): cells at the load
+// factor with up to 2x for power-of-two and uniform sizing, the next-chain
+// and the payloads; the widest buckets whose share stays within a fifth of
+// L2 are taken (16M x 256M: 6 bits, 6.83 ms against 7.12 ms at the
+// configuration's 8 and 7.35 ms at 5).  "probe_pass_bits" overrides it.
+static uint32_t probe_pass_bits(const phj_ctx * ctx, uint32_t total, const phj_table & build)
+{
+    const uint32_t most = std::min<uint32_t>(total, 11);
+    if (ctx->probe_pass_bits)
+        return std::min<uint32_t>(ctx->probe_pass_bits, most);
+    const uint64_t ws = build.rows * (16ull * ctx->table_cap_pct / 100 * 2 + 8 + schema_bytes(build.schema));
+    const uint64_t target = std::max<uint64_t>(ctx->l2_bytes / 5, 1);
+    uint32_t b = 1;
+    while (b < most && (ws >> b) > target)
+        ++b;
+    return b;
+}
+
+// One radix pass over the probe side on the side stream, beside the build
+// side's work on the main stream.  `ready` is waited for first; start and
+// stop bracket the pass.  Until the object goes, an error's way out waits
+// for the side stream (its buffers are freed with the scratch).
+struct SideProbePass
+{
+    phj_ctx * ctx;
+    bool running = false;
+
+    explicit SideProbePass(phj_ctx * c)
+        : ctx(c)
+    {
+    }
+    Cols run(Scratch & s, const phj_table & P, uint32_t bits, cudaEvent_t ready, cudaEvent_t start, cudaEvent_t stop)
+    {
+        if (!ctx->side)
+            PHJ_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        struct OnSide
+        {
+            phj_ctx * c;
+            cudaStream_t main;
+            ~OnSide() { c->stream = main; }
+        } on_side{ctx, ctx->stream};
+        PHJ_CUDA(cudaStreamWaitEvent(ctx->side, ready, 0));
+        ctx->stream = ctx->side;
+        running = true;
+        PHJ_CUDA(cudaEventRecord(start, ctx->stream));
+        const Cols part = alloc_cols_like(s, P.schema, P.rows);
+        const Cols tmp = bits > 11 ? alloc_cols_like(s, P.schema, P.rows) : part;
+        uint32_t * off = s.get<uint32_t>((1ull << bits) + 1);
+        radix_partition(ctx, s, cols_of(P), P.rows, {bits}, part, tmp, off, "probe_scatter");
+        PHJ_CUDA(cudaEventRecord(stop, ctx->stream));
+        return part;
+    }
+    // The main stream goes on after the pass.
+    void join(cudaEvent_t stop)
+    {
+        PHJ_CUDA(cudaStreamWaitEvent(ctx->stream, stop, 0));
+        running = false;
+    }
+    ~SideProbePass()
+    {
+        if (running)
+            cudaStreamSynchronize(ctx->side);
+    }
+};
+
+// `cluster`: the probe side is first put in sub-table order by one radix
+// pass (at most the 8 bits that choose a sub-table), beside the build, so
+// that the sub-tables the rows in flight touch stay in L2.  4M x 64M (200 MB
+// of cells, 64 MB of packed build rows): probed in input order 1,960 us,
+// every cell and row a DRAM sector; clustered 980 us after a pass of 665 beside the
+// build (the join 2,310 -> 1,730 us).
+static void run_chj_form(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj_output ** out, phj_chj_result * res, bool cluster)
 {
     begin_run(ctx);
     Scratch s(ctx);
-    cudaEvent_t e0 = take_event(ctx), e1 = take_event(ctx), e2 = take_event(ctx);
+    cudaEvent_t e0 = take_event(ctx), e1 = take_event(ctx), e2 = take_event(ctx), p0 = take_event(ctx), p1 = take_event(ctx);
     PHJ_CUDA(cudaEventRecord(e0, ctx->stream));
+    ProbeArgs a{};
+    a.probe = cols_of(P);
+    SideProbePass pass(ctx);
+    if (cluster)
+        a.probe = pass.run(s, P, probe_pass_bits(ctx, 8, B), e0, p0, p1);
     LeafTables lt;
     lt.next = s.get<uint64_t>(B.rows);
     build_global_table(ctx, s, B, 8, lt);
     PHJ_CUDA(cudaEventRecord(e1, ctx->stream));
-    ProbeArgs a{};
-    a.probe = cols_of(P);
     a.probe_rows = P.rows;
     a.build = payload_cols(cols_of(B));
     a.meta = lt.meta;
@@ -564,6 +644,8 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
     a.any_dup = lt.any_dup;
     a.uniform_log2cap = -1;
     pack_build_payloads(ctx, s, a, B.rows);
+    if (cluster)
+        pass.join(p1);
     phj_output * o =
         ctx->chj_windows > 1 ? probe_chj_windows(ctx, s, a, B.schema, P.schema, ctx->chj_windows) : probe_into_output(ctx, s, a, B.schema, P.schema);
     PHJ_CUDA(cudaEventRecord(e2, ctx->stream));
@@ -572,6 +654,7 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
     debug_timeline(ctx, e0);
     if (res)
     {
+        // the pass beside the build counts with the probe
         fill_phase(res->build, event_ms(e0, e1), B.rows);
         fill_phase(res->probe, event_ms(e1, e2), P.rows);
         res->e2e_wall_ms = event_ms(e0, e2);
@@ -580,38 +663,38 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
     *out = o;
 }
 
+static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj_output ** out, phj_chj_result * res)
+{
+    // Clustered when the cells (32 to 64 bytes a row: 48) and the gathered
+    // build rows (16 bytes packed) are past L2 by a fifth.  Measured, rows of
+    // 12 payload bytes: 1.3M x 5M 300 -> 334 us clustered, 2M x 32M 957 ->
+    // 928, 2.5M x 20M 760 -> 684, 4M x 32M 1,301 -> 1,088; of 4 bytes: 2M x
+    // 32M 819 -> 889, 4M x 16M 717 -> 673; repeated keys 2.5M x 20M 2,293 ->
+    // 2,302, 4M x 32M 3,752 -> 3,598.  "probe_materialize" forces either.
+    const uint64_t payload = schema_bytes(B.schema);
+    const uint64_t gathered = B.schema.n_payloads >= 2 && payload <= 16 ? 16 : payload;
+    const bool past_l2 = B.rows * (48 + gathered) > ctx->l2_bytes / 5 * 6;
+    if (ctx->chj_windows <= 1 && P.rows > 0 && (ctx->probe_materialize < 0 ? past_l2 : ctx->probe_materialize == 1))
+    {
+        try
+        {
+            return run_chj_form(ctx, B, P, out, res, true);
+        }
+        catch (const Error & e)
+        {
+            // no room for the clustered copy of the probe side: without it
+            if (e.status != PHJ_ERR_OUT_OF_MEMORY)
+                throw;
+        }
+    }
+    run_chj_form(ctx, B, P, out, res, false);
+}
+
 phj_output * join_alone(phj_ctx * ctx, const phj_table & B, const phj_table & P)
 {
     phj_output * o = nullptr;
     run_chj(ctx, B, P, &o, nullptr);
     return o;
-}
-
-// Bits of the probe side's first (and only written) radix pass in PHJ-PURE.
-// The lookup takes every row's leaf from the whole hash, so this width is a
-// performance choice, not the configuration's: buckets narrow enough that
-// one bucket's leaf tables and build payloads stay in L2 while its rows are
-// probed, and otherwise as wide as possible (fewer buckets: longer runs per
-// bucket in the scatter's tiles).  The working set is estimated before the
-// tables exist (the pass runs beside the build side): cells at the load
-// factor with up to 2x for power-of-two and uniform sizing, the next-chain
-// and the payloads; the widest buckets whose share stays within a fifth of
-// L2 are taken (16M x 256M: 6 bits, 6.83 ms against 7.12 ms at the
-// configuration's 8 and 7.35 ms at 5).  "probe_pass_bits" overrides it.
-static uint32_t probe_pass_bits(const phj_ctx * ctx, const std::vector<uint32_t> & bits, const phj_table & build)
-{
-    uint32_t total = 0;
-    for (uint32_t b : bits)
-        total += b;
-    const uint32_t most = std::min<uint32_t>(total, 11);
-    if (ctx->probe_pass_bits)
-        return std::min<uint32_t>(ctx->probe_pass_bits, most);
-    const uint64_t ws = build.rows * (16ull * ctx->table_cap_pct / 100 * 2 + 8 + schema_bytes(build.schema));
-    const uint64_t target = std::max<uint64_t>(ctx->l2_bytes / 5, 1);
-    uint32_t b = 1;
-    while (b < most && (ws >> b) > target)
-        ++b;
-    return b;
 }
 
 static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P, const std::vector<uint32_t> & bits, phj_output ** out,
@@ -634,32 +717,9 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     a.probe = cols_of(P);
     const bool mat = materialize_probe_estimate(ctx, B) && P.rows > 0;
     cudaStream_t main_stream = ctx->stream;
+    SideProbePass pass(ctx);
     if (mat)
-    {
-        if (!ctx->side)
-            PHJ_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-        PHJ_CUDA(cudaStreamWaitEvent(ctx->side, ev[0], 0));
-        ctx->stream = ctx->side;
-        try
-        {
-            PHJ_CUDA(cudaEventRecord(ev[5], ctx->stream));
-            const uint32_t pb = probe_pass_bits(ctx, bits, B);
-            const Cols ppart = alloc_cols_like(s, P.schema, P.rows);
-            const bool split = pb > 11;
-            const Cols ptmp = split ? alloc_cols_like(s, P.schema, P.rows) : ppart;
-            uint32_t * poff = s.get<uint32_t>((1ull << pb) + 1);
-            radix_partition(ctx, s, a.probe, P.rows, {pb}, ppart, ptmp, poff, "probe_scatter");
-            a.probe = ppart;
-            PHJ_CUDA(cudaEventRecord(ev[6], ctx->stream));
-        }
-        catch (...)
-        {
-            ctx->stream = main_stream;
-            cudaStreamSynchronize(ctx->side);
-            throw;
-        }
-        ctx->stream = main_stream;
-    }
+        a.probe = pass.run(s, P, probe_pass_bits(ctx, total_bits, B), ev[0], ev[5], ev[6]);
 
     // -------- BUILD SHUFFLE (src/PHJ.cpp:220-223) --------
     const Cols bin = cols_of(B);
@@ -711,15 +771,13 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     }
     catch (...)
     {
-        // the side and aux streams' buffers are freed with the scratch
-        if (mat)
-            cudaStreamSynchronize(ctx->side);
+        // the aux stream's buffers are freed with the scratch
         if (ctx->aux)
             cudaStreamSynchronize(ctx->aux);
         throw;
     }
     if (mat)
-        PHJ_CUDA(cudaStreamWaitEvent(ctx->stream, ev[6], 0));
+        pass.join(ev[6]);
     PHJ_CUDA(cudaStreamWaitEvent(ctx->stream, ev[8], 0));
     PHJ_CUDA(cudaEventRecord(ev[3], ctx->stream));
 
@@ -1205,7 +1263,7 @@ static void run_phj_pure_host(phj_ctx * ctx, const phj_block_stream & hb, const 
     // packing them would only add to the time before the first download)
     const bool mat = materialize_probe(ctx, lt, *B, n_leaves) && P_rows > 0;
     const Cols ppart = mat ? alloc_cols_like(s, hp.schema, C) : Cols{};
-    const uint32_t pb = probe_pass_bits(ctx, bits, *B);
+    const uint32_t pb = probe_pass_bits(ctx, total_bits, *B);
     const Cols ptmp = mat && pb > 11 ? alloc_cols_like(s, hp.schema, C) : ppart;
     uint32_t * poff = s.get<uint32_t>((1ull << pb) + 1);
     uint32_t * heads = s.get<uint32_t>(C);
