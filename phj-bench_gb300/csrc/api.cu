@@ -121,13 +121,19 @@ __global__ void k_read_small(const __grid_constant__ SmallReadArgs r, uint8_t * 
 }
 } // namespace
 
-void read_small(phj_ctx * ctx, std::initializer_list<SmallRead> reads)
+uint8_t * small_host(phj_ctx * ctx)
 {
     if (!ctx->host_small)
     {
         PHJ_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&ctx->host_small), kSmallReadBytes, cudaHostAllocMapped));
         PHJ_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->host_small_dev), ctx->host_small, 0));
     }
+    return ctx->host_small_dev;
+}
+
+void read_small(phj_ctx * ctx, std::initializer_list<SmallRead> reads)
+{
+    small_host(ctx);
     SmallReadArgs r{};
     uint32_t off = 0;
     for (const SmallRead & x : reads)
@@ -663,8 +669,70 @@ static void run_chj_form(phj_ctx * ctx, const phj_table & B, const phj_table & P
     *out = o;
 }
 
+// A join with a small build side in one launch (small.cu), where the rows
+// and the options allow it: an option that pins a form of the general path
+// keeps it.  Returns the output and the launch's events, or nullptr: the
+// general path has to run (build keys repeat and the probe side is long, or
+// the form does not apply).
+static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj_table & P, const char * name, cudaEvent_t (&ev)[3])
+{
+    if (ctx->probe_materialize >= 0 || ctx->probe_pass_bits || ctx->chj_windows > 1 || !ctx->probe_fused || !ctx->pack_build ||
+        ctx->table_cap_pct != 200 || !small_join_eligible(ctx, B.rows, P.rows, false))
+        return nullptr;
+    begin_run(ctx);
+    ev[0] = take_event(ctx);
+    ev[1] = ev[2] = take_event(ctx);
+    // Sized for one output row a probe row, exact for unique build keys; a
+    // join with more runs again into an output of the size it counted.  Its
+    // chains are written a row at a time, so past 400K probe rows a repeated
+    // key leaves the join to the general path before anything is probed
+    // (8K x 128K, four rows a key: 103 us in two launches against 180; 8K x
+    // 512K: 190 against 182).
+    const bool repeats_ok = P.rows <= 400000;
+    phj_output * o = new_output(ctx, B.schema, P.schema, P.rows);
+    for (int run = 0;; ++run)
+    {
+        uint64_t rows = 0;
+        try
+        {
+            rows = small_join(ctx, cols_of(B), B.rows, cols_of(P), P.rows, o->keys, o->lcol, o->rcol, o->cap, name, !repeats_ok,
+                              ev[run], ev[run + 1]);
+        }
+        catch (...)
+        {
+            free_output(ctx, o);
+            throw;
+        }
+        if (rows <= o->cap && rows != kSmallJoinRepeats)
+        {
+            o->rows = rows;
+            return o;
+        }
+        free_output(ctx, o);
+        if (run == 1 || rows == kSmallJoinRepeats)
+            return nullptr;
+        ev[2] = take_event(ctx);
+        o = new_output(ctx, B.schema, P.schema, rows);
+    }
+}
+
 static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj_output ** out, phj_chj_result * res)
 {
+    // (payloads the one-pass probe takes: both forms look up and project in
+    // one kernel and are recorded under its name)
+    cudaEvent_t ev[3];
+    if (phj_output * o = one_pass_schemas(B.schema, P.schema) ? try_small_join(ctx, B, P, "probe_fused", ev) : nullptr)
+    {
+        if (res)
+        {
+            fill_phase(res->build, 0.f, B.rows);
+            fill_phase(res->probe, event_ms(ev[0], ev[2]), P.rows);
+            res->e2e_wall_ms = res->probe.wall_ms;
+            res->peak_mem_bytes = ctx->peak_bytes;
+        }
+        *out = o;
+        return;
+    }
     // Clustered when the cells (32 to 64 bytes a row: 48) and the gathered
     // build rows (16 bytes packed) are past L2 by a fifth.  Measured, rows of
     // 12 payload bytes: 1.3M x 5M 300 -> 334 us clustered, 2M x 32M 957 ->
@@ -700,6 +768,22 @@ phj_output * join_alone(phj_ctx * ctx, const phj_table & B, const phj_table & P)
 static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P, const std::vector<uint32_t> & bits, phj_output ** out,
                          phj_phj_result * res)
 {
+    cudaEvent_t small_ev[3];
+    if (phj_output * o = try_small_join(ctx, B, P, "small_join", small_ev))
+    {
+        if (res)
+        {
+            // one launch: all of it counts as the probe
+            fill_phase(res->build_shuffle, 0.f, B.rows);
+            fill_phase(res->build, 0.f, B.rows);
+            fill_phase(res->probe_shuffle, 0.f, P.rows);
+            fill_phase(res->probe, event_ms(small_ev[0], small_ev[2]), P.rows);
+            res->e2e_wall_ms = res->probe.wall_ms;
+            res->peak_mem_bytes = ctx->peak_bytes;
+        }
+        *out = o;
+        return;
+    }
     begin_run(ctx);
     Scratch s(ctx);
     uint32_t total_bits = 0;
@@ -1695,6 +1779,9 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         PHJ_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
         PHJ_CUDA(cudaMalloc(&ctx->d_err, sizeof(int)));
         PHJ_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
+        PHJ_CUDA(cudaMalloc(&ctx->small_ctr, sizeof(SmallCounters)));
+        PHJ_CUDA(cudaMemset(ctx->small_ctr, 0, sizeof(SmallCounters)));
+        set_small_smem_limits();
         set_partition_smem_limits((int)ctx->smem_optin);
         set_build_smem_limits((int)ctx->smem_optin);
         set_bep_smem_limits((int)ctx->smem_optin);
@@ -1722,6 +1809,8 @@ void phj_ctx_destroy(phj_ctx * ctx)
             cudaFree(ctx->l2_flush);
         if (ctx->d_err)
             cudaFree(ctx->d_err);
+        if (ctx->small_ctr)
+            cudaFree(ctx->small_ctr);
         if (ctx->host_small)
             cudaFreeHost(ctx->host_small);
         for (cudaEvent_t e : ctx->event_pool)

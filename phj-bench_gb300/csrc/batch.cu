@@ -37,6 +37,7 @@
 // Output multisets equal those of the single-join entry points; the order
 // of the rows is not fixed.
 #include "internal.h"
+#include "piece.cuh"
 #include "scatter.cuh"
 
 #include <cstring>
@@ -48,17 +49,12 @@ namespace
 constexpr int kJNT = 256;              // threads of the join kernel
 constexpr uint32_t kPieceRows = 2048;  // build rows a shared table holds
 constexpr uint32_t kPieceSlots = 4096; // its slots (load <= 1/2)
-constexpr uint32_t kEmptySlot = 0xFFFFFFFFu; // a slot: 20 hash bits << 11 | row of the piece
-constexpr uint32_t kNil = 0xFFFFu;     // end of a chain
 
 struct BatchJoin
 {
-    Cols build, probe; // inputs
-    Cols bpart, ppart; // partitioned copies
-    uint64_t * out_keys;
-    void * out_l[kMaxCols];
-    void * out_r[kMaxCols];
-    uint64_t build_rows, probe_rows, out_cap;
+    Cols build, probe;  // inputs
+    ProbeSides part;    // partitioned copies, output
+    uint64_t build_rows, probe_rows;
     uint32_t bits;      // radix bits
     uint32_t part_base; // index of its first partition among all joins'
     uint32_t aligned_b, aligned_p; // every input column starts on a 16-byte boundary
@@ -168,7 +164,7 @@ struct BatchTiles
     }
     __device__ __forceinline__ const BatchJoin & join(const ScatterTile & t) const { return d[t.aux & ~kProbeSide]; }
     __device__ __forceinline__ const Cols & in(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).probe : join(t).build; }
-    __device__ __forceinline__ const Cols & out(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).ppart : join(t).bpart; }
+    __device__ __forceinline__ const Cols & out(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).part.probe : join(t).part.build; }
     __device__ __forceinline__ bool widened(const ScatterTile &) const { return false; }
     __device__ __forceinline__ bool aligned(const ScatterTile & t) const { return t.aux & kProbeSide ? join(t).aligned_p : join(t).aligned_b; }
     __device__ __forceinline__ uint32_t shift(const ScatterTile & t) const { return join(t).bits ? 64u - join(t).bits : 0u; }
@@ -194,244 +190,18 @@ __global__ void __launch_bounds__(kNT, 2) k_bt_scatter(const BatchJoin * __restr
     scatter_tiles<RPT>(s, smem, bar, stages, buf_bytes, nb_max, err);
 }
 
-// Four values of a payload column of at most 8 bytes, in 64-bit registers.
-__device__ __forceinline__ void load4(uint64_t (&v)[4], const void * src, uint32_t width, const uint32_t (&idx)[4], uint32_t one)
-{
-    switch (width)
-    {
-#define PHJ_LOAD4(W, T)                                                                                                                              \
-    case W:                                                                                                                                          \
-        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) v[u] = static_cast<const T *>(src)[idx[u]];                                 \
-        break;
-        PHJ_LOAD4(1, uint8_t)
-        PHJ_LOAD4(2, uint16_t)
-        PHJ_LOAD4(4, uint32_t)
-        default: PHJ_LOAD4(8, uint64_t)
-#undef PHJ_LOAD4
-    }
-}
-
-__device__ __forceinline__ void store4(const uint64_t (&v)[4], void * dst, uint32_t width, uint64_t base, const uint32_t (&rel)[4], uint32_t one)
-{
-    switch (width)
-    {
-#define PHJ_STORE4(W, T)                                                                                                                             \
-    case W:                                                                                                                                          \
-        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) __stcs(static_cast<T *>(dst) + base + rel[u], (T)v[u]);                     \
-        break;
-        PHJ_STORE4(1, uint8_t)
-        PHJ_STORE4(2, uint16_t)
-        PHJ_STORE4(4, uint32_t)
-        default: PHJ_STORE4(8, uint64_t)
-#undef PHJ_STORE4
-    }
-}
-
-// A slot's 20 hash bits, in place (its group of slots is chosen by the low
-// 12).
-__device__ __forceinline__ uint32_t slot_tag(uint64_t h)
-{
-    return (uint32_t)(h >> 1) & 0x7FFFF800u;
-}
-
-// A piece's table in shared memory.
-struct PieceTable
-{
-    const uint32_t * slots;
-    const uint64_t * keys;
-    const uint16_t * nxt;
-    uint32_t mask;
-
-    // The piece's row that heads `key`'s chain, kNil when the key is absent:
-    // groups of four slots are filled from their first slot on, so a group
-    // with an empty slot ends the search.
-    __device__ __forceinline__ uint32_t find(uint64_t key) const
-    {
-        const uint64_t h = int_hash64(key);
-        const uint32_t tag = slot_tag(h);
-        for (uint32_t pos = (uint32_t)h & mask & ~3u;; pos = (pos + 4) & mask) // some group has an empty slot
-        {
-            const uint4 s = *reinterpret_cast<const uint4 *>(slots + pos);
-            const uint32_t v[4] = {s.x, s.y, s.z, s.w};
-            // the group's last slot with the key's hash bits, without branches
-            uint32_t row = kNil;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                row = (v[i] ^ tag) < kPieceRows ? v[i] ^ tag : row;
-            if (row != kNil)
-            {
-                if (keys[row] == key)
-                    return row;
-                // other keys with the same hash bits: one by one
-                for (int i = 0; i < 4; ++i)
-                    if ((v[i] ^ tag) < kPieceRows && keys[v[i] ^ tag] == key)
-                        return v[i] ^ tag;
-            }
-            if (s.w == kEmptySlot)
-                return kNil;
-        }
-    }
-};
-
-__device__ __forceinline__ void prefetch_l2(const void * p)
-{
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// The CTA's warps probe rows [p0, p1) of the partition against the piece
-// whose first build row is c0, 128 rows a warp at a time.  kDup: some key
-// of the piece has more than one row (a row's matches are its chain).
+// The CTA's warps probe rows [p0, p1) of the partition, 128 a warp at a time.
 template <bool kDup>
-__device__ __forceinline__ void probe_piece(const BatchJoin & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable & tab,
-                                            unsigned long long * __restrict__ out_cur, int * __restrict__ over)
+__device__ __forceinline__ void probe_part(const ProbeSides & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable<kPieceRows> & tab,
+                                           unsigned long long * out_cur, int * over)
 {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll 1
-    for (uint32_t base = p0 + warp * 128; base < p1; base += kJNT / 32 * 128)
-    {
-        // the descriptor (in shared memory) is read where it is used: kept
-        // out of the loop its three dozen pointers would be spilled
-        asm volatile("" ::: "memory");
-        const uint64_t * pkeys = J.ppart.keys;
-        const uint64_t out_cap = J.out_cap;
-        uint64_t key[4];
-        uint32_t head[4], rel[4], total = 0, one = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-        {
-            const uint32_t r = base + u * 32 + lane;
-            key[u] = r < p1 ? __ldcs(pkeys + r) : 0ull;
-        }
-        {
-            // the warp's next chunk into L2, a line a lane
-            const uint32_t next = base + kJNT / 32 * 128;
-            const uint32_t rows = next < p1 ? min(128u, p1 - next) : 0u;
-            if (lane * 16 < rows)
-                prefetch_l2(pkeys + next + lane * 16);
-            for (uint32_t c = 0; c < J.ppart.n; ++c)
-                if (lane * 128 < rows * J.ppart.width[c])
-                    prefetch_l2(static_cast<const uint8_t *>(J.ppart.col[c]) + (uint64_t)next * J.ppart.width[c] + lane * 128);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-        {
-            head[u] = base + u * 32 + lane < p1 ? tab.find(key[u]) : kNil;
-            if (head[u] != kNil)
-                one |= 1u << u;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if constexpr (kDup)
-            {
-                uint32_t cnt = 0;
-                for (uint32_t b = head[u]; b != kNil; b = tab.nxt[b])
-                    ++cnt;
-                uint32_t x = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1)
-                {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= (uint32_t)o)
-                        x += y;
-                }
-                rel[u] = total + x - cnt;
-                total += __shfl_sync(0xffffffffu, x, 31);
-            }
-            else
-            {
-                const uint32_t m = __ballot_sync(0xffffffffu, one >> u & 1u);
-                rel[u] = total + __popc(m & ((1u << lane) - 1u));
-                total += __popc(m);
-            }
-        if (total == 0)
-            continue;
-        // the build payloads' columns, then the probe's; the first one's
-        // loads go out before the reservation comes back, each next one's
-        // before the last one's stores
-        const uint32_t nl = J.bpart.n, nc = nl + J.ppart.n;
-        auto load_column = [&](uint32_t c, uint64_t (&v)[4]) {
-            uint32_t idx[4];
-            const bool left = c < nl;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                idx[u] = left ? c0 + head[u] : base + u * 32 + lane;
-            const uint32_t i = left ? c : c - nl;
-            load4(v, left ? J.bpart.col[i] : J.ppart.col[i], left ? J.bpart.width[i] : J.ppart.width[i], idx, one);
-        };
-        unsigned long long o0 = 0;
-        if (lane == 0)
-        {
-            o0 = atomicAdd(out_cur, (unsigned long long)total);
-            if (o0 + total > out_cap)
-                *over = 1;
-        }
-        uint64_t v[4] = {0, 0, 0, 0};
-        if (!kDup && nc)
-            load_column(0, v);
-        o0 = __shfl_sync(0xffffffffu, o0, 0);
-        if constexpr (kDup)
-        {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                uint64_t o = o0 + rel[u];
-                for (uint32_t b = head[u]; b != kNil; b = tab.nxt[b], ++o)
-                    if (o < out_cap)
-                    {
-                        J.out_keys[o] = key[u];
-                        for (uint32_t c = 0; c < J.bpart.n; ++c)
-                            copy_elem(J.out_l[c], o, J.bpart.col[c], c0 + b, J.bpart.width[c]);
-                        for (uint32_t c = 0; c < J.ppart.n; ++c)
-                            copy_elem(J.out_r[c], o, J.ppart.col[c], base + u * 32 + lane, J.ppart.width[c]);
-                    }
-            }
-        }
-        else
-        {
-            uint64_t * out = J.out_keys + o0;
-            uint32_t fits = one;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                if (o0 + rel[u] >= out_cap)
-                    fits &= ~(1u << u);
-                if (fits >> u & 1u)
-                    __stcs(out + rel[u], key[u]);
-            }
-#pragma unroll 1
-            for (uint32_t c = 0; c < nc; ++c)
-            {
-                asm volatile("" ::: "memory");
-                const bool left = c < nl;
-                const uint32_t i = left ? c : c - nl, w = left ? J.bpart.width[i] : J.ppart.width[i];
-                void * dst = left ? J.out_l[i] : J.out_r[i];
-                uint64_t nx[4] = {0, 0, 0, 0};
-                if (c + 1 < nc)
-                    load_column(c + 1, nx);
-                if (w <= 8)
-                    store4(v, dst, w, o0, rel, fits);
-                else
-                {
-                    const uint4 * src = static_cast<const uint4 *>(left ? J.bpart.col[i] : J.ppart.col[i]);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (fits >> u & 1u)
-                            __stcs(static_cast<uint4 *>(dst) + o0 + rel[u], src[left ? c0 + head[u] : base + u * 32 + lane]);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    v[u] = nx[u];
-            }
-        }
-    }
+    probe_piece<kDup, 4>(J, p0 + (threadIdx.x >> 5) * 128, kJNT / 32 * 128, p1, c0, tab, out_cur, over);
 }
-
 // (out of line, so that its registers do not weigh on the unique-key form)
-__device__ __noinline__ void probe_piece_dup(const BatchJoin & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable tab,
-                                             unsigned long long * out_cur, int * over)
+__device__ __noinline__ void probe_part_dup(const ProbeSides & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable<kPieceRows> tab,
+                                            unsigned long long * out_cur, int * over)
 {
-    probe_piece<true>(J, p0, p1, c0, tab, out_cur, over);
+    probe_part<true>(J, p0, p1, c0, tab, out_cur, over);
 }
 
 // The persistent join: CTAs pop (join, partition) items until the queue is
@@ -488,49 +258,12 @@ __global__ void __launch_bounds__(kJNT, 4) k_bt_join(const BatchJoin * __restric
             const uint32_t cap = max(4u, min(kPieceSlots, (uint32_t)bit_ceil64(3ull * rows))), mask = cap - 1;
             if (c0 != b0)
                 __syncthreads(); // the last piece is no longer probed
-            if (threadIdx.x == 0)
-                s_dup = 0;
-            for (uint32_t i = threadIdx.x; i < cap; i += kJNT)
-                slots[i] = kEmptySlot;
-            for (uint32_t i = threadIdx.x; i < rows; i += kJNT)
-                bkeys[i] = J.bpart.keys[c0 + i];
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < rows; i += kJNT)
-            {
-                const uint64_t k = bkeys[i];
-                const uint64_t h = int_hash64(k);
-                const uint32_t tag = slot_tag(h), mine = tag | i;
-                uint32_t pos = (uint32_t)h & mask & ~3u, link = kNil;
-                for (;; pos = (pos + 1) & mask) // fewer rows than slots: an empty one is found
-                {
-                    uint32_t old = slots[pos];
-                    if (old == kEmptySlot)
-                        old = atomicCAS(&slots[pos], kEmptySlot, mine);
-                    if (old == kEmptySlot)
-                        break;
-                    if ((old ^ tag) < kPieceRows && bkeys[old ^ tag] == k)
-                    {
-                        // the key's slot: this row becomes its head (another
-                        // row of the key may have done so meanwhile)
-                        for (;;)
-                        {
-                            const uint32_t seen = atomicCAS(&slots[pos], old, mine);
-                            if (seen == old)
-                                break;
-                            old = seen;
-                        }
-                        link = old ^ tag;
-                        s_dup = 1;
-                        break;
-                    }
-                }
-                nxt[i] = (uint16_t)link;
-            }
-            __syncthreads();
+            build_piece<kPieceRows, kJNT>(J.part.build.keys + c0, rows, slots, bkeys, nxt, mask, &s_dup);
+            const PieceTable<kPieceRows> tab{slots, bkeys, nxt, mask};
             if (s_dup)
-                probe_piece_dup(J, p0, p1, c0, PieceTable{slots, bkeys, nxt, mask}, out_cur + j, over + j);
+                probe_part_dup(J.part, p0, p1, c0, tab, out_cur + j, over + j);
             else
-                probe_piece<false>(J, p0, p1, c0, PieceTable{slots, bkeys, nxt, mask}, out_cur + j, over + j);
+                probe_part<false>(J.part, p0, p1, c0, tab, out_cur + j, over + j);
         }
     }
 }
@@ -814,8 +547,8 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
         J.part_base = (uint32_t)parts[j];
         J.aligned_b = side_aligned(J.build);
         J.aligned_p = side_aligned(J.probe);
-        place(J.bpart, J.build, B.rows);
-        place(J.ppart, J.probe, P.rows);
+        place(J.part.build, J.build, B.rows);
+        place(J.part.probe, J.probe, P.rows);
         parts[j + 1] = parts[j] + (1ull << J.bits);
         most_bits = std::max(most_bits, J.bits);
         row_bytes = std::max<uint32_t>(row_bytes, 8 + (uint32_t)std::max(schema_bytes(B.schema), schema_bytes(P.schema)));
@@ -834,8 +567,8 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
     };
     for (BatchJoin & J : h)
     {
-        based(J.bpart);
-        based(J.ppart);
+        based(J.part.build);
+        based(J.part.probe);
     }
 
     // outputs at one row per probe row (exact for unique build keys)
@@ -846,12 +579,12 @@ void run_batch(phj_ctx * ctx, uint32_t n, const phj_table * const * builds, cons
         {
             made[j] = new_output(ctx, builds[j]->schema, probes[j]->schema, probes[j]->rows);
             BatchJoin & J = h[j];
-            J.out_keys = made[j]->keys;
+            J.part.out_keys = made[j]->keys;
             for (uint32_t c = 0; c < J.build.n; ++c)
-                J.out_l[c] = made[j]->lcol[c];
+                J.part.out_l[c] = made[j]->lcol[c];
             for (uint32_t c = 0; c < J.probe.n; ++c)
-                J.out_r[c] = made[j]->rcol[c];
-            J.out_cap = probes[j]->rows;
+                J.part.out_r[c] = made[j]->rcol[c];
+            J.part.out_cap = probes[j]->rows;
         }
         std::vector<unsigned long long> rows(n, 0);
         std::vector<int> ov(n, 0);

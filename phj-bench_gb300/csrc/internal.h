@@ -75,6 +75,17 @@ struct LeafMark
 
 namespace phjg
 {
+// Counters of the one-launch joins (small.cu): zero between joins.
+struct SmallCounters
+{
+    unsigned long long out_rows;
+    unsigned int done;    // finished CTAs
+    unsigned int repeats; // a piece had a repeated key (unique_only)
+};
+struct SmallResult // at the start of the context's mapped host buffer
+{
+    unsigned long long out_rows;
+};
 struct BatchGraph; // batch.cu: phj_batch_run's workspace and captured chain
 void free_batch_graph(phj_ctx * ctx);
 } // namespace phjg
@@ -118,6 +129,7 @@ struct phj_ctx
     int batch_graph = 1;          // phj_batch_run: 1 replays its chain as a CUDA graph, 0 launches it
     int probe_fused = 1;          // unique build keys, packed payloads: 1 looks up and projects in one kernel
     phjg::BatchGraph * batch_ws = nullptr;
+    phjg::SmallCounters * small_ctr = nullptr;
     uint32_t probe_pass_bits = 0; // PHJ-PURE probe side's written pass (0: the first logical pass's bits)
     int64_t test_stuck_leaf = -1; // test hook: PHJ/BEP leaf left BUILDING before the probe
     int64_t test_engine_stall_wave = -1; // test hook: a BEP engine group holds back from this wave's barrier
@@ -170,6 +182,8 @@ struct SmallRead
 constexpr uint32_t kMaxSmallReads = 8;
 constexpr uint32_t kSmallReadBytes = 512;
 void read_small(phj_ctx * ctx, std::initializer_list<SmallRead> reads);
+// The device address of that buffer (made on first use).
+uint8_t * small_host(phj_ctx * ctx);
 void reset_accounting(phj_ctx * ctx);
 
 template <class T>
@@ -368,6 +382,18 @@ bool bep_engine_supported(uint32_t b1, uint32_t total_bits);
 // One engine run into `out` (rows past out->cap are counted, not written).
 BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput & in, phj_output * out);
 
+// ----- small.cu ---------------------------------------------------------------------
+// Joins of a small build side in one launch.  Returns the join's output
+// rows; at most out_cap of them are written.  start and stop bracket the
+// launch (recorded as `name`); the call waits for the stream.  With
+// unique_only a repeated build key ends the join before it is probed:
+// kSmallJoinRepeats.
+constexpr uint64_t kSmallJoinRepeats = ~0ull;
+bool small_join_eligible(const phj_ctx * ctx, uint64_t build_rows, uint64_t probe_rows, bool noalloc);
+uint64_t small_join(phj_ctx * ctx, const Cols & build, uint64_t build_rows, const Cols & probe, uint64_t probe_rows, uint64_t * out_keys,
+                    void * const * out_l, void * const * out_r, uint64_t out_cap, const char * name, bool unique_only, cudaEvent_t start, cudaEvent_t stop);
+void set_small_smem_limits();
+
 // One join on its own (the CHJ scheme), for a batched join that needs more
 // output rows than the batch gave it.
 phj_output * join_alone(phj_ctx * ctx, const phj_table & B, const phj_table & P);
@@ -379,6 +405,8 @@ phj_output * probe_join(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const p
 void pack_build_payloads(phj_ctx * ctx, Scratch & s, ProbeArgs & a, uint64_t build_rows);
 // The two halves: lookups + chunk-offset scan (returns the output rows), and
 // the projection into `out` from row `out_base` on.
+// Whether the one-pass probe takes these payload columns (unique keys).
+bool one_pass_schemas(const phj_schema & build, const phj_schema & probe);
 uint64_t probe_chunks(uint64_t probe_rows);
 uint64_t probe_lookup(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, uint32_t * heads, uint32_t * counts);
 void probe_project(phj_ctx * ctx, const ProbeArgs & a, phj_output * out, uint64_t out_base, const uint32_t * heads, const uint32_t * offs,

@@ -145,6 +145,36 @@ __global__ void __launch_bounds__(kNaNT) k_na_probe(const __grid_constant__ Cols
     }
 }
 
+// The join through the global table in the scratch array.
+unsigned long long global_table_join(phj_ctx * ctx, const NaScratch & s, const Cols & bc, uint64_t build_rows, const Cols & pc, uint64_t probe_rows,
+                                     uint64_t cap, const Cols & ol, const Cols & orr, uint64_t out_cap)
+{
+    const unsigned fill_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(cap, kNaNT), (uint64_t)ctx->num_sms * 4));
+    {
+        KTimer kt(ctx, "noalloc_clear", cap, cap * sizeof(Cell));
+        k_na_clear<<<fill_grid, kNaNT, 0, ctx->stream>>>(s, cap);
+        PHJ_LAUNCHED(ctx, "noalloc_clear");
+    }
+    if (build_rows)
+    {
+        KTimer kt(ctx, "noalloc_build", build_rows, build_rows * 8);
+        k_na_build<<<(unsigned)std::min<uint64_t>(ceil_div(build_rows, kNaNT), (uint64_t)ctx->num_sms * 4), kNaNT, 0, ctx->stream>>>(bc.keys, build_rows,
+                                                                                                                                 s, cap);
+        PHJ_LAUNCHED(ctx, "noalloc_build");
+    }
+    if (probe_rows)
+    {
+        KTimer kt(ctx, "noalloc_probe", probe_rows, probe_rows * 8);
+        const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(probe_rows, kNaNT), (uint64_t)ctx->num_sms * 8);
+        k_na_probe<<<grid, kNaNT, 0, ctx->stream>>>(pc, probe_rows, bc, s, cap, ol, orr, out_cap);
+        PHJ_LAUNCHED(ctx, "noalloc_probe");
+    }
+    unsigned long long rows = 0;
+    PHJ_CUDA(cudaMemcpyAsync(&rows, s.rows, sizeof(rows), cudaMemcpyDeviceToHost, ctx->stream));
+    PHJ_CUDA(cudaStreamSynchronize(ctx->stream));
+    return rows;
+}
+
 void run_chj_noalloc(phj_ctx * ctx, const phj_table & B, const phj_table & P, uint64_t out_cap, uint64_t * out_keys, void * const * out_left,
                      void * const * out_right, uint64_t * out_rows)
 {
@@ -174,29 +204,16 @@ void run_chj_noalloc(phj_ctx * ctx, const phj_table & B, const phj_table & P, ui
     for (uint32_t c = 0; c < P.schema.n_payloads; ++c)
         orr.col[c] = out_right ? out_right[c] : nullptr;
 
-    const unsigned fill_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(cap, kNaNT), (uint64_t)ctx->num_sms * 4));
-    {
-        KTimer kt(ctx, "noalloc_clear", cap, cap * sizeof(Cell));
-        k_na_clear<<<fill_grid, kNaNT, 0, ctx->stream>>>(s, cap);
-        PHJ_LAUNCHED(ctx, "noalloc_clear");
-    }
-    if (B.rows)
-    {
-        KTimer kt(ctx, "noalloc_build", B.rows, B.rows * 8);
-        k_na_build<<<(unsigned)std::min<uint64_t>(ceil_div(B.rows, kNaNT), (uint64_t)ctx->num_sms * 4), kNaNT, 0, ctx->stream>>>(bc.keys, B.rows,
-                                                                                                                                 s, cap);
-        PHJ_LAUNCHED(ctx, "noalloc_build");
-    }
-    if (P.rows)
-    {
-        KTimer kt(ctx, "noalloc_probe", P.rows, P.rows * 8);
-        const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(P.rows, kNaNT), (uint64_t)ctx->num_sms * 8);
-        k_na_probe<<<grid, kNaNT, 0, ctx->stream>>>(pc, P.rows, bc, s, cap, ol, orr, out_cap);
-        PHJ_LAUNCHED(ctx, "noalloc_probe");
-    }
     unsigned long long rows = 0;
-    PHJ_CUDA(cudaMemcpyAsync(&rows, s.rows, sizeof(rows), cudaMemcpyDeviceToHost, ctx->stream));
-    PHJ_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (small_join_eligible(ctx, B.rows, P.rows, true))
+    {
+        // one launch, its tables in shared memory (small.cu); it allocates
+        // nothing either
+        rows = small_join(ctx, bc, B.rows, pc, P.rows, out_keys, ol.col, orr.col, out_cap, "noalloc_probe", false, take_event(ctx),
+                          take_event(ctx));
+    }
+    else
+        rows = global_table_join(ctx, s, bc, B.rows, pc, P.rows, cap, ol, orr, out_cap);
     if (out_rows)
         *out_rows = rows;
     if (rows > out_cap)

@@ -1175,6 +1175,19 @@ static int fused_gather_bytes(const ProbeArgs & a)
     return -1;
 }
 
+bool one_pass_schemas(const phj_schema & build, const phj_schema & probe)
+{
+    for (uint32_t c = 0; c < probe.n_payloads; ++c)
+        if (probe.types[c] == PHJ_U128)
+            return false;
+    Cols b{};
+    b.n = build.n_payloads;
+    for (uint32_t c = 0; c < b.n; ++c)
+        b.width[c] = (uint8_t)payload_width(build.types[c]);
+    PackSpec pk;
+    return pack_spec_of(b, pk) || b.n == 0 || (b.n == 1 && (b.width[0] == 4 || b.width[0] == 8));
+}
+
 // The fused probe: unique build keys whose payloads it gathers in one
 // piece, no 16-byte probe payload column (its staged values would not fit
 // the kernel's registers).

@@ -1,0 +1,58 @@
+"""Joins of a small build side in one launch against the oracle, and against
+the general path that a pinned option keeps: one row a side, around a warp's
+chunk (32 and 128 probe rows), a CTA's threads (1024) and a piece (8192
+rows), several pieces, keys that repeat inside and across pieces, more
+output rows than probe rows (two launches), a long probe side of a build
+side that repeats (the general path takes over), every payload
+width and no payload, twice in a row (the counter starts cleared)."""
+import numpy as np
+import pytest
+
+import oracle as O
+import phj_datagen as G
+import phj_gpu as P
+
+pytestmark = pytest.mark.gpu
+
+
+def sides(build, probe, tb, tp, repeat, match):
+    distinct = max(build // repeat, 1)
+    bk = np.resize(G.gen_keys(0, distinct, 601, 602), build)
+    pk = G.gen_keys(4, probe, 603, 602, domain=distinct, match_permille=match)
+    return P.BlockStream(tb, bk, G.payload_columns(604, tb, build)), P.BlockStream(tp, pk, G.payload_columns(605, tp, probe))
+
+
+@pytest.mark.parametrize("build,probe,tb,tp,repeat,match", [
+    (1, 1, [P.U64], [P.U32], 1, 1000),
+    (3, 33, [], [], 1, 500),
+    (1023, 127, [P.U32, P.U16, P.U8], [P.U64], 1, 900),
+    (1025, 152 * 1024 + 1, [P.U64, P.U32], [P.U64, P.U8], 1, 600),   # 128 rows a warp instead of 32
+    (8192, 5000, [P.U128, P.U8], [P.U16, P.U128], 1, 700),
+    (8193, 30_001, [P.U64], [P.U64], 1, 800),                        # two pieces
+    (60_000, 20_000, [P.U32] * 8, [P.U8] * 8, 1, 800),               # eight pieces, eight columns a side
+    (20_000, 40_000, [P.U64], [P.U32], 5, 150),                      # repeats, fewer output than probe rows
+    (20_000, 9000, [P.U64, P.U128], [P.U32], 20_000, 1000),          # one key: 20,000 rows a match
+    (3000, 20_000, [P.U16, P.U64], [P.U32], 4, 900),                 # more output rows than probe rows
+    (3000, 400_001, [P.U64], [P.U32], 2, 300),                       # repeats and a long probe side: the general path
+    (65_536, 4000, [P.U64], [P.U32], 1, 900),                        # the most build rows
+])
+def test_rows_equal_the_oracle(ctx, build, probe, tb, tp, repeat, match):
+    b, p = sides(build, probe, tb, tp, repeat, match)
+    if build == 20_000 and repeat == 20_000:
+        p = P.BlockStream(tp, p.keys[:40], [c[:40] for c in p.payloads])
+    expected = O.join_rows(b, p)
+    t, u = ctx.upload(b), ctx.upload(p)
+    general = repeat > 1 and p.total_rows > 400_000
+    for pinned in (False, False, True):
+        for scheme in ("pure", "chj"):
+            if pinned:
+                ctx.set_int("probe_materialize", 0)
+            try:
+                out, _ = ctx.run_phj_pure(t, u, [6]) if scheme == "pure" else ctx.run_chj(t, u)
+            finally:
+                ctx.set_int("probe_materialize", -1)
+            if scheme == "pure":
+                assert ("small_join" in {k["name"] for k in ctx.kernel_times()}) == (not pinned and not general)
+            assert O.compare_outputs(expected, O.serialize_output(out.download())) == ""
+            out.free()
+    t.free(), u.free()
