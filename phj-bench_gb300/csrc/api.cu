@@ -171,6 +171,55 @@ void dfree(phj_ctx * ctx, void * p)
     cudaFreeAsync(p, ctx->stream);
 }
 
+void arena_release(phj_ctx * ctx) noexcept
+{
+    ScratchArena & a = ctx->arena;
+    if (!a.base || a.depth)
+        return;
+    // work that reads it may be in flight: on the main stream, or on another
+    // one when a call ended early
+    cudaDeviceSynchronize();
+    cudaFree(a.base);
+    a.base = nullptr;
+    a.size = a.used = 0;
+}
+
+void arena_begin(phj_ctx * ctx)
+{
+    ScratchArena & a = ctx->arena;
+    a.used = a.asked = 0;
+    if (a.off || a.want <= a.size)
+        return;
+    // grown to what the last call asked for; what the pool kept for that
+    // call goes back first
+    arena_release(ctx);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    void * p = nullptr;
+    if (cudaMalloc(&p, a.want) == cudaSuccess)
+    {
+        a.base = static_cast<uint8_t *>(p);
+        a.size = a.want;
+    }
+    else
+    {
+        // no room: this call's scratch comes from the pool, and a next
+        // attempt asks for less
+        cudaGetLastError();
+        a.most = a.want / 2;
+    }
+    a.want = a.size;
+}
+
+void arena_end(phj_ctx * ctx) noexcept
+{
+    ScratchArena & a = ctx->arena;
+    // an eighth and 2 MiB more than asked for, so that a little more the
+    // next time is no new growth
+    if (!a.off && a.asked > a.size)
+        a.want = std::min<size_t>(a.asked + a.asked / 8 + (2 << 20), a.most) & ~size_t(255);
+    a.used = 0;
+}
+
 void reset_accounting(phj_ctx * ctx)
 {
     ctx->peak_bytes = ctx->cur_bytes;
@@ -1765,6 +1814,7 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         ctx->num_sms = prop.multiProcessorCount;
         ctx->smem_optin = prop.sharedMemPerBlockOptin;
         ctx->l2_bytes = prop.l2CacheSize;
+        ctx->arena.most = prop.totalGlobalMem / 4;
         // the main stream goes first: its kernels take the SMs as the side
         // stream's short CTAs end (probe side's first pass, see k_scatter)
         int prio_least = 0, prio_greatest = 0;
@@ -1813,6 +1863,7 @@ void phj_ctx_destroy(phj_ctx * ctx)
             cudaFree(ctx->small_ctr);
         if (ctx->host_small)
             cudaFreeHost(ctx->host_small);
+        arena_release(ctx);
         for (cudaEvent_t e : ctx->event_pool)
             cudaEventDestroy(e);
         for (auto & lv : ctx->live)

@@ -90,6 +90,22 @@ struct BatchGraph; // batch.cu: phj_batch_run's workspace and captured chain
 void free_batch_graph(phj_ctx * ctx);
 } // namespace phjg
 
+// Scratch memory of a call, kept by the context between calls: one block that
+// a call's scratch buffers are cut from and that is empty again when the call
+// ends.  (From the stream-ordered pool every buffer cost a microsecond or two,
+// and large ones, and the outputs allocated among them, did not find their
+// place again from call to call: the pool mapped memory anew, 0.2 to 1.6 ms.)
+struct ScratchArena
+{
+    uint8_t * base = nullptr;
+    size_t size = 0, used = 0;
+    size_t asked = 0;  // bytes asked for in this call, with those past `size`
+    size_t want = 0;   // size for the next call
+    size_t most = 0;   // bound of `size`
+    int depth = 0;     // Scratch objects alive
+    bool off = false;  // this call runs from the pool alone
+};
+
 struct phj_ctx
 {
     int device = 0;
@@ -106,6 +122,7 @@ struct phj_ctx
     // Allocation accounting of the current run (peak_mem_bytes).
     uint64_t cur_bytes = 0, peak_bytes = 0;
     std::vector<std::pair<void *, uint64_t>> live; // small: a run holds tens of buffers
+    ScratchArena arena;
     // Per-kernel timing of the last run.
     bool time_kernels = true;
     std::vector<phjg::KernelRecord> records;
@@ -192,24 +209,52 @@ T * dalloc_n(phj_ctx * ctx, uint64_t n)
     return static_cast<T *>(dalloc(ctx, (size_t)(n ? n : 1) * sizeof(T)));
 }
 
-// RAII holder for run-scoped scratch.
+// The arena at a call's first Scratch object, and after its last one.
+void arena_begin(phj_ctx * ctx);
+void arena_end(phj_ctx * ctx) noexcept;
+// Gives the arena's memory back (no call may be using it).
+void arena_release(phj_ctx * ctx) noexcept;
+
+// RAII holder for run-scoped scratch: cut from the context's arena while it
+// has room (given back when the call's first Scratch ends), else from the
+// pool.
 struct Scratch
 {
     phj_ctx * ctx;
-    std::vector<void *> ptrs;
+    std::vector<void *> ptrs; // from the pool
+    uint64_t cut = 0;         // bytes from the arena
     explicit Scratch(phj_ctx * c)
         : ctx(c)
     {
+        if (ctx->arena.depth == 0)
+            arena_begin(ctx);
+        ++ctx->arena.depth;
     }
     ~Scratch()
     {
         for (void * p : ptrs)
             dfree(ctx, p);
+        ctx->cur_bytes -= cut;
+        if (--ctx->arena.depth == 0)
+            arena_end(ctx);
     }
     template <class T>
     T * get(uint64_t n)
     {
-        T * p = dalloc_n<T>(ctx, n);
+        const size_t bytes = ((size_t)(n ? n : 1) * sizeof(T) + 255) & ~size_t(255);
+        ScratchArena & a = ctx->arena;
+        a.asked += bytes;
+        if (!a.off && bytes <= a.size - a.used)
+        {
+            T * p = reinterpret_cast<T *>(a.base + a.used);
+            a.used += bytes;
+            cut += bytes;
+            ctx->cur_bytes += bytes;
+            ctx->peak_bytes = std::max(ctx->peak_bytes, ctx->cur_bytes);
+            return p;
+        }
+        ptrs.reserve(ptrs.size() + 1);
+        T * p = static_cast<T *>(dalloc(ctx, bytes));
         ptrs.push_back(p);
         return p;
     }
@@ -477,7 +522,24 @@ inline phj_status guard(phj_ctx * ctx, F && f)
     }
     try
     {
-        f();
+        try
+        {
+            f();
+        }
+        catch (const Error & e)
+        {
+            // out of memory while the arena holds some: once more without it
+            if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || !ctx->arena.base)
+                throw;
+            arena_release(ctx);
+            struct Off
+            {
+                phj_ctx * c;
+                ~Off() { c->arena.off = false; }
+            } off{ctx};
+            ctx->arena.off = true;
+            f();
+        }
         if (ctx)
             ctx->last_error.clear();
         return PHJ_OK;
