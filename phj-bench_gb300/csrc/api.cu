@@ -561,10 +561,11 @@ phj_output * probe_chj_windows(phj_ctx * ctx, Scratch & s, const ProbeArgs & a_i
 
 // A bounded device wait that gave up leaves a code in the error word; the
 // run fails with PHJ_ERR_DEVICE_TIMEOUT and the word is cleared.
-static void check_device_error(phj_ctx * ctx)
+static void check_device_error(phj_ctx * ctx, const ProbeFound * read = nullptr)
 {
-    int e = 0;
-    read_small(ctx, {{&e, ctx->d_err, sizeof(int)}});
+    int e = read ? read->err : 0;
+    if (!read)
+        read_small(ctx, {{&e, ctx->d_err, sizeof(int)}});
     if (e != 0)
     {
         PHJ_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
@@ -857,20 +858,101 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     // -------- BUILD SHUFFLE (src/PHJ.cpp:220-223) --------
     const Cols bin = cols_of(B);
     const Cols bpart = alloc_cols_like(s, B.schema, B.rows);
-    const Cols btmp = alloc_cols_like(s, B.schema, B.rows);
+    // (one physical pass goes straight to bpart; grouping makes its own)
+    Cols btmp = total_bits > 11 ? alloc_cols_like(s, B.schema, B.rows) : bpart;
     uint32_t * leaf_off = s.get<uint32_t>((uint64_t)n_leaves + 1);
     LeafTables lt;
     bool grouped = false;
+    phj_output * o = nullptr;
+    auto fill_tables = [&](ProbeArgs & x) {
+        x.probe_rows = P.rows;
+        x.meta = lt.meta;
+        x.cells = lt.cells;
+        x.next = lt.next;
+        x.leaf_bits = total_bits;
+        x.chj = 0;
+        x.any_dup = lt.any_dup;
+        x.uniform_log2cap = lt.uniform_log2cap;
+    };
+    // `read`: the probe's read has waited for the stream and has the error word
+    auto finish = [&](phj_output * done, const ProbeFound * read) {
+        try
+        {
+            if (!read)
+            {
+                PHJ_CUDA(cudaEventRecord(ev[4], ctx->stream));
+                PHJ_CUDA(cudaEventSynchronize(ev[4]));
+            }
+            check_device_error(ctx, read);
+            debug_timeline(ctx, ev[0]);
+            if (res)
+            {
+                fill_phase(res->build_shuffle, event_ms(ev[0], ev[1]), B.rows);
+                fill_phase(res->build, event_ms(ev[1], ev[2]), B.rows);
+                // the probe side's first pass runs beside the build: its own span
+                fill_phase(res->probe_shuffle, mat ? event_ms(ev[5], ev[6]) : 0.f, P.rows);
+                fill_phase(res->probe, event_ms(ev[3], ev[4]), P.rows);
+                res->e2e_wall_ms = event_ms(ev[0], ev[4]);
+                res->peak_mem_bytes = ctx->peak_bytes;
+            }
+        }
+        catch (...)
+        {
+            free_output(ctx, done);
+            throw;
+        }
+        *out = done;
+    };
     try
     {
         radix_partition(ctx, s, bin, B.rows, bits, bpart, btmp, leaf_off, "build_scatter");
         PHJ_CUDA(cudaEventRecord(ev[1], ctx->stream));
 
+        // -------- inline tables: at most 8 payload bytes, no repeated key;
+        // sized by estimate, so nothing is read back before the probe is
+        // through --------
+        a.build = payload_cols(bpart);
+        a.any_dup = 0;
+        a.probe_rows = P.rows;
+        PackSpec pk;
+        InlineTables it;
+        ProbeFound found;
+        found.done = ev[4];
+        // Whether the probe goes ahead against tables whose flags are not
+        // known yet.  Beside a probe pass on the side stream the flags are
+        // read first: the pass hides the round trip, and a build that has
+        // to be done again does not wait for the pass.
+        auto usable = [&](const int * flags) {
+            if (mat)
+                read_small(ctx, {{&found.flags, flags, sizeof(int)}});
+            return found.flags == 0;
+        };
+        if (ctx->pack_build && pack_columns(a.build, 8, pk))
+        {
+            ProbeArgs q = a;
+            q.build.n = 0; // (the payloads need no gather)
+            if (one_pass_probe(ctx, q))
+            {
+                Scratch si(ctx); // tables that cannot be used go back at once
+                int * bad = si.get<int>(1);
+                PHJ_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
+                if (build_inline_tables(ctx, si, bpart, B.rows, leaf_off, total_bits, pk, it, bad) && usable(bad))
+                {
+                    PHJ_CUDA(cudaEventRecord(ev[2], ctx->stream));
+                    if (mat)
+                        pass.join(ev[6]);
+                    PHJ_CUDA(cudaEventRecord(ev[3], ctx->stream));
+                    o = probe_inline(ctx, si, a.probe, P.rows, it, a.build, pk, B.schema, P.schema, bad, found);
+                }
+            }
+        }
+        if (o)
+            return finish(o, &found);
+        const int inline_found = found.flags;
+
         // build payloads packed for the projection on a third stream,
         // beside the leaf tables (both only read the partitioned rows);
         // dropped if a key repeats
-        a.build = payload_cols(bpart);
-        a.any_dup = 0;
         if (!ctx->aux)
         {
             int least = 0, greatest = 0; // as the main stream's
@@ -894,9 +976,39 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
 
         // -------- BUILD: per-leaf tables (src/PHJ.cpp:260-282) --------
         lt.next = s.get<uint64_t>(B.rows);
-        build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt);
+        build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows);
+        if (lt.estimated)
+        {
+            // the one-pass probe goes ahead; when the tables turn out not
+            // to fit it ends at once, and the build's flags say why
+            found.flags = 0;
+            if (inline_found || !one_pass_probe(ctx, a))
+                read_small(ctx, {{&found.flags, lt.flags, sizeof(int)}});
+            else if (usable(lt.flags))
+            {
+                PHJ_CUDA(cudaEventRecord(ev[2], ctx->stream));
+                if (mat)
+                    pass.join(ev[6]);
+                PHJ_CUDA(cudaStreamWaitEvent(ctx->stream, ev[8], 0));
+                PHJ_CUDA(cudaEventRecord(ev[3], ctx->stream));
+                fill_tables(a);
+                o = probe_estimated(ctx, s, a, B.schema, P.schema, lt.flags, found);
+                if (o)
+                    return finish(o, &found);
+            }
+            if (found.flags & kLeafOverflow)
+            {
+                lt = LeafTables{};
+                lt.next = s.get<uint64_t>(B.rows);
+                build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt);
+            }
+            else
+                lt.any_dup = found.flags & kLeafRepeats;
+        }
         // repeated keys: each key's rows made contiguous, so the probe
         // expands a match as a row range
+        if (lt.any_dup && btmp.keys == bpart.keys)
+            btmp = alloc_cols_like(s, B.schema, B.rows);
         grouped = group_leaf_duplicates(ctx, bpart, btmp, leaf_off, n_leaves, lt);
         if (lt.any_dup)
             a.packed = nullptr;
@@ -915,32 +1027,10 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     PHJ_CUDA(cudaEventRecord(ev[3], ctx->stream));
 
     // -------- PROBE with projection (src/PHJ.cpp:284-299) --------
-    a.probe_rows = P.rows;
     a.build = payload_cols(grouped ? btmp : bpart);
     a.grouped = grouped ? 1 : 0;
-    a.meta = lt.meta;
-    a.cells = lt.cells;
-    a.next = lt.next;
-    a.leaf_bits = total_bits;
-    a.chj = 0;
-    a.any_dup = lt.any_dup;
-    a.uniform_log2cap = lt.uniform_log2cap;
-    phj_output * o = probe_into_output(ctx, s, a, B.schema, P.schema);
-    PHJ_CUDA(cudaEventRecord(ev[4], ctx->stream));
-    PHJ_CUDA(cudaEventSynchronize(ev[4]));
-    check_device_error(ctx);
-    debug_timeline(ctx, ev[0]);
-    if (res)
-    {
-        fill_phase(res->build_shuffle, event_ms(ev[0], ev[1]), B.rows);
-        fill_phase(res->build, event_ms(ev[1], ev[2]), B.rows);
-        // the probe side's first pass runs beside the build: its own span
-        fill_phase(res->probe_shuffle, mat ? event_ms(ev[5], ev[6]) : 0.f, P.rows);
-        fill_phase(res->probe, event_ms(ev[3], ev[4]), P.rows);
-        res->e2e_wall_ms = event_ms(ev[0], ev[4]);
-        res->peak_mem_bytes = ctx->peak_bytes;
-    }
-    *out = o;
+    fill_tables(a);
+    finish(probe_into_output(ctx, s, a, B.schema, P.schema), nullptr);
 }
 
 // PHJ (BEP).  The build side is shuffled to full leaf depth and its leaf

@@ -320,13 +320,43 @@ struct LeafTables
     int any_dup = 0;
     int uniform_log2cap = -1; // >= 0: every leaf table has 2^this cells at leaf << this
     uint32_t * state = nullptr; // lazy build (PHJ/BEP): per leaf NOT_BUILT / BUILDING / BUILT
+    int * flags = nullptr;      // device: kLeafRepeats, kLeafOverflow
+    bool estimated = false;     // sized by estimate: any_dup is unknown until the flags are read
+};
+
+// What a build found: some key has more than one row; some leaf is past its
+// estimated capacity (its table was not built).
+constexpr int kLeafRepeats = 1, kLeafOverflow = 2;
+
+// Leaf tables whose cells {key, packed payload} answer a lookup by
+// themselves: `cap` cells a leaf at leaf * cap.  A lookup starts at the
+// even cell of a pair chosen by the hash's low 32 bits (any even capacity
+// will do) and goes on cell by cell.  An empty cell of a leaf holds a key
+// of the other half of the leaves.
+struct InlineTables
+{
+    ulonglong2 * cells = nullptr;
+    uint32_t cap = 0;
+    uint32_t leaf_shift = 0; // leaf = hash >> leaf_shift
+    uint32_t half_shift = 0; // upper half of the leaves: leaf >> half_shift
+    uint64_t half_key[2] = {0, 0};
+
+    __device__ __forceinline__ uint32_t start(uint64_t hash) const { return __umulhi((uint32_t)hash, cap >> 1) << 1; }
+    __device__ __forceinline__ uint64_t empty_key(uint32_t leaf) const { return half_key[1u - (leaf >> half_shift)]; }
 };
 
 // Per-leaf tables over leaf-partitioned build rows (PHJ-PURE / PHJ).  With
 // `lazy` only the layout is planned; the probe builds each table on first
-// use (PHJ/BEP).
+// use (PHJ/BEP).  With `estimate_rows` (the build rows) the tables are sized
+// by estimate where that costs no more than the usual sizes, without a host
+// round trip: lt.flags then says whether the tables can be used.
 void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, const uint32_t * leaf_off, uint32_t n_leaves,
-                       LeafTables & lt, bool lazy = false);
+                       LeafTables & lt, bool lazy = false, uint64_t estimate_rows = 0);
+// Inline tables over leaf-partitioned build rows, sized by estimate: false
+// (nothing done) when the leaves are too small or too large for them.
+// *bad (device, zero before) receives what the build found.
+bool build_inline_tables(phj_ctx * ctx, Scratch & s, const Cols & part, uint64_t rows, const uint32_t * leaf_off, uint32_t total_bits,
+                         const PackSpec & pk, InlineTables & t, int * bad);
 // Makes the rows of each repeated key contiguous (src -> dst, one CTA per
 // leaf) so the probe expands a match as a row range instead of a chain
 // walk.  Returns false (nothing done) when no key repeats or a leaf table is
@@ -443,6 +473,25 @@ void set_small_smem_limits();
 // output rows than the batch gave it.
 phj_output * join_alone(phj_ctx * ctx, const phj_table & B, const phj_table & P);
 
+// The packed layout of payload columns of at most 8 bytes each, `most` bytes
+// in all; false when they do not fit.
+bool pack_columns(const Cols & payloads, uint32_t most, PackSpec & pk);
+// Whether the one-pass probe applies to unique build keys.
+bool one_pass_probe(const phj_ctx * ctx, const ProbeArgs & a);
+// The one-pass probe against tables that were sized by estimate: nullptr
+// (and the flags) when the build found them unusable.  One read brings the
+// row count, the flags and the error word back; `done` is recorded before it.
+struct ProbeFound
+{
+    cudaEvent_t done = nullptr;
+    int flags = 0; // of the build
+    int err = 0;   // the context's error word
+};
+phj_output * probe_estimated(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const phj_schema & left, const phj_schema & right, const int * flags,
+                             ProbeFound & found);
+// The same against inline tables (pk: the payloads' places).
+phj_output * probe_inline(phj_ctx * ctx, Scratch & s, const Cols & probe, uint64_t probe_rows, const InlineTables & t, const Cols & build,
+                          const PackSpec & pk, const phj_schema & left, const phj_schema & right, const int * flags, ProbeFound & found);
 // Lookups, then an exactly sized output, then the projection.
 phj_output * probe_join(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const phj_schema & left, const phj_schema & right);
 // Sets a.packed (and packed_off) when the plain projection can use packed

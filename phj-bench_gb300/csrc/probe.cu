@@ -686,8 +686,10 @@ template <int kMode, int kGather>
 __global__ void __launch_bounds__(kPNT, 3) k_probe_fused(const __grid_constant__ ProbeArgs a, const __grid_constant__ ProjCols pc,
                                                       const __grid_constant__ PackedCols bc, uint64_t * __restrict__ out_keys,
                                                       unsigned long long * __restrict__ out_rows, unsigned long long * __restrict__ tickets,
-                                                      uint64_t out_cap)
+                                                      uint64_t out_cap, const int * __restrict__ bad)
 {
+    if (bad && *bad)
+        return; // the tables cannot be used
     __shared__ __align__(16) uint8_t fsm[kPWarps * kFWarpBytes];
     const uint32_t lane = threadIdx.x & 31;
     uint8_t * wsm = fsm + (threadIdx.x >> 5) * kFWarpBytes;
@@ -778,6 +780,230 @@ __global__ void __launch_bounds__(kPNT, 3) k_probe_fused(const __grid_constant__
             base += running;
             __syncwarp(); // the stage is refilled by the next half
         }
+        chunk = (uint32_t)__shfl_sync(0xffffffffu, tn, 0);
+    }
+}
+
+// Four values a lane of a probe payload column of at most 8 bytes, in 64-bit
+// registers: rows row0 + idx[u].
+__device__ __forceinline__ void load_list(uint64_t (&v)[4], const void * src, uint32_t width, uint64_t row0, const uint32_t (&idx)[4], uint32_t one)
+{
+    switch (width)
+    {
+#define PHJ_LOAD_LIST(W, T)                                                                                                                          \
+    case W:                                                                                                                                          \
+        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) v[u] = __ldcs(static_cast<const T *>(src) + row0 + idx[u]);                 \
+        break;
+        PHJ_LOAD_LIST(1, uint8_t)
+        PHJ_LOAD_LIST(2, uint16_t)
+        PHJ_LOAD_LIST(4, uint32_t)
+        default: PHJ_LOAD_LIST(8, uint64_t)
+#undef PHJ_LOAD_LIST
+    }
+}
+
+// Four values a lane to output rows out + 32 * u of a column.
+__device__ __forceinline__ void store_list(const uint64_t (&v)[4], void * dst, uint32_t width, uint64_t out, uint32_t one)
+{
+    switch (width)
+    {
+#define PHJ_STORE_LIST(W, T)                                                                                                                         \
+    case W:                                                                                                                                          \
+        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) __stcs(static_cast<T *>(dst) + out + 32 * u, (T)v[u]);                      \
+        break;
+        PHJ_STORE_LIST(1, uint8_t)
+        PHJ_STORE_LIST(2, uint16_t)
+        PHJ_STORE_LIST(4, uint32_t)
+        default: PHJ_STORE_LIST(8, uint64_t)
+#undef PHJ_STORE_LIST
+    }
+}
+
+// The one-pass probe against inline tables (unique keys, at most 8 payload
+// bytes, InlineTables): the cell pair a row's lookup loads holds its build
+// payloads, so a probe row costs one random request instead of two, and no
+// build row is gathered.  Chunks and keys as k_probe_fused.  The chunk's
+// matching rows are listed in shared memory and written 128 at a time, every
+// lane with a row of its own, whatever the match rate; the probe payloads'
+// loads go out before the output reservation comes back.
+// Bound by instructions and the latency of a chunk's chain of steps (230
+// instructions for 32 rows, issue 50% busy; the request path from L1 to the
+// crossbar is half idle).  1M x 8M rows 131 -> 100 us, 3M x 37M (five
+// payload columns, half of the rows match) 500 -> 430.  With 64 registers a
+// thread and four CTAs a SM it spills: 143 and 572 us.
+constexpr uint32_t kIKeys = 0, kIPay = 2048, kIQueue = 4096, kIHits = 4608, kIList = 4640, kIWarpBytes = 4896;
+__global__ void __launch_bounds__(kPNT, 3) k_probe_inline(const uint64_t * __restrict__ keys, uint64_t probe_rows,
+                                                          const __grid_constant__ InlineTables t, const __grid_constant__ ProjCols pc,
+                                                          const __grid_constant__ PackedCols bc, uint64_t * __restrict__ out_keys,
+                                                          unsigned long long * __restrict__ out_rows, unsigned long long * __restrict__ tickets,
+                                                          uint64_t out_cap, const int * __restrict__ bad)
+{
+    if (*bad)
+        return; // the tables cannot be used
+    __shared__ __align__(16) uint8_t ism[kPWarps * kIWarpBytes];
+    const uint32_t lane = threadIdx.x & 31;
+    uint8_t * wsm = ism + (threadIdx.x >> 5) * kIWarpBytes;
+    uint64_t * key_s = reinterpret_cast<uint64_t *>(wsm + kIKeys);
+    uint64_t * pay_s = reinterpret_cast<uint64_t *>(wsm + kIPay);
+    uint16_t * qrow = reinterpret_cast<uint16_t *>(wsm + kIQueue);
+    uint32_t * hits = reinterpret_cast<uint32_t *>(wsm + kIHits); // bit `lane` of word k: row k * 32 + lane
+    uint8_t * list = wsm + kIList;                                // matching rows of the chunk
+    const uint32_t n_chunks = (uint32_t)ceil_div(probe_rows, kWChunk); // probe rows < 2^32
+    unsigned long long t0 = 0;
+    if (lane == 0)
+        t0 = atomicAdd(tickets, 1ull);
+    uint32_t chunk = (uint32_t)__shfl_sync(0xffffffffu, t0, 0);
+    const uint64_t stream = l2_evict_first(); // keys are read once
+    while (chunk < n_chunks)
+    {
+        unsigned long long tn = 0; // the next chunk's ticket, taken early
+        if (lane == 0)
+            tn = atomicAdd(tickets, 1ull);
+        const uint64_t row0 = (uint64_t)chunk * kWChunk;
+        const uint32_t rows = (uint32_t)(probe_rows - row0 < kWChunk ? probe_rows - row0 : kWChunk);
+#pragma unroll
+        for (int k = 0; k < kPRPT; ++k)
+            if ((uint32_t)k * 32 + lane < rows)
+                cp_async8(key_s + k * 32 + lane, keys + row0 + (uint32_t)k * 32 + lane, stream);
+        cp_async_wait_all();
+        uint32_t qn = 0;
+#pragma unroll 1
+        for (uint32_t g = 0; g < kWChunk; g += 128)
+        {
+            uint64_t key[4];
+            CellPair cell[4];
+            uint32_t upper = 0; // bit u: the key's leaf is in the upper half
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const uint32_t i = g + u * 32 + lane;
+                key[u] = 0;
+                if (i < rows)
+                {
+                    key[u] = ld_shared_u64(key_s + i);
+                    const uint64_t h = int_hash64(key[u]);
+                    upper |= (uint32_t)(h >> 63) << u;
+                    cell[u] = load_pair<false>(reinterpret_cast<const Cell *>(t.cells + (h >> t.leaf_shift) * t.cap + t.start(h)));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const uint32_t i = g + u * 32 + lane;
+                const uint64_t none = upper >> u & 1u ? t.half_key[0] : t.half_key[1];
+                const bool first = cell[u].a.x == key[u], hit = i < rows && (first || cell[u].b.x == key[u]);
+                // a full pair of other keys: on to the cells after it (a pair
+                // fills from its first cell on)
+                const bool more = i < rows && !hit && cell[u].b.x != none;
+                if (hit)
+                    pay_s[i] = first ? cell[u].a.y : cell[u].b.y;
+                const uint32_t mh = __ballot_sync(0xffffffffu, hit), mq = __ballot_sync(0xffffffffu, more);
+                if (lane == 0)
+                    hits[g / 32 + u] = mh;
+                if (more)
+                    qrow[qn + __popc(mq & ((1u << lane) - 1u))] = (uint16_t)i;
+                qn += __popc(mq);
+            }
+        }
+        __syncwarp();
+        for (uint32_t j = lane; j < qn; j += 32)
+        {
+            const uint32_t i = qrow[j];
+            const uint64_t qk = key_s[i];
+            const uint64_t h = int_hash64(qk);
+            const uint64_t none = h >> 63 ? t.half_key[0] : t.half_key[1];
+            const ulonglong2 * tab = t.cells + (h >> t.leaf_shift) * t.cap;
+            uint32_t pos = t.start(h) + 2;
+            for (uint32_t step = 2; step < t.cap; step += 2)
+            {
+                pos = pos >= t.cap ? 0 : pos; // cap is even: pairs do not straddle the end
+                const CellPair c = load_pair<false>(reinterpret_cast<const Cell *>(tab + pos));
+                if (c.a.x == qk || c.b.x == qk)
+                {
+                    pay_s[i] = c.a.x == qk ? c.a.y : c.b.y;
+                    atomicOr(hits + (i >> 5), 1u << (i & 31));
+                    break;
+                }
+                if (c.b.x == none)
+                    break;
+                pos += 2;
+            }
+        }
+        __syncwarp();
+        uint32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < kPRPT; ++k)
+        {
+            const uint32_t m = hits[k];
+            if (m >> lane & 1u)
+                list[total + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(k * 32 + lane);
+            total += __popc(m);
+        }
+        __syncwarp();
+        if (total)
+        {
+            unsigned long long b0 = 0;
+            if (lane == 0)
+                b0 = atomicAdd(out_rows, (unsigned long long)total);
+            uint64_t base = 0;
+#pragma unroll 1
+            for (uint32_t j0 = 0; j0 < total; j0 += 128)
+            {
+                uint32_t idx[4], one = 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const uint32_t j = j0 + u * 32 + lane;
+                    idx[u] = 0;
+                    if (j < total)
+                    {
+                        idx[u] = list[j];
+                        one |= 1u << u;
+                    }
+                }
+                uint64_t v[4];
+                if (pc.n)
+                    load_list(v, pc.src[0], pc.width[0], row0, idx, one);
+                if (j0 == 0)
+                    base = __shfl_sync(0xffffffffu, b0, 0);
+                const uint64_t out = base + j0 + lane;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (out + 32 * u >= out_cap)
+                        one &= ~(1u << u);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (one >> u & 1u)
+                        __stcs(out_keys + out + 32 * u, key_s[idx[u]]);
+#pragma unroll 1
+                for (uint32_t c = 0; c < pc.n; ++c)
+                {
+                    uint64_t nx[4];
+                    if (c + 1 < pc.n)
+                        load_list(nx, pc.src[c + 1], pc.width[c + 1], row0, idx, one);
+                    store_list(v, pc.dst[c], pc.width[c], out, one);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        v[u] = nx[u];
+                }
+                if (bc.n)
+                {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        v[u] = pay_s[idx[u]];
+#pragma unroll 1
+                    for (uint32_t c = 0; c < bc.n; ++c)
+                    {
+                        uint64_t x[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            x[u] = v[u] >> (bc.off[c] * 8u);
+                        store_list(x, bc.dst[c], bc.width[c], out, one);
+                    }
+                }
+            }
+        }
+        __syncwarp(); // the warp's shared memory is filled again by the next chunk
         chunk = (uint32_t)__shfl_sync(0xffffffffu, tn, 0);
     }
 }
@@ -1078,13 +1304,9 @@ uint64_t probe_lookup(phj_ctx * ctx, Scratch & s, const ProbeArgs & a_in, uint32
     return total;
 }
 
-// The packed layout of payload columns, when they pack: 2+ columns of 1-8
-// bytes, 16 bytes in all.
-static bool pack_spec_of(const Cols & payloads, PackSpec & pk)
+bool pack_columns(const Cols & payloads, uint32_t most, PackSpec & pk)
 {
     pk = PackSpec{};
-    if (payloads.n < 2)
-        return false;
     // widest column first, so every offset is a multiple of its width
     uint32_t order[kMaxCols];
     for (uint32_t c = 0; c < payloads.n; ++c)
@@ -1099,10 +1321,17 @@ static bool pack_spec_of(const Cols & payloads, PackSpec & pk)
         pk.off[c] = (uint8_t)off;
         off += payloads.width[c];
     }
-    if (off > 16)
+    if (off > most)
         return false;
     pk.n = payloads.n;
     return true;
+}
+
+// The packed layout of payload columns, when they pack: 2+ columns of 1-8
+// bytes, 16 bytes in all.
+static bool pack_spec_of(const Cols & payloads, PackSpec & pk)
+{
+    return payloads.n >= 2 && pack_columns(payloads, 16, pk);
 }
 
 void pack_build_payloads(phj_ctx * ctx, Scratch & s, ProbeArgs & a, uint64_t build_rows)
@@ -1202,7 +1431,10 @@ static bool probe_fused_eligible(const phj_ctx * ctx, const ProbeArgs & a)
 
 // Unique build keys, packed build payloads: one pass that looks up and
 // projects (k_probe_fused) into an output of one row per probe row.
-static phj_output * probe_fused(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const phj_schema & left, const phj_schema & right)
+// With `flags` (tables sized by estimate) the kernel does nothing when they
+// are set: nullptr, and *found gets them.
+static phj_output * probe_fused(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const phj_schema & left, const phj_schema & right,
+                                const int * flags = nullptr, ProbeFound * found = nullptr)
 {
     unsigned long long * counter = s.get<unsigned long long>(2); // output rows, chunk tickets
     PHJ_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), ctx->stream));
@@ -1241,7 +1473,7 @@ static phj_output * probe_fused(phj_ctx * ctx, Scratch & s, const ProbeArgs & a,
             if (std::getenv("PHJ_DEBUG"))
                 std::fprintf(stderr, "[phj] probe_fused: grid %u x %d threads, %d CTAs/SM, chunks %llu\n", grid, kPNT, per_sm,
                              (unsigned long long)n_chunks);
-            kernel<<<grid, kPNT, 0, ctx->stream>>>(a, pc, bc, o.keys, counter, counter + 1, a.probe_rows);
+            kernel<<<grid, kPNT, 0, ctx->stream>>>(a, pc, bc, o.keys, counter, counter + 1, a.probe_rows, flags);
         };
         if ((a.uniform_log2cap >= 0 && a.uniform_log2cap < 1) || (reinterpret_cast<uintptr_t>(a.cells) & 31) != 0)
             throw Error(PHJ_ERR_CUDA, "internal: leaf tables need aligned pairs of cells");
@@ -1268,13 +1500,98 @@ static phj_output * probe_fused(phj_ctx * ctx, Scratch & s, const ProbeArgs & a,
             PHJ_LAUNCHED(ctx, "probe_fused");
         }
         unsigned long long total = 0;
-        read_small(ctx, {{&total, counter, sizeof(total)}});
+        if (flags)
+        {
+            PHJ_CUDA(cudaEventRecord(found->done, ctx->stream));
+            read_small(ctx, {{&total, counter, sizeof(total)}, {&found->flags, flags, sizeof(int)}, {&found->err, ctx->d_err, sizeof(int)}});
+            if (found->flags)
+            {
+                if (rec >= 0)
+                    ctx->records.erase(ctx->records.begin() + rec);
+                free_output(ctx, out);
+                return nullptr;
+            }
+        }
+        else
+            read_small(ctx, {{&total, counter, sizeof(total)}});
         if (total > out->cap)
             throw Error(PHJ_ERR_CUDA, "internal: the one-pass probe counted more output rows than probe rows");
         out->rows = total;
         // algorithmic bytes: every probe row read, every output row written
         if (rec >= 0)
             ctx->records[rec].bytes = a.probe_rows * row_bytes_of(a.probe, true) + total * (8 + row_bytes_of(a.build, false) + row_bytes_of(a.probe, false));
+    }
+    catch (...)
+    {
+        free_output(ctx, out);
+        throw;
+    }
+    return out;
+}
+
+bool one_pass_probe(const phj_ctx * ctx, const ProbeArgs & a)
+{
+    return probe_fused_eligible(ctx, a);
+}
+
+phj_output * probe_estimated(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const phj_schema & left, const phj_schema & right, const int * flags,
+                             ProbeFound & found)
+{
+    return probe_fused(ctx, s, a, left, right, flags, &found);
+}
+
+phj_output * probe_inline(phj_ctx * ctx, Scratch & s, const Cols & probe, uint64_t probe_rows, const InlineTables & t, const Cols & build,
+                          const PackSpec & pk, const phj_schema & left, const phj_schema & right, const int * flags, ProbeFound & found)
+{
+    unsigned long long * counter = s.get<unsigned long long>(2); // output rows, chunk tickets
+    PHJ_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), ctx->stream));
+    phj_output * out = new_output(ctx, left, right, probe_rows);
+    try
+    {
+        ProjCols pc{};
+        for (uint32_t c = 0; c < probe.n; ++c)
+        {
+            pc.src[pc.n] = probe.col[c];
+            pc.dst[pc.n] = out->rcol[c];
+            pc.width[pc.n] = probe.width[c];
+            pc.by_build[pc.n++] = 0;
+        }
+        PackedCols bc{};
+        for (uint32_t c = 0; c < build.n; ++c)
+        {
+            bc.dst[c] = out->lcol[c];
+            bc.width[c] = (uint8_t)build.width[c];
+            bc.off[c] = pk.off[c];
+        }
+        bc.n = build.n;
+        int per_sm = 0;
+        PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_probe_inline, kPNT, 0));
+        const unsigned grid = (unsigned)std::max<uint64_t>(
+            1, std::min<uint64_t>(ceil_div(ceil_div(probe_rows, kWChunk), kPWarps), (uint64_t)ctx->num_sms * (uint64_t)std::max(per_sm, 1)));
+        int rec = -1;
+        {
+            // (a single 1- or 2-byte column is nothing k_probe_fused takes)
+            KTimer kt(ctx, one_pass_schemas(left, right) ? "probe_fused" : "probe_inline", probe_rows, 0);
+            rec = kt.idx;
+            k_probe_inline<<<grid, kPNT, 0, ctx->stream>>>(probe.keys, probe_rows, t, pc, bc, out->keys, counter, counter + 1, probe_rows, flags);
+            PHJ_LAUNCHED(ctx, "probe_inline");
+        }
+        unsigned long long total = 0;
+        PHJ_CUDA(cudaEventRecord(found.done, ctx->stream));
+        read_small(ctx, {{&total, counter, sizeof(total)}, {&found.flags, flags, sizeof(int)}, {&found.err, ctx->d_err, sizeof(int)}});
+        if (found.flags)
+        {
+            if (rec >= 0)
+                ctx->records.erase(ctx->records.begin() + rec);
+            free_output(ctx, out);
+            return nullptr;
+        }
+        if (total > out->cap)
+            throw Error(PHJ_ERR_CUDA, "internal: the one-pass probe counted more output rows than probe rows");
+        out->rows = total;
+        // algorithmic bytes: every probe row read, every output row written
+        if (rec >= 0)
+            ctx->records[rec].bytes = probe_rows * row_bytes_of(probe, true) + total * (8 + row_bytes_of(build, false) + row_bytes_of(probe, false));
     }
     catch (...)
     {
