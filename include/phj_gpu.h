@@ -176,8 +176,8 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *        group of consecutive top-8-bit sub-tables, so the tables a sweep
  *        touches can stay in L2; 0 or 1 (default): one sweep.  Same output
  *        rows, in another order;
- *   "bep_engine": PHJ (BEP) form; 0 (default) the device budget engine: one
- *        persistent grid whose CTA groups (one per SM) each hold a share of
+ *   "bep_engine": PHJ (BEP) form; 0 (default) the device budget engine:
+ *        CTA groups (one per SM) each hold a share of
  *        bep_budget_mib, scatter their slice of the probe side into
  *        first-pass chains, refine at the reference's water marks and
  *        evict leaves round-robin (first pass 1..11 bits with at most 13

@@ -1294,6 +1294,7 @@ static void run_phj_bep_engine(phj_ctx * ctx, const phj_table & B, const phj_tab
     in.probe = cols_of(P);
     in.probe_rows = P.rows;
     in.build = bpart;
+    in.build_rows = B.rows;
     in.lt = &lt;
     in.leaf_off = leaf_off;
     in.b1 = bits[0];

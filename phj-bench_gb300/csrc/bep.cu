@@ -170,12 +170,123 @@ __global__ void __launch_bounds__(kBepNT) k_bep_build(BepLeaves b, int * __restr
             return;
     }
 }
+
+// Small tables (at most kWarpCells cells): a warp per leaf.  A table of 32
+// rows leaves seven of a CTA's eight warps waiting at its barriers (8M build
+// rows in 262,144 leaves, both evictions: claims and builds 620 us with a CTA
+// a leaf, 350 us with a warp).  A warp claims kClaim leaves at once, one a lane, so
+// their descriptors are read and their states changed side by side; nothing
+// but the build itself is then serial.
+constexpr uint32_t kWarpCells = 256;
+
+__global__ void __launch_bounds__(kBepNT) k_bep_build_warps(BepLeaves b, int * __restrict__ err)
+{
+    extern __shared__ __align__(16) Cell sh_cells[];
+    Cell * tab = sh_cells + (uint64_t)(threadIdx.x >> 5) * b.smem_cells;
+    const uint32_t lane = threadIdx.x & 31;
+    for (;;)
+    {
+        uint32_t base = 0;
+        if (lane == 0)
+            base = atomicAdd(b.queue_len + 1, kClaim);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t qlen = *reinterpret_cast<volatile uint32_t *>(b.queue_len);
+        if (base >= qlen)
+            return;
+        const bool mine = lane < min(kClaim, qlen - base);
+        uint32_t L = 0, r0 = 0, r1 = 0, cap = 0;
+        uint64_t off = 0;
+        bool won = false, dup = false;
+        if (mine)
+        {
+            L = b.queue[base + lane];
+            won = atomicCAS(b.state + L, kNotBuilt, kBuilding) == kNotBuilt;
+            const LeafMeta m = b.meta[L];
+            if (m.has_table)
+            {
+                cap = 1u << m.log2cap; // (at most smem_cells)
+                off = m.table_off;
+                r0 = m.row_off;
+                r1 = b.leaf_off[L + 1];
+            }
+        }
+        for (uint32_t todo = __ballot_sync(0xffffffffu, won && cap); todo; todo &= todo - 1)
+        {
+            const int i = __ffs(todo) - 1;
+            const uint32_t c = __shfl_sync(0xffffffffu, cap, i), q0 = __shfl_sync(0xffffffffu, r0, i), q1 = __shfl_sync(0xffffffffu, r1, i);
+            Cell * out = b.cells + __shfl_sync(0xffffffffu, off, i);
+            uint64_t k = q0 + lane < q1 ? b.build_keys[q0 + lane] : 0ull;
+            for (uint32_t j = lane; j < c; j += 32)
+                reinterpret_cast<ulonglong2 *>(tab)[j] = make_ulonglong2(0ull, INVALID_REF);
+            __syncwarp();
+            bool rep = false;
+            for (uint32_t r = q0 + lane; r < q1; r += 32)
+            {
+                const uint64_t ahead = r + 32 < q1 ? b.build_keys[r + 32] : 0ull;
+                const uint64_t prev = table_insert<true>(tab, c, int_hash64(k), k, make_ref(0, r));
+                b.next[r] = prev;
+                rep |= ref_valid(prev);
+                k = ahead;
+            }
+            rep = __any_sync(0xffffffffu, rep);
+            if ((int)lane == i)
+                dup = rep;
+            for (uint32_t j = lane; j < c; j += 32)
+                reinterpret_cast<ulonglong2 *>(out)[j] = reinterpret_cast<const ulonglong2 *>(tab)[j];
+            __syncwarp(); // the shared table is reused by the next leaf
+        }
+        // (BUILT needs no fence, as above)
+        if (won)
+        {
+            b.meta[L].dup = dup ? 1 : 0;
+            atomicExch(b.state + L, dup ? kBuiltDup : kBuilt);
+        }
+        const uint32_t n_won = __popc(__ballot_sync(0xffffffffu, won));
+        const bool any = __any_sync(0xffffffffu, dup);
+        if (lane == 0)
+        {
+            atomicAdd(b.ctr + 0, (unsigned long long)n_won);
+            if (any)
+                atomicExch(b.any_dup, 1);
+        }
+        // a leaf that another builder has is waited for (bounded)
+        bool stop = false;
+        if (mine && !won && load_acquire(b.state + L) < kBuilt)
+        {
+            atomicAdd(b.ctr + 1, 1ull);
+            const uint64_t t0 = global_ns();
+            uint32_t spins = 0;
+            while (load_acquire(b.state + L) < kBuilt)
+                if (++spins >= kWaitLimit || global_ns() - t0 > b.wait_limit_ns)
+                {
+                    atomicExch(err, 4);
+                    stop = true;
+                    break;
+                }
+        }
+        if (__any_sync(0xffffffffu, stop))
+            return;
+    }
+}
 } // namespace
 
 void set_bep_smem_limits(int smem_optin)
 {
     PHJ_CUDA(cudaFuncSetAttribute(k_bep_build, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::min<size_t>((size_t)kBepSmemCellsMax * sizeof(Cell), (size_t)smem_optin - 1024)));
+}
+
+void bep_build_queue(phj_ctx * ctx, const BepLeaves & b)
+{
+    // smem_cells is at least the largest table's cells while that is no more
+    // than kBepSmemCellsMax, so up to kWarpCells every table fits a warp's
+    const bool warps = b.smem_cells <= kWarpCells;
+    const auto kernel = warps ? k_bep_build_warps : k_bep_build;
+    const size_t smem = (size_t)b.smem_cells * sizeof(Cell) * (warps ? kBepNT / 32 : 1);
+    int per_sm = 0;
+    PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBepNT, smem));
+    kernel<<<(unsigned)(ctx->num_sms * std::max(per_sm, 1)), kBepNT, smem, ctx->stream>>>(b, ctx->d_err);
+    PHJ_LAUNCHED(ctx, "bep_build");
 }
 
 bool bep_build_touched(phj_ctx * ctx, const BepLeaves & b)
@@ -185,10 +296,7 @@ bool bep_build_touched(phj_ctx * ctx, const BepLeaves & b)
     PHJ_LAUNCHED(ctx, "bep_collect");
     {
         KTimer kt(ctx, "bep_build", 0, 0);
-        int per_sm = 0;
-        PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bep_build, kBepNT, (size_t)b.smem_cells * sizeof(Cell)));
-        k_bep_build<<<(unsigned)(ctx->num_sms * std::max(per_sm, 1)), kBepNT, (size_t)b.smem_cells * sizeof(Cell), ctx->stream>>>(b, ctx->d_err);
-        PHJ_LAUNCHED(ctx, "bep_build");
+        bep_build_queue(ctx, b);
     }
     int dup = 0;
     read_small(ctx, {{&dup, b.any_dup, sizeof(int)}});

@@ -1,63 +1,73 @@
 // bep_engine.cu -- PHJ (best-effort partitioning, src/PHJBep.cpp:113-790)
 // with the probe side's byte budget kept on the device.
 //
-// One persistent grid, one CTA per SM; each CTA is one of the reference's
-// workers (a "CTA group") with its own contiguous slice of the probe input
-// and its own share of the budget (bep_budget_mib / groups).  Probe rows
-// live in fixed-size blocks of `page` rows (column-major inside a block)
-// taken from one device pool through a free-block stack.
+// One CTA per SM is one of the reference's workers (a "CTA group") with its
+// own contiguous slice of the probe input and its own share of the budget
+// (bep_budget_mib / groups).  Probe rows live in fixed-size blocks of `page`
+// rows (column-major inside a block) taken from one device pool through a
+// free-block stack.
 //
-// The grid runs in waves separated by grid-wide barriers:
-//   S  each group scatters the next tile of its slice by the first radix
-//      pass into its private pass-1 bucket chains (the reference's
-//      per-worker `unrefined` chains) and adds the tile's bytes to its
-//      unrefined count.  At the per-group high water (half the group's
-//      budget) it refines its largest bucket, again and again until the
-//      count is below the low water (a quarter): refining a bucket sorts
-//      each of its blocks by leaf (passes 2..N) in shared memory and
-//      publishes the block as a refined block of that bucket; the rows go
-//      to the per-leaf counts (leaf_rows) and to the global leaf count.
+// The run alternates between two steps, S and E, until the input is through:
+//   S  k_bep_scatter, a cooperative launch of the groups.  In waves separated
+//      by grid-wide barriers, each group scatters the next tile of its slice
+//      by the first radix pass into its private pass-1 bucket chains (the
+//      reference's per-worker `unrefined` chains) and adds the tile's bytes
+//      to its unrefined count.  At the per-group high water (half the
+//      group's budget) it refines its largest bucket, again and again until
+//      the count is below the low water (a quarter): refining a bucket
+//      counts its rows by leaf (leaf_rows, the global leaf count) and
+//      publishes its blocks as refined blocks of that bucket.  (The rows
+//      are not moved: a leaf's rows are found in its bucket's blocks by
+//      their hash when the leaf is evicted.)
 //      (src/PHJBep.cpp:397-450 refinePartition, :508-528 evictAsNeeded
-//      phase 1, :582-605 the main loop.)
-//   E  when the global leaf bytes reach the leaf high water (5/8 of the
-//      budget), the round-robin eviction cursor (next_evict_leaf) advances
-//      over the leaves until the leaves it passed hold enough rows to take
-//      the global count below the low water (5/8 of the high water); each
-//      leaf passed is claimed with a CAS on its lock word and counted as an
-//      eviction when it held rows; the claimed leaves whose table is
-//      NOT_BUILT are built (NOT_BUILT -> BUILDING by CAS, BUILT when done; a
-//      leaf found BUILDING is waited for, bounded); then every refined
-//      block's rows of the claimed leaves are probed and projected, the
-//      blocks in bucket order so one bucket's leaf tables stay in L2; a
-//      block whose rows are all probed goes back to the pool.
-//      (src/PHJBep.cpp:453-505 tryEvictOneLeaf, :530-571 phase 2.)
-// After the last input wave every group refines what it still holds
-// (:662-676), and a final E over all leaves drains the rest (the post-probe
-// drain, :689-727).  The reference's cooperative end-of-slice drain
-// (:619-655) has no separate form: the slices are equal and every group
-// takes part in every E, so no group idles while another scatters.
+//      phase 1, :582-605 the main loop.)  When the global leaf bytes reach
+//      the leaf high water (5/8 of the budget), or the input is through and
+//      every group has refined what it held (:662-676), the launch ends; the
+//      groups' state stays in memory.
+//   E  the round-robin eviction cursor (next_evict_leaf) advances over the
+//      leaves until the leaves it passed hold enough rows to take the global
+//      count below the low water (5/8 of the high water; every leaf in the
+//      final drain): k_bep_range.  Each leaf passed is claimed with a CAS on
+//      its lock word and counted as an eviction when it held rows
+//      (k_bep_claim); the claimed leaves whose table is NOT_BUILT are built
+//      (k_bep_build of bep.cu: NOT_BUILT -> BUILDING by CAS, BUILT when
+//      done; a leaf found BUILDING is waited for, bounded); then every
+//      refined block's rows of the claimed leaves are probed and projected
+//      (k_bep_probe), the blocks in bucket order so one bucket's leaf tables
+//      stay in L2; a block whose rows are all probed goes back to the pool.
+//      (src/PHJBep.cpp:453-505 tryEvictOneLeaf, :530-571 phase 2; the
+//      post-probe drain, :689-727.)
+// The host enqueues S and E in turn, one pair and then more at a time, and
+// reads the control block between; steps past the end find nothing to do.
+// The reference's cooperative end-of-slice drain (:619-655) has no separate
+// form: the slices are equal and every group takes part in every E, so no
+// group idles while another scatters.
 //
 // Counters as the reference defines them (src/PHJBep.h:13-39): evictions
 // (leaves that held rows when claimed), refinements (bucket refines), peak
 // (the largest global leaf bytes, seen after each wave's refines), skip
 // retries (claims that found the leaf locked, and waits on a BUILDING leaf).
 //
-// Every wait is bounded: the grid barrier and the BUILDING wait give up
-// after the context's wait limit, set an error code and end the grid.  A
-// group that finds too few free blocks for its tile refines what it holds
-// and the wave ends in a drain of every leaf (which frees every refined
-// block); a second shortage right after such a drain ends the grid with a
-// capacity error.  Each group takes its free blocks from a cache of its own,
-// refilled from the pool's stack a batch at a time.
+// Every wait is bounded: the grid barrier, the bulk copies and the BUILDING
+// wait give up after the context's wait limit (the copies after a poll
+// limit), set an error code and end the run.  A group that finds too few
+// free blocks for its tile refines what it holds and the wave ends in a
+// drain of every leaf (which frees every refined block); a second shortage
+// right after such a drain ends the run with a capacity error.  Each group
+// takes its free blocks from a cache of its own, refilled from the pool's
+// stack a batch at a time.
 //
-// Pool blocks, control words, per-leaf and per-block state and the lazily
-// built tables are written by one group and read by others during the
-// launch, so they are read through L2 (ld.global.cg): an SM's L1 may hold
-// an older copy of the line.
+// Measured (64M x 512M rows, Zipf keys, 32 MiB a group): 14.8 ms (S 5.9,
+// claims and builds 1.4, probes 6.7 ms); one persistent grid of 1024-thread
+// CTAs for both steps, whose refines sorted every block by leaf, took 28.1 ms
+// (S 11.6, claims and builds 3.9, probes 12.3).  8M x 64M rows: 2.85 ms
+// (S 1.1, 0.35, 0.88) against 6.06 ms.
 #include "internal.h"
+#include "list.cuh"
 
 #include <cstdio>
 #include <cstdlib>
+#include <type_traits>
 
 namespace phjg
 {
@@ -65,13 +75,17 @@ namespace
 {
 constexpr int kENT = 1024; // threads of a group's CTA
 constexpr uint32_t kNone = 0xFFFFFFFFu;
-constexpr uint32_t kNotBuilt = 0, kBuilding = 1, kBuilt = 2, kBuiltDup = 3;
+constexpr uint32_t kBuilt = 2, kBuiltDup = 3; // (0 NOT_BUILT, 1 BUILDING)
 
 // error codes written to the context's error word
-constexpr int kErrWait = 4;    // a BUILDING leaf was not published in time
+// (1: a bulk copy, 4: a BUILDING leaf was not there in time)
 constexpr int kErrBarrier = 5; // a grid barrier was not reached in time
 constexpr int kErrPool = 6;    // the block pool ran out
 constexpr int kErrChain = 7;   // a bucket chain outgrew its directory
+
+constexpr uint32_t kETile = 4096;  // most input rows of one scatter step
+constexpr uint32_t kRefill = 64;   // free blocks a group takes beyond its need
+constexpr uint32_t kPersistScal = 8;
 
 struct EngineCtl
 {
@@ -89,11 +103,17 @@ struct EngineCtl
     unsigned int work_n;
     unsigned int build_n, build_next;
     unsigned long long work_next;
-    unsigned long long evictions, refinements, skip_retries, tables_built, evict_phases;
+    unsigned long long evictions, refinements, skip_retries, evict_phases;
     unsigned long long ns_shuffle, ns_evict, ns_probe; // group 0's time in S, E bookkeeping, E probing
     unsigned long long rows_scattered, rows_refined, rows_probed, rows_claimed; // row totals per step (checks)
     unsigned int groups_done; // groups whose slice is scattered
-    int more_input;           // some group still has input (decided at each wave's barrier)
+    int ev_mode;              // the E to come: 0 none, 1 down to the low water, 2 every leaf
+    int input_done;           // the final drain is the E to come, or is done
+    int finished;             // the final drain is claimed: nothing is left to do
+    int started;              // an S step has run: the groups' state is in memory
+    unsigned long long t_evict0, t_probe0; // start of this E, of its probes (0: none)
+    int no_more_input;        // every group's slice is scattered (decided at each wave's barrier)
+    unsigned int waves;       // waves so far
     int pool_low;             // a group found too few free blocks for its tile this wave
     int forced_last;          // the previous E was a drain forced by a low pool
     int any_dup;              // some leaf built so far has a repeated key
@@ -115,7 +135,6 @@ struct EngineArgs
     uint64_t * next;
     const uint32_t * leaf_off;
     int ulog;            // >= 0: uniform tables of 2^ulog cells at leaf << ulog
-    uint32_t smem_cells; // tables up to this many cells are built in shared memory
     uint32_t b1;         // first-pass bits
     uint32_t total_bits; // leaf bits
     uint32_t lb_log2;    // leaf-in-bucket bits (total_bits - b1)
@@ -131,8 +150,6 @@ struct EngineArgs
     uint32_t * blk_rows;
     uint32_t * blk_rem;
     uint32_t * blk_bucket; // the bucket of a refined block (kept after the block is freed)
-    uint32_t * blk_lfirst; // leaf-in-bucket of a refined block's first and last row
-    uint32_t * blk_llast;
     // the eviction cursor when the block was refined: the block's rows of
     // leaf L are probed when the cursor first passes L after that point
     unsigned long long * blk_c0;
@@ -148,7 +165,11 @@ struct EngineArgs
     uint64_t unref_high, unref_low, leaf_high, leaf_low;
     uint32_t rb;        // bytes of a probe row
     uint64_t tile_rows; // input rows a group scatters per wave
-    uint32_t waves;
+    uint32_t stage_rows;                 // rows of a scatter step (<= kETile)
+    uint32_t stage_off[kMaxCols], stage_bytes; // a step's columns in shared memory (keys at 0)
+    int use_tma;                         // the input columns start on 16-byte boundaries
+    uint32_t * group_state; // per group: the words of Smem::persist
+    uint32_t persist_words, bcache_words, fresh_words, half_bytes;
     // output
     uint64_t * out_keys;
     void * out_l[kMaxCols];
@@ -193,22 +214,7 @@ __device__ __forceinline__ T vload(const T * p)
 
 __device__ __forceinline__ uint64_t umin64(uint64_t x, uint64_t y) { return x < y ? x : y; }
 
-// Element src_i of a pool column (read through L2) to element dst_i of an
-// output column of the same width (a streaming store: output rows are not
-// read again, so they should not push pool pages and tables out of L2).
-__device__ __forceinline__ void copy_elem_cg(void * dst, uint64_t dst_i, const void * src, uint64_t src_i, uint32_t w)
-{
-    switch (w)
-    {
-        case 1: __stcs(static_cast<unsigned char *>(dst) + dst_i, (unsigned char)__ldcg(static_cast<const signed char *>(src) + src_i)); break;
-        case 2: __stcs(static_cast<unsigned short *>(dst) + dst_i, __ldcg(static_cast<const unsigned short *>(src) + src_i)); break;
-        case 4: __stcs(static_cast<unsigned int *>(dst) + dst_i, __ldcg(static_cast<const unsigned int *>(src) + src_i)); break;
-        case 8: __stcs(static_cast<unsigned long long *>(dst) + dst_i, __ldcg(static_cast<const unsigned long long *>(src) + src_i)); break;
-        default: __stcs(static_cast<uint4 *>(dst) + dst_i, __ldcg(static_cast<const uint4 *>(src) + src_i)); break;
-    }
-}
-
-// Element src_i of a build payload column (written before the launch) to
+// Element src_i of a column (written by an earlier kernel) to
 // element dst_i of an output column, with a streaming store.
 __device__ __forceinline__ void copy_elem_out(void * dst, uint64_t dst_i, const void * src, uint64_t src_i, uint32_t w)
 {
@@ -265,11 +271,6 @@ __device__ bool grid_sync(const EngineArgs & a, uint32_t & gen, F last)
     return !aborted(a);
 }
 
-struct NoOp
-{
-    __device__ void operator()() const {}
-};
-
 // Block-wide exclusive scan over `n` u32 bins in shared memory (in place);
 // returns the total.  `ws` holds kENT/32 words.
 __device__ uint32_t scan_bins(uint32_t * bins, uint32_t n, uint32_t * ws)
@@ -299,308 +300,355 @@ __device__ __forceinline__ uint8_t * block_ptr(const EngineArgs & a, uint32_t bl
     return a.pool + (uint64_t)blk * a.block_bytes;
 }
 
-// Copies row `src_i` of a column-major tile in shared memory (keys at 0,
-// payload c at col_off[c]) to row `dst_i` of a block of the same layout.
-__device__ __forceinline__ void copy_row(const EngineArgs & a, uint8_t * dst, uint32_t dst_i, const uint8_t * src, uint32_t src_i)
-{
-    reinterpret_cast<uint64_t *>(dst)[dst_i] = reinterpret_cast<const uint64_t *>(src)[src_i];
-    for (uint32_t c = 0; c < a.pin.n; ++c)
-        copy_elem(dst + a.col_off[c], dst_i, src + a.col_off[c], src_i, a.pin.width[c]);
-}
+// An S CTA scatters in two halves of 512 threads, a step each at a time.
+constexpr int kHNT = kENT / 2;
+constexpr int kHRows = (int)kETile / kHNT; // rows a thread of a step
 
-// Column c of rows i0 + u * kENT + threadIdx.x (u < 4, below n) from `src`
-// (row r0 + i) into the stage column `dst`: the four loads are issued
-// before any store.  kL2: the source was written during this launch (read
-// through L2).
-template <class T, bool kL2>
-__device__ __forceinline__ void stage4(T * dst, const T * src, uint64_t r0, uint32_t i0, uint32_t n)
+// One half's shared memory.
+struct Half
 {
-    T v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-    {
-        const uint32_t i = i0 + u * kENT + threadIdx.x;
-        if (i < n)
-            v[u] = kL2 ? __ldcg(src + r0 + i) : __ldcs(src + r0 + i); // the input is read once
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-    {
-        const uint32_t i = i0 + u * kENT + threadIdx.x;
-        if (i < n)
-            dst[i] = v[u];
-    }
-}
-
-template <bool kL2>
-__device__ __forceinline__ void stage4_column(void * dst, const void * src, uint64_t r0, uint32_t i0, uint32_t n, uint32_t w)
-{
-    switch (w)
-    {
-        case 1: stage4<unsigned char, kL2>(static_cast<unsigned char *>(dst), static_cast<const unsigned char *>(src), r0, i0, n); break;
-        case 2: stage4<unsigned short, kL2>(static_cast<unsigned short *>(dst), static_cast<const unsigned short *>(src), r0, i0, n); break;
-        case 4: stage4<unsigned int, kL2>(static_cast<unsigned int *>(dst), static_cast<const unsigned int *>(src), r0, i0, n); break;
-        case 8: stage4<unsigned long long, kL2>(static_cast<unsigned long long *>(dst), static_cast<const unsigned long long *>(src), r0, i0, n); break;
-        default: stage4<uint4, kL2>(static_cast<uint4 *>(dst), static_cast<const uint4 *>(src), r0, i0, n); break;
-    }
-}
-
-struct Smem
-{
-    uint8_t * stage;  // page rows in the block layout; the leaf builds' cells
-    uint16_t * perm;  // page entries
-    uint16_t * src;   // page entries: the stage row of each sorted position
-    uint32_t * bins;  // max(buckets, leaves per bucket, page) entries
-    uint32_t * boff;  // buckets: scatter offsets
-    uint32_t * nbpre; // buckets: new blocks per bucket, then their prefix
-    uint32_t * fill;  // buckets: rows in each chain's last block (page: no block)
-    uint32_t * clen;  // buckets: blocks in each chain
-    uint32_t * urows; // buckets: unrefined rows per bucket
-    uint32_t * acc;   // leaves per bucket: rows a refine adds to each leaf
-    uint32_t * bcache; // the group's free blocks: 2 x buckets + 2 x kRefill entries
-    uint32_t * ws;    // scan scratch (kENT / 32 words)
-    uint32_t * scal;  // scalars (32 words, 8-byte aligned)
+    uint8_t * stage;  // a step's rows, column-major
+    uint32_t * perm;  // a step's rows in bucket order: row | bucket << 12
+    uint32_t * bins;  // buckets: rows of the step
+    uint32_t * off;   // buckets: first position in the step's bucket order (and the total)
+    uint32_t * nb0;   // buckets: first of the step's new blocks (and the total)
+    uint32_t * fill;  // buckets: rows in the chain's last block before the step
+    uint32_t * last;  // buckets: the chain's last block before the step
+    uint32_t * fresh; // the step's new blocks
+    uint32_t * wsum;  // the warps' sums of a scan
+    uint32_t * scal;  // [0] the step's outcome, [1,2] where its new blocks come from
 };
 
-// ---------------------------------------------------------------------------
-// S: scatter `n` (<= page) input rows from `r0` into the group's chains.
-// ---------------------------------------------------------------------------
-constexpr int kTileDone = 0, kTileNoRoom = 1, kTileFailed = 2;
-constexpr uint32_t kRefill = 64; // free blocks a group takes beyond its need
+// Shared memory of an S CTA.
+struct Smem
+{
+    Half hf;          // this thread's half's
+    uint32_t * acc;   // leaves per bucket: rows a refine adds to each leaf
+    uint32_t * scal;  // scalars (32 words, 8-byte aligned)
+    // kept in memory between launches, one run of words:
+    uint32_t * persist;
+    uint32_t * fill;   // buckets: rows in each chain's last block (page: no block)
+    uint32_t * clen;   // buckets: blocks in each chain
+    uint32_t * urows;  // buckets: unrefined rows per bucket
+    uint32_t * last;   // buckets: each chain's last block
+    uint32_t * bcache; // the group's free blocks
+    uint32_t * pscal;  // [0] blocks in bcache, [1] counted in groups_done, [2,3] next input row, [4,5] unrefined bytes
+};
 
-// Returns kTileDone, kTileNoRoom (too few free blocks: nothing done) or
-// kTileFailed (the grid is ending).  sm.bins[0, buckets) is zero on entry
-// and on a kTileDone return.
-__device__ int scatter_tile(const EngineArgs & a, const Smem & sm, uint32_t g, uint64_t r0, uint32_t n)
+// Barriers of one half (hardware barrier 1 + half).
+__device__ __forceinline__ void half_sync(uint32_t half)
+{
+    asm volatile("barrier.sync %0, %1;" ::"r"(1u + half), "n"(kHNT) : "memory");
+}
+__device__ __forceinline__ bool half_sync_and(uint32_t half, bool v)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "barrier.red.and.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"(1u + half), "n"(kHNT), "r"((uint32_t)v)
+        : "memory");
+    return r != 0;
+}
+
+// ---------------------------------------------------------------------------
+// S: one scatter step -- the `n` rows in a half's stage into the group's
+// chains.
+// ---------------------------------------------------------------------------
+enum : uint32_t
+{
+    kTileDone = 0,
+    kTileNoRoom = 1,
+    kTileFailed = 2
+};
+// words of Smem::scal that order the halves' steps: the step whose turn it is
+// to allocate, the outcome of the first step that was not taken, and which
+constexpr uint32_t kTurn = 8, kStop = 9, kStopStep = 10;
+
+template <class T>
+__device__ __forceinline__ void block_column(const EngineArgs & a, const uint8_t * src_v, uint32_t col_off, const uint32_t (&row)[4],
+                                             const uint32_t (&blk)[4], const uint32_t (&slot)[4], uint32_t live)
+{
+    const T * src = reinterpret_cast<const T *>(src_v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (live >> j & 1u)
+            reinterpret_cast<T *>(block_ptr(a, blk[j]) + col_off)[slot[j]] = src[row[j]];
+}
+
+// The step's places, by its half: the bucket counts scanned, the blocks its
+// chains need (an empty chain counts as a full last block) taken from the
+// group's cache of free blocks, and the chains brought to their state after
+// the step.  A half runs this in its turn, so steps allocate in input order.
+// hf.bins is zero on a kTileDone return.
+__device__ __forceinline__ uint32_t allocate_step(const EngineArgs & a, const Smem & sm, uint32_t half, uint32_t g, uint32_t n)
+{
+    const Half & hf = sm.hf;
+    const uint32_t page = 1u << a.page_log2, P1 = a.n_buckets;
+    const uint32_t tid = threadIdx.x & (kHNT - 1), lane = tid & 31, warp = tid >> 5;
+    const uint32_t per = (P1 + kHNT - 1) / kHNT, p0 = tid * per; // at most kPer
+    constexpr uint32_t kPer = 2048 / kHNT;
+    // rows (low half: at most 4096) and new blocks (at most 4096 + 2048)
+    uint32_t cnt[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j)
+    {
+        cnt[j] = 0;
+        if (j < per && p0 + j < P1)
+        {
+            const uint32_t c = hf.bins[p0 + j];
+            if (c)
+                cnt[j] = c | (((sm.fill[p0 + j] + c + page - 1) >> a.page_log2) - 1u) << 16;
+            sum += cnt[j];
+        }
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o)
+            incl += y;
+    }
+    if (lane == 31)
+        hf.wsum[warp] = incl;
+    half_sync(half);
+    static_assert(kHNT / 32 == 16, "the scan of the warps' sums");
+    uint32_t w = hf.wsum[lane & 15];
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o, 16);
+        if ((lane & 15) >= (uint32_t)o)
+            w += y;
+    }
+    const uint32_t need = __shfl_sync(0xffffffffu, w, 15) >> 16;
+    const uint32_t before = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0);
+    uint32_t run = incl - sum + (warp ? before : 0u);
+    // the cache is refilled from the pool's stack kRefill blocks beyond the
+    // need at a time, so the groups rarely meet on the stack
+    uint32_t have = sm.pscal[0];
+    if (need > have)
+    {
+        if (tid == 0)
+        {
+            const uint32_t lack = need - have, want = lack + kRefill;
+            unsigned long long * top = reinterpret_cast<unsigned long long *>(&a.ctl->free_top);
+            long long cur = (long long)vload(top), t;
+            for (;;)
+            {
+                t = cur >= (long long)want ? (long long)want : (cur >= (long long)lack ? cur : 0);
+                if (t == 0)
+                    break; // too few free blocks
+                const long long seen = (long long)atomicCAS(top, (unsigned long long)cur, (unsigned long long)(cur - t));
+                if (seen == cur)
+                    break;
+                cur = seen;
+            }
+            hf.scal[0] = t ? kTileDone : kTileNoRoom;
+            hf.scal[1] = (uint32_t)(cur - t);
+            hf.scal[2] = (uint32_t)t;
+        }
+        half_sync(half);
+        if (hf.scal[0] != kTileDone)
+            return kTileNoRoom;
+        const uint32_t from = hf.scal[1], got = hf.scal[2];
+        for (uint32_t i = tid; i < got; i += kHNT)
+            sm.bcache[have + i] = __ldcg(a.free_stack + from + i);
+        have += got;
+        half_sync(half);
+    }
+    const uint32_t base = have - need; // this step's blocks: bcache[base, +need)
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j)
+        if (j < per && p0 + j < P1)
+        {
+            const uint32_t p = p0 + j, c = cnt[j] & 0xFFFFu, nb = cnt[j] >> 16;
+            const uint32_t rb = run >> 16, fill = sm.fill[p], last = sm.last[p];
+            hf.off[p] = run & 0xFFFFu;
+            hf.nb0[p] = rb;
+            hf.fill[p] = fill;
+            hf.last[p] = last;
+            if (c)
+            {
+                hf.bins[p] = 0;
+                const uint32_t len = sm.clen[p];
+                if (len + nb > a.maxb)
+                {
+                    fail(a, kErrChain);
+                    hf.scal[0] = kTileFailed;
+                }
+                else
+                {
+                    uint32_t blk = last;
+                    for (uint32_t i = 0; i < nb; ++i)
+                    {
+                        blk = sm.bcache[base + rb + i];
+                        a.chain[((uint64_t)g * P1 + p) * a.maxb + len + i] = blk;
+                        hf.fresh[rb + i] = blk;
+                    }
+                    sm.last[p] = blk;
+                    sm.fill[p] = ((fill + c - 1) & (page - 1)) + 1;
+                    sm.clen[p] = len + nb;
+                    sm.urows[p] += c;
+                }
+            }
+            run += cnt[j];
+        }
+    if (tid == 0)
+    {
+        hf.off[P1] = n;
+        hf.nb0[P1] = need;
+    }
+    half_sync(half);
+    if (tid == 0)
+        sm.pscal[0] = base;
+    return hf.scal[0];
+}
+
+// One half's step `k` of the launch.  Consecutive rows of a bucket go to
+// consecutive rows of its blocks.  A step is a chain of latencies (shared
+// atomics, the scan, the permutation, the stores); the other half's step
+// fills them: 5.9 us a step of 4096 rows of 12 bytes, against 8.6 us for
+// steps of all 1024 threads, whose first warp scanned the buckets alone.
+// What bounds it now is the instructions of a row (issue slots 40% busy, DRAM
+// 21%, 8 to 9 warps of 32 at a barrier).  hf.bins is zero on entry and on a kTileDone return.
+__device__ uint32_t scatter_step(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t half, uint32_t k, uint32_t n, bool ok)
+{
+    const Half & hf = sm.hf;
+    const uint32_t page = 1u << a.page_log2, tid = threadIdx.x & (kHNT - 1);
+    const uint64_t * keys = reinterpret_cast<const uint64_t *>(hf.stage);
+    volatile uint32_t * turn = sm.scal + kTurn;
+    volatile uint32_t * stop = sm.scal + kStop;
+    uint32_t dr[kHRows]; // bucket | rank << 11
+#pragma unroll
+    for (int j = 0; j < kHRows; ++j)
+    {
+        const uint32_t i = j * kHNT + tid;
+        dr[j] = kNone;
+        if (ok && i < n)
+        {
+            const uint32_t p = (uint32_t)(int_hash64(keys[i]) >> (64u - a.b1));
+            dr[j] = p | atomicAdd(&hf.bins[p], 1u) << 11;
+        }
+    }
+    if (tid == 0)
+    {
+        // the steps before this one allocate first (bounded: a step that
+        // gives up passes the turn on)
+        uint32_t spin = 0;
+        while (*turn != k && ++spin < kWaitLimit)
+        {
+        }
+        __threadfence_block();
+        hf.scal[0] = *turn == k ? *stop : kTileFailed;
+    }
+    if (!half_sync_and(half, ok) && tid == 0)
+        hf.scal[0] = kTileFailed; // a bulk copy was not there in time
+    half_sync(half);
+    uint32_t state = hf.scal[0];
+    if (state == kTileDone)
+        state = allocate_step(a, sm, half, g, n);
+    if (tid == 0)
+    {
+        if (state == kTileFailed)
+        {
+            if (!aborted(a))
+                fail(a, 1);
+            *stop = kTileFailed;
+        }
+        else if (state == kTileNoRoom && *stop == kTileDone)
+        {
+            *stop = kTileNoRoom;
+            sm.scal[kStopStep] = k; // the first step not taken
+        }
+        __threadfence_block();
+        *turn = k + 1;
+    }
+    if (state != kTileDone)
+        return state;
+#pragma unroll
+    for (int j = 0; j < kHRows; ++j)
+        if (dr[j] != kNone)
+            hf.perm[hf.off[dr[j] & 2047u] + (dr[j] >> 11)] = (j * kHNT + tid) | (dr[j] & 2047u) << 12;
+    half_sync(half);
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < n; s0 += 4 * kHNT)
+    {
+        uint32_t row[4], blk[4], slot[4], live = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const uint32_t s = s0 + j * kHNT + tid;
+            row[j] = blk[j] = slot[j] = 0;
+            if (s < n)
+            {
+                const uint32_t e = hf.perm[s], p = e >> 12;
+                const uint32_t q = hf.fill[p] + (s - hf.off[p]); // slot counted from the chain's last block
+                row[j] = e & 4095u;
+                blk[j] = q < page ? hf.last[p] : hf.fresh[hf.nb0[p] + (q >> a.page_log2) - 1u];
+                slot[j] = q & (page - 1);
+                live |= 1u << j;
+            }
+        }
+        block_column<uint64_t>(a, hf.stage, 0, row, blk, slot, live);
+        for (uint32_t c = 0; c < a.pin.n; ++c)
+            switch (a.pin.width[c])
+            {
+                case 1: block_column<uint8_t>(a, hf.stage + a.stage_off[c], a.col_off[c], row, blk, slot, live); break;
+                case 2: block_column<uint16_t>(a, hf.stage + a.stage_off[c], a.col_off[c], row, blk, slot, live); break;
+                case 4: block_column<uint32_t>(a, hf.stage + a.stage_off[c], a.col_off[c], row, blk, slot, live); break;
+                case 8: block_column<uint64_t>(a, hf.stage + a.stage_off[c], a.col_off[c], row, blk, slot, live); break;
+                default: block_column<uint4>(a, hf.stage + a.stage_off[c], a.col_off[c], row, blk, slot, live); break;
+            }
+    }
+    return kTileDone;
+}
+
+// ---------------------------------------------------------------------------
+// S: refine bucket p of group g -- its rows counted by leaf, its blocks
+// published as refined.  Returns the rows refined.
+// ---------------------------------------------------------------------------
+__device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p)
 {
     const uint32_t page = 1u << a.page_log2;
-    const uint32_t P1 = a.n_buckets;
-    // the tile into the stage in input order (one read of the input), and
-    // the first-pass bucket of every row
-    for (uint32_t i0 = 0; i0 < n; i0 += 4 * kENT)
+    const uint32_t LB = 1u << a.lb_log2, shift = 64u - a.total_bits;
+    const uint32_t len = sm.clen[p], rows = sm.urows[p], tail = sm.fill[p];
+    const uint32_t * ch = a.chain + ((uint64_t)g * a.n_buckets + p) * a.maxb;
+    for (uint32_t l = threadIdx.x; l < LB; l += kENT)
+        sm.acc[l] = 0;
+    __syncthreads();
+    // the chain's rows in one run, four loads in flight a thread
+    for (uint32_t i0 = 0; i0 < rows; i0 += 4 * kENT)
     {
         uint64_t k[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
         {
             const uint32_t i = i0 + u * kENT + threadIdx.x;
-            k[u] = i < n ? __ldcs(a.pin.keys + r0 + i) : 0ull;
+            k[u] = 0;
+            if (i < rows)
+                k[u] = __ldcg(reinterpret_cast<const unsigned long long *>(block_ptr(a, ch[i >> a.page_log2])) + (i & (page - 1)));
         }
-        for (uint32_t c = 0; c < a.pin.n; ++c)
-            stage4_column<false>(sm.stage + a.col_off[c], a.pin.col[c], r0, i0, n, a.pin.width[c]);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-        {
-            const uint32_t i = i0 + u * kENT + threadIdx.x;
-            if (i < n)
-            {
-                reinterpret_cast<uint64_t *>(sm.stage)[i] = k[u];
-                const uint32_t p = (uint32_t)(int_hash64(k[u]) >> (64u - a.b1));
-                sm.perm[i] = (uint16_t)p;
-                atomicAdd(&sm.bins[p], 1u);
-            }
-        }
+            if (i0 + u * kENT + threadIdx.x < rows)
+                atomicAdd(&sm.acc[(uint32_t)(int_hash64(k[u]) >> shift) & (LB - 1u)], 1u);
+    }
+    const unsigned long long c0 = vload(&a.ctl->cursor); // the cursor stands still outside E
+    for (uint32_t j = threadIdx.x; j < len; j += kENT)
+    {
+        const uint32_t blk = ch[j], n = j + 1 == len ? tail : page;
+        a.blk_rows[blk] = n;
+        a.blk_rem[blk] = n;
+        a.blk_bucket[blk] = p;
+        a.blk_c0[blk] = c0;
+        a.blk_state[blk] = p;
     }
     __syncthreads();
-    // per bucket its rows (high half) and the blocks its chain needs (low
-    // half; an empty chain counts as a full last block), scanned at once
-    for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-    {
-        const uint32_t c = sm.bins[p];
-        const uint32_t nb = c == 0 ? 0u : (sm.fill[p] + c + page - 1) / page - 1u;
-        sm.boff[p] = (c << 16) | nb;
-    }
-    __syncthreads();
-    const uint32_t tot = scan_bins(sm.boff, P1, sm.ws);
-    const uint32_t nb_total = tot & 0xFFFFu;
-    // blocks come from the group's cache of free blocks (sm.bcache, its
-    // length in scal[16]), refilled from the pool's stack kRefill blocks
-    // beyond the need at a time, so the groups rarely meet on the stack
-    if (threadIdx.x == 0)
-    {
-        sm.scal[0] = 0;
-        sm.scal[1] = 0;
-        sm.scal[2] = 0;
-        const uint32_t have = sm.scal[16];
-        if (nb_total > have)
-        {
-            const uint32_t need = nb_total - have, want = need + kRefill;
-            unsigned long long * top = reinterpret_cast<unsigned long long *>(&a.ctl->free_top);
-            long long cur = (long long)vload(top);
-            for (;;)
-            {
-                const long long take = cur >= (long long)want ? (long long)want : (cur >= (long long)need ? cur : 0);
-                if (take == 0)
-                {
-                    sm.scal[0] = 2; // too few free blocks
-                    break;
-                }
-                const long long seen = (long long)atomicCAS(top, (unsigned long long)cur, (unsigned long long)(cur - take));
-                if (seen == cur)
-                {
-                    sm.scal[1] = (uint32_t)(cur - take);
-                    sm.scal[2] = (uint32_t)take;
-                    break;
-                }
-                cur = seen;
-            }
-        }
-    }
-    __syncthreads();
-    if (sm.scal[0])
-    {
-        for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-            sm.bins[p] = 0;
-        __syncthreads();
-        return kTileNoRoom;
-    }
-    if (sm.scal[2])
-    {
-        const uint32_t have = sm.scal[16];
-        for (uint32_t i = threadIdx.x; i < sm.scal[2]; i += kENT)
-            sm.bcache[have + i] = __ldcg(a.free_stack + sm.scal[1] + i);
-        __syncthreads();
-        if (threadIdx.x == 0)
-            sm.scal[16] = have + sm.scal[2];
-        __syncthreads();
-    }
-    const uint32_t cache_base = sm.scal[16] - nb_total; // this tile's blocks: bcache[cache_base, +nb_total)
-    // new blocks onto the chains; the cursors of the sorted tile
-    for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-    {
-        const uint32_t off = sm.boff[p] >> 16, nb0 = sm.boff[p] & 0xFFFFu;
-        const uint32_t nb = ((p + 1 < P1 ? sm.boff[p + 1] : tot) & 0xFFFFu) - nb0;
-        sm.bins[p] = off;
-        if (nb == 0)
-            continue;
-        const uint32_t len = sm.clen[p];
-        if (len + nb > a.maxb)
-        {
-            fail(a, kErrChain);
-            sm.scal[0] = 1;
-            continue;
-        }
-        uint32_t * ch = a.chain + ((uint64_t)g * P1 + p) * a.maxb;
-        for (uint32_t j = 0; j < nb; ++j)
-            ch[len + j] = sm.bcache[cache_base + nb0 + j];
-    }
-    __syncthreads();
-    if (sm.scal[0])
-        return kTileFailed;
-    if (threadIdx.x == 0)
-        sm.scal[16] = cache_base; // read by no thread before the next tile's syncs
-    // the stage row of every sorted position
-    for (uint32_t i = threadIdx.x; i < n; i += kENT)
-        sm.src[atomicAdd(&sm.bins[sm.perm[i]], 1u)] = (uint16_t)i;
-    __syncthreads();
-    // the rows out to the chains' blocks in sorted order: consecutive rows
-    // of a bucket go to consecutive rows of its blocks
-    for (uint32_t s = threadIdx.x; s < n; s += kENT)
-    {
-        const uint32_t r = sm.src[s];
-        const uint64_t key = reinterpret_cast<const uint64_t *>(sm.stage)[r];
-        const uint32_t p = (uint32_t)(int_hash64(key) >> (64u - a.b1));
-        const uint32_t q = sm.fill[p] + (s - (sm.boff[p] >> 16)); // slot counted from the chain's last block
-        const uint32_t idx = sm.clen[p] + (q >> a.page_log2) - 1u;
-        const uint32_t blk = a.chain[((uint64_t)g * P1 + p) * a.maxb + idx];
-        copy_row(a, block_ptr(a, blk), q & (page - 1), sm.stage, r);
-    }
-    __syncthreads();
-    for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-    {
-        sm.bins[p] = 0;
-        const uint32_t c = (sm.boff[p + 1 < P1 ? p + 1 : p] >> 16) - (sm.boff[p] >> 16);
-        const uint32_t cnt = p + 1 < P1 ? c : n - (sm.boff[p] >> 16);
-        if (cnt == 0)
-            continue;
-        const uint32_t nb = ((p + 1 < P1 ? sm.boff[p + 1] : tot) & 0xFFFFu) - (sm.boff[p] & 0xFFFFu);
-        sm.fill[p] = ((sm.fill[p] + cnt - 1) & (page - 1)) + 1;
-        sm.clen[p] += nb;
-        sm.urows[p] += cnt;
-    }
-    __syncthreads();
-    return kTileDone;
-}
-
-// ---------------------------------------------------------------------------
-// S: refine bucket p of group g -- each block of its chain sorted by leaf
-// in place and published as a refined block.  Returns the rows refined.
-// ---------------------------------------------------------------------------
-__device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p)
-{
-    const uint32_t page = 1u << a.page_log2;
-    const uint32_t LB = 1u << a.lb_log2;
-    const uint32_t len = sm.clen[p], rows = sm.urows[p];
-    const uint32_t * ch = a.chain + ((uint64_t)g * a.n_buckets + p) * a.maxb;
-    const uint32_t shift = 64u - a.total_bits;
-    // the rows each leaf gains, summed over the bucket's blocks
-    for (uint32_t l = threadIdx.x; l < LB; l += kENT)
-        sm.acc[l] = 0;
-    for (uint32_t j = 0; j < len; ++j)
-    {
-        const uint32_t blk = ch[j];
-        const uint32_t n = j + 1 == len ? sm.fill[p] : page;
-        uint8_t * B = block_ptr(a, blk);
-        for (uint32_t l = threadIdx.x; l < LB; l += kENT)
-            sm.bins[l] = 0;
-        __syncthreads();
-        for (uint32_t i0 = 0; i0 < n; i0 += 4 * kENT)
-        {
-            uint64_t k[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                const uint32_t i = i0 + u * kENT + threadIdx.x;
-                k[u] = i < n ? __ldcg(reinterpret_cast<const unsigned long long *>(B) + i) : 0ull;
-            }
-            for (uint32_t c = 0; c < a.pin.n; ++c)
-                stage4_column<true>(sm.stage + a.col_off[c], B + a.col_off[c], 0, i0, n, a.pin.width[c]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                const uint32_t i = i0 + u * kENT + threadIdx.x;
-                if (i < n)
-                {
-                    reinterpret_cast<uint64_t *>(sm.stage)[i] = k[u];
-                    const uint32_t l = (uint32_t)(int_hash64(k[u]) >> shift) & (LB - 1u);
-                    sm.perm[i] = (uint16_t)l;
-                    atomicAdd(&sm.bins[l], 1u);
-                }
-            }
-        }
-        __syncthreads();
-        for (uint32_t l = threadIdx.x; l < LB; l += kENT)
-            sm.acc[l] += sm.bins[l];
-        scan_bins(sm.bins, LB, sm.ws);
-        // every row's sorted position (a row's order within its leaf does
-        // not matter), inverted into the source row of every position
-        // (bins reused: page entries), then the block written back in
-        // sorted order with consecutive stores
-        for (uint32_t i = threadIdx.x; i < n; i += kENT)
-            sm.perm[i] = (uint16_t)atomicAdd(&sm.bins[sm.perm[i]], 1u);
-        __syncthreads();
-        uint32_t * src = sm.bins;
-        for (uint32_t i = threadIdx.x; i < n; i += kENT)
-            src[sm.perm[i]] = i;
-        __syncthreads();
-        for (uint32_t s = threadIdx.x; s < n; s += kENT)
-            copy_row(a, B, s, sm.stage, src[s]);
-        if (threadIdx.x == 0)
-        {
-            // the leaves of its first and last rows: E probes a block that
-            // lies wholly inside its range without searching it
-            a.blk_lfirst[blk] = (uint32_t)(int_hash64(reinterpret_cast<const uint64_t *>(sm.stage)[src[0]]) >> shift) & (LB - 1u);
-            a.blk_llast[blk] = (uint32_t)(int_hash64(reinterpret_cast<const uint64_t *>(sm.stage)[src[n - 1]]) >> shift) & (LB - 1u);
-            a.blk_rows[blk] = n;
-            a.blk_rem[blk] = n;
-            a.blk_bucket[blk] = p;
-            a.blk_c0[blk] = vload(&a.ctl->cursor); // the cursor stands still outside E
-            if (g == 0)
-                a.ctl->blocks0 += 1;
-            a.blk_state[blk] = p;
-        }
-        __syncthreads();
-    }
     for (uint32_t l = threadIdx.x; l < LB; l += kENT)
         if (sm.acc[l])
             atomicAdd(a.leaf_rows + ((uint64_t)p << a.lb_log2) + l, sm.acc[l]);
@@ -609,6 +657,8 @@ __device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_
         atomicAdd(&a.ctl->global_leaf_rows, (unsigned long long)rows);
         atomicAdd(&a.ctl->rows_refined, (unsigned long long)rows);
         atomicAdd(&a.ctl->refinements, 1ull);
+        if (g == 0)
+            a.ctl->blocks0 += len;
         sm.clen[p] = 0;
         sm.fill[p] = page;
         sm.urows[p] = 0;
@@ -658,12 +708,29 @@ __device__ void refine_down_to(const EngineArgs & a, const Smem & sm, uint32_t g
 }
 
 // ---------------------------------------------------------------------------
-// E0 (group 0 alone): the eviction range.  From the cursor on, leaves are
+// E: the eviction range (one CTA).  From the cursor on, leaves are
 // taken until the rows they hold take the global leaf bytes below the low
 // water (every leaf in the final drain).
 // ---------------------------------------------------------------------------
-__device__ void evict_range(const EngineArgs & a, const Smem & sm, bool final_drain)
+__global__ void __launch_bounds__(kENT) k_bep_range(const __grid_constant__ EngineArgs a)
 {
+    __shared__ uint32_t ws[kENT / 32];
+    __shared__ uint32_t s_hit;
+    const int mode = vload(&a.ctl->ev_mode);
+    __syncthreads(); // (cleared below)
+    if (threadIdx.x == 0)
+    {
+        a.ctl->ev_mode = 0;
+        a.ctl->ev_len = 0;
+        a.ctl->work_n = 0;
+        a.ctl->work_next = 0;
+        a.ctl->build_n = 0;
+        a.ctl->build_next = 0;
+        a.ctl->t_evict0 = mode ? now_ns() : 0ull;
+    }
+    if (mode == 0)
+        return; // no E: the following kernels find nothing to do
+    const bool final_drain = mode == 2;
     const uint64_t n = a.n_leaves;
     const uint64_t lo_abs = vload(&a.ctl->cursor), lo = lo_abs % n;
     const uint64_t g_rows = vload(&a.ctl->global_leaf_rows);
@@ -687,9 +754,9 @@ __device__ void evict_range(const EngineArgs & a, const Smem & sm, bool final_dr
                 mine += v[u];
             }
             uint32_t tot;
-            const uint32_t ex = block_excl_scan<kENT>(mine, sm.ws, &tot);
+            const uint32_t ex = block_excl_scan<kENT>(mine, ws, &tot);
             if (threadIdx.x == 0)
-                sm.scal[6] = kNone;
+                s_hit = kNone;
             __syncthreads();
             // the leaf whose inclusive prefix first reaches `need`
             if (taken + ex < need && taken + ex + mine >= need)
@@ -702,10 +769,10 @@ __device__ void evict_range(const EngineArgs & a, const Smem & sm, bool final_dr
                     if (run >= need)
                         break;
                 }
-                sm.scal[6] = threadIdx.x * kPer + u;
+                s_hit = threadIdx.x * kPer + u;
             }
             __syncthreads();
-            const uint32_t hit = sm.scal[6];
+            const uint32_t hit = s_hit;
             __syncthreads();
             if (hit != kNone)
             {
@@ -724,10 +791,9 @@ __device__ void evict_range(const EngineArgs & a, const Smem & sm, bool final_dr
         a.ctl->ev_lo = lo_abs;
         a.ctl->ev_len = len;
         a.ctl->cursor = lo_abs + len;
-        a.ctl->work_next = 0;
-        a.ctl->build_n = 0;
-        a.ctl->build_next = 0;
         a.ctl->evict_phases += 1;
+        if (a.ctl->input_done)
+            a.ctl->finished = 1; // the post-probe drain
     }
     for (uint32_t p = threadIdx.x; p <= a.n_buckets; p += kENT)
     {
@@ -777,110 +843,6 @@ __device__ __forceinline__ uint64_t block_len(const EngineArgs & a, unsigned lon
 {
     const uint64_t end = c0 + a.n_leaves;
     return end <= lo_abs ? 0 : umin64(len, end - lo_abs);
-}
-
-// Builds the table of leaf L in place (this warp won NOT_BUILT ->
-// BUILDING) and threads the next-chain.  Returns whether a key repeats.
-__device__ bool build_leaf_warp(const EngineArgs & a, uint32_t L, uint32_t lane)
-{
-    const LeafMeta m = a.meta[L]; // its place and size are planned before the launch
-    bool dup = false;
-    if (m.has_table)
-    {
-        const uint64_t cap = 1ull << m.log2cap;
-        Cell * tab = a.cells + m.table_off;
-        for (uint64_t j = lane; j < cap; j += 32)
-            reinterpret_cast<ulonglong2 *>(tab)[j] = make_ulonglong2(0ull, INVALID_REF);
-        __syncwarp();
-        const uint32_t r0 = m.row_off, r1 = a.leaf_off[L + 1];
-        for (uint32_t r = r0 + lane; r < r1; r += 32)
-        {
-            const uint64_t k = a.bpart.keys[r];
-            const uint64_t prev = table_insert<false>(tab, cap, int_hash64(k), k, make_ref(0, r));
-            a.next[r] = prev;
-            dup |= ref_valid(prev);
-        }
-    }
-    return __any_sync(0xffffffffu, dup);
-}
-
-// E1b: every warp takes claimed leaves from the queue and builds those it
-// wins NOT_BUILT -> BUILDING for; a leaf another warp is building is waited
-// for, bounded (the grid then ends with kErrWait).
-__device__ void build_claimed(const EngineArgs & a)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    for (;;)
-    {
-        uint32_t L = kNone, won = 0;
-        if (lane == 0)
-        {
-            const uint32_t i = atomicAdd(&a.ctl->build_next, 1u);
-            L = i < vload(&a.ctl->build_n) ? __ldcg(a.build_queue + i) : kNone;
-            if (L != kNone)
-            {
-                if (atomicCAS(a.state + L, kNotBuilt, kBuilding) == kNotBuilt)
-                    won = 1;
-                else if (ld_acquire_u32(a.state + L) < kBuilt)
-                {
-                    atomicAdd(&a.ctl->skip_retries, 1ull);
-                    const uint64_t t0 = now_ns();
-                    uint32_t spins = 0;
-                    while (ld_acquire_u32(a.state + L) < kBuilt)
-                    {
-                        if (aborted(a))
-                            break;
-                        if ((++spins & 255u) == 0 && now_ns() - t0 > a.wait_limit_ns)
-                        {
-                            fail(a, kErrWait);
-                            break;
-                        }
-                        __nanosleep(64);
-                    }
-                }
-            }
-        }
-        L = __shfl_sync(0xffffffffu, L, 0);
-        won = __shfl_sync(0xffffffffu, won, 0);
-        if (L == kNone || aborted(a))
-            return;
-        if (won)
-        {
-            const bool dup = build_leaf_warp(a, L, lane);
-            if (lane == 0)
-            {
-                a.meta[L].dup = dup ? 1 : 0;
-                if (dup)
-                    atomicExch(&a.ctl->any_dup, 1);
-                __threadfence();
-                atomicExch(a.state + L, dup ? kBuiltDup : kBuilt);
-                atomicAdd(&a.ctl->tables_built, 1ull);
-            }
-        }
-    }
-}
-
-// First row of the leaf-sorted block B (rows [lo, hi)) whose leaf-in-bucket
-// is >= l: a 32-way search by one warp.
-__device__ uint32_t lower_bound_warp(const EngineArgs & a, const uint8_t * B, uint32_t lo, uint32_t hi, uint32_t l, uint32_t lane)
-{
-    const uint32_t mask = (1u << a.lb_log2) - 1u, shift = 64u - a.total_bits;
-    const unsigned long long * keys = reinterpret_cast<const unsigned long long *>(B);
-    while (hi - lo > 32)
-    {
-        const uint32_t step = (hi - lo + 31) / 32;
-        const uint32_t x = lo + lane * step;
-        const bool below = x < hi && ((uint32_t)(int_hash64(__ldcg(keys + x)) >> shift) & mask) < l;
-        const uint32_t c = __popc(__ballot_sync(0xffffffffu, below));
-        // rows before lo are below l, rows from hi on are not
-        const uint32_t nlo = c ? lo + (c - 1) * step + 1 : lo;
-        const uint32_t nhi = c < 32 && lo + c * step < hi ? lo + c * step : hi;
-        lo = nlo;
-        hi = nhi;
-    }
-    const uint32_t x = lo + lane;
-    const bool below = x < hi && ((uint32_t)(int_hash64(__ldcg(keys + x)) >> shift) & mask) < l;
-    return lo + __popc(__ballot_sync(0xffffffffu, below));
 }
 
 // A lookup in two halves, so that several rows' first loads are in flight
@@ -961,262 +923,483 @@ __device__ __forceinline__ uint32_t probe_finish(const EngineArgs & a, uint64_t 
     return c;
 }
 
-// E2: one warp probes rows [r0, r1) of refined block B and projects the
-// matches, 256 rows a step with one reservation of output rows; a step's
-// output rows are placed round by round so each store instruction writes
-// consecutive rows.
-constexpr uint32_t kWarpRows = 4; // rows per lane per step
-__device__ void probe_rows_warp(const EngineArgs & a, const uint8_t * B, uint32_t r0, uint32_t r1, uint32_t lane, bool chains)
+// Every claim of this E's range: the leaf's rows leave the global count, a
+// leaf that held rows is an eviction, and one whose table is not built is
+// queued; the refined blocks to probe are counted per bucket.
+__global__ void __launch_bounds__(512) k_bep_claim(const __grid_constant__ EngineArgs a)
 {
-    const unsigned long long * keys = reinterpret_cast<const unsigned long long *>(B);
-    for (uint32_t base = r0; base < r1; base += 32 * kWarpRows)
+    const uint64_t lo_abs = vload(&a.ctl->ev_lo), len = vload(&a.ctl->ev_len);
+    if (len == 0)
+        return;
+    const uint64_t n = a.n_leaves, lo = lo_abs % n;
+    const uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    unsigned long long rows = 0, ev = 0, skips = 0;
+    for (uint64_t i = i0; i < len; i += stride)
     {
-        uint64_t key[kWarpRows];
-        uint32_t head[kWarpRows], cnt[kWarpRows];
-#pragma unroll
-        for (uint32_t k = 0; k < kWarpRows; ++k)
+        const uint32_t L = (uint32_t)((lo + i) % n);
+        if (atomicCAS(a.leaf_lock + L, 0u, 1u) != 0u)
         {
-            const uint32_t i = base + k * 32 + lane;
-            key[k] = i < r1 ? __ldcg(keys + i) : 0ull;
-        }
-        // four first loads in flight, then their comparisons
-#pragma unroll
-        for (uint32_t g = 0; g < kWarpRows; g += 4)
-        {
-            CellPair pr[4];
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u)
-            {
-                const uint32_t i = base + (g + u) * 32 + lane;
-                if (i < r1)
-                    pr[u] = probe_issue(a, int_hash64(key[g + u]));
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u)
-            {
-                const uint32_t i = base + (g + u) * 32 + lane;
-                head[g + u] = 0;
-                cnt[g + u] = i < r1 ? probe_finish(a, key[g + u], int_hash64(key[g + u]), pr[u], chains, head[g + u]) : 0u;
-            }
-        }
-        // placement: a warp scan per round, rounds one after another
-        uint32_t rel[kWarpRows], total = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < kWarpRows; ++k)
-        {
-            uint32_t x = cnt[k];
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1)
-            {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= (uint32_t)d)
-                    x += y;
-            }
-            rel[k] = total + x - cnt[k];
-            total += __shfl_sync(0xffffffffu, x, 31);
-        }
-        if (total == 0)
+            ++skips; // held elsewhere
             continue;
-        unsigned long long out0 = 0;
-        if (lane == 0)
-            out0 = atomicAdd(&a.ctl->out_rows, (unsigned long long)total);
-        out0 = __shfl_sync(0xffffffffu, out0, 0);
-#pragma unroll 1
-        for (uint32_t k = 0; k < kWarpRows; ++k)
-        {
-            if (cnt[k] == 0)
-                continue;
-            const uint32_t i = base + k * 32 + lane;
-            uint64_t o = out0 + rel[k];
-            uint32_t b = head[k];
-            for (uint32_t m = 0; m < cnt[k]; ++m, ++o)
-            {
-                if (o < a.out_cap)
-                {
-                    __stcs(a.out_keys + o, (unsigned long long)key[k]);
-                    for (uint32_t c = 0; c < a.bpart.n; ++c)
-                        copy_elem_out(a.out_l[c], o, a.bpart.col[c], b, a.bpart.width[c]);
-                    for (uint32_t c = 0; c < a.pin.n; ++c)
-                        copy_elem_cg(a.out_r[c], o, B + a.col_off[c], i, a.pin.width[c]);
-                }
-                if (m + 1 < cnt[k])
-                    b = ref_row(__ldcg(reinterpret_cast<const unsigned long long *>(a.next) + b));
-            }
         }
+        const uint32_t r = __ldcg(a.leaf_rows + L);
+        if (r)
+        {
+            a.leaf_rows[L] = 0;
+            rows += r;
+            ++ev;
+            const uint32_t st = ld_acquire_u32(a.state + L);
+            if (st < kBuilt)
+                a.build_queue[atomicAdd(&a.ctl->build_n, 1u)] = L;
+            else if (st == kBuiltDup)
+                atomicExch(&a.ctl->any_dup, 1); // built by an earlier run over these tables
+        }
+        atomicExch(a.leaf_lock + L, 0u);
+    }
+    for (uint64_t b = i0; b < a.n_blocks; b += stride)
+    {
+        const uint32_t p = a.blk_state[b];
+        if (p != kNone && bucket_in_range(a, p, lo, block_len(a, a.blk_c0[b], lo_abs, len)))
+            atomicAdd(a.bucket_cnt + p, 1u);
+    }
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        rows += __shfl_xor_sync(0xffffffffu, rows, o);
+        ev += __shfl_xor_sync(0xffffffffu, ev, o);
+        skips += __shfl_xor_sync(0xffffffffu, skips, o);
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+        if (rows)
+        {
+            atomicAdd(&a.ctl->global_leaf_rows, (unsigned long long)(-(long long)rows));
+            atomicAdd(&a.ctl->rows_claimed, rows);
+        }
+        if (ev)
+            atomicAdd(&a.ctl->evictions, ev);
+        if (skips)
+            atomicAdd(&a.ctl->skip_retries, skips);
     }
 }
 
-// ---------------------------------------------------------------------------
-// One E: range, claims, builds, probes.  False when the grid is ending.
-// ---------------------------------------------------------------------------
-__device__ bool evict_phase(const EngineArgs & a, const Smem & sm, uint32_t & gen, bool final_drain)
+// Block counts per bucket into work offsets, the buckets in the range's
+// order (one CTA).
+__global__ void __launch_bounds__(kENT) k_bep_offsets(const __grid_constant__ EngineArgs a)
 {
-    const uint64_t t0 = now_ns();
-    if (blockIdx.x == 0)
-        evict_range(a, sm, final_drain);
-    if (!grid_sync(a, gen, NoOp{}))
-        return false;
+    __shared__ uint32_t bins[1u << 11];
+    __shared__ uint32_t ws[kENT / 32];
+    if (vload(&a.ctl->ev_len) == 0)
+        return;
+    const uint32_t P1 = a.n_buckets, first = (uint32_t)((vload(&a.ctl->ev_lo) % a.n_leaves) >> a.lb_log2);
+    for (uint32_t q = threadIdx.x; q < P1; q += kENT)
+        bins[q] = a.bucket_cnt[(first + q) % P1];
+    __syncthreads();
+    const uint32_t total = scan_bins(bins, P1, ws);
+    for (uint32_t q = threadIdx.x; q < P1; q += kENT)
+        a.bucket_cnt[(first + q) % P1] = bins[q];
+    if (threadIdx.x == 0)
+        a.ctl->work_n = total;
+}
+
+// The refined blocks of the range's buckets into the work list.
+__global__ void __launch_bounds__(512) k_bep_list(const __grid_constant__ EngineArgs a)
+{
     const uint64_t lo_abs = vload(&a.ctl->ev_lo), len = vload(&a.ctl->ev_len);
-    const uint64_t n = a.n_leaves, lo = lo_abs % n;
-    const uint64_t stride = (uint64_t)gridDim.x * kENT;
-    // E1: claim every leaf of the range; count the refined blocks to probe
-    // per bucket
+    if (blockIdx.x == 0 && threadIdx.x == 0)
     {
-        unsigned long long rows = 0, ev = 0, skips = 0;
-        for (uint64_t i = (uint64_t)blockIdx.x * kENT + threadIdx.x; i < len; i += stride)
-        {
-            const uint32_t L = (uint32_t)((lo + i) % n);
-            if (atomicCAS(a.leaf_lock + L, 0u, 1u) != 0u)
-            {
-                ++skips; // held elsewhere
-                continue;
-            }
-            const uint32_t r = __ldcg(a.leaf_rows + L);
-            if (r)
-            {
-                a.leaf_rows[L] = 0;
-                rows += r;
-                ++ev;
-                const uint32_t st = ld_acquire_u32(a.state + L);
-                if (st < kBuilt)
-                    a.build_queue[atomicAdd(&a.ctl->build_n, 1u)] = L;
-                else if (st == kBuiltDup)
-                    atomicExch(&a.ctl->any_dup, 1); // built by an earlier run over these tables
-            }
-            atomicExch(a.leaf_lock + L, 0u);
-        }
-        for (uint64_t b = (uint64_t)blockIdx.x * kENT + threadIdx.x; b < a.n_blocks; b += stride)
-        {
-            const uint32_t p = __ldcg(a.blk_state + b);
-            if (p != kNone && bucket_in_range(a, p, lo, block_len(a, __ldcg(a.blk_c0 + b), lo_abs, len)))
-                atomicAdd(a.bucket_cnt + p, 1u);
-        }
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            rows += __shfl_xor_sync(0xffffffffu, rows, o);
-            ev += __shfl_xor_sync(0xffffffffu, ev, o);
-            skips += __shfl_xor_sync(0xffffffffu, skips, o);
-        }
-        if ((threadIdx.x & 31) == 0)
-        {
-            if (rows)
-            {
-                atomicAdd(&a.ctl->global_leaf_rows, (unsigned long long)(-(long long)rows));
-                atomicAdd(&a.ctl->rows_claimed, rows);
-            }
-            if (ev)
-                atomicAdd(&a.ctl->evictions, ev);
-            if (skips)
-                atomicAdd(&a.ctl->skip_retries, skips);
-        }
+        const unsigned long long t = now_ns(), t0 = a.ctl->t_evict0;
+        if (t0)
+            a.ctl->ns_evict += t - t0;
+        a.ctl->t_probe0 = t0 ? t : 0ull;
     }
-    if (!grid_sync(a, gen, NoOp{}))
-        return false;
-    // E1b: group 0 turns the counts into work offsets, the buckets in the
-    // range's order; every group builds claimed leaves
-    if (blockIdx.x == 0)
+    if (len == 0)
+        return;
+    const uint64_t lo = lo_abs % a.n_leaves, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < a.n_blocks; b += stride)
     {
-        const uint32_t P1 = a.n_buckets, first = (uint32_t)(lo >> a.lb_log2);
-        for (uint32_t q = threadIdx.x; q < P1; q += kENT)
-            sm.bins[q] = __ldcg(a.bucket_cnt + (first + q) % P1);
-        __syncthreads();
-        const uint32_t total = scan_bins(sm.bins, P1, sm.ws);
-        for (uint32_t q = threadIdx.x; q < P1; q += kENT)
-            a.bucket_cnt[(first + q) % P1] = sm.bins[q];
-        if (threadIdx.x == 0)
-            a.ctl->work_n = total;
-        __syncthreads();
+        const uint32_t p = a.blk_state[b];
+        if (p != kNone && bucket_in_range(a, p, lo, block_len(a, a.blk_c0[b], lo_abs, len)))
+            a.work[a.bucket_cnt[p] + atomicAdd(a.bucket_fill + p, 1u)] = (uint32_t)b;
     }
-    build_claimed(a);
-    if (!grid_sync(a, gen, NoOp{}))
+}
+
+// Work items of the probe kernels: a part of at most 256 rows of a listed
+// block, in list order (bucket by bucket), so the warps in flight cover
+// little more than one bucket and its leaf tables and build rows stay in L2.
+constexpr uint32_t kPartRows = 256;
+struct PartItem
+{
+    uint32_t blk, first, rows; // rows [first, first + rows) of the block
+    uint32_t x0, x1, y0, y1;   // the range's leaves of its bucket
+    bool whole;                // ... are all of them
+};
+
+__device__ __forceinline__ bool part_item(const EngineArgs & a, uint64_t w, uint64_t n_blocks_listed, uint64_t lo_abs, uint64_t len, PartItem & it)
+{
+    const uint32_t page = 1u << a.page_log2, part_rows = page < kPartRows ? page : kPartRows, parts = page / part_rows;
+    if (w >= n_blocks_listed * parts)
         return false;
-    // E1c: the refined blocks of the range's buckets into the work list
-    for (uint64_t b = (uint64_t)blockIdx.x * kENT + threadIdx.x; b < a.n_blocks; b += stride)
+    it.blk = a.work[w / parts];
+    it.first = (uint32_t)(w % parts) * part_rows;
+    const uint32_t nrows = a.blk_rows[it.blk];
+    it.rows = it.first < nrows ? min(part_rows, nrows - it.first) : 0u;
+    const uint32_t p = a.blk_bucket[it.blk];
+    bucket_intervals(a, p, lo_abs % a.n_leaves, block_len(a, a.blk_c0[it.blk], lo_abs, len), it.x0, it.x1, it.y0, it.y1);
+    it.whole = it.x0 == 0 && it.x1 == (1u << a.lb_log2);
+    return true;
+}
+
+__device__ __forceinline__ bool leaf_in(const PartItem & it, uint32_t l)
+{
+    return it.whole || l - it.x0 < it.x1 - it.x0 || l - it.y0 < it.y1 - it.y0;
+}
+
+// `done` of the block's rows are probed; a block whose rows all are goes
+// back to the pool.
+__device__ __forceinline__ void rows_done(const EngineArgs & a, uint32_t blk, uint32_t done)
+{
+    if (done && atomicSub(a.blk_rem + blk, done) == done)
     {
-        const uint32_t p = __ldcg(a.blk_state + b);
-        if (p != kNone && bucket_in_range(a, p, lo, block_len(a, __ldcg(a.blk_c0 + b), lo_abs, len)))
-            a.work[__ldcg(a.bucket_cnt + p) + atomicAdd(a.bucket_fill + p, 1u)] = (uint32_t)b;
+        a.blk_state[blk] = kNone;
+        const long long slot = (long long)atomicAdd(reinterpret_cast<unsigned long long *>(&a.ctl->free_top), 1ull);
+        a.free_stack[slot] = blk;
     }
-    if (!grid_sync(a, gen, NoOp{}))
-        return false;
-    const uint64_t t1 = now_ns();
-    // E2: every warp takes a 1024-row part of a listed block at a time and
-    // probes the range's rows in it.  Parts are handed out in list order
-    // (bucket by bucket), so the warps in flight cover little more than one
-    // bucket and its leaf tables and build rows stay in L2.
+}
+
+// E's probes when no key repeats and the build payloads are gathered in one
+// piece (kGather 16: packed rows; 4 or 8: the one column; 0: none): per part
+// the lookups, one reservation of its output rows, then its matches 128 at a
+// time, as k_probe_inline (probe.cu) writes them, the build rows gathered to
+// shared memory meanwhile.  Bound as k_probe_fused by the request path from
+// L1 to the crossbar: a cell pair and a build row a probe row.  Measured:
+// 6.7 ms for the 512M rows against 64M build rows and 0.88 ms for 64M rows
+// against 8M, where the chain-following warps of the persistent grid took
+// 12.3 and 1.9 ms.
+constexpr int kBPNT = 256;
+constexpr uint32_t kBKeys = 0, kBRow = 2048, kBStage = 3072, kBQueue = 5120, kBList = 5632, kBWarpBytes = 5888;
+template <int kGather, bool kUniform>
+__global__ void __launch_bounds__(kBPNT, 3) k_bep_probe(const __grid_constant__ EngineArgs a, const void * __restrict__ gathered,
+                                                        const __grid_constant__ PackSpec pk)
+{
+    __shared__ __align__(16) uint8_t bsm[kBPNT / 32 * kBWarpBytes];
+    if (vload(a.err))
+        return; // a leaf's build gave up: its table cannot be read
+    if (vload(&a.ctl->any_dup))
+        return; // chains have to be followed: k_bep_probe_chains
+    const uint32_t lane = threadIdx.x & 31;
+    uint8_t * wsm = bsm + (threadIdx.x >> 5) * kBWarpBytes;
+    uint64_t * key_s = reinterpret_cast<uint64_t *>(wsm + kBKeys);
+    uint32_t * brow_s = reinterpret_cast<uint32_t *>(wsm + kBRow);
+    uint4 * stage = reinterpret_cast<uint4 *>(wsm + kBStage);
+    uint16_t * qrow = reinterpret_cast<uint16_t *>(wsm + kBQueue);
+    uint8_t * list = wsm + kBList;
+    const uint64_t lo_abs = vload(&a.ctl->ev_lo), len = vload(&a.ctl->ev_len);
+    const uint64_t listed = len ? vload(&a.ctl->work_n) : 0u;
+    const uint32_t shift = 64u - a.total_bits, lmask = (1u << a.lb_log2) - 1u;
+    const uint64_t ucap = kUniform ? 1ull << a.ulog : 0ull;
+    unsigned long long probed = 0;
+    for (;;)
     {
-        constexpr uint32_t kPart = 1024;
-        const uint32_t lane = threadIdx.x & 31;
-        const bool chains = vload(&a.ctl->any_dup) != 0; // some leaf table has a repeated key
-        const uint32_t parts = (1u << a.page_log2) > kPart ? (1u << a.page_log2) / kPart : 1u;
-        const uint32_t part_rows = (1u << a.page_log2) / parts;
-        const uint64_t n_items = (uint64_t)vload(&a.ctl->work_n) * parts;
-        for (;;)
+        unsigned long long w = 0;
+        if (lane == 0)
+            w = atomicAdd(&a.ctl->work_next, 1ull);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        PartItem it;
+        if (!part_item(a, w, listed, lo_abs, len, it))
+            break;
+        const uint8_t * B = block_ptr(a, it.blk);
+        const uint64_t * keys = reinterpret_cast<const uint64_t *>(B) + it.first;
+#pragma unroll
+        for (int k = 0; k < (int)kPartRows / 32; ++k)
+            if ((uint32_t)k * 32 + lane < it.rows)
+                cp_async_small<8>(key_s + k * 32 + lane, keys + k * 32 + lane);
+        cp_async_wait_all();
+        uint32_t qn = 0, done = 0;
+#pragma unroll 1
+        for (uint32_t g = 0; g < it.rows; g += 128)
         {
-            unsigned long long w = 0;
-            if (lane == 0)
-                w = atomicAdd(&a.ctl->work_next, 1ull);
-            w = __shfl_sync(0xffffffffu, w, 0);
-            if (w >= n_items)
-                break;
-            const uint32_t blk = __ldcg(a.work + w / parts);
-            const uint32_t c0r = (uint32_t)(w % parts) * part_rows; // the part's first row
-            // (blk_state may already be cleared by the warp that probed the
-            // block's last rows; the bucket stays)
-            const uint32_t p = __ldcg(a.blk_bucket + blk);
-            const uint32_t nrows = __ldcg(a.blk_rows + blk);
-            if (c0r >= nrows)
-                continue;
-            const uint32_t c1r = c0r + part_rows < nrows ? c0r + part_rows : nrows;
-            const uint32_t lf = __ldcg(a.blk_lfirst + blk), ll = __ldcg(a.blk_llast + blk);
-            const uint8_t * B = block_ptr(a, blk);
-            uint32_t x0, x1, y0, y1;
-            bucket_intervals(a, p, lo, block_len(a, __ldcg(a.blk_c0 + blk), lo_abs, len), x0, x1, y0, y1);
-            uint32_t done = 0;
-            for (int part = 0; part < 2; ++part)
+            uint64_t key[4];
+            CellPair cell[4];
+            uint32_t live = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
             {
-                const uint32_t l0 = part ? y0 : x0, l1 = part ? y1 : x1;
-                if (l1 <= l0 || l1 <= lf || l0 > ll)
-                    continue; // no row of the block in these leaves
-                uint32_t ra = l0 > lf ? lower_bound_warp(a, B, 0, nrows, l0, lane) : 0u;
-                uint32_t rb = l1 <= ll ? lower_bound_warp(a, B, ra, nrows, l1, lane) : nrows;
-                ra = ra > c0r ? ra : c0r;
-                rb = rb < c1r ? rb : c1r;
-                if (rb <= ra)
-                    continue;
-                probe_rows_warp(a, B, ra, rb, lane, chains);
-                done += rb - ra;
-            }
-            if (lane == 0 && done)
-            {
-                atomicAdd(&a.ctl->rows_probed, (unsigned long long)done);
-                const uint32_t left = atomicSub(a.blk_rem + blk, done) - done;
-                if (left == 0)
+                const uint32_t i = g + u * 32 + lane;
+                key[u] = 0;
+                cell[u].a = make_ulonglong2(0ull, INVALID_REF);
+                cell[u].b = cell[u].a;
+                if (i < it.rows)
                 {
-                    // every row probed: the block goes back to the pool
-                    a.blk_state[blk] = kNone;
-                    const long long slot = (long long)atomicAdd(reinterpret_cast<unsigned long long *>(&a.ctl->free_top), 1ull);
-                    a.free_stack[slot] = blk;
+                    key[u] = ld_shared_u64(key_s + i);
+                    const uint64_t h = int_hash64(key[u]);
+                    const uint32_t L = (uint32_t)(h >> shift);
+                    if (leaf_in(it, L & lmask))
+                    {
+                        live |= 1u << u;
+                        if (kUniform)
+                            cell[u] = load_pair<false>(a.cells + ((uint64_t)L << a.ulog) + probe_start(h, ucap));
+                        else
+                        {
+                            const ulonglong2 m = __ldg(reinterpret_cast<const ulonglong2 *>(a.meta + L));
+                            if ((m.y >> 40) & 0xffu)
+                                cell[u] = load_pair<false>(a.cells + m.x + probe_start(h, 1ull << ((uint32_t)(m.y >> 32) & 0xffu)));
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const uint32_t i = g + u * 32 + lane;
+                uint64_t head = INVALID_REF;
+                bool more = false;
+                if ((live >> u & 1u) && ref_valid(cell[u].a.y))
+                {
+                    if (cell[u].a.x == key[u])
+                        head = cell[u].a.y;
+                    else if (ref_valid(cell[u].b.y))
+                    {
+                        if (cell[u].b.x == key[u])
+                            head = cell[u].b.y;
+                        else
+                            more = true;
+                    }
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, more);
+                if (more)
+                    qrow[qn + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
+                qn += __popc(m);
+                done += __popc(__ballot_sync(0xffffffffu, live >> u & 1u));
+                brow_s[i] = ref_valid(head) ? ref_row(head) : kNone;
+            }
+        }
+        __syncwarp();
+        for (uint32_t j = lane; j < qn; j += 32)
+        {
+            const uint32_t i = qrow[j];
+            const uint64_t qk = key_s[i], h = int_hash64(qk);
+            const Cell * tab;
+            uint64_t cap = ucap;
+            if (kUniform)
+                tab = a.cells + ((h >> shift) << a.ulog);
+            else
+                tab = leaf_table(a, h, cap);
+            uint64_t pos = (probe_start(h, cap) + 2) & (cap - 1);
+            for (uint64_t step = 2; step < cap; step += 2)
+            {
+                const CellPair c = load_pair<false>(tab + pos);
+                if (!ref_valid(c.a.y))
+                    break;
+                if (c.a.x == qk || (ref_valid(c.b.y) && c.b.x == qk))
+                {
+                    brow_s[i] = ref_row(c.a.x == qk ? c.a.y : c.b.y);
+                    break;
+                }
+                if (!ref_valid(c.b.y))
+                    break;
+                pos = (pos + 2) & (cap - 1);
+            }
+        }
+        __syncwarp();
+        uint32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < (int)kPartRows / 32; ++k)
+        {
+            const uint32_t i = (uint32_t)k * 32 + lane;
+            const bool hit = i < it.rows && brow_s[i] != kNone;
+            const uint32_t m = __ballot_sync(0xffffffffu, hit);
+            if (hit)
+                list[total + __popc(m & ((1u << lane) - 1u))] = (uint8_t)i;
+            total += __popc(m);
+        }
+        __syncwarp();
+        if (total)
+        {
+            unsigned long long b0 = 0;
+            if (lane == 0)
+                b0 = atomicAdd(&a.ctl->out_rows, (unsigned long long)total);
+            uint64_t base = 0;
+#pragma unroll 1
+            for (uint32_t j0 = 0; j0 < total; j0 += 128)
+            {
+                uint32_t idx[4], one = 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    const uint32_t j = j0 + u * 32 + lane;
+                    idx[u] = 0;
+                    if (j < total)
+                    {
+                        idx[u] = list[j];
+                        one |= 1u << u;
+                        if constexpr (kGather == 16)
+                            cp_async16(stage + u * 32 + lane, static_cast<const uint4 *>(gathered) + brow_s[idx[u]]);
+                        else if constexpr (kGather != 0)
+                            cp_async_small<kGather>(stage + u * 32 + lane, static_cast<const uint8_t *>(gathered) + (uint64_t)brow_s[idx[u]] * kGather);
+                    }
+                }
+                uint64_t v[4];
+                if (a.pin.n)
+                    load_list(v, B + a.col_off[0], a.pin.width[0], it.first, idx, one);
+                if (j0 == 0)
+                    base = __shfl_sync(0xffffffffu, b0, 0);
+                const uint64_t out = base + j0 + lane;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                {
+                    if (out + 32 * u >= a.out_cap)
+                        one &= ~(1u << u);
+                    if (one >> u & 1u)
+                        __stcs(a.out_keys + out + 32 * u, key_s[idx[u]]);
+                }
+#pragma unroll 1
+                for (uint32_t c = 0; c < a.pin.n; ++c)
+                {
+                    uint64_t nx[4];
+                    if (c + 1 < a.pin.n)
+                        load_list(nx, B + a.col_off[c + 1], a.pin.width[c + 1], it.first, idx, one);
+                    store_list(v, a.out_r[c], a.pin.width[c], out, one);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        v[u] = nx[u];
+                }
+                if constexpr (kGather != 0)
+                {
+                    cp_async_wait_all();
+#pragma unroll 1
+                    for (uint32_t c = 0; c < a.bpart.n; ++c)
+                    {
+                        uint64_t x[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            x[u] = reinterpret_cast<const uint64_t *>(stage + u * 32 + lane)[pk.off[c] >> 3] >> ((pk.off[c] & 7u) * 8u);
+                        store_list(x, a.out_l[c], a.bpart.width[c], out, one);
+                    }
+                }
+                __syncwarp(); // the stage is refilled by the next batch
+            }
+        }
+        if (lane == 0)
+            rows_done(a, it.blk, done);
+        probed += done;
+        __syncwarp(); // the warp's shared memory is filled again by the next part
+    }
+    if (lane == 0 && probed)
+        atomicAdd(&a.ctl->rows_probed, probed);
+}
+
+// E's probes in every other case: chains are followed, columns of any width
+// are copied row by row.  `only_dup`: k_bep_probe has done the work unless a
+// key repeats.
+__global__ void __launch_bounds__(kBPNT, 4) k_bep_probe_chains(const __grid_constant__ EngineArgs a, int only_dup)
+{
+    const bool chains = vload(&a.ctl->any_dup) != 0; // some leaf table has a repeated key
+    if ((only_dup && !chains) || vload(a.err))
+        return; // (err: a leaf's build gave up)
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t lo_abs = vload(&a.ctl->ev_lo), len = vload(&a.ctl->ev_len);
+    const uint64_t listed = len ? vload(&a.ctl->work_n) : 0u;
+    const uint32_t shift = 64u - a.total_bits, lmask = (1u << a.lb_log2) - 1u;
+    unsigned long long probed = 0;
+    for (;;)
+    {
+        unsigned long long w = 0;
+        if (lane == 0)
+            w = atomicAdd(&a.ctl->work_next, 1ull);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        PartItem it;
+        if (!part_item(a, w, listed, lo_abs, len, it))
+            break;
+        const uint8_t * B = block_ptr(a, it.blk);
+        const uint64_t * keys = reinterpret_cast<const uint64_t *>(B) + it.first;
+        uint32_t done = 0;
+#pragma unroll 1
+        for (uint32_t r0 = 0; r0 < it.rows; r0 += 128)
+        {
+            uint64_t key[4];
+            uint32_t head[4], cnt[4], live = 0;
+            CellPair pr[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                const uint32_t i = r0 + u * 32 + lane;
+                key[u] = i < it.rows ? keys[i] : 0ull;
+                const uint64_t h = int_hash64(key[u]);
+                if (i < it.rows && leaf_in(it, (uint32_t)(h >> shift) & lmask))
+                {
+                    live |= 1u << u;
+                    pr[u] = probe_issue(a, h);
+                }
+            }
+            uint32_t rel[4], total = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                head[u] = 0;
+                cnt[u] = (live >> u & 1u) ? probe_finish(a, key[u], int_hash64(key[u]), pr[u], chains, head[u]) : 0u;
+                done += __popc(__ballot_sync(0xffffffffu, live >> u & 1u));
+                uint32_t x = cnt[u];
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1)
+                {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                    if (lane >= (uint32_t)d)
+                        x += y;
+                }
+                rel[u] = total + x - cnt[u];
+                total += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (total == 0)
+                continue;
+            unsigned long long out0 = 0;
+            if (lane == 0)
+                out0 = atomicAdd(&a.ctl->out_rows, (unsigned long long)total);
+            out0 = __shfl_sync(0xffffffffu, out0, 0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+            {
+                uint64_t o = out0 + rel[u];
+                uint32_t b = head[u];
+                for (uint32_t m = 0; m < cnt[u]; ++m, ++o)
+                {
+                    if (o < a.out_cap)
+                    {
+                        __stcs(a.out_keys + o, key[u]);
+                        for (uint32_t c = 0; c < a.bpart.n; ++c)
+                            copy_elem_out(a.out_l[c], o, a.bpart.col[c], b, a.bpart.width[c]);
+                        for (uint32_t c = 0; c < a.pin.n; ++c)
+                            copy_elem_out(a.out_r[c], o, B + a.col_off[c], it.first + r0 + u * 32 + lane, a.pin.width[c]);
+                    }
+                    if (m + 1 < cnt[u])
+                        b = ref_row(__ldg(reinterpret_cast<const unsigned long long *>(a.next) + b));
                 }
             }
         }
+        if (lane == 0)
+            rows_done(a, it.blk, done);
+        probed += done;
     }
-    const uint64_t t2 = now_ns();
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-    {
-        a.ctl->ns_evict += t1 - t0;
-        a.ctl->ns_probe += t2 - t1;
-    }
-    return grid_sync(a, gen, NoOp{});
+    if (lane == 0 && probed)
+        atomicAdd(&a.ctl->rows_probed, probed);
+}
+
+// After the last E: its probes' time.
+__global__ void k_bep_stamp(EngineCtl * c)
+{
+    if (c->t_probe0)
+        c->ns_probe += now_ns() - c->t_probe0;
+    c->t_probe0 = 0;
 }
 
 // The last group to arrive after a wave's S: records the peak, decides
 // whether an E follows (the leaf high water, or a drain of every leaf when
 // a group found too few free blocks) and whether input is left.  A low pool
-// right after a forced drain cannot be helped: the grid ends.
+// right after a forced drain cannot be helped: the run ends.  At the end of
+// the input the E is the drain of every leaf.
 struct WaveEnd
 {
     const EngineArgs * a;
+    bool end_of_input;
     __device__ void operator()() const
     {
         EngineCtl * c = a->ctl;
@@ -1236,94 +1419,198 @@ struct WaveEnd
         c->evict_now = low ? 2 : (r > 0 && r * a->rb >= a->leaf_high ? 1 : 0);
         c->ns_s_crit += c->wave_s_max;
         c->wave_s_max = 0;
-        c->more_input = vload(&c->groups_done) < gridDim.x;
+        c->waves += 1;
+        c->no_more_input = vload(&c->groups_done) >= gridDim.x;
+        c->started = 1;
+        c->ev_mode = end_of_input ? 2 : c->evict_now;
+        if (end_of_input)
+            c->input_done = 1;
     }
 };
 
-__global__ void __launch_bounds__(kENT, 1) k_bep_engine(const __grid_constant__ EngineArgs a)
+__global__ void __launch_bounds__(kENT, 1) k_bep_scatter(const __grid_constant__ EngineArgs a)
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bar[2];
+    if (vload(&a.ctl->finished) || aborted(a) || vload(a.err))
+        return; // nothing is left to do (no group changes these before a barrier of this launch)
     const uint32_t page = 1u << a.page_log2;
     const uint32_t P1 = a.n_buckets, LB = 1u << a.lb_log2;
+    const uint32_t g = blockIdx.x, G = gridDim.x;
+    const uint32_t half = threadIdx.x / kHNT, tid = threadIdx.x & (kHNT - 1);
     Smem sm;
     {
         uint8_t * p = smem_raw;
-        const uint64_t cells_bytes = (uint64_t)a.smem_cells * sizeof(Cell), rows_bytes = (uint64_t)page * a.rb;
-        const uint64_t stage = rows_bytes > cells_bytes ? rows_bytes : cells_bytes;
-        sm.stage = p;
-        p += (stage + 15) & ~15ull;
-        sm.perm = reinterpret_cast<uint16_t *>(p);
-        p += ((uint64_t)page * 2 + 15) & ~15ull;
-        sm.src = reinterpret_cast<uint16_t *>(p);
-        p += ((uint64_t)page * 2 + 15) & ~15ull;
-        const uint32_t nbins = P1 > LB ? (P1 > page ? P1 : page) : (LB > page ? LB : page);
-        sm.bins = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)nbins * 4 + 15) & ~15ull;
-        sm.boff = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)P1 * 4 + 15) & ~15ull;
-        sm.nbpre = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)P1 * 4 + 15) & ~15ull;
-        sm.fill = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)P1 * 4 + 15) & ~15ull;
-        sm.clen = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)P1 * 4 + 15) & ~15ull;
-        sm.urows = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)P1 * 4 + 15) & ~15ull;
-        sm.acc = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)LB * 4 + 15) & ~15ull;
-        sm.bcache = reinterpret_cast<uint32_t *>(p);
-        p += ((uint64_t)(2 * P1 + 2 * kRefill) * 4 + 15) & ~15ull;
-        sm.ws = reinterpret_cast<uint32_t *>(p);
-        p += (kENT / 32) * 4;
-        sm.scal = reinterpret_cast<uint32_t *>(p);
+        auto take = [&](uint64_t bytes) {
+            uint8_t * q = p;
+            p += (bytes + 15) & ~15ull;
+            return q;
+        };
+        auto words = [&](uint64_t n) { return reinterpret_cast<uint32_t *>(take(4 * n)); };
+        p += half * a.half_bytes;
+        sm.hf.stage = take(a.stage_bytes);
+        sm.hf.perm = words(a.stage_rows);
+        sm.hf.bins = words(P1);
+        sm.hf.off = words(P1 + 1);
+        sm.hf.nb0 = words(P1 + 1);
+        sm.hf.fill = words(P1);
+        sm.hf.last = words(P1);
+        sm.hf.fresh = words(a.fresh_words);
+        sm.hf.wsum = words(kHNT / 32);
+        sm.hf.scal = words(4);
+        p = smem_raw + 2 * a.half_bytes;
+        sm.acc = words(LB);
+        sm.scal = words(32);
+        sm.persist = words(a.persist_words);
+        sm.fill = sm.persist;
+        sm.clen = sm.fill + P1;
+        sm.urows = sm.clen + P1;
+        sm.last = sm.urows + P1;
+        sm.pscal = sm.last + P1; // (an even number of words before it)
+        sm.bcache = sm.pscal + kPersistScal;
     }
-    const uint32_t g = blockIdx.x, G = gridDim.x;
-    for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-    {
-        sm.fill[p] = page; // no block yet
-        sm.clen[p] = 0;
-        sm.urows[p] = 0;
-    }
-    for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-        sm.bins[p] = 0;
-    if (threadIdx.x < 32)
-        sm.scal[threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t lo = a.probe_rows * g / G, hi = a.probe_rows * (g + 1) / G;
+    const uint64_t lo = (a.probe_rows * g / G) & ~15ull, hi = g + 1 == G ? a.probe_rows : (a.probe_rows * (g + 1) / G) & ~15ull;
     uint64_t pos = lo, unref_bytes = 0;
-    uint32_t gen = 0;
     bool counted = false; // this group is counted in groups_done
-    for (uint32_t wave = 0;; ++wave)
+    uint32_t * kept = a.group_state + (uint64_t)g * a.persist_words;
+    const bool resumed = vload(&a.ctl->started) != 0;
+    for (uint32_t i = threadIdx.x; i < a.persist_words; i += kENT)
+        sm.persist[i] = resumed ? __ldcg(kept + i) : (i < P1 ? page : 0u); // (fill = page: no block yet)
+    for (uint32_t p = tid; p < P1; p += kHNT)
+        sm.hf.bins[p] = 0;
+    if (threadIdx.x == 0)
+    {
+        sm.scal[kTurn] = 0;
+        sm.scal[kStop] = kTileDone;
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if (resumed)
+    {
+        pos = *reinterpret_cast<const uint64_t *>(sm.pscal + 2);
+        unref_bytes = *reinterpret_cast<const uint64_t *>(sm.pscal + 4);
+        counted = sm.pscal[1] != 0;
+    }
+    // (every group reads these before the launch's first barrier lets any
+    // group go on)
+    uint32_t gen = vload(&a.ctl->bar_gen), wave = (uint32_t)vload(&a.ctl->waves);
+    bool more = vload(&a.ctl->no_more_input) == 0;
+    unsigned long long t_probe = 0;
+    if (g == 0 && threadIdx.x == 0 && a.ctl->t_probe0)
+    {
+        t_probe = now_ns() - a.ctl->t_probe0; // the E before this launch
+        a.ctl->t_probe0 = 0;
+        a.ctl->ns_probe += t_probe;
+    }
+
+    // Steps of the launch: step k is rows [pos0 + k * stage_rows, ..), the
+    // half k & 1's.  A half's next step is copied in once its stage is free.
+    const uint64_t pos0 = pos;
+    auto step_row = [&](uint32_t k) -> uint64_t { return umin64(hi, pos0 + (uint64_t)k * a.stage_rows); };
+    auto step_rows = [&](uint32_t k) -> uint32_t { return (uint32_t)(step_row(k + 1) - step_row(k)); };
+    auto tma_ok = [&](uint32_t n) -> bool {
+        if (!a.use_tma || n == 0 || ((n * 8u) & 15u))
+            return false;
+        for (uint32_t c = 0; c < a.pin.n; ++c)
+            if ((n * a.pin.width[c]) & 15u)
+                return false;
+        return true;
+    };
+    uint32_t parity = 0;     // phase of bar[half] to wait for
+    uint32_t mine = half;    // this half's next step
+    bool in_flight = false;  // its copies are under way
+    uint8_t * stage = sm.hf.stage;
+    auto issue = [&] {
+        const uint32_t n = step_rows(mine);
+        in_flight = tma_ok(n);
+        if (!in_flight || tid != 0)
+            return;
+        const uint64_t r = step_row(mine);
+        uint32_t bytes = n * 8u;
+        for (uint32_t c = 0; c < a.pin.n; ++c)
+            bytes += n * a.pin.width[c];
+        fence_proxy_async_smem();
+        mbar_arrive_expect_tx(&bar[half], bytes);
+        bulk_copy_g2s(stage, a.pin.keys + r, n * 8u, &bar[half]);
+        for (uint32_t c = 0; c < a.pin.n; ++c)
+            bulk_copy_g2s(stage + a.stage_off[c], static_cast<const uint8_t *>(a.pin.col[c]) + r * a.pin.width[c], n * a.pin.width[c], &bar[half]);
+    };
+    if (more)
+        issue();
+    // before the launch ends, the copies in flight have to land
+    auto land = [&] {
+        if (in_flight)
+            (void)mbar_wait(&bar[half], parity, a.err, 1);
+        __syncthreads();
+    };
+    auto keep = [&] {
+        if (threadIdx.x == 0)
+        {
+            sm.pscal[1] = counted ? 1u : 0u;
+            *reinterpret_cast<uint64_t *>(sm.pscal + 2) = pos;
+            *reinterpret_cast<uint64_t *>(sm.pscal + 4) = unref_bytes;
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < a.persist_words; i += kENT)
+            kept[i] = sm.persist[i];
+    };
+    const uint32_t wave_steps = (uint32_t)(a.tile_rows / a.stage_rows);
+    for (uint32_t k_end = wave_steps; more; ++wave, k_end += wave_steps)
     {
         // -------- S: this wave's tile of the slice, then the refine trigger --------
         const uint64_t t0 = now_ns();
-        for (uint32_t p = threadIdx.x; p < P1; p += kENT)
-            sm.bins[p] = 0; // refines and E use the bins too
-        __syncthreads();
-        const uint64_t end = umin64(hi, pos + a.tile_rows);
-        while (pos < end)
+        const uint64_t end = step_row(k_end);
+        while (mine < k_end && step_rows(mine) != 0)
         {
-            const uint32_t n = (uint32_t)umin64(page, end - pos);
-            const int st = scatter_tile(a, sm, g, pos, n);
-            if (st == kTileFailed)
-                return;
-            if (st == kTileNoRoom)
+            const uint32_t n = step_rows(mine);
+            bool ok = true;
+            if (in_flight)
             {
-                // too few free blocks: the rest of the tile waits for the
-                // drain this forces after the wave
-                if (threadIdx.x == 0)
-                    atomicExch(&a.ctl->pool_low, 1);
+                ok = mbar_wait(&bar[half], parity, a.err, 1);
+                if (ok)
+                {
+                    parity ^= 1u;
+                    in_flight = false;
+                }
+            }
+            else
+            {
+                const uint64_t r = step_row(mine);
+                for (uint32_t i = tid; i < n; i += kHNT)
+                    reinterpret_cast<uint64_t *>(stage)[i] = a.pin.keys[r + i];
+                for (uint32_t c = 0; c < a.pin.n; ++c)
+                    for (uint32_t i = tid; i < n; i += kHNT)
+                        copy_elem(stage + a.stage_off[c], i, a.pin.col[c], r + i, a.pin.width[c]);
+                half_sync(half);
+            }
+            if (scatter_step(a, sm, g, half, mine, n, ok) != kTileDone)
                 break;
-            }
-            pos += n;
-            unref_bytes += (uint64_t)n * a.rb;
-            if (threadIdx.x == 0)
-            {
-                atomicAdd(&a.ctl->rows_scattered, (unsigned long long)n);
-                if (g == 0)
-                    a.ctl->tiles0 += 1;
-            }
+            half_sync(half); // the stage is free
+            mine += 2;
+            issue();
         }
+        __syncthreads(); // both halves' steps, and the chains' state
+        const uint32_t stop = sm.scal[kStop];
+        if (stop == kTileFailed)
+        {
+            land();
+            return;
+        }
+        // (a step without room ends the wave: the steps from it on were not
+        // taken, and wait for the drain this forces after the wave)
+        const uint64_t done = stop == kTileDone ? end : step_row(sm.scal[kStopStep]);
+        if (threadIdx.x == 0)
+        {
+            if (stop != kTileDone)
+                atomicExch(&a.ctl->pool_low, 1);
+            atomicAdd(&a.ctl->rows_scattered, (unsigned long long)(done - pos));
+            if (g == 0)
+                a.ctl->tiles0 += ceil_div(done - pos, a.stage_rows);
+        }
+        unref_bytes += (done - pos) * a.rb;
+        pos = done;
         if (pos >= hi && !counted)
         {
             counted = true;
@@ -1335,13 +1622,14 @@ __global__ void __launch_bounds__(kENT, 1) k_bep_engine(const __grid_constant__ 
             refine_down_to(a, sm, g, unref_bytes, 0); // stalled: everything it holds goes to the drain
         else if (unref_bytes >= a.unref_high)
             refine_down_to(a, sm, g, unref_bytes, a.unref_low);
-        if (g == 0 && threadIdx.x == 0)
-            a.ctl->ns_refine0 += now_ns() - t_ref;
         if (threadIdx.x == 0)
         {
-            const unsigned long long dt = now_ns() - t0;
+            const unsigned long long t = now_ns(), dt = t - t0;
             if (g == 0)
+            {
+                a.ctl->ns_refine0 += t - t_ref;
                 a.ctl->ns_shuffle += dt;
+            }
             atomicMax(&a.ctl->wave_s_max, dt);
         }
         if (wave == a.test_stall_wave && g == 0 && threadIdx.x == 0)
@@ -1353,27 +1641,35 @@ __global__ void __launch_bounds__(kENT, 1) k_bep_engine(const __grid_constant__ 
                 __nanosleep(1000);
         }
         // the last group to arrive records the peak and decides the E
-        if (!grid_sync(a, gen, WaveEnd{&a}))
+        if (!grid_sync(a, gen, WaveEnd{&a, false}))
+        {
+            land();
             return;
+        }
         const int ev = vload(&a.ctl->evict_now);
-        const bool more = vload(&a.ctl->more_input) != 0;
+        const bool left = vload(&a.ctl->no_more_input) == 0;
         if (ev)
-            if (!evict_phase(a, sm, gen, ev == 2))
-                return;
-        if (!more)
+        {
+            land();
+            keep();
+            return;
+        }
+        if (!left)
             break;
     }
-    // -------- end of the slice: refine every bucket that holds rows --------
+    if (more)
+        land();
+    // -------- end of the slices: refine every bucket that holds rows; the
+    // post-probe drain follows --------
     {
         const uint64_t t0 = now_ns();
         refine_down_to(a, sm, g, unref_bytes, 0);
         if (g == 0 && threadIdx.x == 0)
             a.ctl->ns_shuffle += now_ns() - t0;
     }
-    if (!grid_sync(a, gen, WaveEnd{&a}))
+    if (!grid_sync(a, gen, WaveEnd{&a, true}))
         return;
-    // -------- the post-probe drain: every leaf that holds rows --------
-    evict_phase(a, sm, gen, true);
+    keep();
 }
 
 __global__ void k_engine_init(uint32_t * __restrict__ free_stack, uint32_t * __restrict__ blk_state, uint32_t n_blocks, EngineCtl * ctl)
@@ -1426,14 +1722,10 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
     const uint64_t P1 = a.n_buckets, LB = 1ull << a.lb_log2;
     const uint64_t high_rows = a.unref_high / rb;
     // block rows: a power of two, 64..8192, about what one bucket of a group
-    // gathers before its group refines (so a refined block is mostly
-    // full), and whose rows fit 96 KiB of shared memory (the refine sorts a
-    // whole block there)
+    // gathers before its group refines (so a refined block is mostly full)
     uint32_t page_log2 = 6;
     while (page_log2 < 13 && (2ull << page_log2) <= std::max<uint64_t>(high_rows / P1, 1))
         ++page_log2;
-    while (page_log2 > 6 && ((uint64_t)rb << page_log2) > (96u << 10))
-        --page_log2;
     a.page_log2 = page_log2;
     const uint64_t page = 1ull << page_log2;
     uint64_t off = page * 8;
@@ -1443,13 +1735,42 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
         off += page * in.probe.width[c];
     }
     a.block_bytes = (off + 255) & ~255ull;
-    a.smem_cells = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>((page * rb) / sizeof(Cell), 2048));
     // input rows a group scatters between two looks at the global leaf
-    // count: half its unrefined high water, within [256, 64K], so one wave
-    // overshoots the marks by little
-    a.tile_rows = std::min<uint64_t>(std::min<uint64_t>(page * 16, 65536), std::max<uint64_t>(256, (high_rows / 2) & ~255ull));
-    const uint64_t slice = ceil_div(std::max<uint64_t>(in.probe_rows, 1), G);
-    a.waves = (uint32_t)std::max<uint64_t>(1, ceil_div(slice, a.tile_rows));
+    // count: half its unrefined high water, at least 256 and at most 16
+    // blocks (4096 to 64K rows), so one wave overshoots the marks by little;
+    // in steps of at most 4096 rows, at least two a wave (one for each half
+    // of the CTA), both in shared memory beside the rest
+    a.tile_rows = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(page * 16, 4096), 65536), std::max<uint64_t>(256, (high_rows / 2) & ~255ull));
+    auto smem_of = [&](uint32_t rows) -> uint64_t {
+        auto room = [](uint64_t bytes) { return (bytes + 15) & ~15ull; };
+        a.stage_rows = rows;
+        uint64_t at = 8ull * rows;
+        for (uint32_t c = 0; c < in.probe.n; ++c)
+        {
+            a.stage_off[c] = (uint32_t)at;
+            at += ((uint64_t)rows * in.probe.width[c] + 15) & ~15ull;
+        }
+        a.stage_bytes = (uint32_t)((at + 127) & ~127ull);
+        a.fresh_words = (uint32_t)(rows / page + P1 + 1);
+        a.bcache_words = a.fresh_words + 2 * kRefill + 2;
+        a.persist_words = (uint32_t)((4 * P1 + kPersistScal + a.bcache_words + 1) & ~1ull);
+        a.half_bytes = (uint32_t)(
+            a.stage_bytes + room(4ull * rows) + 3 * room(4 * P1) + 2 * room(4 * (P1 + 1)) + room(4ull * a.fresh_words) + room(kHNT / 8) + room(16));
+        return 2ull * a.half_bytes + room(4 * LB) + room(32 * 4) + room(4ull * a.persist_words);
+    };
+    size_t smem = 0;
+    uint32_t step = 64;
+    for (uint32_t rows = 128; rows <= kETile && 2 * rows <= a.tile_rows; rows *= 2)
+        if (smem_of(rows) + 1024 <= (size_t)ctx->smem_optin)
+            step = rows;
+    smem = smem_of(step);
+    if (smem + 1024 > (size_t)ctx->smem_optin)
+        throw Error(PHJ_ERR_UNSUPPORTED, "PHJ (BEP): the device budget engine's shared memory does not fit this configuration");
+    a.tile_rows = a.tile_rows / step * step;
+    a.use_tma = (reinterpret_cast<uintptr_t>(in.probe.keys) & 15u) == 0;
+    for (uint32_t c = 0; c < in.probe.n; ++c)
+        a.use_tma = a.use_tma && (reinterpret_cast<uintptr_t>(in.probe.col[c]) & 15u) == 0;
+    const uint64_t slice = ceil_div(std::max<uint64_t>(in.probe_rows, 1), G) + 16; // (slices start on multiples of 16 rows)
     // pool, in blocks: a group's unrefined chains hold at most its high
     // water plus a tile in full blocks and one part block per bucket; the
     // refined blocks hold the leaf rows (up to the leaf high water plus one
@@ -1471,8 +1792,6 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
     a.blk_state = s.get<uint32_t>(a.n_blocks);
     a.blk_rows = s.get<uint32_t>(a.n_blocks);
     a.blk_rem = s.get<uint32_t>(a.n_blocks);
-    a.blk_lfirst = s.get<uint32_t>(a.n_blocks);
-    a.blk_llast = s.get<uint32_t>(a.n_blocks);
     a.blk_bucket = s.get<uint32_t>(a.n_blocks);
     a.blk_c0 = s.get<unsigned long long>(a.n_blocks);
     a.chain = s.get<uint32_t>((uint64_t)G * P1 * a.maxb);
@@ -1490,6 +1809,7 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
     a.out_cap = out->cap;
     a.wait_limit_ns = (uint64_t)ctx->wait_limit_ms * 1000000ull;
     a.test_stall_wave = ctx->test_engine_stall_wave >= 0 ? (uint32_t)ctx->test_engine_stall_wave : kNone;
+    a.group_state = s.get<uint32_t>((uint64_t)G * a.persist_words);
     a.ctl = s.get<EngineCtl>(1);
     a.err = ctx->d_err;
     PHJ_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(EngineCtl), ctx->stream));
@@ -1498,31 +1818,122 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
     k_engine_init<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(a.n_blocks, 256), (uint64_t)ctx->num_sms * 8)), 256, 0,
                     ctx->stream>>>(a.free_stack, a.blk_state, a.n_blocks, a.ctl);
     PHJ_LAUNCHED(ctx, "bep_engine_init");
-    // shared memory: stage, permutation, bins, the per-bucket state
-    const uint64_t stage = std::max<uint64_t>(page * rb, (uint64_t)a.smem_cells * sizeof(Cell));
-    const uint64_t nbins = std::max(std::max(P1, LB), page);
-    const size_t smem = ((stage + 15) & ~15ull) + 2 * ((page * 2 + 15) & ~15ull) + ((nbins * 4 + 15) & ~15ull) + 5 * ((P1 * 4 + 15) & ~15ull) +
-                        ((LB * 4 + 15) & ~15ull) + (((2 * P1 + 2 * kRefill) * 4 + 15) & ~15ull) + (kENT / 32) * 4 + 32 * 4;
-    if (smem + 1024 > (size_t)ctx->smem_optin)
-        throw Error(PHJ_ERR_UNSUPPORTED, "PHJ (BEP): the device budget engine's shared memory does not fit this configuration");
-    PHJ_CUDA(cudaFuncSetAttribute(k_bep_engine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PHJ_CUDA(cudaFuncSetAttribute(k_bep_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bep_engine, kENT, smem));
+    PHJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bep_scatter, kENT, smem));
     if (per_sm < 1)
         throw Error(PHJ_ERR_UNSUPPORTED, "PHJ (BEP): the device budget engine does not fit on an SM");
     if (std::getenv("PHJ_DEBUG"))
-        std::fprintf(stderr, "[phj] bep_engine: %u groups, page %llu rows (%llu B), %u blocks (%.2f GB), maxb %u, waves %u, tile %llu, smem %zu\n", G,
-                     (unsigned long long)page, (unsigned long long)a.block_bytes, a.n_blocks, a.n_blocks * (double)a.block_bytes / 1e9, a.maxb,
-                     a.waves, (unsigned long long)a.tile_rows, smem);
+        std::fprintf(stderr, "[phj] bep_engine: %u groups, page %llu rows (%llu B), %u blocks (%.2f GB), maxb %u, wave %llu rows in steps of %u, smem %zu\n",
+                     G, (unsigned long long)page, (unsigned long long)a.block_bytes, a.n_blocks, a.n_blocks * (double)a.block_bytes / 1e9, a.maxb,
+                     (unsigned long long)a.tile_rows, a.stage_rows, smem);
+    // the leaf builds (bep.cu), from the claims' queue
+    BepLeaves bl{};
+    bl.state = a.state;
+    bl.leaf_off = a.leaf_off;
+    bl.build_keys = a.bpart.keys;
+    bl.meta = a.meta;
+    bl.cells = a.cells;
+    bl.next = a.next;
+    bl.leaf_bits = a.total_bits;
+    bl.n_leaves = a.n_leaves;
+    bl.smem_cells = (uint32_t)std::min<uint64_t>(
+        a.ulog >= 0 ? (1ull << a.ulog) : bit_ceil64(2ull * std::max<uint32_t>(in.lt->max_rows, 1)), 8192);
+    bl.wait_limit_ns = a.wait_limit_ns;
+    bl.ctr = s.get<unsigned long long>(4);
+    PHJ_CUDA(cudaMemsetAsync(bl.ctr, 0, 4 * sizeof(unsigned long long), ctx->stream));
+    bl.queue = a.build_queue;
+    bl.queue_len = &a.ctl->build_n; // build_n, build_next
+    bl.any_dup = &a.ctl->any_dup;
+    // the probes: one gather a build row where the payloads allow it
+    ProbeArgs pa{};
+    pa.build = in.build;
+    pa.build.keys = nullptr;
+    pack_build_payloads(ctx, s, pa, in.build_rows);
+    PackSpec pk{};
+    int gather = -1;
+    const void * gathered = nullptr;
+    if (pa.packed)
     {
-        KTimer kt(ctx, "bep_engine", in.probe_rows, 0);
-        void * args[] = {&a};
-        PHJ_CUDA(cudaLaunchCooperativeKernel((const void *)k_bep_engine, dim3(G), dim3(kENT), args, smem, ctx->stream));
-        PHJ_LAUNCHED(ctx, "bep_engine");
+        gather = 16;
+        gathered = pa.packed;
+        for (uint32_t c = 0; c < in.build.n; ++c)
+            pk.off[c] = pa.packed_off[c];
     }
+    else if (in.build.n == 0)
+        gather = 0;
+    else if (in.build.n == 1 && (in.build.width[0] == 4 || in.build.width[0] == 8))
+    {
+        gather = (int)in.build.width[0];
+        gathered = in.build.col[0];
+    }
+    for (uint32_t c = 0; c < in.probe.n; ++c)
+        if (in.probe.width[c] > 8)
+            gather = -1;
+    void (*probe)(EngineArgs, const void *, PackSpec) = nullptr;
+    auto pick = [&](auto uniform) {
+        constexpr bool kU = decltype(uniform)::value;
+        switch (gather)
+        {
+            case 16: return k_bep_probe<16, kU>;
+            case 8: return k_bep_probe<8, kU>;
+            case 4: return k_bep_probe<4, kU>;
+            default: return k_bep_probe<0, kU>;
+        }
+    };
+    if (gather >= 0)
+        probe = a.ulog >= 0 ? pick(std::true_type{}) : pick(std::false_type{});
+    const unsigned sms = (unsigned)ctx->num_sms;
+    const unsigned block_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(std::max<uint64_t>(a.n_blocks, a.n_leaves), 512), sms * 4));
     EngineCtl c{};
     int e = 0;
-    read_small(ctx, {{&c, a.ctl, sizeof(c)}, {&e, ctx->d_err, sizeof(e)}});
+    int rec = -1;
+    {
+        KTimer kt(ctx, "bep_engine", in.probe_rows, 0);
+        rec = kt.idx;
+        unsigned int waves = 0;
+        for (uint32_t round = 0;; ++round)
+        {
+            // S and E in turn; the first E's read-back says whether more
+            // than the final drain is to come, then pairs go out in growing
+            // numbers (a pair past the end costs its launches)
+            const uint32_t pairs = round < 2 ? 1u : std::min<uint32_t>(1u << (round - 1), 8u);
+            for (uint32_t k = 0; k < pairs; ++k)
+            {
+                void * args[] = {&a};
+                PHJ_CUDA(cudaLaunchCooperativeKernel((const void *)k_bep_scatter, dim3(G), dim3(kENT), args, smem, ctx->stream));
+                PHJ_LAUNCHED(ctx, "bep_scatter");
+                k_bep_range<<<1, kENT, 0, ctx->stream>>>(a);
+                PHJ_LAUNCHED(ctx, "bep_range");
+                k_bep_claim<<<block_grid, 512, 0, ctx->stream>>>(a);
+                PHJ_LAUNCHED(ctx, "bep_claim");
+                k_bep_offsets<<<1, kENT, 0, ctx->stream>>>(a);
+                PHJ_LAUNCHED(ctx, "bep_offsets");
+                bep_build_queue(ctx, bl);
+                k_bep_list<<<block_grid, 512, 0, ctx->stream>>>(a);
+                PHJ_LAUNCHED(ctx, "bep_list");
+                if (probe)
+                {
+                    probe<<<sms * 3, kBPNT, 0, ctx->stream>>>(a, gathered, pk);
+                    PHJ_LAUNCHED(ctx, "bep_probe");
+                }
+                k_bep_probe_chains<<<sms * 4, kBPNT, 0, ctx->stream>>>(a, probe ? 1 : 0);
+                PHJ_LAUNCHED(ctx, "bep_probe_chains");
+            }
+            k_bep_stamp<<<1, 1, 0, ctx->stream>>>(a.ctl);
+            PHJ_LAUNCHED(ctx, "bep_stamp");
+            read_small(ctx, {{&c, a.ctl, sizeof(c)}, {&e, ctx->d_err, sizeof(e)}});
+            if (c.finished || e != 0 || c.abort)
+                break;
+            if (c.waves == waves)
+                throw Error(PHJ_ERR_CUDA, "internal: the device budget engine stands still");
+            waves = c.waves;
+        }
+    }
+    unsigned long long built[2] = {0, 0}; // tables built, waits on a BUILDING leaf
+    read_small(ctx, {{built, bl.ctr, sizeof(built)}});
+    if (e == 0)
+        e = c.abort;
     // the launch's algorithmic bytes, as the join's: every probe row read
     // once, every output row written once
     {
@@ -1531,19 +1942,15 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
             orow += in.build.width[c2];
         for (uint32_t c2 = 0; c2 < in.probe.n; ++c2)
             orow += in.probe.width[c2];
-        for (size_t i = ctx->records.size(); i-- > 0;)
-            if (ctx->records[i].name == "bep_engine")
-            {
-                ctx->records[i].bytes = in.probe_rows * rb + std::min<uint64_t>(c.out_rows, a.out_cap) * orow;
-                break;
-            }
+        if (rec >= 0)
+            ctx->records[rec].bytes = in.probe_rows * rb + std::min<uint64_t>(c.out_rows, a.out_cap) * orow;
     }
     res.err = e;
     res.out_rows = c.out_rows;
     res.evictions = c.evictions;
     res.refinements = c.refinements;
-    res.skip_retries = c.skip_retries;
-    res.tables_built = c.tables_built;
+    res.skip_retries = c.skip_retries + built[1];
+    res.tables_built = built[0];
     res.evict_phases = c.evict_phases;
     res.peak_bytes = c.peak_leaf_rows * rb;
     res.ms_shuffle = c.ns_shuffle * 1e-6;

@@ -427,6 +427,8 @@ struct BepLeaves
 // The batch's leaves are flagged in b.touched by its first radix pass
 // (ctx->leaf_mark) before this runs.
 bool bep_build_touched(phj_ctx * ctx, const BepLeaves & b);
+// The builds alone, of the leaves in b.queue (b.queue_len[0] of them, [1] zero).
+void bep_build_queue(phj_ctx * ctx, const BepLeaves & b);
 void set_bep_smem_limits(int smem_optin);
 
 // ----- bep_engine.cu ------------------------------------------------------------------
@@ -438,6 +440,7 @@ struct BepEngineInput
     Cols probe; // probe side in input order
     uint64_t probe_rows;
     Cols build; // leaf-partitioned build side (keys and payloads)
+    uint64_t build_rows;
     const LeafTables * lt; // lazily built tables (lt->state set)
     const uint32_t * leaf_off;
     uint32_t b1, total_bits;

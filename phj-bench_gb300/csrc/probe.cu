@@ -27,6 +27,7 @@
 //                    row counter, then the projection from shared memory;
 //                    the output is sized by the probe rows beforehand.
 #include "internal.h"
+#include "list.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -781,41 +782,6 @@ __global__ void __launch_bounds__(kPNT, 3) k_probe_fused(const __grid_constant__
             __syncwarp(); // the stage is refilled by the next half
         }
         chunk = (uint32_t)__shfl_sync(0xffffffffu, tn, 0);
-    }
-}
-
-// Four values a lane of a probe payload column of at most 8 bytes, in 64-bit
-// registers: rows row0 + idx[u].
-__device__ __forceinline__ void load_list(uint64_t (&v)[4], const void * src, uint32_t width, uint64_t row0, const uint32_t (&idx)[4], uint32_t one)
-{
-    switch (width)
-    {
-#define PHJ_LOAD_LIST(W, T)                                                                                                                          \
-    case W:                                                                                                                                          \
-        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) v[u] = __ldcs(static_cast<const T *>(src) + row0 + idx[u]);                 \
-        break;
-        PHJ_LOAD_LIST(1, uint8_t)
-        PHJ_LOAD_LIST(2, uint16_t)
-        PHJ_LOAD_LIST(4, uint32_t)
-        default: PHJ_LOAD_LIST(8, uint64_t)
-#undef PHJ_LOAD_LIST
-    }
-}
-
-// Four values a lane to output rows out + 32 * u of a column.
-__device__ __forceinline__ void store_list(const uint64_t (&v)[4], void * dst, uint32_t width, uint64_t out, uint32_t one)
-{
-    switch (width)
-    {
-#define PHJ_STORE_LIST(W, T)                                                                                                                         \
-    case W:                                                                                                                                          \
-        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) __stcs(static_cast<T *>(dst) + out + 32 * u, (T)v[u]);                      \
-        break;
-        PHJ_STORE_LIST(1, uint8_t)
-        PHJ_STORE_LIST(2, uint16_t)
-        PHJ_STORE_LIST(4, uint32_t)
-        default: PHJ_STORE_LIST(8, uint64_t)
-#undef PHJ_STORE_LIST
     }
 }
 
