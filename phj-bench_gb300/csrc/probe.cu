@@ -983,7 +983,11 @@ __global__ void __launch_bounds__(kPNT, 3) k_probe_inline(const uint64_t * __res
 // binary search of the offsets.  Every output row costs the same whatever
 // the match counts, the stores of a step are consecutive, and every step is
 // full (expanding 32 probe rows at a time left most slots of a step empty
-// at two matches a row: 4.9 ms against 3.6 ms for 32M x 128M).
+// at two matches a row: 4.9 ms against 3.6 ms for 32M x 128M).  Bound by the
+// latency of a step's columns and by L1, where consecutive output rows of a
+// key find each other's sectors: steps of 64 or 256 rows took 3.7 and 5.9 ms
+// against 3.2, loads without an L1 line 4.3, and build rows packed into one
+// 32-byte gather 3.5.
 template <bool kFlat>
 __global__ void __launch_bounds__(kPNT, kProjMinBlocks) k_probe_project_window(const __grid_constant__ ProbeArgs a,
                                                                          const __grid_constant__ ProjCols pc, const uint32_t * __restrict__ heads,
@@ -1004,27 +1008,37 @@ __global__ void __launch_bounds__(kPNT, kProjMinBlocks) k_probe_project_window(c
         // of the next row, so the search lands on the matching one
         uint32_t running = 0;
 #pragma unroll 1
-        for (int k = 0; k < kPRPT; ++k)
+        for (int k0 = 0; k0 < kPRPT; k0 += 4)
         {
-            const uint64_t row = chunk * kWChunk + (uint64_t)k * 32 + lane;
-            uint32_t first = 0, cnt = 0;
-            if (row < a.probe_rows)
-            {
-                first = __ldcs(heads + row);
-                if (first != kNoMatch)
-                    cnt = __ldcs(a.row_cnt + row);
-            }
-            uint32_t incl = cnt;
+            uint32_t first[4], cnt[4];
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1)
+            for (int k = 0; k < 4; ++k)
             {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= (uint32_t)d)
-                    incl += y;
+                const uint64_t row = chunk * kWChunk + (uint64_t)(k0 + k) * 32 + lane;
+                first[k] = kNoMatch;
+                cnt[k] = 0;
+                if (row < a.probe_rows)
+                {
+                    first[k] = __ldcs(heads + row);
+                    cnt[k] = __ldcs(a.row_cnt + row);
+                }
             }
-            st[k * 32 + lane] = running + incl - cnt;
-            sf[k * 32 + lane] = first;
-            running += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                const uint32_t own = first[k] != kNoMatch ? cnt[k] : 0u;
+                uint32_t incl = own;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1)
+                {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= (uint32_t)d)
+                        incl += y;
+                }
+                st[(k0 + k) * 32 + lane] = running + incl - own;
+                sf[(k0 + k) * 32 + lane] = first[k];
+                running += __shfl_sync(0xffffffffu, incl, 31);
+            }
         }
         __syncwarp();
         const uint32_t T = running;
@@ -1047,11 +1061,11 @@ __global__ void __launch_bounds__(kPNT, kProjMinBlocks) k_probe_project_window(c
                 else
                     brow[u] = sf[L] + (j - st[L]);
                 prow[u] = (uint32_t)(chunk * kWChunk + L);
-                rel[u] = j;
+                rel[u] = u * 32;
                 if (j < T && base + j < out_cap)
                     one |= 1u << u;
             }
-            project_all(pc, brow, prow, base, rel, one);
+            project_all(pc, brow, prow, base + t + lane, rel, one);
         }
         __syncwarp();
     }
