@@ -976,7 +976,9 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
 
         // -------- BUILD: per-leaf tables (src/PHJ.cpp:260-282) --------
         lt.next = s.get<uint64_t>(B.rows);
-        build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows);
+        // (grouping needs a place for the payloads: the partition's temporary)
+        const Cols * group_dst = btmp.keys != bpart.keys ? &btmp : nullptr;
+        build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows, group_dst);
         if (lt.estimated)
         {
             // the one-pass probe goes ahead; when the tables turn out not
@@ -1000,7 +1002,7 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
             {
                 lt = LeafTables{};
                 lt.next = s.get<uint64_t>(B.rows);
-                build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt);
+                build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, 0, group_dst);
             }
             else
                 lt.any_dup = found.flags & kLeafRepeats;
@@ -1469,7 +1471,7 @@ static void run_phj_pure_host(phj_ctx * ctx, const phj_block_stream & hb, const 
     PHJ_CUDA(cudaEventRecord(ev[1], S));
     LeafTables lt;
     lt.next = s.get<uint64_t>(B_rows);
-    build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt);
+    build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, 0, &btmp);
     const bool grouped = group_leaf_duplicates(ctx, bpart, btmp, leaf_off, n_leaves, lt);
     PHJ_CUDA(cudaEventRecord(ev[2], S));
 

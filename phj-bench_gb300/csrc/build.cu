@@ -50,18 +50,49 @@ __device__ __forceinline__ uint32_t log2u(uint64_t x)
     return 63u - (uint32_t)__clzll((long long)x);
 }
 
+// Position of `key` in a finished table (the key is present).
+__device__ __forceinline__ uint32_t cell_of(const Cell * tab, uint64_t cap, uint64_t h, uint64_t key)
+{
+    uint64_t pos = probe_start(h, cap);
+    for (uint64_t step = 0; step < cap; ++step)
+    {
+        if (tab[pos].key == key && ref_valid(tab[pos].ref))
+            return (uint32_t)pos;
+        pos = (pos + 1) & (cap - 1);
+    }
+    return 0; // unreachable: every row's key was inserted
+}
+
+// The payloads of row `si`, to row `di`.
+__device__ __forceinline__ void copy_row(const Cols & src, uint64_t si, const Cols & dst, uint64_t di)
+{
+    for (uint32_t c = 0; c < src.n; ++c)
+        copy_elem(dst.col[c], di, src.col[c], si, src.width[c]);
+}
+
 // One CTA per leaf.  Tables are either uniform (every leaf 2^ulog cells at
 // leaf << ulog, ulog >= 0) or sized per leaf through table_off (ulog < 0).
 // The RowRefCell of a build row is {0, row}: block 0 is the whole
 // leaf-partitioned build side, row its index there.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_build_leaf(const uint64_t * __restrict__ keys, const uint32_t * __restrict__ leaf_off,
+// With kGroup (every table in shared memory) a leaf whose keys repeat is
+// grouped while its table is at hand: the payloads of one key's rows become
+// contiguous in `dst` and the key's cell holds {row count, first row}
+// (block_no, always 0 for the single partitioned build block, carries the
+// count).  Nothing follows a chain then, and none is written.  33.5M rows of
+// 27 bytes in 131,072 leaves, beside the probe side's pass: 1,082 us, against
+// 566 for the tables and 820 for a second kernel that found every row's cell
+// again in memory (the join 7,260 -> 6,990).  Bound by the latency of a
+// leaf's steps.
+template <int NT, bool kGroup>
+__global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols part, const __grid_constant__ Cols dst, const uint32_t * __restrict__ leaf_off,
                                                          const uint32_t * __restrict__ table_off, int ulog, uint32_t smem_cells,
                                                          Cell * __restrict__ cells, uint64_t * __restrict__ next, LeafMeta * __restrict__ meta,
                                                          int * __restrict__ any_dup)
 {
-    extern __shared__ __align__(16) Cell sh_cells[];
+    extern __shared__ __align__(16) Cell sh_cells[]; // | (kGroup) cnt[smem_cells] | place of each row[smem_cells]
     __shared__ int dup;
+    __shared__ uint32_t warp_sums[NT / 32];
+    const uint64_t * keys = part.keys;
     const uint32_t l = blockIdx.x;
     const uint32_t r0 = leaf_off[l], r = leaf_off[l + 1] - r0;
     const uint64_t t0 = ulog >= 0 ? ((uint64_t)l << ulog) : table_off[l];
@@ -100,12 +131,51 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const uint64_t * __restrict__
         const uint64_t h = int_hash64(k);
         const uint64_t ref = make_ref(0, r0 + i);
         const uint64_t prev = in_smem ? table_insert<true>(tab, cap, h, k, ref) : table_insert<false>(tab, cap, h, k, ref);
-        next[r0 + i] = prev;
+        if constexpr (!kGroup)
+            next[r0 + i] = prev;
         my_dup |= ref_valid(prev);
     }
     if (__any_sync(0xffffffffu, my_dup) && (threadIdx.x & 31) == 0)
         dup = 1;
     __syncthreads();
+    if constexpr (kGroup)
+        if (dup)
+        {
+            uint32_t * cnt = reinterpret_cast<uint32_t *>(sh_cells + smem_cells); // rows of each cell, then its first
+            uint32_t * place = cnt + smem_cells;                                 // each row's cell | its rank in the cell << 13
+            static_assert(kSmemCellsMax <= 1u << 13, "a cell and a rank in 32 bits");
+            const uint32_t c_n = (uint32_t)cap;
+            for (uint32_t i = threadIdx.x; i < c_n; i += NT)
+                cnt[i] = 0;
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < r; i += NT)
+            {
+                const uint64_t k = keys[r0 + i];
+                const uint32_t c = cell_of(tab, cap, int_hash64(k), k);
+                place[i] = c | atomicAdd(&cnt[c], 1u) << 13;
+            }
+            __syncthreads();
+            // one block scan: thread t owns cells [t * per, (t + 1) * per)
+            const uint32_t per = (c_n + NT - 1) / NT, c0 = threadIdx.x * per;
+            uint32_t local = 0;
+            for (uint32_t j = 0; j < per; ++j)
+                if (c0 + j < c_n)
+                    local += cnt[c0 + j];
+            uint32_t tot;
+            uint32_t run = block_excl_scan<NT>(local, warp_sums, &tot);
+            for (uint32_t j = 0; j < per; ++j)
+                if (c0 + j < c_n)
+                {
+                    const uint32_t v = cnt[c0 + j];
+                    cnt[c0 + j] = run;
+                    if (v)
+                        tab[c0 + j].ref = make_ref(v, r0 + run);
+                    run += v;
+                }
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < r; i += NT)
+                copy_row(part, r0 + i, dst, (uint64_t)r0 + cnt[place[i] & (kSmemCellsMax - 1u)] + (place[i] >> 13));
+        }
     if (in_smem)
     {
         ulonglong2 * dst = reinterpret_cast<ulonglong2 *>(cells + t0);
@@ -197,31 +267,13 @@ __global__ void __launch_bounds__(NT) k_build_inline(const __grid_constant__ Col
 }
 
 // ---- grouped duplicates (PHJ-PURE with repeated build keys) ----------------
-// Position of `key` in a finished table (the key is present).
-__device__ __forceinline__ uint32_t cell_of(const Cell * tab, uint64_t cap, uint64_t h, uint64_t key)
-{
-    uint64_t pos = probe_start(h, cap);
-    for (uint64_t step = 0; step < cap; ++step)
-    {
-        if (tab[pos].key == key && ref_valid(tab[pos].ref))
-            return (uint32_t)pos;
-        pos = (pos + 1) & (cap - 1);
-    }
-    return 0; // unreachable: every row's key was inserted
-}
-
-__device__ __forceinline__ void copy_row(const Cols & src, uint64_t si, const Cols & dst, uint64_t di)
-{
-    for (uint32_t c = 0; c < src.n; ++c)
-        copy_elem(dst.col[c], di, src.col[c], si, src.width[c]);
-}
-
 // One CTA per leaf.  The payloads of one key's rows become contiguous in
 // `dst`; the key's cell then holds {row count, first row} (block_no, which is
 // always 0 for the single partitioned build block, carries the count).
 // Leaves without repeated keys are copied unchanged.  A grouped leaf is read
 // through its cells only, so neither keys nor a next-chain are written.
-// Bound by the latency of a leaf's steps (a row's cell, its place, its
+// For builds that did not group (LeafTables::groups): at most 11 radix bits
+// (no second set of columns at hand), or tables built in place.  Bound by the latency of a leaf's steps (a row's cell, its place, its
 // payloads).  33.5M rows of 27 bytes in 131,072 leaves, beside the probe
 // side's pass: 946 us with keys and next-chain, 820 without.
 __global__ void __launch_bounds__(kBuildNT) k_group_leaf(const __grid_constant__ Cols src, const __grid_constant__ Cols dst,
@@ -358,6 +410,18 @@ __global__ void k_chj_insert(const uint64_t * __restrict__ keys, uint64_t n, uin
         }
     }
 }
+
+// The leaves without repeated keys of a build that grouped the others: their
+// payloads in the same order, a warp per leaf.
+__global__ void k_copy_leaves(const __grid_constant__ Cols src, const __grid_constant__ Cols dst, const uint32_t * __restrict__ leaf_off, uint32_t n_leaves,
+                              const LeafMeta * __restrict__ meta)
+{
+    const uint32_t l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (l >= n_leaves || meta[l].dup)
+        return;
+    for (uint32_t i = leaf_off[l] + (threadIdx.x & 31); i < leaf_off[l + 1]; i += 32)
+        copy_row(src, i, dst, i);
+}
 } // namespace
 
 // Rows of the largest leaf, with a margin of six standard deviations of a
@@ -407,8 +471,9 @@ void set_build_smem_limits(int smem_optin)
     PHJ_CUDA(cudaFuncSetAttribute(k_build_inline<kBuildNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
     PHJ_CUDA(cudaFuncSetAttribute(k_build_inline<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
     const size_t need = (size_t)kSmemCellsMax * sizeof(Cell);
-    PHJ_CUDA(cudaFuncSetAttribute(k_build_leaf<kBuildNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(need, (size_t)smem_optin - 1024)));
-    PHJ_CUDA(cudaFuncSetAttribute(k_build_leaf<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(need, (size_t)smem_optin - 1024)));
+    for (const auto kernel : {k_build_leaf<kBuildNT, false>, k_build_leaf<1024, false>, k_build_leaf<kBuildNT, true>, k_build_leaf<1024, true>})
+        PHJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)std::min<size_t>(need + need / 2, (size_t)smem_optin - 1024)));
     PHJ_CUDA(cudaFuncSetAttribute(k_group_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::min<size_t>((size_t)kSmemCellsMax * 12, (size_t)smem_optin - 1024)));
 }
@@ -419,6 +484,12 @@ bool group_leaf_duplicates(phj_ctx * ctx, const Cols & src, const Cols & dst, co
     if (!lt.any_dup || max_cap > kSmemCellsMax || lt.state)
         return false;
     KTimer kt(ctx, "group_leaf", 0, 0);
+    if (lt.groups)
+    {
+        k_copy_leaves<<<(unsigned)ceil_div(n_leaves, 8), 256, 0, ctx->stream>>>(src, dst, leaf_off, n_leaves, lt.meta);
+        PHJ_LAUNCHED(ctx, "copy_leaves");
+        return true;
+    }
     k_group_leaf<<<n_leaves, kBuildNT, (size_t)max_cap * 12, ctx->stream>>>(src, dst, leaf_off, lt.meta, lt.cells);
     PHJ_LAUNCHED(ctx, "group_leaf");
     return true;
@@ -440,7 +511,7 @@ __global__ void k_leaf_plan(const uint32_t * __restrict__ leaf_off, const uint32
 }
 
 void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, const uint32_t * leaf_off, uint32_t n_leaves, LeafTables & lt,
-                       bool lazy, uint64_t estimate_rows)
+                       bool lazy, uint64_t estimate_rows, const Cols * group_dst)
 {
     uint32_t * table_off = nullptr;
     uint32_t * small = s.get<uint32_t>(4); // [0] max rows, [1] flags (kLeafRepeats, kLeafOverflow)
@@ -499,9 +570,12 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
     {
         KTimer kt(ctx, "build_leaf_tables", 0, 0);
         // leaves of more than 1024 rows get 1024 threads
-        auto kb = lt.max_rows > 1024 ? k_build_leaf<1024> : k_build_leaf<kBuildNT>;
-        kb<<<n_leaves, lt.max_rows > 1024 ? 1024 : kBuildNT, (size_t)smem_cells * sizeof(Cell), ctx->stream>>>(build_part.keys, leaf_off, table_off, lt.uniform_log2cap,
-                                                                                            smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
+        const bool large = lt.max_rows > 1024;
+        lt.groups = group_dst && smem_cells && smem_cells == max_cap;
+        const auto kb = lt.groups ? (large ? k_build_leaf<1024, true> : k_build_leaf<kBuildNT, true>)
+                                  : (large ? k_build_leaf<1024, false> : k_build_leaf<kBuildNT, false>);
+        kb<<<n_leaves, large ? 1024 : kBuildNT, (size_t)smem_cells * (lt.groups ? sizeof(Cell) + 8 : sizeof(Cell)), ctx->stream>>>(
+            build_part, group_dst ? *group_dst : Cols{}, leaf_off, table_off, lt.uniform_log2cap, smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
         PHJ_LAUNCHED(ctx, "build_leaf");
     }
     lt.any_dup = 0; // unknown until the flags are read

@@ -321,6 +321,7 @@ struct LeafTables
     int uniform_log2cap = -1; // >= 0: every leaf table has 2^this cells at leaf << this
     uint32_t * state = nullptr; // lazy build (PHJ/BEP): per leaf NOT_BUILT / BUILDING / BUILT
     int * flags = nullptr;      // device: kLeafRepeats, kLeafOverflow
+    bool groups = false;        // leaves whose keys repeat were grouped by the build
     bool estimated = false;     // sized by estimate: any_dup is unknown until the flags are read
 };
 
@@ -349,9 +350,11 @@ struct InlineTables
 // `lazy` only the layout is planned; the probe builds each table on first
 // use (PHJ/BEP).  With `estimate_rows` (the build rows) the tables are sized
 // by estimate where that costs no more than the usual sizes, without a host
-// round trip: lt.flags then says whether the tables can be used.
+// round trip: lt.flags then says whether the tables can be used.  With
+// `group_dst` (payload columns) the build may group leaves whose keys repeat
+// (lt.groups): they are then followed through group_leaf_duplicates only.
 void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, const uint32_t * leaf_off, uint32_t n_leaves,
-                       LeafTables & lt, bool lazy = false, uint64_t estimate_rows = 0);
+                       LeafTables & lt, bool lazy = false, uint64_t estimate_rows = 0, const Cols * group_dst = nullptr);
 // Inline tables over leaf-partitioned build rows, sized by estimate: false
 // (nothing done) when the leaves are too small or too large for them.
 // *bad (device, zero before) receives what the build found.
