@@ -57,11 +57,11 @@
 // takes its free blocks from a cache of its own, refilled from the pool's
 // stack a batch at a time.
 //
-// Measured (64M x 512M rows, Zipf keys, 32 MiB a group): 14.8 ms (S 5.9,
-// claims and builds 1.4, probes 6.7 ms); one persistent grid of 1024-thread
+// Measured (64M x 512M rows, Zipf keys, 32 MiB a group): 14.4 ms (S 5.7,
+// claims and builds 1.4, probes 6.5 ms); one persistent grid of 1024-thread
 // CTAs for both steps, whose refines sorted every block by leaf, took 28.1 ms
-// (S 11.6, claims and builds 3.9, probes 12.3).  8M x 64M rows: 2.85 ms
-// (S 1.1, 0.35, 0.88) against 6.06 ms.
+// (S 11.6, claims and builds 3.9, probes 12.3).  8M x 64M rows: 2.81 ms
+// (S 1.08, 0.35, 0.87) against 6.06 ms.
 #include "internal.h"
 #include "list.cuh"
 
@@ -379,6 +379,128 @@ __device__ __forceinline__ void block_column(const EngineArgs & a, const uint8_t
             reinterpret_cast<T *>(block_ptr(a, blk[j]) + col_off)[slot[j]] = src[row[j]];
 }
 
+// Takes `lack` blocks and up to kRefill beyond from the pool's stack: the
+// first of them in *from, their number returned (0: too few free blocks).
+__device__ __forceinline__ uint32_t take_blocks(const EngineArgs & a, uint32_t lack, uint32_t * from)
+{
+    const uint32_t want = lack + kRefill;
+    unsigned long long * top = reinterpret_cast<unsigned long long *>(&a.ctl->free_top);
+    long long cur = (long long)vload(top), t;
+    for (;;)
+    {
+        t = cur >= (long long)want ? (long long)want : (cur >= (long long)lack ? cur : 0);
+        if (t == 0)
+            break;
+        const long long seen = (long long)atomicCAS(top, (unsigned long long)cur, (unsigned long long)(cur - t));
+        if (seen == cur)
+            break;
+        cur = seen;
+    }
+    *from = (uint32_t)(cur - t);
+    return (uint32_t)t;
+}
+
+// Bucket p's share of a step: c rows and nb new blocks, of them bcache[first,
+// +nb); its rows start at `row` of the step's bucket order, its new blocks at
+// `rb` of hf.fresh.  False: the chain outgrew its directory.
+__device__ __forceinline__ bool place_bucket(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p, uint32_t c, uint32_t nb, uint32_t row,
+                                             uint32_t rb, uint32_t first)
+{
+    const Half & hf = sm.hf;
+    const uint32_t fill = sm.fill[p], last = sm.last[p];
+    hf.off[p] = row;
+    hf.nb0[p] = rb;
+    hf.fill[p] = fill;
+    hf.last[p] = last;
+    if (c == 0)
+        return true;
+    hf.bins[p] = 0;
+    const uint32_t len = sm.clen[p];
+    if (len + nb > a.maxb)
+        return false;
+    uint32_t blk = last;
+    for (uint32_t i = 0; i < nb; ++i)
+    {
+        blk = sm.bcache[first + i];
+        a.chain[((uint64_t)g * a.n_buckets + p) * a.maxb + len + i] = blk;
+        hf.fresh[rb + i] = blk;
+    }
+    sm.last[p] = blk;
+    sm.fill[p] = ((fill + c - 1) & ((1u << a.page_log2) - 1)) + 1;
+    sm.clen[p] = len + nb;
+    sm.urows[p] += c;
+    return true;
+}
+
+// A step's places for few buckets (at most 32 * kLanePer), by one warp, the
+// others of its half at a barrier: two barriers of 512 threads fewer (64
+// buckets: 4,500 cycles of a step's 20,000 were spent here by the general form;
+// S 5.9 -> 5.7 ms for 512M rows).
+constexpr uint32_t kLanePer = 4;
+__device__ __forceinline__ uint32_t allocate_few(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t n)
+{
+    const Half & hf = sm.hf;
+    const uint32_t page = 1u << a.page_log2, P1 = a.n_buckets, lane = threadIdx.x & 31;
+    uint32_t cnt[kLanePer], at[kLanePer], run = 0; // bucket j * 32 + lane
+#pragma unroll
+    for (uint32_t j = 0; j < kLanePer; ++j)
+    {
+        const uint32_t p = j * 32 + lane;
+        cnt[j] = 0;
+        if (p < P1)
+        {
+            const uint32_t c = hf.bins[p];
+            if (c)
+                cnt[j] = c | (((sm.fill[p] + c + page - 1) >> a.page_log2) - 1u) << 16;
+        }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kLanePer; ++j)
+    {
+        uint32_t incl = cnt[j];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o)
+                incl += y;
+        }
+        at[j] = run + incl - cnt[j];
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    const uint32_t need = run >> 16;
+    uint32_t have = sm.pscal[0];
+    if (need > have)
+    {
+        uint32_t from = 0, got = 0;
+        if (lane == 0)
+            got = take_blocks(a, need - have, &from);
+        got = __shfl_sync(0xffffffffu, got, 0);
+        from = __shfl_sync(0xffffffffu, from, 0);
+        if (got == 0)
+            return kTileNoRoom;
+        for (uint32_t i = lane; i < got; i += 32)
+            sm.bcache[have + i] = __ldcg(a.free_stack + from + i);
+        have += got;
+        __syncwarp();
+    }
+    bool ok = true;
+#pragma unroll
+    for (uint32_t j = 0; j < kLanePer; ++j)
+        if (j * 32 + lane < P1)
+            ok = place_bucket(a, sm, g, j * 32 + lane, cnt[j] & 0xFFFFu, cnt[j] >> 16, at[j] & 0xFFFFu, at[j] >> 16, have - need + (at[j] >> 16)) && ok;
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0)
+    {
+        if (!ok)
+            fail(a, kErrChain);
+        hf.off[P1] = n;
+        hf.nb0[P1] = need;
+        sm.pscal[0] = have - need;
+    }
+    return ok ? kTileDone : kTileFailed;
+}
+
 // The step's places, by its half: the bucket counts scanned, the blocks its
 // chains need (an empty chain counts as a full last block) taken from the
 // group's cache of free blocks, and the chains brought to their state after
@@ -435,22 +557,11 @@ __device__ __forceinline__ uint32_t allocate_step(const EngineArgs & a, const Sm
     {
         if (tid == 0)
         {
-            const uint32_t lack = need - have, want = lack + kRefill;
-            unsigned long long * top = reinterpret_cast<unsigned long long *>(&a.ctl->free_top);
-            long long cur = (long long)vload(top), t;
-            for (;;)
-            {
-                t = cur >= (long long)want ? (long long)want : (cur >= (long long)lack ? cur : 0);
-                if (t == 0)
-                    break; // too few free blocks
-                const long long seen = (long long)atomicCAS(top, (unsigned long long)cur, (unsigned long long)(cur - t));
-                if (seen == cur)
-                    break;
-                cur = seen;
-            }
+            uint32_t from;
+            const uint32_t t = take_blocks(a, need - have, &from);
             hf.scal[0] = t ? kTileDone : kTileNoRoom;
-            hf.scal[1] = (uint32_t)(cur - t);
-            hf.scal[2] = (uint32_t)t;
+            hf.scal[1] = from;
+            hf.scal[2] = t;
         }
         half_sync(half);
         if (hf.scal[0] != kTileDone)
@@ -466,35 +577,10 @@ __device__ __forceinline__ uint32_t allocate_step(const EngineArgs & a, const Sm
     for (uint32_t j = 0; j < kPer; ++j)
         if (j < per && p0 + j < P1)
         {
-            const uint32_t p = p0 + j, c = cnt[j] & 0xFFFFu, nb = cnt[j] >> 16;
-            const uint32_t rb = run >> 16, fill = sm.fill[p], last = sm.last[p];
-            hf.off[p] = run & 0xFFFFu;
-            hf.nb0[p] = rb;
-            hf.fill[p] = fill;
-            hf.last[p] = last;
-            if (c)
+            if (!place_bucket(a, sm, g, p0 + j, cnt[j] & 0xFFFFu, cnt[j] >> 16, run & 0xFFFFu, run >> 16, base + (run >> 16)))
             {
-                hf.bins[p] = 0;
-                const uint32_t len = sm.clen[p];
-                if (len + nb > a.maxb)
-                {
-                    fail(a, kErrChain);
-                    hf.scal[0] = kTileFailed;
-                }
-                else
-                {
-                    uint32_t blk = last;
-                    for (uint32_t i = 0; i < nb; ++i)
-                    {
-                        blk = sm.bcache[base + rb + i];
-                        a.chain[((uint64_t)g * P1 + p) * a.maxb + len + i] = blk;
-                        hf.fresh[rb + i] = blk;
-                    }
-                    sm.last[p] = blk;
-                    sm.fill[p] = ((fill + c - 1) & (page - 1)) + 1;
-                    sm.clen[p] = len + nb;
-                    sm.urows[p] += c;
-                }
+                fail(a, kErrChain);
+                hf.scal[0] = kTileFailed;
             }
             run += cnt[j];
         }
@@ -512,7 +598,7 @@ __device__ __forceinline__ uint32_t allocate_step(const EngineArgs & a, const Sm
 // One half's step `k` of the launch.  Consecutive rows of a bucket go to
 // consecutive rows of its blocks.  A step is a chain of latencies (shared
 // atomics, the scan, the permutation, the stores); the other half's step
-// fills them: 5.9 us a step of 4096 rows of 12 bytes, against 8.6 us for
+// fills them: 5.4 us a step of 4096 rows of 12 bytes, against 8.6 us for
 // steps of all 1024 threads, whose first warp scanned the buckets alone.
 // What bounds it now is the instructions of a row (issue slots 40% busy, DRAM
 // 21%, 8 to 9 warps of 32 at a barrier).  hf.bins is zero on entry and on a kTileDone return.
@@ -548,10 +634,29 @@ __device__ uint32_t scatter_step(const EngineArgs & a, const Smem & sm, uint32_t
     }
     if (!half_sync_and(half, ok) && tid == 0)
         hf.scal[0] = kTileFailed; // a bulk copy was not there in time
-    half_sync(half);
-    uint32_t state = hf.scal[0];
-    if (state == kTileDone)
-        state = allocate_step(a, sm, half, g, n);
+    uint32_t state;
+    if (a.n_buckets <= 32 * kLanePer)
+    {
+        if (tid < 32)
+        {
+            __syncwarp();
+            state = hf.scal[0];
+            if (state == kTileDone)
+                state = allocate_few(a, sm, g, n);
+            __syncwarp();
+            if (tid == 0)
+                hf.scal[0] = state;
+        }
+        half_sync(half);
+        state = hf.scal[0];
+    }
+    else
+    {
+        half_sync(half);
+        state = hf.scal[0];
+        if (state == kTileDone)
+            state = allocate_step(a, sm, half, g, n);
+    }
     if (tid == 0)
     {
         if (state == kTileFailed)
