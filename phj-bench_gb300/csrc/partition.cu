@@ -355,14 +355,17 @@ uint64_t row_bytes_of(const Cols & c)
 
 // Launches the scatter over at most `tiles` tiles.  CTAs take a few tiles
 // each and end, so that a kernel of another stream gets its turn on the
-// SMs; the tiles in flight at a time are neighbours.
+// SMs; the tiles in flight at a time are neighbours.  (Up to 8 tiles each, a
+// build side of 3M rows waited for the probe side's pass of 37M again and
+// again: the join took 925 us against 905 with up to 4; with 1 or 2 it takes
+// 910 to 919.  Passes on their own take the same.)
 void launch_scatter(phj_ctx * ctx, const Cols & src, const Cols & dst, ScatterGeom g, const TileShape & sh, uint64_t tiles, const uint32_t * offs,
                     uint32_t * counts, const char * phase, uint64_t n)
 {
     g.stages = sh.stages;
     g.buf_bytes = sh.buf_bytes;
     g.wave = (uint32_t)ctx->num_sms * 2;
-    g.tiles_per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(8, tiles / g.wave / 4));
+    g.tiles_per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(4, tiles / g.wave / 4));
     const uint64_t waves = ceil_div(tiles, (uint64_t)g.wave * g.tiles_per_cta);
     const unsigned grid = (unsigned)(waves == 1 ? std::min<uint64_t>(g.wave, tiles) : waves * g.wave);
     auto kern = g.desc ? (sh.rpt == 8 ? k_scatter<8, true> : sh.rpt == 4 ? k_scatter<4, true> : k_scatter<2, true>)
