@@ -198,13 +198,17 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
 // or a leaf of cap rows or more sets *bad (the table is then unusable).
 // Bound by the write of the tables (16 bytes a cell, 2.2 to 2.9 cells a
 // row): 3M rows in 16,384 leaves 60 us, 2.9 TB/s, where the general tables,
-// their next-chain and the payload packing took 115.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_build_inline(const __grid_constant__ Cols part, const uint32_t * __restrict__ leaf_off,
+// their next-chain and the payload packing took 115.  kRows: shared memory
+// holds the keys and their rows only (10 bytes a cell).
+template <int NT, bool kRows>
+__global__ void __launch_bounds__(NT, kRows ? 2 : 1) k_build_inline(const __grid_constant__ Cols part, const uint32_t * __restrict__ leaf_off,
                                                      const __grid_constant__ PackSpec pk, const __grid_constant__ InlineTables t,
                                                      int * __restrict__ bad)
 {
-    extern __shared__ __align__(16) ulonglong2 icells[];
+    extern __shared__ __align__(16) ulonglong2 icells[]; // (kRows: keys[cap] | rows[cap])
+    uint64_t * ikeys = reinterpret_cast<uint64_t *>(icells);
+    uint16_t * irows = reinterpret_cast<uint16_t *>(ikeys + t.cap);
+    constexpr uint32_t kStride = kRows ? 1 : 2; // 8-byte words from key to key
     const uint32_t l = blockIdx.x;
     const uint32_t r0 = leaf_off[l], r = leaf_off[l + 1] - r0;
     const uint64_t none = t.empty_key(l);
@@ -218,13 +222,15 @@ __global__ void __launch_bounds__(NT) k_build_inline(const __grid_constant__ Col
         return;
     }
     for (uint32_t i = threadIdx.x; i < t.cap; i += NT)
-        icells[i] = make_ulonglong2(none, 0ull);
+    {
+        if constexpr (kRows)
+            ikeys[i] = none;
+        else
+            icells[i] = make_ulonglong2(none, 0ull);
+    }
     if (__syncthreads_or(stop))
         return;
-    bool repeats = false;
-    for (uint32_t i = threadIdx.x; i < r && !repeats; i += NT)
-    {
-        const uint64_t k = part.keys[r0 + i];
+    auto payload = [&](uint32_t i) -> uint64_t {
         uint64_t v = 0;
         for (uint32_t c = 0; c < part.n; ++c)
         {
@@ -238,13 +244,23 @@ __global__ void __launch_bounds__(NT) k_build_inline(const __grid_constant__ Col
             }
             v |= x << (pk.off[c] * 8u);
         }
+        return v;
+    };
+    bool repeats = false;
+    for (uint32_t i = threadIdx.x; i < r && !repeats; i += NT)
+    {
+        const uint64_t k = part.keys[r0 + i];
+        const uint64_t v = kRows ? 0ull : payload(i);
         uint32_t pos = t.start(int_hash64(k));
         for (;;) // r < cap: an empty cell is found
         {
-            const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long *>(&icells[pos].x), none, k);
+            const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long *>(ikeys + pos * kStride), none, k);
             if (old == none)
             {
-                icells[pos].y = v;
+                if constexpr (kRows)
+                    irows[pos] = (uint16_t)i;
+                else
+                    icells[pos].y = v;
                 break;
             }
             if (old == k)
@@ -263,7 +279,15 @@ __global__ void __launch_bounds__(NT) k_build_inline(const __grid_constant__ Col
     }
     ulonglong2 * dst = t.cells + (uint64_t)l * t.cap;
     for (uint32_t i = threadIdx.x; i < t.cap; i += NT)
-        dst[i] = icells[i];
+    {
+        if constexpr (kRows)
+        {
+            const uint64_t key = ikeys[i];
+            dst[i] = make_ulonglong2(key, key != none ? payload(irows[i]) : 0ull);
+        }
+        else
+            dst[i] = icells[i];
+    }
 }
 
 // ---- grouped duplicates (PHJ-PURE with repeated build keys) ----------------
@@ -457,19 +481,25 @@ bool build_inline_tables(phj_ctx * ctx, Scratch & s, const Cols & part, uint64_t
     t.half_shift = total_bits - 1;
     t.cells = reinterpret_cast<ulonglong2 *>(s.get<Cell>(n_leaves * t.cap));
     KTimer kt(ctx, "build_inline", rows, rows * 16 + n_leaves * t.cap * 16);
-    // leaves of more than 1024 rows get 1024 threads
-    if (est > 1024)
-        k_build_inline<1024><<<(unsigned)n_leaves, 1024, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
+    // leaves of more than 1024 rows get 1024 threads; where two such CTAs do
+    // not fit on a SM with cells in shared memory, keys and rows are held
+    // there and the payloads are read as the cells go out (256 leaves of
+    // 4096 rows: 24 us against 28, in one wave of CTAs)
+    const size_t lean = (size_t)t.cap * 10, two = (ctx->smem_optin + 1024) / 2 - 2048;
+    if (est > 1024 && smem > two && lean <= two)
+        k_build_inline<1024, true><<<(unsigned)n_leaves, 1024, lean, ctx->stream>>>(part, leaf_off, pk, t, bad);
+    else if (est > 1024)
+        k_build_inline<1024, false><<<(unsigned)n_leaves, 1024, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
     else
-        k_build_inline<kBuildNT><<<(unsigned)n_leaves, kBuildNT, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
+        k_build_inline<kBuildNT, false><<<(unsigned)n_leaves, kBuildNT, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
     PHJ_LAUNCHED(ctx, "build_inline");
     return true;
 }
 
 void set_build_smem_limits(int smem_optin)
 {
-    PHJ_CUDA(cudaFuncSetAttribute(k_build_inline<kBuildNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    PHJ_CUDA(cudaFuncSetAttribute(k_build_inline<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
+    for (const auto kernel : {k_build_inline<kBuildNT, false>, k_build_inline<1024, false>, k_build_inline<1024, true>})
+        PHJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
     const size_t need = (size_t)kSmemCellsMax * sizeof(Cell);
     for (const auto kernel : {k_build_leaf<kBuildNT, false>, k_build_leaf<1024, false>, k_build_leaf<kBuildNT, true>, k_build_leaf<1024, true>})
         PHJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -38,7 +38,8 @@ def test_payload_widths(ctx, bt, mat):
     assert ("build_inline" in names) == (bt != [P.U64, P.U32])
 
 
-@pytest.mark.parametrize("build,probe,bits", [(33_000, 1, [10]), (4096, 255, [7]), (4096, 257, [1]), (70_000, 5000, [11]), (70_000, 5000, [4, 3])])
+@pytest.mark.parametrize("build,probe,bits", [(33_000, 1, [10]), (4096, 255, [7]), (4096, 257, [1]), (70_000, 5000, [11]), (70_000, 5000, [4, 3]), (9000, 3000, [1]),
+                                              (70_000, 5000, [4])])
 def test_leaf_sizes_and_chunk_edges(ctx, build, probe, bits):
     bk = G.gen_keys(0, build, 706, 707)
     names = join(ctx, bk, G.gen_keys(4, probe, 708, 707, domain=build, match_permille=800), [P.U64], [P.U64], bits, 0)
