@@ -161,7 +161,9 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *   "time_kernels": 1 (default) records CUDA events around each kernel;
  *   "wait_limit_ms": bound of a device wait on another warp's work
  *        (PHJ/BEP leaf builds), 1..60000, default 1000;
- *   "host_chunk_rows": probe rows per chunk of phj_run_phj_pure_host (>= 4096);
+ *   "host_chunk_rows": probe rows per chunk of phj_run_phj_pure_host (>= 4096;
+ *        at the default of 16M it is the most: short probe sides go in
+ *        smaller chunks);
  *   "table_cap_pct": leaf table cells >= rows * pct / 100, rounded up to a
  *        power of two (110..800, default 200: the reference's bit_ceil(2 rows));
  *   "p1_tile_rows", "p1_stages": tile rows (1024/2048/4096) and bulk-copy
@@ -290,7 +292,7 @@ phj_status phj_run_phj_pure(phj_ctx *ctx, const phj_table *build, const phj_tabl
 /* runPHJ with the BlockStreams and the JoinOutput in host memory (pinned
  * for full speed), the form a host caller of runPHJ uses.  The build side is
  * uploaded whole; the probe side streams through in chunks of
- * "host_chunk_rows" rows (context option, default 16M) with the upload of
+ * at most "host_chunk_rows" rows (context option, default 16M) with the upload of
  * the next chunk, the join of this one and the download of the previous
  * output overlapped.  Output rows go to the host columns (`out_keys`,
  * `out_left[build payloads]`, `out_right[probe payloads]`, `out_capacity`

@@ -1386,6 +1386,22 @@ struct CopyDrain
     }
 };
 
+// Probe rows a chunk, at the option's default: 96 MiB of uploads, at least a
+// sixteenth of the probe side and at most the option.  The first upload and
+// the last download overlap nothing, so a short probe side wants small
+// chunks; a chunk's launches and round trips take 0.1 to 0.25 ms, which its
+// copies (0.45 ms of uploads) have to cover.  2M x 24M rows of 16 bytes: 5.37
+// ms in chunks of 16M rows, 4.66 of 6M, 4.77 of 2M, 5.94 of 1M; 4M x 64M 11.6,
+// 11.0, 11.6 and 15.0; 1M x 12M of 12 bytes, a fifth matching: 1.30 of 16M,
+// 1.28 of 8M, 1.39 of 4M; 16M x 256M 41.7 of 16M or 8M, 42.2 of 6M.
+static uint64_t host_chunk_rows(const phj_ctx * ctx, const phj_block_stream & probe)
+{
+    const uint64_t most = (uint64_t)ctx->host_chunk_rows;
+    if (ctx->host_chunk_rows != kHostChunkRows)
+        return most; // pinned
+    return std::min<uint64_t>(most, std::max<uint64_t>((96ull << 20) / (8 + schema_bytes(probe.schema)), probe.total_rows / 16));
+}
+
 // PHJ-PURE with the inputs and the output in host memory.  The build side
 // is uploaded whole; the probe side streams through in chunks on three
 // streams: chunk c+1 uploads (h2d) while chunk c is partitioned by the first
@@ -2391,7 +2407,7 @@ phj_status phj_run_phj_pure_host(phj_ctx * ctx, const phj_block_stream * build, 
         for (uint32_t c = 0; c < probe->schema.n_payloads; ++c)
             if ((probe->total_rows && !probe->payloads[c]) || (out_capacity && (!out_right || !out_right[c])))
                 throw Error(PHJ_ERR_INVALID_ARGUMENT, "null probe payload column");
-        run_phj_pure_host(ctx, *build, *probe, bits, out_capacity, out_keys, out_left, out_right, out_rows, result, (uint64_t)ctx->host_chunk_rows);
+        run_phj_pure_host(ctx, *build, *probe, bits, out_capacity, out_keys, out_left, out_right, out_rows, result, host_chunk_rows(ctx, *probe));
     });
 }
 

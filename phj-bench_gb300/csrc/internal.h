@@ -106,6 +106,8 @@ struct ScratchArena
     bool off = false;  // this call runs from the pool alone
 };
 
+constexpr int64_t kHostChunkRows = 16ll << 20; // default of "host_chunk_rows"
+
 struct phj_ctx
 {
     int device = 0;
@@ -136,7 +138,7 @@ struct phj_ctx
     // Options (phj_ctx_set_int).
     int probe_materialize = -1; // -1 auto, 0 never, 1 always
     int64_t wait_limit_ms = 1000; // bound of a device wait on another warp's work
-    int64_t host_chunk_rows = 16ll << 20; // probe rows per chunk of the host-buffer entry points
+    int64_t host_chunk_rows = kHostChunkRows; // probe rows per chunk of the host-buffer entry points
     uint32_t table_cap_pct = 200; // leaf table cells >= rows * pct / 100 (power of two)
     uint32_t p1_tile_rows = 0;    // first radix pass: rows per staged tile (0: chosen per row width)
     uint32_t p1_stages = 0;       // first radix pass: depth of the bulk-copy ring (0: chosen per row width)
