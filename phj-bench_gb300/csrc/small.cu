@@ -86,15 +86,18 @@ __global__ void __launch_bounds__(kSNT, 1) k_small_join(const __grid_constant__ 
 // of one 8-byte payload): partitioned joins take about 100 us + 10.5 us a
 // million probe rows, so the launch wins while (pieces - 1) x probe rows
 // stay under about 7.6M (64K x 512K: 74 us against 142; 64K x 2M: 177
-// against 159); the no-allocation join's global table 50 us + 38 us a
-// million, under (pieces - 3) x probe rows of 2.6M (16K x 256K: 40 against
-// 64; 64K x 1M: 107 against 90).
+// against 159).  The no-allocation join's global table takes 50 us + 38 us a
+// million, less the more build rows there are; with 8 to 20 payload bytes a
+// side the launch wins up to four pieces (16K x 256K: 40 against 64 us; 32K x
+// 786K 63-73 against 76-80) and beyond them while (pieces - 1) x probe rows
+// stay under 1.4M (40K x 320K: 50-55 against 56-60; 40K x 512K 59-67 against
+// 61-63; 57K x 256K 54-61 against 60; 57K x 456K 65-74 against 64-67).
 bool small_join_eligible(const phj_ctx * ctx, uint64_t build_rows, uint64_t probe_rows, bool noalloc)
 {
     const uint64_t pieces = ceil_div(build_rows, kSRows), free_pieces = noalloc ? 3 : 1;
-    const uint64_t most = (uint64_t)ctx->num_sms * (noalloc ? 17000 : 50000);
+    const uint64_t most = (uint64_t)ctx->num_sms * (!noalloc ? 50000 : pieces <= 4 ? 20400 : 9200);
     return build_rows > 0 && probe_rows > 0 && pieces <= 8 && probe_rows < (1ull << 31) &&
-           (pieces <= free_pieces || (pieces - free_pieces) * probe_rows <= most);
+           (pieces <= free_pieces || (pieces - 1) * probe_rows <= most);
 }
 
 uint64_t small_join(phj_ctx * ctx, const Cols & build, uint64_t build_rows, const Cols & probe, uint64_t probe_rows, uint64_t * out_keys,
