@@ -60,8 +60,8 @@
 // Measured (64M x 512M rows, Zipf keys, 32 MiB a group): 14.4 ms (S 5.7,
 // claims and builds 1.4, probes 6.5 ms); one persistent grid of 1024-thread
 // CTAs for both steps, whose refines sorted every block by leaf, took 28.1 ms
-// (S 11.6, claims and builds 3.9, probes 12.3).  8M x 64M rows: 2.81 ms
-// (S 1.08, 0.35, 0.87) against 6.06 ms.
+// (S 11.6, claims and builds 3.9, probes 12.3).  8M x 64M rows: 2.60 ms
+// (S 1.0, 0.36, 0.87) against 6.06 ms.
 #include "internal.h"
 #include "list.cuh"
 
@@ -325,6 +325,7 @@ struct Smem
     Half hf;          // this thread's half's
     uint32_t * acc;   // leaves per bucket: rows a refine adds to each leaf
     uint32_t * scal;  // scalars (32 words, 8-byte aligned)
+    uint32_t * list;  // buckets: refine_down_to's lists (half 0's `off`, between steps)
     // kept in memory between launches, one run of words:
     uint32_t * persist;
     uint32_t * fill;   // buckets: rows in each chain's last block (page: no block)
@@ -367,6 +368,7 @@ enum : uint32_t
 // words of Smem::scal that order the halves' steps: the step whose turn it is
 // to allocate, the outcome of the first step that was not taken, and which
 constexpr uint32_t kTurn = 8, kStop = 9, kStopStep = 10;
+constexpr uint32_t kRefineSlot = 16; // refine_down_to's words
 
 template <class T>
 __device__ __forceinline__ void block_column(const EngineArgs & a, const uint8_t * src_v, uint32_t col_off, const uint32_t (&row)[4],
@@ -717,7 +719,7 @@ __device__ uint32_t scatter_step(const EngineArgs & a, const Smem & sm, uint32_t
 // S: refine bucket p of group g -- its rows counted by leaf, its blocks
 // published as refined.  Returns the rows refined.
 // ---------------------------------------------------------------------------
-__device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p)
+__device__ void refine_bucket(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p, unsigned long long c0)
 {
     const uint32_t page = 1u << a.page_log2;
     const uint32_t LB = 1u << a.lb_log2, shift = 64u - a.total_bits;
@@ -743,7 +745,6 @@ __device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_
             if (i0 + u * kENT + threadIdx.x < rows)
                 atomicAdd(&sm.acc[(uint32_t)(int_hash64(k[u]) >> shift) & (LB - 1u)], 1u);
     }
-    const unsigned long long c0 = vload(&a.ctl->cursor); // the cursor stands still outside E
     for (uint32_t j = threadIdx.x; j < len; j += kENT)
     {
         const uint32_t blk = ch[j], n = j + 1 == len ? tail : page;
@@ -759,9 +760,6 @@ __device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_
             atomicAdd(a.leaf_rows + ((uint64_t)p << a.lb_log2) + l, sm.acc[l]);
     if (threadIdx.x == 0)
     {
-        atomicAdd(&a.ctl->global_leaf_rows, (unsigned long long)rows);
-        atomicAdd(&a.ctl->rows_refined, (unsigned long long)rows);
-        atomicAdd(&a.ctl->refinements, 1ull);
         if (g == 0)
             a.ctl->blocks0 += len;
         sm.clen[p] = 0;
@@ -769,47 +767,143 @@ __device__ uint32_t refine_bucket(const EngineArgs & a, const Smem & sm, uint32_
         sm.urows[p] = 0;
     }
     __syncthreads();
-    return rows;
 }
 
 // Refines the group's largest bucket (src/PHJBep.cpp:376-395) until its
 // unrefined bytes are below `low` (every bucket that holds rows when low
 // is 0).
+// A warp's refine of a bucket of few rows: as refine_bucket, counted without
+// shared memory (rows of one leaf in a step of 32 rows together).
+__device__ __forceinline__ void refine_small(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p, unsigned long long c0)
+{
+    const uint32_t page = 1u << a.page_log2, shift = 64u - a.total_bits, lane = threadIdx.x & 31;
+    const uint32_t len = sm.clen[p], rows = sm.urows[p], tail = sm.fill[p];
+    const uint32_t * ch = a.chain + ((uint64_t)g * a.n_buckets + p) * a.maxb;
+    for (uint32_t i0 = 0; i0 < rows; i0 += 128)
+    {
+        uint64_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const uint32_t i = i0 + u * 32 + lane;
+            k[u] = 0;
+            if (i < rows)
+                k[u] = __ldcg(reinterpret_cast<const unsigned long long *>(block_ptr(a, ch[i >> a.page_log2])) + (i & (page - 1)));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const bool on = i0 + u * 32 + lane < rows;
+            const uint32_t leaf = on ? (uint32_t)(int_hash64(k[u]) >> shift) : kNone;
+            const uint32_t same = __match_any_sync(0xffffffffu, leaf);
+            if (on && (uint32_t)__ffs(same) - 1u == lane)
+                atomicAdd(a.leaf_rows + leaf, (uint32_t)__popc(same));
+        }
+    }
+    for (uint32_t j = lane; j < len; j += 32)
+    {
+        const uint32_t blk = ch[j], n = j + 1 == len ? tail : page;
+        a.blk_rows[blk] = n;
+        a.blk_rem[blk] = n;
+        a.blk_bucket[blk] = p;
+        a.blk_c0[blk] = c0;
+        a.blk_state[blk] = p;
+    }
+    __syncwarp();
+    if (lane == 0)
+    {
+        sm.clen[p] = 0;
+        sm.fill[p] = page;
+        sm.urows[p] = 0;
+    }
+}
+
+// (Of equal buckets the first.)  The buckets so refined are the first ones
+// in that order, so they are found at once -- by a binary search of the
+// order's last key -- and refined side by side: those of few rows a warp
+// each, the others by the whole CTA.  One after the other they took 2 to 5
+// us each, most of it barriers and the search for the largest (2M x 10M Zipf
+// rows, 256 buckets, 116 MiB, 82,475 refines: a join of 4,370 us against
+// 2,260; 8M x 64M rows, 64 buckets, 20,983 refines: 3,150 against 2,920).
+constexpr uint32_t kSmallRows = 1024;
 __device__ void refine_down_to(const EngineArgs & a, const Smem & sm, uint32_t g, uint64_t & unref_bytes, uint64_t low)
 {
-    unsigned long long * best_slot = reinterpret_cast<unsigned long long *>(sm.scal + 4);
-    for (;;)
+    if (unref_bytes == 0 || (low && unref_bytes < low))
+        return;
+    // order: rows, then the lower bucket
+    uint32_t * slot = sm.scal + kRefineSlot; // three sums in turn, the two lists' lengths
+    auto key = [&](uint32_t p, uint32_t r) -> uint64_t { return (uint64_t)r << 11 | (2047u - p); };
+    constexpr uint32_t kMine = 2048 / kENT;
+    uint32_t mine[kMine];
+#pragma unroll
+    for (uint32_t j = 0; j < kMine; ++j)
+        mine[j] = j * kENT + threadIdx.x < a.n_buckets ? sm.urows[j * kENT + threadIdx.x] : 0u;
+    uint64_t last = 2048; // refined: keys from this one on
+    __syncthreads();      // (the slots are no longer read)
+    if (threadIdx.x < 5)
+        slot[threadIdx.x] = 0;
+    __syncthreads();
+    if (low)
     {
-        if (unref_bytes == 0 || (low && unref_bytes < low))
-            return;
-        if (threadIdx.x == 0)
-            *best_slot = 0ull;
-        __syncthreads();
-        unsigned long long best = 0;
-        for (uint32_t p = threadIdx.x; p < a.n_buckets; p += kENT)
+        uint64_t none = (unref_bytes / a.rb + 1) << 11; // a key past all
+        for (uint32_t it = 0; none - last > 1; ++it)
         {
-            // ties go to the lowest bucket
-            const unsigned long long v = ((unsigned long long)sm.urows[p] << 32) | (0xFFFFFFFFu - p);
-            if (sm.urows[p] && v > best)
-                best = v;
+            const uint64_t mid = last + (none - last) / 2;
+            uint32_t sum = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < kMine; ++j)
+                sum += key(j * kENT + threadIdx.x, mine[j]) >= mid ? mine[j] : 0u;
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if ((threadIdx.x & 31) == 0 && sum)
+                atomicAdd(slot + it % 3, sum);
+            if (threadIdx.x == 0)
+                slot[(it + 1) % 3] = 0;
+            __syncthreads();
+            // (a slot is cleared again two steps on, past the next barrier)
+            if ((uint64_t)*reinterpret_cast<volatile uint32_t *>(slot + it % 3) * a.rb + low > unref_bytes)
+                last = mid;
+            else
+                none = mid;
         }
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            const unsigned long long y = __shfl_xor_sync(0xffffffffu, best, o);
-            best = y > best ? y : best;
-        }
-        if ((threadIdx.x & 31) == 0 && best)
-            atomicMax(best_slot, best);
-        __syncthreads();
-        const unsigned long long top = *reinterpret_cast<volatile unsigned long long *>(best_slot);
-        __syncthreads();
-        if (top == 0)
-            return;
-        const uint32_t p = 0xFFFFFFFFu - (uint32_t)(top & 0xFFFFFFFFull);
-        const uint32_t rows = refine_bucket(a, sm, g, p);
-        const uint64_t b = (uint64_t)rows * a.rb;
-        unref_bytes = unref_bytes > b ? unref_bytes - b : 0;
     }
+    // the lists: small ones from the front, the others from the back
+    uint32_t rows = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kMine; ++j)
+    {
+        const uint32_t p = j * kENT + threadIdx.x;
+        if (mine[j] && key(p, mine[j]) >= last)
+        {
+            rows += mine[j];
+            if (mine[j] <= kSmallRows)
+                sm.list[atomicAdd(slot + 3, 1u)] = p;
+            else
+                sm.list[a.n_buckets - 1u - atomicAdd(slot + 4, 1u)] = p;
+        }
+    }
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    __syncthreads(); // the lists; the sums are no longer read
+    if (threadIdx.x == 0)
+        slot[0] = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && rows)
+        atomicAdd(slot, rows);
+    const uint32_t n_small = slot[3], n_large = slot[4];
+    const unsigned long long c0 = vload(&a.ctl->cursor); // the cursor stands still outside E
+    for (uint32_t i = threadIdx.x >> 5; i < n_small; i += kENT / 32)
+        refine_small(a, sm, g, sm.list[i], c0);
+    __syncthreads();
+    for (uint32_t i = 0; i < n_large; ++i)
+        refine_bucket(a, sm, g, sm.list[a.n_buckets - 1u - i], c0);
+    const uint32_t total = slot[0];
+    if (threadIdx.x == 0)
+    {
+        atomicAdd(&a.ctl->global_leaf_rows, (unsigned long long)total);
+        atomicAdd(&a.ctl->rows_refined, (unsigned long long)total);
+        atomicAdd(&a.ctl->refinements, (unsigned long long)(n_small + n_large));
+    }
+    const uint64_t bytes = (uint64_t)total * a.rb;
+    unref_bytes = unref_bytes > bytes ? unref_bytes - bytes : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1564,6 +1658,7 @@ __global__ void __launch_bounds__(kENT, 1) k_bep_scatter(const __grid_constant__
         sm.hf.wsum = words(kHNT / 32);
         sm.hf.scal = words(4);
         p = smem_raw + 2 * a.half_bytes;
+        sm.list = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(sm.hf.off) - (uint64_t)half * a.half_bytes);
         sm.acc = words(LB);
         sm.scal = words(32);
         sm.persist = words(a.persist_words);
