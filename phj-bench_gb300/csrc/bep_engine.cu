@@ -312,8 +312,7 @@ struct Half
     uint32_t * bins;  // buckets: rows of the step
     uint32_t * off;   // buckets: first position in the step's bucket order (and the total)
     uint32_t * nb0;   // buckets: first of the step's new blocks (and the total)
-    uint32_t * fill;  // buckets: rows in the chain's last block before the step
-    uint32_t * last;  // buckets: the chain's last block before the step
+    uint2 * fl;       // buckets: {rows in the chain's last block before the step - off, that block}
     uint32_t * fresh; // the step's new blocks
     uint32_t * wsum;  // the warps' sums of a scan
     uint32_t * scal;  // [0] the step's outcome, [1,2] where its new blocks come from
@@ -412,8 +411,7 @@ __device__ __forceinline__ bool place_bucket(const EngineArgs & a, const Smem & 
     const uint32_t fill = sm.fill[p], last = sm.last[p];
     hf.off[p] = row;
     hf.nb0[p] = rb;
-    hf.fill[p] = fill;
-    hf.last[p] = last;
+    hf.fl[p] = make_uint2(fill - row, last);
     if (c == 0)
         return true;
     hf.bins[p] = 0;
@@ -437,7 +435,8 @@ __device__ __forceinline__ bool place_bucket(const EngineArgs & a, const Smem & 
 // A step's places for few buckets (at most 32 * kLanePer), by one warp, the
 // others of its half at a barrier: two barriers of 512 threads fewer (64
 // buckets: 4,500 cycles of a step's 20,000 were spent here by the general form;
-// S 5.9 -> 5.7 ms for 512M rows).
+// S 5.9 -> 5.7 ms for 512M rows; with 256 buckets a warp alone takes longer:
+// 2M x 10M rows 2,310 us against 2,214).
 constexpr uint32_t kLanePer = 4;
 __device__ __forceinline__ uint32_t allocate_few(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t n)
 {
@@ -694,9 +693,10 @@ __device__ uint32_t scatter_step(const EngineArgs & a, const Smem & sm, uint32_t
             if (s < n)
             {
                 const uint32_t e = hf.perm[s], p = e >> 12;
-                const uint32_t q = hf.fill[p] + (s - hf.off[p]); // slot counted from the chain's last block
+                const uint2 fl = hf.fl[p];
+                const uint32_t q = fl.x + s; // slot counted from the chain's last block
                 row[j] = e & 4095u;
-                blk[j] = q < page ? hf.last[p] : hf.fresh[hf.nb0[p] + (q >> a.page_log2) - 1u];
+                blk[j] = q < page ? fl.y : hf.fresh[hf.nb0[p] + (q >> a.page_log2) - 1u];
                 slot[j] = q & (page - 1);
                 live |= 1u << j;
             }
@@ -1652,8 +1652,7 @@ __global__ void __launch_bounds__(kENT, 1) k_bep_scatter(const __grid_constant__
         sm.hf.bins = words(P1);
         sm.hf.off = words(P1 + 1);
         sm.hf.nb0 = words(P1 + 1);
-        sm.hf.fill = words(P1);
-        sm.hf.last = words(P1);
+        sm.hf.fl = reinterpret_cast<uint2 *>(words(2 * P1));
         sm.hf.fresh = words(a.fresh_words);
         sm.hf.wsum = words(kHNT / 32);
         sm.hf.scal = words(4);
@@ -1955,7 +1954,7 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
         a.bcache_words = a.fresh_words + 2 * kRefill + 2;
         a.persist_words = (uint32_t)((4 * P1 + kPersistScal + a.bcache_words + 1) & ~1ull);
         a.half_bytes = (uint32_t)(
-            a.stage_bytes + room(4ull * rows) + 3 * room(4 * P1) + 2 * room(4 * (P1 + 1)) + room(4ull * a.fresh_words) + room(kHNT / 8) + room(16));
+            a.stage_bytes + room(4ull * rows) + room(4 * P1) + room(8 * P1) + 2 * room(4 * (P1 + 1)) + room(4ull * a.fresh_words) + room(kHNT / 8) + room(16));
         return 2ull * a.half_bytes + room(4 * LB) + room(32 * 4) + room(4ull * a.persist_words);
     };
     size_t smem = 0;
