@@ -378,6 +378,54 @@ __global__ void k_slot_hist(const uint64_t * __restrict__ keys, uint64_t n, uint
             atomicAdd(&counts[i], bins[i]);
 }
 
+// Rows of each of 2^slot_bits (at most 1024) sub-tables, and by the last CTA
+// to finish the tables themselves: their cells (as table_cells) laid end to
+// end in meta, the sum in counts[nb + 1] (counts[nb] counts CTAs; all zero
+// before).  Bound by the keys' latency and one global atomic a CTA and
+// sub-table: one CTA of 1024 threads a SM, four loads in flight (669K rows
+// 10.7 us; 1,216 CTAs of 256 threads, a load at a time, 16.4).
+__global__ void __launch_bounds__(1024) k_slot_plan(const uint64_t * __restrict__ keys, uint64_t n, uint32_t slot_bits, uint32_t * __restrict__ counts,
+                                                    LeafMeta * __restrict__ meta)
+{
+    __shared__ uint32_t bins[1024];
+    __shared__ uint32_t warp_sums[32];
+    __shared__ uint32_t s_last;
+    const uint32_t nb = 1u << slot_bits, t = threadIdx.x;
+    bins[t] = 0;
+    __syncthreads();
+    const uint64_t stride = (uint64_t)gridDim.x * 1024;
+    for (uint64_t i = (uint64_t)blockIdx.x * 1024 + t; i < n; i += 4 * stride)
+    {
+        uint64_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            k[u] = i + u * stride < n ? keys[i + u * stride] : 0ull;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * stride < n)
+                atomicAdd(&bins[int_hash64(k[u]) >> (64 - slot_bits)], 1u);
+    }
+    __syncthreads();
+    if (t < nb && bins[t])
+        atomicAdd(&counts[t], bins[t]);
+    __threadfence();
+    __syncthreads();
+    if (t == 0)
+        s_last = atomicAdd(&counts[nb], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last)
+        return;
+    __threadfence();
+    const uint32_t r = t < nb ? __ldcg(counts + t) : 0u;
+    const uint32_t cap = (uint32_t)table_cells(r, 200);
+    uint32_t total;
+    const uint32_t off = block_excl_scan<1024>(cap, warp_sums, &total);
+    if (t < nb)
+        meta[t] = LeafMeta{off, 0u, cap ? (uint8_t)log2u(cap) : (uint8_t)0, (uint8_t)(r != 0), 0, 0};
+    if (t == 0)
+        counts[nb + 1] = total;
+}
+
 __global__ void k_slot_meta(const uint32_t * __restrict__ counts, const uint32_t * __restrict__ table_off, uint32_t n_slots, LeafMeta * __restrict__ meta)
 {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -387,8 +435,11 @@ __global__ void k_slot_meta(const uint32_t * __restrict__ counts, const uint32_t
     meta[s] = LeafMeta{table_off[s], 0u, cap ? (uint8_t)log2u(cap) : (uint8_t)0, (uint8_t)(counts[s] != 0), 0, 0};
 }
 
-__global__ void k_fill_empty(Cell * __restrict__ cells, uint64_t n)
+// n cells, or *n_dev.
+__global__ void k_fill_empty(Cell * __restrict__ cells, uint64_t n, const uint32_t * __restrict__ n_dev)
 {
+    if (n_dev)
+        n = *n_dev;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         reinterpret_cast<ulonglong2 *>(cells)[i] = make_ulonglong2(0ull, INVALID_REF);
 }
@@ -616,39 +667,56 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
 void build_global_table(phj_ctx * ctx, Scratch & s, const phj_table & build, uint32_t slot_bits, LeafTables & lt)
 {
     const uint32_t n_slots = 1u << slot_bits;
-    uint32_t * counts = s.get<uint32_t>(n_slots + 1);
-    uint32_t * caps = s.get<uint32_t>(n_slots + 1);
-    uint32_t * table_off = s.get<uint32_t>(n_slots + 1);
-    int * any_dup = s.get<int>(1);
-    PHJ_CUDA(cudaMemsetAsync(counts, 0, (n_slots + 1) * sizeof(uint32_t), ctx->stream));
-    PHJ_CUDA(cudaMemsetAsync(any_dup, 0, sizeof(int), ctx->stream));
     const uint64_t n = build.rows;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 256), (uint64_t)ctx->num_sms * 8));
+    uint32_t * counts = s.get<uint32_t>(n_slots + 3); // and the plan's CTA count and total; the repeated-key flag
+    int * any_dup = reinterpret_cast<int *>(counts + n_slots + 2);
+    PHJ_CUDA(cudaMemsetAsync(counts, 0, (n_slots + 3) * sizeof(uint32_t), ctx->stream));
+    lt.meta = s.get<LeafMeta>(n_slots);
+    // Up to 16M rows the cells are allocated at the most they can be (four a
+    // row, 1 GiB), so their number is not read back and one launch counts and
+    // plans: the tables' fill starts 12 us after the count did instead of 47
+    // (342K x 3.6M rows: 208 -> 170 us a join, 669K x 2.7M 213 -> 177).  More
+    // rows are counted first: the exact size is then worth the round trip.
+    const bool plan = n <= (16u << 20) && n_slots <= 1024;
+    if (plan)
     {
+        lt.total_cells = std::max<uint64_t>(4 * n, 2);
+        lt.cells = s.get<Cell>(lt.total_cells);
         KTimer kt(ctx, "chj_slot_hist", n, n * 8);
-        k_slot_hist<<<grid, 256, n_slots * sizeof(uint32_t), ctx->stream>>>(build.keys, n, slot_bits, counts);
+        k_slot_plan<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 4096), (uint64_t)ctx->num_sms)), 1024, 0, ctx->stream>>>(
+            build.keys, n, slot_bits, counts, lt.meta);
         PHJ_LAUNCHED(ctx, "chj_slot_hist");
     }
-    uint32_t * max_rows = s.get<uint32_t>(1);
-    PHJ_CUDA(cudaMemsetAsync(max_rows, 0, sizeof(uint32_t), ctx->stream));
-    // counts -> capacities -> offsets: the offsets of leaf_off-style caps
-    // reuse k_leaf_caps on a prefix of the counts.
-    uint32_t * cnt_off = s.get<uint32_t>(n_slots + 1);
-    scan_u32(ctx, s, counts, cnt_off, n_slots);
-    k_leaf_caps<<<(unsigned)ceil_div(n_slots, 256), 256, 0, ctx->stream>>>(cnt_off, n_slots, 200u, caps, max_rows);
-    PHJ_LAUNCHED(ctx, "chj_caps");
-    scan_u32(ctx, s, caps, table_off, n_slots);
-    uint32_t total = 0;
-    read_small(ctx, {{&total, table_off + n_slots, sizeof(uint32_t)}});
-    lt.total_cells = total;
-    lt.meta = s.get<LeafMeta>(n_slots);
-    lt.cells = s.get<Cell>(total);
-    k_slot_meta<<<(unsigned)ceil_div(n_slots, 256), 256, 0, ctx->stream>>>(counts, table_off, n_slots, lt.meta);
-    PHJ_LAUNCHED(ctx, "chj_meta");
+    else
     {
-        KTimer kt(ctx, "chj_fill", 0, total * 16ull);
-        k_fill_empty<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(total, 256), (uint64_t)ctx->num_sms * 16)), 256, 0, ctx->stream>>>(
-            lt.cells, total);
+        uint32_t * caps = s.get<uint32_t>(n_slots + 1);
+        uint32_t * table_off = s.get<uint32_t>(n_slots + 1);
+        {
+            KTimer kt(ctx, "chj_slot_hist", n, n * 8);
+            k_slot_hist<<<grid, 256, n_slots * sizeof(uint32_t), ctx->stream>>>(build.keys, n, slot_bits, counts);
+            PHJ_LAUNCHED(ctx, "chj_slot_hist");
+        }
+        uint32_t * max_rows = s.get<uint32_t>(1);
+        PHJ_CUDA(cudaMemsetAsync(max_rows, 0, sizeof(uint32_t), ctx->stream));
+        // counts -> capacities -> offsets: the offsets of leaf_off-style caps
+        // reuse k_leaf_caps on a prefix of the counts.
+        uint32_t * cnt_off = s.get<uint32_t>(n_slots + 1);
+        scan_u32(ctx, s, counts, cnt_off, n_slots);
+        k_leaf_caps<<<(unsigned)ceil_div(n_slots, 256), 256, 0, ctx->stream>>>(cnt_off, n_slots, 200u, caps, max_rows);
+        PHJ_LAUNCHED(ctx, "chj_caps");
+        scan_u32(ctx, s, caps, table_off, n_slots);
+        uint32_t total = 0;
+        read_small(ctx, {{&total, table_off + n_slots, sizeof(uint32_t)}});
+        lt.total_cells = total;
+        lt.cells = s.get<Cell>(total);
+        k_slot_meta<<<(unsigned)ceil_div(n_slots, 256), 256, 0, ctx->stream>>>(counts, table_off, n_slots, lt.meta);
+        PHJ_LAUNCHED(ctx, "chj_meta");
+    }
+    {
+        KTimer kt(ctx, "chj_fill", 0, plan ? 0 : lt.total_cells * 16ull);
+        k_fill_empty<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(lt.total_cells, 256), (uint64_t)ctx->num_sms * 16)), 256, 0,
+                       ctx->stream>>>(lt.cells, lt.total_cells, plan ? counts + n_slots + 1 : nullptr);
         PHJ_LAUNCHED(ctx, "chj_fill");
     }
     {
