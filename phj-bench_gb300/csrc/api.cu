@@ -361,7 +361,27 @@ phj_output * new_output(phj_ctx * ctx, const phj_schema & left, const phj_schema
         auto column = [&](uint64_t w) -> void * {
             o->bytes += cap * w;
             if (!o->slab)
-                return dalloc(ctx, room(w));
+            {
+                // in steps of a 32nd to a 64th, so that the output of a join
+                // of nearly as many rows finds the place of the last one
+                // (7.5M x 228M rows, 7.5 GB of output whose size changes a
+                // little from call to call: 8.8 ms at exact sizes, 2.1 of
+                // them mapping memory, and 6.7 in steps)
+                const uint64_t bytes = room(w);
+                uint64_t step = 256;
+                while (step * 64 <= bytes)
+                    step *= 2;
+                try
+                {
+                    return dalloc(ctx, (bytes + step - 1) & ~(step - 1));
+                }
+                catch (const Error & e)
+                {
+                    if (e.status != PHJ_ERR_OUT_OF_MEMORY)
+                        throw;
+                    return dalloc(ctx, bytes);
+                }
+            }
             uint8_t * p = at;
             at += room(w);
             return p;
