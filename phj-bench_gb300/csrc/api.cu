@@ -1960,6 +1960,7 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         PHJ_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
         PHJ_CUDA(cudaMalloc(&ctx->small_ctr, sizeof(SmallCounters)));
         PHJ_CUDA(cudaMemset(ctx->small_ctr, 0, sizeof(SmallCounters)));
+        small_host(ctx); // (the no-allocation join uses both)
         set_small_smem_limits();
         set_partition_smem_limits((int)ctx->smem_optin);
         set_build_smem_limits((int)ctx->smem_optin);

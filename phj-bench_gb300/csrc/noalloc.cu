@@ -170,8 +170,8 @@ unsigned long long global_table_join(phj_ctx * ctx, const NaScratch & s, const C
         PHJ_LAUNCHED(ctx, "noalloc_probe");
     }
     unsigned long long rows = 0;
-    PHJ_CUDA(cudaMemcpyAsync(&rows, s.rows, sizeof(rows), cudaMemcpyDeviceToHost, ctx->stream));
-    PHJ_CUDA(cudaStreamSynchronize(ctx->stream));
+    // (through mapped memory: 54K x 1.1M rows 90 -> 87 us, 48K x 400K 67 -> 63)
+    read_small(ctx, {{&rows, s.rows, sizeof(rows)}});
     return rows;
 }
 
