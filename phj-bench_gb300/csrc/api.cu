@@ -1177,8 +1177,7 @@ static void run_phj_bep(phj_ctx * ctx, const phj_table & B, const phj_table & P,
     bl.next = lt.next;
     bl.leaf_bits = total_bits;
     bl.n_leaves = n_leaves;
-    bl.smem_cells = (uint32_t)std::min<uint64_t>(lt.uniform_log2cap >= 0 ? (1ull << lt.uniform_log2cap) : bit_ceil64(2ull * std::max<uint32_t>(lt.max_rows, 1)),
-                                                 8192);
+    bl.smem_cells = bep_smem_cells(lt);
     bl.wait_limit_ns = (uint64_t)ctx->wait_limit_ms * 1000000ull;
     bl.ctr = ctr;
     bl.queue = s.get<uint32_t>(n_leaves);
@@ -1771,8 +1770,7 @@ static void run_phj_bep_host(phj_ctx * ctx, const phj_block_stream & hb, const p
     bl.next = lt.next;
     bl.leaf_bits = total_bits;
     bl.n_leaves = n_leaves;
-    bl.smem_cells = (uint32_t)std::min<uint64_t>(lt.uniform_log2cap >= 0 ? (1ull << lt.uniform_log2cap) : bit_ceil64(2ull * std::max<uint32_t>(lt.max_rows, 1)),
-                                                 8192);
+    bl.smem_cells = bep_smem_cells(lt);
     bl.wait_limit_ns = (uint64_t)ctx->wait_limit_ms * 1000000ull;
     bl.ctr = ctr;
     bl.queue = s.get<uint32_t>(n_leaves);

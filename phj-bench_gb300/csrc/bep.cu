@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kBepNT) k_bep_build_warps(BepLeaves b, int * _
             const LeafMeta m = b.meta[L];
             if (m.has_table)
             {
-                cap = 1u << m.log2cap; // (at most smem_cells)
+                cap = 1u << m.log2cap;
                 off = m.table_off;
                 r0 = m.row_off;
                 r1 = b.leaf_off[L + 1];
@@ -216,14 +216,17 @@ __global__ void __launch_bounds__(kBepNT) k_bep_build_warps(BepLeaves b, int * _
             const uint32_t c = __shfl_sync(0xffffffffu, cap, i), q0 = __shfl_sync(0xffffffffu, r0, i), q1 = __shfl_sync(0xffffffffu, r1, i);
             Cell * out = b.cells + __shfl_sync(0xffffffffu, off, i);
             uint64_t k = q0 + lane < q1 ? b.build_keys[q0 + lane] : 0ull;
+            const bool in_smem = c <= b.smem_cells; // (otherwise in place, as above)
+            Cell * t = in_smem ? tab : out;
             for (uint32_t j = lane; j < c; j += 32)
-                reinterpret_cast<ulonglong2 *>(tab)[j] = make_ulonglong2(0ull, INVALID_REF);
+                reinterpret_cast<ulonglong2 *>(t)[j] = make_ulonglong2(0ull, INVALID_REF);
             __syncwarp();
             bool rep = false;
             for (uint32_t r = q0 + lane; r < q1; r += 32)
             {
                 const uint64_t ahead = r + 32 < q1 ? b.build_keys[r + 32] : 0ull;
-                const uint64_t prev = table_insert<true>(tab, c, int_hash64(k), k, make_ref(0, r));
+                const uint64_t h = int_hash64(k), ref = make_ref(0, r);
+                const uint64_t prev = in_smem ? table_insert<true>(t, c, h, k, ref) : table_insert<false>(t, c, h, k, ref);
                 b.next[r] = prev;
                 rep |= ref_valid(prev);
                 k = ahead;
@@ -231,8 +234,9 @@ __global__ void __launch_bounds__(kBepNT) k_bep_build_warps(BepLeaves b, int * _
             rep = __any_sync(0xffffffffu, rep);
             if ((int)lane == i)
                 dup = rep;
-            for (uint32_t j = lane; j < c; j += 32)
-                reinterpret_cast<ulonglong2 *>(out)[j] = reinterpret_cast<const ulonglong2 *>(tab)[j];
+            if (in_smem)
+                for (uint32_t j = lane; j < c; j += 32)
+                    reinterpret_cast<ulonglong2 *>(out)[j] = reinterpret_cast<const ulonglong2 *>(tab)[j];
             __syncwarp(); // the shared table is reused by the next leaf
         }
         // (BUILT needs no fence, as above)
@@ -276,10 +280,14 @@ void set_bep_smem_limits(int smem_optin)
                                   (int)std::min<size_t>((size_t)kBepSmemCellsMax * sizeof(Cell), (size_t)smem_optin - 1024)));
 }
 
+uint32_t bep_smem_cells(const LeafTables & lt)
+{
+    return (uint32_t)std::min<uint64_t>(lt.max_cells, kBepSmemCellsMax);
+}
+
 void bep_build_queue(phj_ctx * ctx, const BepLeaves & b)
 {
-    // smem_cells is at least the largest table's cells while that is no more
-    // than kBepSmemCellsMax, so up to kWarpCells every table fits a warp's
+    // (up to kWarpCells, smem_cells holds the largest table)
     const bool warps = b.smem_cells <= kWarpCells;
     const auto kernel = warps ? k_bep_build_warps : k_bep_build;
     const size_t smem = (size_t)b.smem_cells * sizeof(Cell) * (warps ? kBepNT / 32 : 1);

@@ -2036,8 +2036,7 @@ BepEngineResult bep_engine_run(phj_ctx * ctx, Scratch & s, const BepEngineInput 
     bl.next = a.next;
     bl.leaf_bits = a.total_bits;
     bl.n_leaves = a.n_leaves;
-    bl.smem_cells = (uint32_t)std::min<uint64_t>(
-        a.ulog >= 0 ? (1ull << a.ulog) : bit_ceil64(2ull * std::max<uint32_t>(in.lt->max_rows, 1)), 8192);
+    bl.smem_cells = bep_smem_cells(*in.lt);
     bl.wait_limit_ns = a.wait_limit_ns;
     bl.ctr = s.get<unsigned long long>(4);
     PHJ_CUDA(cudaMemsetAsync(bl.ctr, 0, 4 * sizeof(unsigned long long), ctx->stream));

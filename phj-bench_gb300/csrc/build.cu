@@ -630,6 +630,7 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
         lt.uniform_log2cap = uniform ? (int)(63 - __builtin_clzll(max_cap)) : -1;
         lt.total_cells = uniform ? uniform_cells : host[1];
     }
+    lt.max_cells = max_cap;
     lt.meta = s.get<LeafMeta>(n_leaves);
     lt.cells = s.get<Cell>(lt.total_cells);
     if (lazy)

@@ -318,6 +318,7 @@ struct LeafTables
     Cell * cells = nullptr;
     uint64_t * next = nullptr; // next-chain, one RowRefCell per build row (BlockStore next_chain_)
     uint64_t total_cells = 0;
+    uint64_t max_cells = 0; // cells of the largest table
     uint32_t max_rows = 0;
     int any_dup = 0;
     int uniform_log2cap = -1; // >= 0: every leaf table has 2^this cells at leaf << this
@@ -420,7 +421,7 @@ struct BepLeaves
     uint64_t * next;
     uint32_t leaf_bits;
     uint32_t n_leaves;
-    uint32_t smem_cells;          // tables up to this many cells are built in shared memory
+    uint32_t smem_cells;          // tables up to this many cells are built in shared memory (bep_smem_cells)
     uint64_t wait_limit_ns;
     unsigned long long * ctr;
     uint32_t * queue;             // n_leaves entries
@@ -434,6 +435,9 @@ struct BepLeaves
 bool bep_build_touched(phj_ctx * ctx, const BepLeaves & b);
 // The builds alone, of the leaves in b.queue (b.queue_len[0] of them, [1] zero).
 void bep_build_queue(phj_ctx * ctx, const BepLeaves & b);
+// BepLeaves::smem_cells for planned tables: the largest table's cells as they
+// were laid out, whatever the load factor, as far as shared memory takes them.
+uint32_t bep_smem_cells(const LeafTables & lt);
 void set_bep_smem_limits(int smem_optin);
 
 // ----- bep_engine.cu ------------------------------------------------------------------
