@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(kBepNT) k_bep_build_warps(BepLeaves b, int * _
             rep = __any_sync(0xffffffffu, rep);
             if ((int)lane == i)
                 dup = rep;
+            __syncwarp(); // every lane's inserts, before the table is copied out (a vote orders no memory)
             if (in_smem)
                 for (uint32_t j = lane; j < c; j += 32)
                     reinterpret_cast<ulonglong2 *>(out)[j] = reinterpret_cast<const ulonglong2 *>(tab)[j];
