@@ -210,8 +210,9 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *        joins return PHJ_ERR_CUDA right after the build shuffle, with
  *        their uploads still queued. */
 phj_status phj_ctx_set_int(phj_ctx *ctx, const char *name, int64_t value);
-/* Reads an option above, or a device property: "device", "num_sms",
- * "l2_bytes", "wait_limit_ms". */
+/* Reads an option above, a device property ("device", "num_sms",
+ * "l2_bytes"), or "scratch_bytes": the block of device memory the context
+ * keeps for the scratch of its calls. */
 phj_status phj_ctx_get_int(const phj_ctx *ctx, const char *name, int64_t *value);
 
 /* ---- radix configuration: src/CLI.cpp:330-355 ---------------------------- */

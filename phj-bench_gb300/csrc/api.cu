@@ -7,6 +7,7 @@
 #include <memory>
 #include <cstring>
 #include <new>
+#include <optional>
 
 namespace phjg
 {
@@ -174,7 +175,7 @@ void dfree(phj_ctx * ctx, void * p)
 void arena_release(phj_ctx * ctx) noexcept
 {
     ScratchArena & a = ctx->arena;
-    if (!a.base || a.depth)
+    if (!a.base || a.top)
         return;
     // work that reads it may be in flight: on the main stream, or on another
     // one when a call ended early
@@ -187,7 +188,7 @@ void arena_release(phj_ctx * ctx) noexcept
 void arena_begin(phj_ctx * ctx)
 {
     ScratchArena & a = ctx->arena;
-    a.used = a.asked = 0;
+    a.used = a.held = a.asked = 0;
     if (a.off || a.want <= a.size)
         return;
     // grown to what the last call asked for; what the pool kept for that
@@ -213,11 +214,10 @@ void arena_begin(phj_ctx * ctx)
 void arena_end(phj_ctx * ctx) noexcept
 {
     ScratchArena & a = ctx->arena;
-    // an eighth and 2 MiB more than asked for, so that a little more the
+    // an eighth and 2 MiB more than was held, so that a little more the
     // next time is no new growth
     if (!a.off && a.asked > a.size)
         a.want = std::min<size_t>(a.asked + a.asked / 8 + (2 << 20), a.most) & ~size_t(255);
-    a.used = 0;
 }
 
 void reset_accounting(phj_ctx * ctx)
@@ -882,6 +882,7 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
     Cols btmp = total_bits > 11 ? alloc_cols_like(s, B.schema, B.rows) : bpart;
     uint32_t * leaf_off = s.get<uint32_t>((uint64_t)n_leaves + 1);
     LeafTables lt;
+    std::optional<Scratch> st; // the tables'
     bool grouped = false;
     phj_output * o = nullptr;
     auto fill_tables = [&](ProbeArgs & x) {
@@ -995,10 +996,11 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
         ctx->stream = main_stream;
 
         // -------- BUILD: per-leaf tables (src/PHJ.cpp:260-282) --------
-        lt.next = s.get<uint64_t>(B.rows);
+        st.emplace(ctx); // tables that cannot be used go back at once
+        lt.next = st->get<uint64_t>(B.rows);
         // (grouping needs a place for the payloads: the partition's temporary)
         const Cols * group_dst = btmp.keys != bpart.keys ? &btmp : nullptr;
-        build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows, group_dst);
+        build_leaf_tables(ctx, *st, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows, group_dst);
         if (lt.estimated)
         {
             // the one-pass probe goes ahead; when the tables turn out not
@@ -1014,15 +1016,17 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
                 PHJ_CUDA(cudaStreamWaitEvent(ctx->stream, ev[8], 0));
                 PHJ_CUDA(cudaEventRecord(ev[3], ctx->stream));
                 fill_tables(a);
-                o = probe_estimated(ctx, s, a, B.schema, P.schema, lt.flags, found);
+                o = probe_estimated(ctx, *st, a, B.schema, P.schema, lt.flags, found);
                 if (o)
                     return finish(o, &found);
             }
             if (found.flags & kLeafOverflow)
             {
                 lt = LeafTables{};
-                lt.next = s.get<uint64_t>(B.rows);
-                build_leaf_tables(ctx, s, bpart, leaf_off, n_leaves, lt, false, 0, group_dst);
+                st.reset();
+                st.emplace(ctx);
+                lt.next = st->get<uint64_t>(B.rows);
+                build_leaf_tables(ctx, *st, bpart, leaf_off, n_leaves, lt, false, 0, group_dst);
             }
             else
                 lt.any_dup = found.flags & kLeafRepeats;
@@ -2107,6 +2111,8 @@ phj_status phj_ctx_get_int(const phj_ctx * ctx, const char * name, int64_t * val
         *value = ctx->num_sms;
     else if (std::strcmp(name, "l2_bytes") == 0)
         *value = (int64_t)ctx->l2_bytes;
+    else if (std::strcmp(name, "scratch_bytes") == 0)
+        *value = (int64_t)ctx->arena.size;
     else
         return PHJ_ERR_INVALID_ARGUMENT;
     return PHJ_OK;

@@ -86,23 +86,25 @@ struct SmallResult // at the start of the context's mapped host buffer
 {
     unsigned long long out_rows;
 };
+struct Scratch;
 struct BatchGraph; // batch.cu: phj_batch_run's workspace and captured chain
 void free_batch_graph(phj_ctx * ctx);
 } // namespace phjg
 
 // Scratch memory of a call, kept by the context between calls: one block that
-// a call's scratch buffers are cut from and that is empty again when the call
-// ends.  (From the stream-ordered pool every buffer cost a microsecond or two,
+// a call's scratch buffers are cut from as from a stack and that is empty
+// again when the call ends.  (From the stream-ordered pool every buffer cost a microsecond or two,
 // and large ones, and the outputs allocated among them, did not find their
 // place again from call to call: the pool mapped memory anew, 0.2 to 1.6 ms.)
 struct ScratchArena
 {
     uint8_t * base = nullptr;
     size_t size = 0, used = 0;
-    size_t asked = 0;  // bytes asked for in this call, with those past `size`
+    size_t held = 0;   // scratch bytes held now, with those from the pool
+    size_t asked = 0;  // the most held at a time in this call
     size_t want = 0;   // size for the next call
     size_t most = 0;   // bound of `size`
-    int depth = 0;     // Scratch objects alive
+    phjg::Scratch * top = nullptr; // innermost Scratch alive
     bool off = false;  // this call runs from the pool alone
 };
 
@@ -218,26 +220,47 @@ void arena_end(phj_ctx * ctx) noexcept;
 void arena_release(phj_ctx * ctx) noexcept;
 
 // RAII holder for run-scoped scratch: cut from the context's arena while it
-// has room (given back when the call's first Scratch ends), else from the
-// pool.
+// has room, else from the pool.  Scratch objects end in the reverse order of
+// their making, and an ending one's buffers are free for the next: what ran
+// on them is ordered before what comes, as it is for buffers that go back to
+// the pool (both in the main stream's order; other streams wait for an event
+// of it before they touch a buffer taken later).  A buffer that an outer
+// Scratch took meanwhile lies above them in the arena; they then go back with
+// the next outer one.
 struct Scratch
 {
     phj_ctx * ctx;
-    std::vector<void *> ptrs; // from the pool
-    uint64_t cut = 0;         // bytes from the arena
+    Scratch * outer;
+    std::vector<void *> ptrs;  // from the pool
+    uint64_t cut = 0;          // bytes from the arena
+    uint64_t pooled = 0;       // bytes from the pool
+    size_t mark = 0;           // the arena's bytes in use before
+    bool covered = false;      // an outer Scratch's buffer lies above
     explicit Scratch(phj_ctx * c)
         : ctx(c)
+        , outer(c->arena.top)
     {
-        if (ctx->arena.depth == 0)
+        if (!outer)
             arena_begin(ctx);
-        ++ctx->arena.depth;
+        mark = ctx->arena.used;
+        ctx->arena.top = this;
     }
     ~Scratch()
     {
+        ScratchArena & a = ctx->arena;
         for (void * p : ptrs)
             dfree(ctx, p);
-        ctx->cur_bytes -= cut;
-        if (--ctx->arena.depth == 0)
+        a.held -= pooled;
+        a.top = outer;
+        if (covered && outer)
+            outer->cut += cut;
+        else
+        {
+            a.used = mark;
+            a.held -= cut;
+            ctx->cur_bytes -= cut;
+        }
+        if (!outer)
             arena_end(ctx);
     }
     template <class T>
@@ -245,19 +268,26 @@ struct Scratch
     {
         const size_t bytes = ((size_t)(n ? n : 1) * sizeof(T) + 255) & ~size_t(255);
         ScratchArena & a = ctx->arena;
-        a.asked += bytes;
+        T * p;
         if (!a.off && bytes <= a.size - a.used)
         {
-            T * p = reinterpret_cast<T *>(a.base + a.used);
+            for (Scratch * t = a.top; t != this; t = t->outer)
+                t->covered = true;
+            p = reinterpret_cast<T *>(a.base + a.used);
             a.used += bytes;
             cut += bytes;
             ctx->cur_bytes += bytes;
             ctx->peak_bytes = std::max(ctx->peak_bytes, ctx->cur_bytes);
-            return p;
         }
-        ptrs.reserve(ptrs.size() + 1);
-        T * p = static_cast<T *>(dalloc(ctx, bytes));
-        ptrs.push_back(p);
+        else
+        {
+            ptrs.reserve(ptrs.size() + 1);
+            p = static_cast<T *>(dalloc(ctx, bytes));
+            ptrs.push_back(p);
+            pooled += bytes;
+        }
+        a.held += bytes;
+        a.asked = std::max(a.asked, a.held);
         return p;
     }
     Scratch(const Scratch &) = delete;

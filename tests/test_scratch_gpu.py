@@ -1,0 +1,53 @@
+"""The scratch memory a context keeps between calls ("scratch_bytes"): it is
+sized by what a call holds at a time, so the scratch of one step is the next
+one's again."""
+import numpy as np
+import pytest
+
+import oracle as O
+import phj_datagen as G
+import phj_gpu as P
+
+pytestmark = pytest.mark.gpu
+
+
+def sides(ctx, build, probe, repeat=1, types=(P.U64,)):
+    distinct = build // repeat
+    bk = np.resize(G.gen_keys(0, distinct, 901, 902), build)
+    b = P.BlockStream(list(types), bk, G.payload_columns(903, list(types), build))
+    p = P.BlockStream([P.U32], G.gen_keys(4, probe, 904, 902, domain=distinct, match_permille=500), G.payload_columns(905, [P.U32], probe))
+    return b, p, ctx.upload(b), ctx.upload(p)
+
+
+def kept(options, build, probe, call, repeat=1):
+    """The block a new context keeps once a first call has said how much it
+    needs: it is there for the second, and the third finds it large enough."""
+    with P.Context(0) as c:
+        for k, v in options.items():
+            c.set_int(k, v)
+        b, p, t, u = sides(c, build, probe, repeat)
+        fp = O.join_fingerprint(b, p)
+        sizes = []
+        for _ in range(3):
+            out, _ = call(c, t, u)
+            sizes.append(c.get_int("scratch_bytes"))
+            assert tuple(out.fingerprint()) == tuple(fp)
+            out.free()
+        t.free(), u.free()
+        assert sizes[0] == 0 and sizes[1] == sizes[2] > 0
+        return sizes[2]
+
+
+def test_batches_use_the_same_scratch():
+    # 24 batches of 1 MiB keep no more than 3 do
+    call = lambda c, t, u: c.run_phj_bep(t, u, [6, 6], 1)  # noqa: E731
+    few, many = (kept({"bep_engine": 1}, 100_000, n, call) for n in (262_144, 2_097_152))
+    assert many == few
+
+
+def test_tables_that_cannot_be_used_go_back():
+    # repeated keys: the tables tried first (one 8-byte payload in the cells)
+    # are not held beside the ones that are used
+    call = lambda c, t, u: c.run_phj_pure(t, u, [12])  # noqa: E731
+    tried, plain = (kept({"probe_materialize": 0, "pack_build": pack}, 1 << 20, 1 << 20, call, repeat=4) for pack in (1, 0))
+    assert tried <= plain * 1.01
