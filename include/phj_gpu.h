@@ -208,7 +208,10 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *        the run fails with PHJ_ERR_DEVICE_TIMEOUT;
  *   "test_fail_build": test hook, 0 (default) off; 1 makes the host-buffer
  *        joins return PHJ_ERR_CUDA right after the build shuffle, with
- *        their uploads still queued. */
+ *        their uploads still queued;
+ *   "test_memory_limit_mib": test hook, 0 (default) off; an allocation that
+ *        takes the device memory this context holds (tables, outputs,
+ *        scratch) past so many MiB fails as out of memory. */
 phj_status phj_ctx_set_int(phj_ctx *ctx, const char *name, int64_t value);
 /* Reads an option above, a device property ("device", "num_sms",
  * "l2_bytes"), or "scratch_bytes": the block of device memory the context

@@ -85,11 +85,16 @@ float event_ms(cudaEvent_t a, cudaEvent_t b)
 // ---------------------------------------------------------------------------
 // allocation: the context's stream-ordered pool, with per-run accounting
 // ---------------------------------------------------------------------------
+static bool over_test_limit(const phj_ctx * ctx, size_t bytes)
+{
+    return ctx->test_memory_limit && ctx->device_bytes + bytes > ctx->test_memory_limit;
+}
+
 void * dalloc(phj_ctx * ctx, size_t bytes)
 {
     void * p = nullptr;
     const size_t rounded = (bytes + 255) & ~size_t(255);
-    const cudaError_t e = cudaMallocFromPoolAsync(&p, rounded, ctx->pool, ctx->stream);
+    const cudaError_t e = over_test_limit(ctx, rounded) ? cudaErrorMemoryAllocation : cudaMallocFromPoolAsync(&p, rounded, ctx->pool, ctx->stream);
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -98,6 +103,7 @@ void * dalloc(phj_ctx * ctx, size_t bytes)
         throw Error(PHJ_ERR_OUT_OF_MEMORY, buf);
     }
     ctx->live.emplace_back(p, rounded);
+    ctx->device_bytes += rounded;
     ctx->cur_bytes += rounded;
     ctx->peak_bytes = std::max(ctx->peak_bytes, ctx->cur_bytes);
     return p;
@@ -165,6 +171,7 @@ void dfree(phj_ctx * ctx, void * p)
         if (ctx->live[i].first == p)
         {
             ctx->cur_bytes -= ctx->live[i].second;
+            ctx->device_bytes -= ctx->live[i].second;
             ctx->live[i] = ctx->live.back();
             ctx->live.pop_back();
             break;
@@ -181,8 +188,18 @@ void arena_release(phj_ctx * ctx) noexcept
     // one when a call ended early
     cudaDeviceSynchronize();
     cudaFree(a.base);
+    ctx->device_bytes -= a.size;
     a.base = nullptr;
     a.size = a.used = 0;
+}
+
+void arena_retreat(phj_ctx * ctx) noexcept
+{
+    ScratchArena & a = ctx->arena;
+    a.most = std::max(a.size, a.want) / 2;
+    a.calls = 0;
+    arena_release(ctx);
+    a.want = 0;
 }
 
 void arena_begin(phj_ctx * ctx)
@@ -196,17 +213,18 @@ void arena_begin(phj_ctx * ctx)
     arena_release(ctx);
     cudaMemPoolTrimTo(ctx->pool, 0);
     void * p = nullptr;
-    if (cudaMalloc(&p, a.want) == cudaSuccess)
+    if (!over_test_limit(ctx, a.want) && cudaMalloc(&p, a.want) == cudaSuccess)
     {
         a.base = static_cast<uint8_t *>(p);
         a.size = a.want;
+        ctx->device_bytes += a.size;
     }
     else
     {
         // no room: this call's scratch comes from the pool, and a next
         // attempt asks for less
         cudaGetLastError();
-        a.most = a.want / 2;
+        arena_retreat(ctx);
     }
     a.want = a.size;
 }
@@ -214,9 +232,16 @@ void arena_begin(phj_ctx * ctx)
 void arena_end(phj_ctx * ctx) noexcept
 {
     ScratchArena & a = ctx->arena;
+    if (a.off)
+        return;
+    if (a.most < a.bound && ++a.calls >= 64)
+    {
+        a.most = std::min(a.bound, std::max<size_t>(a.most, 1 << 20) * 2);
+        a.calls = 0;
+    }
     // an eighth and 2 MiB more than was held, so that a little more the
     // next time is no new growth
-    if (!a.off && a.asked > a.size)
+    if (a.asked > a.size)
         a.want = std::min<size_t>(a.asked + a.asked / 8 + (2 << 20), a.most) & ~size_t(255);
 }
 
@@ -1945,7 +1970,7 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         ctx->num_sms = prop.multiProcessorCount;
         ctx->smem_optin = prop.sharedMemPerBlockOptin;
         ctx->l2_bytes = prop.l2CacheSize;
-        ctx->arena.most = prop.totalGlobalMem / 4;
+        ctx->arena.most = ctx->arena.bound = prop.totalGlobalMem / 4;
         // the main stream goes first: its kernels take the SMs as the side
         // stream's short CTAs end (probe side's first pass, see k_scatter)
         int prio_least = 0, prio_greatest = 0;
@@ -2064,6 +2089,8 @@ phj_status phj_ctx_set_int(phj_ctx * ctx, const char * name, int64_t value)
         ctx->test_engine_stall_wave = value;
     else if (std::strcmp(name, "test_fail_build") == 0 && (value == 0 || value == 1))
         ctx->test_fail_build = (int)value;
+    else if (std::strcmp(name, "test_memory_limit_mib") == 0 && value >= 0 && value < (1ll << 40))
+        ctx->test_memory_limit = (uint64_t)value << 20;
     else
         return PHJ_ERR_INVALID_ARGUMENT;
     return PHJ_OK;
@@ -2105,6 +2132,8 @@ phj_status phj_ctx_get_int(const phj_ctx * ctx, const char * name, int64_t * val
         *value = ctx->test_engine_stall_wave;
     else if (std::strcmp(name, "test_fail_build") == 0)
         *value = ctx->test_fail_build;
+    else if (std::strcmp(name, "test_memory_limit_mib") == 0)
+        *value = (int64_t)(ctx->test_memory_limit >> 20);
     else if (std::strcmp(name, "device") == 0)
         *value = ctx->device;
     else if (std::strcmp(name, "num_sms") == 0)

@@ -103,7 +103,9 @@ struct ScratchArena
     size_t held = 0;   // scratch bytes held now, with those from the pool
     size_t asked = 0;  // the most held at a time in this call
     size_t want = 0;   // size for the next call
-    size_t most = 0;   // bound of `size`
+    size_t most = 0;   // bound of `size`: `bound`, less after a call ran out of memory
+    size_t bound = 0;
+    uint32_t calls = 0; // since `most` was lowered
     phjg::Scratch * top = nullptr; // innermost Scratch alive
     bool off = false;  // this call runs from the pool alone
 };
@@ -125,6 +127,7 @@ struct phj_ctx
     uint64_t launches = 0;
     // Allocation accounting of the current run (peak_mem_bytes).
     uint64_t cur_bytes = 0, peak_bytes = 0;
+    uint64_t device_bytes = 0; // held now, the arena's whole block included
     std::vector<std::pair<void *, uint64_t>> live; // small: a run holds tens of buffers
     ScratchArena arena;
     // Per-kernel timing of the last run.
@@ -155,6 +158,7 @@ struct phj_ctx
     int64_t test_stuck_leaf = -1; // test hook: PHJ/BEP leaf left BUILDING before the probe
     int64_t test_engine_stall_wave = -1; // test hook: a BEP engine group holds back from this wave's barrier
     int test_fail_build = 0;      // test hook: host-buffer joins fail on the host after the build shuffle
+    uint64_t test_memory_limit = 0; // test hook: device_bytes past this are out of memory (0: off)
     LeafMark leaf_mark;           // consumed by the next first radix pass
 };
 
@@ -218,6 +222,9 @@ void arena_begin(phj_ctx * ctx);
 void arena_end(phj_ctx * ctx) noexcept;
 // Gives the arena's memory back (no call may be using it).
 void arena_release(phj_ctx * ctx) noexcept;
+// The same after a call ran out of memory beside it: the next calls keep at
+// most half as much, twice that again after each 64 that did not.
+void arena_retreat(phj_ctx * ctx) noexcept;
 
 // RAII holder for run-scoped scratch: cut from the context's arena while it
 // has room, else from the pool.  Scratch objects end in the reverse order of
@@ -622,7 +629,7 @@ inline phj_status guard(phj_ctx * ctx, F && f)
             // out of memory while the arena holds some: once more without it
             if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || !ctx->arena.base)
                 throw;
-            arena_release(ctx);
+            arena_retreat(ctx);
             struct Off
             {
                 phj_ctx * c;

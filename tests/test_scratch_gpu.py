@@ -1,6 +1,6 @@
 """The scratch memory a context keeps between calls ("scratch_bytes"): it is
 sized by what a call holds at a time, so the scratch of one step is the next
-one's again."""
+one's again, and a call that runs out of memory beside it goes on without."""
 import numpy as np
 import pytest
 
@@ -51,3 +51,31 @@ def test_tables_that_cannot_be_used_go_back():
     call = lambda c, t, u: c.run_phj_pure(t, u, [12])  # noqa: E731
     tried, plain = (kept({"probe_materialize": 0, "pack_build": pack}, 1 << 20, 1 << 20, call, repeat=4) for pack in (1, 0))
     assert tried <= plain * 1.01
+
+
+def test_a_call_out_of_memory_beside_the_block_is_run_again_once():
+    # a large join's block, then a join whose output does not fit beside it
+    # but does without it: the first call is run again, the later ones are not
+    with P.Context(0) as c:
+        c.set_int("probe_materialize", 0)
+        _, _, t, u = sides(c, 1 << 21, 1 << 12)
+        for _ in range(3):
+            c.run_phj_pure(t, u, [12])[0].free()
+        block = c.get_int("scratch_bytes")
+        assert block > (64 << 20)
+        t.free(), u.free()
+        b, p, t, u = sides(c, 1 << 18, 1 << 20)
+        fp = tuple(O.join_fingerprint(b, p))
+        inputs = (1 << 18) * 16 + (1 << 20) * 12
+        out = (1 << 20) * 20
+        c.set_int("test_memory_limit_mib", (inputs + out + block - (8 << 20)) >> 20)
+        launches = []
+        for _ in range(6):
+            n0 = c.launch_count()
+            o, _ = c.run_phj_pure(t, u, [10])
+            launches.append(c.launch_count() - n0)
+            assert tuple(o.fingerprint()) == fp
+            o.free()
+        c.set_int("test_memory_limit_mib", 0)
+        assert launches[0] > launches[1] and launches[1:] == [launches[1]] * 5, launches
+        t.free(), u.free()
