@@ -184,10 +184,9 @@ void arena_release(phj_ctx * ctx) noexcept
     ScratchArena & a = ctx->arena;
     if (!a.base || a.top)
         return;
-    // work that reads it may be in flight: on the main stream, or on another
-    // one when a call ended early
-    cudaDeviceSynchronize();
-    cudaFree(a.base);
+    // (in the main stream's order: a call ends, also early, only when its
+    // other streams' work is done or waited for)
+    cudaFreeAsync(a.base, ctx->stream);
     ctx->device_bytes -= a.size;
     a.base = nullptr;
     a.size = a.used = 0;
@@ -208,12 +207,13 @@ void arena_begin(phj_ctx * ctx)
     a.used = a.held = a.asked = 0;
     if (a.off || a.want <= a.size)
         return;
-    // grown to what the last call asked for; what the pool kept for that
-    // call goes back first
+    // grown to what the last call held; what the pool kept for that call goes
+    // back first.  Only this context's streams are waited for.
     arena_release(ctx);
+    cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
     void * p = nullptr;
-    if (!over_test_limit(ctx, a.want) && cudaMalloc(&p, a.want) == cudaSuccess)
+    if (!over_test_limit(ctx, a.want) && cudaMallocFromPoolAsync(&p, a.want, ctx->pool, ctx->stream) == cudaSuccess)
     {
         a.base = static_cast<uint8_t *>(p);
         a.size = a.want;

@@ -79,3 +79,25 @@ def test_a_call_out_of_memory_beside_the_block_is_run_again_once():
         c.set_int("test_memory_limit_mib", 0)
         assert launches[0] > launches[1] and launches[1:] == [launches[1]] * 5, launches
         t.free(), u.free()
+
+
+def test_growing_the_block_waits_for_no_other_stream():
+    torch = pytest.importorskip("torch")
+    with P.Context(0) as c:
+        small, large = (sides(c, n, 4 * n) for n in (1 << 17, 1 << 20))
+        for s in (small, large):  # every kernel once, and the first block's size
+            c.run_phj_pure(s[2], s[3], [10])[0].free()
+        c.run_phj_pure(small[2], small[3], [10])[0].free()
+        before = c.get_int("scratch_bytes")
+        huge = sides(c, 1 << 21, 1 << 22)
+        c.run_phj_pure(huge[2], huge[3], [10])[0].free()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(1_000_000_000)  # about half a second
+            done = torch.cuda.Event()
+            done.record()
+        c.run_phj_pure(huge[2], huge[3], [10])[0].free()
+        assert not done.query()
+        assert c.get_int("scratch_bytes") > before
+        torch.cuda.synchronize()
+        for s in (small, large, huge):
+            s[2].free(), s[3].free()
