@@ -100,7 +100,7 @@ typedef struct phj_chj_result {
     phj_phase_timing build;
     phj_phase_timing probe;
     double e2e_wall_ms;
-    uint64_t peak_mem_bytes; /* peak device bytes held by the run */
+    uint64_t peak_mem_bytes; /* peak device bytes held by the run (of the context's kept scratch, what the run used) */
 } phj_chj_result;
 
 /* PhjResult minus the output, src/PHJ.h:13-22. */
@@ -144,9 +144,18 @@ typedef struct phj_output phj_output; /* a device-resident JoinOutput (src/JoinO
 
 /* ---- context ---------------------------------------------------------- */
 
-/* Opens `device`, creates the context's stream and stream-ordered pool. */
+/* Opens `device`, creates the context's stream and stream-ordered pool.
+ * What a call frees stays with the context for its next calls: the pool's
+ * memory, and one block for the calls' scratch, sized by the most that a call
+ * held of it and an eighth more, at most a quarter of the device's memory.
+ * The block grows at the start of the call after the one that needed more,
+ * which then waits for this context's stream; a call that runs out of memory
+ * beside the block runs again without it. */
 phj_status phj_ctx_create(int device, phj_ctx **out);
 void phj_ctx_destroy(phj_ctx *ctx);
+/* Waits for the context's stream and gives that memory back to the device
+ * (tables and outputs stay).  The next calls take theirs anew. */
+phj_status phj_ctx_trim(phj_ctx *ctx);
 /* Message of the last failing call on this context ("" if none). */
 const char *phj_last_error(const phj_ctx *ctx);
 uint32_t phj_abi_version(void);

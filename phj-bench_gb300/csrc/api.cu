@@ -201,6 +201,14 @@ void arena_retreat(phj_ctx * ctx) noexcept
     a.want = 0;
 }
 
+// What both pools hold free, back to the device.
+static void pools_trim(phj_ctx * ctx)
+{
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    cudaMemPoolTrimTo(ctx->scratch_pool, 0);
+}
+
 void arena_begin(phj_ctx * ctx)
 {
     ScratchArena & a = ctx->arena;
@@ -210,10 +218,9 @@ void arena_begin(phj_ctx * ctx)
     // grown to what the last call held; what the pool kept for that call goes
     // back first.  Only this context's streams are waited for.
     arena_release(ctx);
-    cudaStreamSynchronize(ctx->stream);
-    cudaMemPoolTrimTo(ctx->pool, 0);
+    pools_trim(ctx);
     void * p = nullptr;
-    if (!over_test_limit(ctx, a.want) && cudaMallocFromPoolAsync(&p, a.want, ctx->pool, ctx->stream) == cudaSuccess)
+    if (!over_test_limit(ctx, a.want) && cudaMallocFromPoolAsync(&p, a.want, ctx->scratch_pool, ctx->stream) == cudaSuccess)
     {
         a.base = static_cast<uint8_t *>(p);
         a.size = a.want;
@@ -1980,9 +1987,12 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         pp.allocType = cudaMemAllocationTypePinned;
         pp.location.type = cudaMemLocationTypeDevice;
         pp.location.id = device;
-        PHJ_CUDA(cudaMemPoolCreate(&ctx->pool, &pp));
         uint64_t keep = ~0ull; // keep freed memory in the pool across runs
-        PHJ_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        for (cudaMemPool_t * pool : {&ctx->pool, &ctx->scratch_pool})
+        {
+            PHJ_CUDA(cudaMemPoolCreate(pool, &pp));
+            PHJ_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
         PHJ_CUDA(cudaMalloc(&ctx->d_err, sizeof(int)));
         PHJ_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
         PHJ_CUDA(cudaMalloc(&ctx->small_ctr, sizeof(SmallCounters)));
@@ -2027,8 +2037,9 @@ void phj_ctx_destroy(phj_ctx * ctx)
             cudaFreeAsync(lv.first, ctx->stream);
         if (ctx->stream)
             cudaStreamSynchronize(ctx->stream);
-        if (ctx->pool)
-            cudaMemPoolDestroy(ctx->pool);
+        for (cudaMemPool_t pool : {ctx->pool, ctx->scratch_pool})
+            if (pool)
+                cudaMemPoolDestroy(pool);
         if (ctx->stream)
             cudaStreamDestroy(ctx->stream);
         if (ctx->h2d)
@@ -2041,6 +2052,18 @@ void phj_ctx_destroy(phj_ctx * ctx)
             cudaStreamDestroy(ctx->aux);
     }
     delete ctx;
+}
+
+phj_status phj_ctx_trim(phj_ctx * ctx)
+{
+    if (!ctx)
+        return PHJ_ERR_INVALID_ARGUMENT;
+    return guard(ctx, [&] {
+        arena_release(ctx);
+        ctx->arena.want = 0;
+        pools_trim(ctx);
+        PHJ_CUDA(cudaGetLastError());
+    });
 }
 
 const char * phj_last_error(const phj_ctx * ctx)

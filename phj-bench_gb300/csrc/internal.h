@@ -123,6 +123,7 @@ struct phj_ctx
     cudaStream_t side = nullptr;               // second compute stream: probe-side first pass beside the build
     cudaStream_t aux = nullptr;                // third compute stream: build payload packing beside the leaf tables
     cudaMemPool_t pool = nullptr;
+    cudaMemPool_t scratch_pool = nullptr; // the arena's block alone, so that all of it goes back when it is freed
     std::string last_error;
     uint64_t launches = 0;
     // Allocation accounting of the current run (peak_mem_bytes).

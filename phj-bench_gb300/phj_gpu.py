@@ -128,6 +128,7 @@ def load() -> C.CDLL:
         "phj_abi_version": (C.c_uint32, []),
         "phj_ctx_create": (C.c_int, [C.c_int, C.POINTER(P)]),
         "phj_ctx_destroy": (None, [P]),
+        "phj_ctx_trim": (C.c_int, [P]),
         "phj_last_error": (C.c_char_p, [P]),
         "phj_ctx_stream": (P, [P]),
         "phj_ctx_set_int": (C.c_int, [P, C.c_char_p, C.c_int64]),
@@ -389,6 +390,10 @@ class Context:
             self._pinned = []
             self.lib.phj_ctx_destroy(self.ptr)
             self.ptr = None
+
+    def trim(self):
+        """Gives the memory the context keeps between calls back to the device."""
+        self._check(self.lib.phj_ctx_trim(self.ptr))
 
     def __enter__(self):
         return self

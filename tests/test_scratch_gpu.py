@@ -101,3 +101,26 @@ def test_growing_the_block_waits_for_no_other_stream():
         torch.cuda.synchronize()
         for s in (small, large, huge):
             s[2].free(), s[3].free()
+
+
+def test_trim_gives_the_kept_memory_back():
+    torch = pytest.importorskip("torch")
+    with P.Context(0) as c:
+        b, p, t, u = sides(c, 1 << 21, 1 << 23)
+        fp = tuple(O.join_fingerprint(b, p))
+        for _ in range(3):
+            c.run_phj_pure(t, u, [12])[0].free()
+        out, _ = c.run_phj_pure(t, u, [12])
+        block = c.get_int("scratch_bytes")
+        assert block > (64 << 20)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        c.trim()
+        assert c.get_int("scratch_bytes") == 0
+        assert torch.cuda.mem_get_info()[0] >= free + block - (4 << 20)
+        assert tuple(out.fingerprint()) == fp
+        out.free()
+        out, _ = c.run_phj_pure(t, u, [12])
+        assert tuple(out.fingerprint()) == fp
+        for o in (out, t, u):
+            o.free()
