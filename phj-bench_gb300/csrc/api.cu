@@ -791,7 +791,23 @@ static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj
     // (8K x 128K, four rows a key: 103 us in two launches against 180; 8K x
     // 512K: 190 against 182).
     const bool repeats_ok = P.rows <= 400000;
-    phj_output * o = new_output(ctx, B.schema, P.schema, P.rows);
+    // (the general path sizes its output exactly where keys repeat or the
+    // payloads do not suit the one-pass probe: few matches may fit there)
+    auto output = [&](uint64_t cap) -> phj_output * {
+        try
+        {
+            return new_output(ctx, B.schema, P.schema, cap);
+        }
+        catch (const Error & e)
+        {
+            if (e.status != PHJ_ERR_OUT_OF_MEMORY)
+                throw;
+            return nullptr;
+        }
+    };
+    phj_output * o = output(P.rows);
+    if (!o)
+        return nullptr;
     for (int run = 0;; ++run)
     {
         uint64_t rows = 0;
@@ -814,7 +830,9 @@ static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj
         if (run == 1 || rows == kSmallJoinRepeats)
             return nullptr;
         ev[2] = take_event(ctx);
-        o = new_output(ctx, B.schema, P.schema, rows);
+        o = output(rows);
+        if (!o)
+            return nullptr;
     }
 }
 

@@ -56,3 +56,21 @@ def test_rows_equal_the_oracle(ctx, build, probe, tb, tp, repeat, match):
             assert O.compare_outputs(expected, O.serialize_output(out.download())) == ""
             out.free()
     t.free(), u.free()
+
+
+def test_an_output_of_the_probe_rows_does_not_fit():
+    # few of the rows match, and memory holds the join's rows but not one for
+    # each probe row: the general path counts them first
+    with P.Context(0) as c:
+        tb, tp = [P.U128, P.U128], [P.U32]
+        b, p = sides(1000, 4_000_000, tb, tp, 1, 20)
+        expected = O.join_rows(b, p)
+        t, u = c.upload(b), c.upload(p)
+        inputs = 1000 * 40 + 4_000_000 * 12
+        c.set_int("test_memory_limit_mib", (inputs >> 20) + 100)  # (one row each: 168 MiB)
+        for _ in range(2):
+            out, _ = c.run_phj_pure(t, u, [6])
+            assert "small_join" not in {k["name"] for k in c.kernel_times()}
+            assert O.compare_outputs(expected, O.serialize_output(out.download())) == ""
+            out.free()
+        t.free(), u.free()
