@@ -827,7 +827,8 @@ static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj
             return o;
         }
         free_output(ctx, o);
-        if (run == 1 || rows == kSmallJoinRepeats)
+        // (a join of 2^32 rows or more is the general path's to refuse)
+        if (run == 1 || rows == kSmallJoinRepeats || rows >= (1ull << 32))
             return nullptr;
         ev[2] = take_event(ctx);
         o = output(rows);

@@ -74,3 +74,14 @@ def test_an_output_of_the_probe_rows_does_not_fit():
             assert O.compare_outputs(expected, O.serialize_output(out.download())) == ""
             out.free()
         t.free(), u.free()
+
+
+@pytest.mark.parametrize("scheme", ["pure", "chj"])
+def test_a_join_of_2_32_rows_is_refused(ctx, scheme):
+    # one key on both sides: 65,536 x 70,000 output rows
+    t = ctx.upload(P.BlockStream([P.U32], np.full(65_536, 9, np.uint64), [np.arange(65_536, dtype=np.uint32)]))
+    u = ctx.upload(P.BlockStream([], np.full(70_000, 9, np.uint64), []))
+    with pytest.raises(P.PhjError) as e:
+        ctx.run_phj_pure(t, u, [6]) if scheme == "pure" else ctx.run_chj(t, u)
+    assert e.value.status == P.ERR_CAPACITY and str(65_536 * 70_000) in str(e.value)
+    t.free(), u.free()
