@@ -191,17 +191,17 @@ __global__ void __launch_bounds__(kNT, 2) k_bt_scatter(const BatchJoin * __restr
 }
 
 // The CTA's warps probe rows [p0, p1) of the partition, 128 a warp at a time.
-template <bool kDup>
+template <Repeats kRepeats>
 __device__ __forceinline__ void probe_part(const ProbeSides & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable<kPieceRows> & tab,
                                            unsigned long long * out_cur, int * over)
 {
-    probe_piece<kDup, 4>(J, p0 + (threadIdx.x >> 5) * 128, kJNT / 32 * 128, p1, c0, tab, out_cur, over);
+    probe_piece<kRepeats, 4>(J, p0 + (threadIdx.x >> 5) * 128, kJNT / 32 * 128, p1, c0, tab, out_cur, over);
 }
 // (out of line, so that its registers do not weigh on the unique-key form)
 __device__ __noinline__ void probe_part_dup(const ProbeSides & J, uint32_t p0, uint32_t p1, uint32_t c0, const PieceTable<kPieceRows> tab,
                                             unsigned long long * out_cur, int * over)
 {
-    probe_part<true>(J, p0, p1, c0, tab, out_cur, over);
+    probe_part<kLaneWrites>(J, p0, p1, c0, tab, out_cur, over);
 }
 
 // The persistent join: CTAs pop (join, partition) items until the queue is
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kJNT, 4) k_bt_join(const BatchJoin * __restric
     __shared__ uint16_t nxt[kPieceRows];
     __shared__ BatchJoin J; // the item's join
     __shared__ uint32_t s_item;
-    __shared__ int s_dup;
+    __shared__ int s_linked;
     const uint32_t n = *d_n;
     const uint64_t n_items = parts[n];
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -258,12 +258,12 @@ __global__ void __launch_bounds__(kJNT, 4) k_bt_join(const BatchJoin * __restric
             const uint32_t cap = max(4u, min(kPieceSlots, (uint32_t)bit_ceil64(3ull * rows))), mask = cap - 1;
             if (c0 != b0)
                 __syncthreads(); // the last piece is no longer probed
-            build_piece<kPieceRows, kJNT>(J.part.build.keys + c0, rows, slots, bkeys, nxt, mask, &s_dup);
+            build_piece<kPieceRows, kJNT, false>(J.part.build.keys + c0, rows, slots, bkeys, nxt, mask, &s_linked);
             const PieceTable<kPieceRows> tab{slots, bkeys, nxt, mask};
-            if (s_dup)
+            if (s_linked)
                 probe_part_dup(J.part, p0, p1, c0, tab, out_cur + j, over + j);
             else
-                probe_part<false>(J.part, p0, p1, c0, tab, out_cur + j, over + j);
+                probe_part<kUnique>(J.part, p0, p1, c0, tab, out_cur + j, over + j);
         }
     }
 }

@@ -103,18 +103,20 @@ __device__ __forceinline__ void prefetch_l2(const void * p)
 
 // Builds the table of `rows` build keys (`keys`, in memory) with all NT
 // threads of the CTA: mask + 1 slots (a power of two, at least 4, more than
-// the rows).  *dup (shared) is set when a key repeats.  Ends with a barrier.
-template <uint32_t kRows, int NT>
+// the rows).  *linked (shared): 0 when no key repeats, otherwise 1 or, with
+// kCount, the rows whose key was there already.  Ends with a barrier.
+template <uint32_t kRows, int NT, bool kCount>
 __device__ __forceinline__ void build_piece(const uint64_t * __restrict__ keys, uint32_t rows, uint32_t * slots, uint64_t * skeys, uint16_t * nxt,
-                                            uint32_t mask, int * dup)
+                                            uint32_t mask, int * linked)
 {
     if (threadIdx.x == 0)
-        *dup = 0;
+        *linked = 0;
     for (uint32_t i = threadIdx.x; i <= mask; i += NT)
         slots[i] = kEmptySlot;
     for (uint32_t i = threadIdx.x; i < rows; i += NT)
         skeys[i] = keys[i];
     __syncthreads();
+    int mine_linked = 0;
     for (uint32_t i = threadIdx.x; i < rows; i += NT)
     {
         const uint64_t k = skeys[i];
@@ -130,22 +132,22 @@ __device__ __forceinline__ void build_piece(const uint64_t * __restrict__ keys, 
                 break;
             if ((old ^ tag) < kRows && skeys[old ^ tag] == k)
             {
-                // the key's slot: this row becomes its head (another row of
-                // the key may have done so meanwhile)
-                for (;;)
-                {
-                    const uint32_t seen = atomicCAS(&slots[pos], old, mine);
-                    if (seen == old)
-                        break;
-                    old = seen;
-                }
-                link = old ^ tag;
-                *dup = 1;
+                // the key's slot, which stays the key's: this row becomes its
+                // head in one exchange, whoever else does so meanwhile (with
+                // compare-and-swaps 8,000 rows of one key took 6.5 ms, this
+                // way 1.4)
+                link = atomicExch(&slots[pos], mine) ^ tag;
+                if constexpr (kCount)
+                    ++mine_linked;
+                else
+                    *linked = 1;
                 break;
             }
         }
         nxt[i] = (uint16_t)link;
     }
+    if (kCount && mine_linked)
+        atomicAdd(linked, mine_linked);
     __syncthreads();
 }
 
@@ -159,15 +161,144 @@ struct ProbeSides
     uint64_t out_cap;
 };
 
+// Four values a lane of an output column, to rows out[u].
+__device__ __forceinline__ void store_at(const uint64_t (&v)[4], void * dst, uint32_t width, const uint64_t (&out)[4], uint32_t one)
+{
+    switch (width)
+    {
+#define PHJ_STORE_AT(W, T)                                                                                                                           \
+    case W:                                                                                                                                          \
+        _Pragma("unroll") for (int u = 0; u < 4; ++u) if (one >> u & 1u) static_cast<T *>(dst)[out[u]] = (T)v[u];                                     \
+        break;
+        PHJ_STORE_AT(1, uint8_t)
+        PHJ_STORE_AT(2, uint16_t)
+        PHJ_STORE_AT(4, uint32_t)
+        default: PHJ_STORE_AT(8, uint64_t)
+#undef PHJ_STORE_AT
+    }
+}
+
+// The output rows of a probe row (`row`, of key `key`) whose matches are the
+// chain from row b of the piece at c0 (kNil: none), o and those after it.
+__device__ __forceinline__ void write_chain(const ProbeSides & J, uint64_t o, uint32_t b, uint64_t key, uint32_t row, uint32_t c0, const uint16_t * nxt)
+{
+    for (; b != kNil; b = nxt[b], ++o)
+        if (o < J.out_cap)
+        {
+            J.out_keys[o] = key;
+            for (uint32_t c = 0; c < J.build.n; ++c)
+                copy_elem(J.out_l[c], o, J.build.col[c], c0 + b, J.build.width[c]);
+            for (uint32_t c = 0; c < J.probe.n; ++c)
+                copy_elem(J.out_r[c], o, J.probe.col[c], row, J.probe.width[c]);
+        }
+}
+
+// The same for the 32 probe rows of a warp, one a lane, when one of them has
+// more than four matches.  Every lane walks four rows of its chain; the warp
+// then writes them eight chains at a time, four neighbouring lanes the four
+// rows of one, at output rows that start at a multiple of four: a store fills
+// sectors.  Bound by the stores and the build rows' gathers in L1.  A lane
+// writing its chain alone waits for each row's loads, and its stores are
+// quarters of sectors, which L2 reads back from memory when they do not meet
+// (12.8M output rows, 8K build rows of 64 a key x 400K: 859 us a join of 20-byte
+// rows and 1,429 of 32-byte ones, this way 200 and 300; 13.4M of 67 a key
+// 1,217 and 347).
+static __device__ __noinline__ void write_chains(const ProbeSides & J, uint64_t o, uint32_t b, uint64_t key, uint32_t row, uint32_t c0,
+                                                 const uint16_t * nxt)
+{
+    const uint32_t lane = threadIdx.x & 31, e = lane & 3;
+    const uint64_t out_cap = J.out_cap;
+    uint32_t fifth = b;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        fifth = fifth != kNil ? nxt[fifth] : kNil;
+    if (!__any_sync(0xffffffffu, fifth != kNil))
+    {
+        write_chain(J, o, b, key, row, c0, nxt);
+        return;
+    }
+    uint32_t skip = (uint32_t)o & 3u; // groups of four start at multiples of four
+    for (o -= skip;; o += 4, skip = 0)
+    {
+        uint32_t at[4];
+        if (o >= out_cap)
+            b = kNil;
+        if (!__any_sync(0xffffffffu, b != kNil))
+            return;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+        {
+            at[k] = k >= skip ? b : kNil;
+            if (at[k] != kNil)
+                b = nxt[b];
+        }
+        uint64_t out[4], v[4];
+        uint32_t brow[4], prow[4], one = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int from = u * 8 + (int)(lane >> 2);
+            uint32_t x = kNil;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k)
+            {
+                const uint32_t y = __shfl_sync(0xffffffffu, at[k], from);
+                x = e == k ? y : x;
+            }
+            brow[u] = c0 + x;
+            prow[u] = __shfl_sync(0xffffffffu, row, from);
+            out[u] = __shfl_sync(0xffffffffu, o, from) + e;
+            v[u] = __shfl_sync(0xffffffffu, key, from);
+            if (x != kNil && out[u] < out_cap)
+                one |= 1u << u;
+        }
+        store_at(v, J.out_keys, 8, out, one);
+        const uint32_t nl = J.build.n, nc = nl + J.probe.n;
+#pragma unroll 1
+        for (uint32_t c = 0; c < nc; ++c)
+        {
+            const bool left = c < nl;
+            const uint32_t i = left ? c : c - nl, w = left ? J.build.width[i] : J.probe.width[i];
+            const void * src = left ? J.build.col[i] : J.probe.col[i];
+            void * dst = left ? J.out_l[i] : J.out_r[i];
+            uint32_t idx[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                idx[u] = left ? brow[u] : prow[u];
+            if (w <= 8)
+            {
+                load_rows(v, src, w, idx, one);
+                store_at(v, dst, w, out, one);
+            }
+            else
+            {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (one >> u & 1u)
+                        static_cast<uint4 *>(dst)[out[u]] = static_cast<const uint4 *>(src)[idx[u]];
+            }
+        }
+    }
+}
+
+// Whether a piece's keys repeat, and how a probe row's matches, a chain, are
+// then written.
+enum Repeats
+{
+    kUnique,
+    kLaneWrites, // by its lane
+    kWarpWrites  // by the whole warp, if a chain has more than four rows
+};
+
 // One warp probes rows first, first + step, ... of [.., p1), 32 * kU rows at
-// a time, against the piece whose first build row is c0.  kDup: some key of
-// the piece has more than one row (a row's matches are its chain).  Output
+// a time, against the piece whose first build row is c0.  Output
 // rows are reserved on *out_cur, a chunk at a time; rows past the capacity
 // are counted and not written (and *over is set).
-template <bool kDup, int kU, uint32_t kRows>
+template <Repeats kRepeats, int kU, uint32_t kRows>
 __device__ __forceinline__ void probe_piece(const ProbeSides & J, uint32_t first, uint32_t step, uint32_t p1, uint32_t c0,
                                             const PieceTable<kRows> & tab, unsigned long long * __restrict__ out_cur, int * __restrict__ over)
 {
+    constexpr bool kDup = kRepeats != kUnique;
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll 1
     for (uint32_t base = first; base < p1; base += step)
@@ -257,18 +388,10 @@ __device__ __forceinline__ void probe_piece(const ProbeSides & J, uint32_t first
         {
 #pragma unroll
             for (int u = 0; u < kU; ++u)
-            {
-                uint64_t o = o0 + rel[u];
-                for (uint32_t b = head[u]; b != kNil; b = tab.nxt[b], ++o)
-                    if (o < out_cap)
-                    {
-                        J.out_keys[o] = key[u];
-                        for (uint32_t c = 0; c < J.build.n; ++c)
-                            copy_elem(J.out_l[c], o, J.build.col[c], c0 + b, J.build.width[c]);
-                        for (uint32_t c = 0; c < J.probe.n; ++c)
-                            copy_elem(J.out_r[c], o, J.probe.col[c], base + u * 32 + lane, J.probe.width[c]);
-                    }
-            }
+                if constexpr (kRepeats == kLaneWrites)
+                    write_chain(J, o0 + rel[u], head[u], key[u], base + u * 32 + lane, c0, tab.nxt);
+                else
+                    write_chains(J, o0 + rel[u], head[u], key[u], base + u * 32 + lane, c0, tab.nxt);
         }
         else
         {

@@ -28,6 +28,7 @@ struct SmallArgs
     ProbeSides sides;
     uint32_t build_rows, probe_rows;
     uint32_t pieces, piece_rows, slots; // slots of a piece's table
+    int dup_wide;                       // chunks of kU * 32 rows also where keys have more than four rows
     int unique_only;                    // a piece with a repeated key is not probed
     SmallCounters * ctr;
     SmallResult * host;                 // mapped host memory
@@ -37,13 +38,14 @@ struct SmallArgs
 // Bound by its chain of dependent steps: key load, table build (rows / 1024
 // inserts a thread), probe key load, lookup, reservation, payload loads,
 // stores.  One chunk of 32 rows a warp (kU 1) spreads a short probe side
-// over all SMs; 128 rows (kU 4) keep more loads in flight on a long one.
+// over all SMs; 128 rows (kU 4) keep more loads in flight on a long one.  (Only
+// that form counts the rows of repeated keys: it costs half a microsecond.)
 template <int kU>
 __global__ void __launch_bounds__(kSNT, 1) k_small_join(const __grid_constant__ SmallArgs a)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ ProbeSides J;
-    __shared__ int s_dup;
+    __shared__ int s_linked; // 0 when no key repeats
     __shared__ int s_over;
     uint64_t * keys = reinterpret_cast<uint64_t *>(smem);
     uint32_t * slots = reinterpret_cast<uint32_t *>(smem + 8ull * kSRows);
@@ -53,19 +55,22 @@ __global__ void __launch_bounds__(kSNT, 1) k_small_join(const __grid_constant__ 
     const uint32_t piece = blockIdx.x % a.pieces, share = blockIdx.x / a.pieces, shares = gridDim.x / a.pieces;
     const uint32_t c0 = piece * a.piece_rows, rows = min(a.piece_rows, a.build_rows - min(c0, a.build_rows));
     // (J is visible after this call's barriers)
-    build_piece<kSRows, kSNT>(a.sides.build.keys + c0, rows, slots, keys, nxt, a.slots - 1, &s_dup);
+    build_piece<kSRows, kSNT, (kU > 1)>(a.sides.build.keys + c0, rows, slots, keys, nxt, a.slots - 1, &s_linked);
     const PieceTable<kSRows> tab{slots, keys, nxt, a.slots - 1};
-    constexpr uint32_t kChunk = 32 * kU;
-    const uint32_t first = (share * (kSNT / 32) + (threadIdx.x >> 5)) * kChunk, step = shares * (kSNT / 32) * kChunk;
-    if (s_dup && a.unique_only)
+    // the CTAs take a warp's chunk each in turn: a short probe side is spread
+    // over all of them
+    const uint32_t first = ((threadIdx.x >> 5) * shares + share) * 32, step = shares * (kSNT / 32) * 32;
+    if (s_linked && a.unique_only)
     {
         if (threadIdx.x == 0)
             atomicOr(&a.ctr->repeats, 1u);
     }
-    else if (s_dup)
-        probe_piece<true, kU>(J, first, step, a.probe_rows, c0, tab, &a.ctr->out_rows, &s_over);
+    else if (s_linked && kU > 1 && (a.dup_wide || s_linked * 4 <= (int)rows * 3))
+        probe_piece<kWarpWrites, kU>(J, first * kU, step * kU, a.probe_rows, c0, tab, &a.ctr->out_rows, &s_over);
+    else if (s_linked)
+        probe_piece<kWarpWrites, 1>(J, first, step, a.probe_rows, c0, tab, &a.ctr->out_rows, &s_over);
     else
-        probe_piece<false, kU>(J, first, step, a.probe_rows, c0, tab, &a.ctr->out_rows, &s_over);
+        probe_piece<kUnique, kU>(J, first * kU, step * kU, a.probe_rows, c0, tab, &a.ctr->out_rows, &s_over);
     __syncthreads();
     if (threadIdx.x == 0)
     {
@@ -121,8 +126,14 @@ uint64_t small_join(phj_ctx * ctx, const Cols & build, uint64_t build_rows, cons
     a.ctr = ctx->small_ctr;
     a.host = reinterpret_cast<SmallResult *>(small_host(ctx));
     const bool wide = probe_rows > (uint64_t)ctx->num_sms / a.pieces * kSNT;
-    const uint64_t rows_cta = (uint64_t)kSNT * (wide ? 4 : 1);
+    const uint64_t rows_cta = (uint64_t)kSNT * (wide ? 2 : 1);
     const uint32_t shares = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(probe_rows, rows_cta), (uint64_t)ctx->num_sms / a.pieces));
+    // Keys of more than four rows make a chunk's output rows many: a warp then
+    // takes 128 probe rows at a time only if it has two such chunks to do, and
+    // else 32 (8K rows of 64 a key x 400K: 300 us a join against 420).  Fewer
+    // rows a key want the loads in flight (64K rows of two a key and piece x
+    // 400K: 151 against 218).
+    a.dup_wide = ceil_div(probe_rows, 128) >= 2ull * shares * (kSNT / 32);
     const size_t smem = 8ull * kSRows + 4ull * a.slots + 2ull * a.piece_rows;
     if (ctx->time_kernels)
     {

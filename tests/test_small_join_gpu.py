@@ -85,3 +85,47 @@ def test_a_join_of_2_32_rows_is_refused(ctx, scheme):
         ctx.run_phj_pure(t, u, [6]) if scheme == "pure" else ctx.run_chj(t, u)
     assert e.value.status == P.ERR_CAPACITY and str(65_536 * 70_000) in str(e.value)
     t.free(), u.free()
+
+
+@pytest.mark.parametrize("build,probe,distinct,tb,tp,match", [
+    (1000, 3000, 200, [P.U64], [P.U32], 900),                  # five rows a key: one more than a lane writes alone
+    (1000, 3001, 15, [P.U64, P.U32], [P.U16], 700),            # 66 or 67 rows: chains start at any row
+    (1003, 500, 1, [P.U128, P.U8], [P.U128], 800),             # one key, 16-byte columns on both sides
+    (8192, 200_001, 125, [P.U16], [P.U8, P.U64], 30),          # long probe side, few chunks of 128 a warp
+    (60_000, 300_000, 3000, [P.U32], [], 100),                 # ... and many, eight pieces
+    (60_000, 300_000, 30_000, [P.U32], [P.U32], 300),          # two rows a key, in pieces of their own
+])
+def test_long_chains(ctx, build, probe, distinct, tb, tp, match):
+    bk = np.resize(G.gen_keys(0, distinct, 611, 612), build)
+    bk[build // 2:build // 2 + 40] = bk[3]                     # and one key more often than the others
+    b = P.BlockStream(tb, bk, G.payload_columns(613, tb, build))
+    p = P.BlockStream(tp, G.gen_keys(4, probe, 614, 612, domain=distinct, match_permille=match), G.payload_columns(615, tp, probe))
+    expected = O.join_fingerprint(b, p)
+    t, u = ctx.upload(b), ctx.upload(p)
+    for _ in range(2):
+        out, _ = ctx.run_phj_pure(t, u, [6])
+        assert "small_join" in {k["name"] for k in ctx.kernel_times()}
+        assert out.fingerprint() == expected
+        out.free()
+    t.free(), u.free()
+
+
+@pytest.mark.parametrize("cap", [1, 4097, 33_002])
+def test_chains_past_the_capacity(ctx, cap):
+    # the no-allocation join: rows past the caller's columns are counted, and
+    # nothing is written behind them
+    torch = pytest.importorskip("torch")
+    b, p = sides(1000, 2000, [P.U64], [P.U32], 67, 900)
+    rows = O.join_fingerprint(b, p)[0]
+    t, u = ctx.upload(b), ctx.upload(p)
+    keys, left = (torch.full((rows,), -7, dtype=torch.int64, device="cuda") for _ in range(2))
+    right = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+    with pytest.raises(P.PhjError) as e:
+        ctx.run_chj_noalloc(t, u, cap, keys.data_ptr(), [left.data_ptr()], [right.data_ptr()])
+    assert e.value.status == P.ERR_CAPACITY and e.value.rows == rows > cap
+    assert all((c[cap:] == -7).all() for c in (keys, left, right))
+    of = {}
+    for k, v in zip(b.keys.tolist(), b.payloads[0].tolist()):
+        of.setdefault(k, set()).add(v)
+    assert all(v % 2**64 in of[k % 2**64] for k, v in zip(keys[:cap].tolist(), left[:cap].tolist()))
+    t.free(), u.free()
