@@ -85,7 +85,7 @@ __device__ __forceinline__ void copy_row(const Cols & src, uint64_t si, const Co
 // leaf's steps.
 template <int NT, bool kGroup>
 __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols part, const __grid_constant__ Cols dst, const uint32_t * __restrict__ leaf_off,
-                                                         const uint32_t * __restrict__ table_off, int ulog, uint32_t smem_cells,
+                                                         const uint32_t * __restrict__ table_off, int ulog, uint32_t most_rows, uint32_t smem_cells,
                                                          Cell * __restrict__ cells, uint64_t * __restrict__ next, LeafMeta * __restrict__ meta,
                                                          int * __restrict__ any_dup)
 {
@@ -108,10 +108,10 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
             meta[l] = LeafMeta{t0, r0, cap ? (uint8_t)log2u(cap) : (uint8_t)0, 0, 0, 0};
         return;
     }
-    if (r >= cap)
+    if (r > most_rows)
     {
-        // a leaf past an estimated capacity: nothing is inserted, the build
-        // runs again at the counted sizes
+        // a leaf past the estimate: nothing is inserted, the build runs again
+        // at the counted sizes
         if (threadIdx.x == 0)
         {
             meta[l] = LeafMeta{t0, r0, (uint8_t)log2u(cap), 0, 0, 0};
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
 // One CTA per leaf; a table of `cap` cells {key, packed payload} at leaf *
 // cap, built in shared memory with 64-bit compare-and-swaps on the keys and
 // streamed out.  An empty cell holds a key of another leaf.  A repeated key
-// or a leaf of cap rows or more sets *bad (the table is then unusable).
+// or a leaf of more than most_rows rows sets *bad (the table is then unusable).
 // Bound by the write of the tables (16 bytes a cell, 2.2 to 2.9 cells a
 // row): 3M rows in 16,384 leaves 60 us, 2.9 TB/s, where the general tables,
 // their next-chain and the payload packing took 115.  kRows: shared memory
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
 template <int NT, bool kRows>
 __global__ void __launch_bounds__(NT, kRows ? 2 : 1) k_build_inline(const __grid_constant__ Cols part, const uint32_t * __restrict__ leaf_off,
                                                      const __grid_constant__ PackSpec pk, const __grid_constant__ InlineTables t,
-                                                     int * __restrict__ bad)
+                                                     uint32_t most_rows, int * __restrict__ bad)
 {
     extern __shared__ __align__(16) ulonglong2 icells[]; // (kRows: keys[cap] | rows[cap])
     uint64_t * ikeys = reinterpret_cast<uint64_t *>(icells);
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(NT, kRows ? 2 : 1) k_build_inline(const __grid
     // another leaf's build may have found the tables unusable (one thread
     // asks: every warp of 16K CTAs reading one word took 60 us)
     const int stop = threadIdx.x == 0 ? *reinterpret_cast<volatile int *>(bad) : 0;
-    if (r >= t.cap)
+    if (r > most_rows) // (fewer than t.cap)
     {
         if (threadIdx.x == 0)
             atomicOr(bad, kLeafOverflow);
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(NT, kRows ? 2 : 1) k_build_inline(const __grid
         const uint64_t k = part.keys[r0 + i];
         const uint64_t v = kRows ? 0ull : payload(i);
         uint32_t pos = t.start(int_hash64(k));
-        for (;;) // r < cap: an empty cell is found
+        for (;;) // fewer rows than cells: an empty one is found
         {
             const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long *>(ikeys + pos * kStride), none, k);
             if (old == none)
@@ -508,6 +508,12 @@ static uint64_t leaf_rows_estimate(uint64_t rows, uint64_t n_leaves)
     return (uint64_t)(m + 6.0 * std::sqrt(m) + 8.0);
 }
 
+// Rows that a table of `cells` may hold at the load the option allows.
+static uint32_t rows_at_load(uint64_t cells, uint32_t pct)
+{
+    return (uint32_t)std::min<uint64_t>(std::min(cells - 1, cells * 100 / pct), 0xFFFFFFFFu);
+}
+
 bool build_inline_tables(phj_ctx * ctx, Scratch & s, const Cols & part, uint64_t rows, const uint32_t * leaf_off, uint32_t total_bits,
                          const PackSpec & pk, InlineTables & t, int * bad)
 {
@@ -536,13 +542,14 @@ bool build_inline_tables(phj_ctx * ctx, Scratch & s, const Cols & part, uint64_t
     // not fit on a SM with cells in shared memory, keys and rows are held
     // there and the payloads are read as the cells go out (256 leaves of
     // 4096 rows: 24 us against 28, in one wave of CTAs)
+    const uint32_t most = rows_at_load(t.cap, ctx->table_cap_pct);
     const size_t lean = (size_t)t.cap * 10, two = (ctx->smem_optin + 1024) / 2 - 2048;
     if (est > 1024 && smem > two && lean <= two)
-        k_build_inline<1024, true><<<(unsigned)n_leaves, 1024, lean, ctx->stream>>>(part, leaf_off, pk, t, bad);
+        k_build_inline<1024, true><<<(unsigned)n_leaves, 1024, lean, ctx->stream>>>(part, leaf_off, pk, t, most, bad);
     else if (est > 1024)
-        k_build_inline<1024, false><<<(unsigned)n_leaves, 1024, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
+        k_build_inline<1024, false><<<(unsigned)n_leaves, 1024, smem, ctx->stream>>>(part, leaf_off, pk, t, most, bad);
     else
-        k_build_inline<kBuildNT, false><<<(unsigned)n_leaves, kBuildNT, smem, ctx->stream>>>(part, leaf_off, pk, t, bad);
+        k_build_inline<kBuildNT, false><<<(unsigned)n_leaves, kBuildNT, smem, ctx->stream>>>(part, leaf_off, pk, t, most, bad);
     PHJ_LAUNCHED(ctx, "build_inline");
     return true;
 }
@@ -651,13 +658,14 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
         max_cap * sizeof(Cell) * 2 <= ctx->smem_optin ? (uint32_t)std::min<uint64_t>(max_cap, kSmemCellsMax) : 0u;
     {
         KTimer kt(ctx, "build_leaf_tables", 0, 0);
+        const uint32_t most = lt.estimated ? rows_at_load(max_cap, ctx->table_cap_pct) : 0xFFFFFFFFu; // (counted sizes hold every leaf)
         // leaves of more than 1024 rows get 1024 threads
         const bool large = lt.max_rows > 1024;
         lt.groups = group_dst && smem_cells && smem_cells == max_cap;
         const auto kb = lt.groups ? (large ? k_build_leaf<1024, true> : k_build_leaf<kBuildNT, true>)
                                   : (large ? k_build_leaf<1024, false> : k_build_leaf<kBuildNT, false>);
         kb<<<n_leaves, large ? 1024 : kBuildNT, (size_t)smem_cells * (lt.groups ? sizeof(Cell) + 8 : sizeof(Cell)), ctx->stream>>>(
-            build_part, group_dst ? *group_dst : Cols{}, leaf_off, table_off, lt.uniform_log2cap, smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
+            build_part, group_dst ? *group_dst : Cols{}, leaf_off, table_off, lt.uniform_log2cap, most, smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
         PHJ_LAUNCHED(ctx, "build_leaf");
     }
     lt.any_dup = 0; // unknown until the flags are read

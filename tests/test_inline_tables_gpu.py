@@ -62,3 +62,25 @@ def test_builds_the_estimate_does_not_hold_for(ctx, bt, mat, how):
     skewed = np.concatenate([keys[leaf == 3][:9000], keys[leaf != 3][:8000]])
     bk = {"skew": skewed, "repeats": np.resize(keys[:9000], 20_000), "both": np.resize(skewed, 25_000)}[how]
     join(ctx, bk, np.concatenate([keys[:9000], skewed[::2]]), bt, [P.U32], [5], mat)
+
+
+@pytest.mark.parametrize("bt", [[P.U32], [P.U64, P.U32]])
+@pytest.mark.parametrize("rows,kept", [(400, True), (600, False)])
+def test_a_crowded_leaf_is_not_kept_past_the_load(ctx, bt, rows, kept):
+    # 32 leaves of about 300 rows, the estimate 411 (cells for 412 rows at the
+    # default load in an inline table, for 512 in a general one): a leaf of
+    # 600 rows fits neither at that load, though it has fewer rows than cells
+    keys = G.gen_keys(0, 400_000, 721, 722)
+    leaf = O.leaf_ids(keys, 5)
+    bk = np.concatenate([keys[leaf == 3][:rows], keys[leaf != 3][: 9600 - rows]])
+    b = P.BlockStream(bt, bk, G.payload_columns(723, bt, len(bk)))
+    p = P.BlockStream([P.U32], bk[::3], G.payload_columns(724, [P.U32], len(bk[::3])))
+    ctx.set_int("probe_materialize", 0)
+    try:
+        r = P.runPHJ(b, p, [5], ctx=ctx)
+    finally:
+        ctx.set_int("probe_materialize", -1)
+    names = [k["name"] for k in ctx.kernel_times()]
+    general = names.count("build_leaf_tables")
+    assert general == (0 if kept else 1) + (bt == [P.U64, P.U32]), names
+    assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
