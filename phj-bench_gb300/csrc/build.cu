@@ -22,6 +22,7 @@ namespace
 {
 constexpr int kBuildNT = 256;
 constexpr uint32_t kSmemCellsMax = 8192; // 128 KiB of cells per CTA
+constexpr uint32_t kLookers = 1024;
 
 // Cells of a table for r rows: the power of two at or above r * pct / 100
 // (pct 200: load <= 1/2, the reference's JoinHashTable::reserve), and above r.
@@ -70,6 +71,28 @@ __device__ __forceinline__ void copy_row(const Cols & src, uint64_t si, const Co
         copy_elem(dst.col[c], di, src.col[c], si, src.width[c]);
 }
 
+// Tables sized by estimate: whether a leaf has more rows than its table may
+// hold is found out before any is built (a hot key of 100,000 rows among 8M: a
+// build of 150 us that was thrown away when the leaf's own CTA found out; now
+// 45 us of CTAs that end at once).
+__device__ __forceinline__ bool past_estimate(const uint32_t * __restrict__ leaf_off, uint32_t l0, uint32_t l1, uint32_t stride, uint32_t most_rows)
+{
+    bool over = false;
+    for (uint32_t l = l0 + threadIdx.x; l < l1; l += stride)
+        over |= leaf_off[l + 1] - leaf_off[l] > most_rows;
+    return over;
+}
+
+__global__ void k_leaf_check(const uint32_t * __restrict__ leaf_off, uint32_t n_leaves, uint32_t most_rows, int * __restrict__ flags, int * __restrict__ stop)
+{
+    const uint32_t l0 = blockIdx.x * blockDim.x;
+    if (past_estimate(leaf_off, l0, min(n_leaves, l0 + blockDim.x), blockDim.x, most_rows))
+    {
+        atomicOr(flags, kLeafOverflow);
+        *stop = 1;
+    }
+}
+
 // One CTA per leaf.  Tables are either uniform (every leaf 2^ulog cells at
 // leaf << ulog, ulog >= 0) or sized per leaf through table_off (ulog < 0).
 // The RowRefCell of a build row is {0, row}: block 0 is the whole
@@ -85,7 +108,7 @@ __device__ __forceinline__ void copy_row(const Cols & src, uint64_t si, const Co
 // leaf's steps.
 template <int NT, bool kGroup>
 __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols part, const __grid_constant__ Cols dst, const uint32_t * __restrict__ leaf_off,
-                                                         const uint32_t * __restrict__ table_off, int ulog, uint32_t most_rows, uint32_t smem_cells,
+                                                         const uint32_t * __restrict__ table_off, int ulog, const int * __restrict__ stop, uint32_t smem_cells,
                                                          Cell * __restrict__ cells, uint64_t * __restrict__ next, LeafMeta * __restrict__ meta,
                                                          int * __restrict__ any_dup)
 {
@@ -99,6 +122,7 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
     const uint64_t cap = ulog >= 0 ? (1ull << ulog) : table_off[l + 1] - t0;
     if (threadIdx.x == 0)
         dup = 0;
+    const int stopped = stop ? __ldg(stop) : 0; // (looked at when the table is cleared)
     const Cell empty{0ull, INVALID_REF};
     if (r == 0)
     {
@@ -108,22 +132,19 @@ __global__ void __launch_bounds__(NT) k_build_leaf(const __grid_constant__ Cols 
             meta[l] = LeafMeta{t0, r0, cap ? (uint8_t)log2u(cap) : (uint8_t)0, 0, 0, 0};
         return;
     }
-    if (r > most_rows)
-    {
-        // a leaf past the estimate: nothing is inserted, the build runs again
-        // at the counted sizes
-        if (threadIdx.x == 0)
-        {
-            meta[l] = LeafMeta{t0, r0, (uint8_t)log2u(cap), 0, 0, 0};
-            atomicOr(any_dup, kLeafOverflow);
-        }
+    // (Only where `stopped`: the bound is for the compiler.  With it this form
+    // has 31 registers and no spills, 1,080 us for the workload above against
+    // 1,160; the other form is better without: the table of a leaf with a key
+    // of 100,000 rows takes 565 us, 1,070 with it.)
+    if (kGroup && r >= cap)
         return;
-    }
     const bool in_smem = cap <= smem_cells;
     Cell * tab = in_smem ? sh_cells : cells + t0;
     for (uint64_t i = threadIdx.x; i < cap; i += NT)
         tab[i] = empty;
     __syncthreads();
+    if (stopped)
+        return; // some leaf is past the estimate: all are built again at the counted sizes
     bool my_dup = false;
     for (uint32_t i = threadIdx.x; i < r; i += NT)
     {
@@ -214,6 +235,14 @@ __global__ void __launch_bounds__(NT, kRows ? 2 : 1) k_build_inline(const __grid
     const uint64_t none = t.empty_key(l);
     // another leaf's build may have found the tables unusable (one thread
     // asks: every warp of 16K CTAs reading one word took 60 us)
+    // (the first kLookers CTAs look through all leaves, a share each)
+    if (blockIdx.x < kLookers)
+    {
+        const uint32_t lookers = min(gridDim.x, kLookers);
+        const uint32_t l0 = (uint32_t)((uint64_t)gridDim.x * blockIdx.x / lookers), l1 = (uint32_t)((uint64_t)gridDim.x * (blockIdx.x + 1) / lookers);
+        if (past_estimate(leaf_off, l0, l1, NT, most_rows))
+            atomicOr(bad, kLeafOverflow);
+    }
     const int stop = threadIdx.x == 0 ? *reinterpret_cast<volatile int *>(bad) : 0;
     if (r > most_rows) // (fewer than t.cap)
     {
@@ -602,7 +631,7 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
                        bool lazy, uint64_t estimate_rows, const Cols * group_dst)
 {
     uint32_t * table_off = nullptr;
-    uint32_t * small = s.get<uint32_t>(4); // [0] max rows, [1] flags (kLeafRepeats, kLeafOverflow)
+    uint32_t * small = s.get<uint32_t>(4); // [0] max rows, [1] flags (kLeafRepeats, kLeafOverflow), [2] a leaf is past the estimate
     PHJ_CUDA(cudaMemsetAsync(small, 0, 4 * sizeof(uint32_t), ctx->stream));
     lt.flags = reinterpret_cast<int *>(small + 1);
     uint64_t max_cap;
@@ -658,14 +687,19 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
         max_cap * sizeof(Cell) * 2 <= ctx->smem_optin ? (uint32_t)std::min<uint64_t>(max_cap, kSmemCellsMax) : 0u;
     {
         KTimer kt(ctx, "build_leaf_tables", 0, 0);
-        const uint32_t most = lt.estimated ? rows_at_load(max_cap, ctx->table_cap_pct) : 0xFFFFFFFFu; // (counted sizes hold every leaf)
+        int * stop = reinterpret_cast<int *>(small + 2);
+        if (lt.estimated)
+        {
+            k_leaf_check<<<(unsigned)ceil_div(n_leaves, 256), 256, 0, ctx->stream>>>(leaf_off, n_leaves, rows_at_load(max_cap, ctx->table_cap_pct), lt.flags, stop);
+            PHJ_LAUNCHED(ctx, "leaf_check");
+        }
         // leaves of more than 1024 rows get 1024 threads
         const bool large = lt.max_rows > 1024;
         lt.groups = group_dst && smem_cells && smem_cells == max_cap;
         const auto kb = lt.groups ? (large ? k_build_leaf<1024, true> : k_build_leaf<kBuildNT, true>)
                                   : (large ? k_build_leaf<1024, false> : k_build_leaf<kBuildNT, false>);
         kb<<<n_leaves, large ? 1024 : kBuildNT, (size_t)smem_cells * (lt.groups ? sizeof(Cell) + 8 : sizeof(Cell)), ctx->stream>>>(
-            build_part, group_dst ? *group_dst : Cols{}, leaf_off, table_off, lt.uniform_log2cap, most, smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
+            build_part, group_dst ? *group_dst : Cols{}, leaf_off, table_off, lt.uniform_log2cap, lt.estimated ? stop : nullptr, smem_cells, lt.cells, lt.next, lt.meta, lt.flags);
         PHJ_LAUNCHED(ctx, "build_leaf");
     }
     lt.any_dup = 0; // unknown until the flags are read

@@ -84,3 +84,18 @@ def test_a_crowded_leaf_is_not_kept_past_the_load(ctx, bt, rows, kept):
     general = names.count("build_leaf_tables")
     assert general == (0 if kept else 1) + (bt == [P.U64, P.U32]), names
     assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
+
+
+@pytest.mark.parametrize("bt", [[P.U32], [P.U64, P.U32]])
+@pytest.mark.parametrize("crowded", [0, 1, 2047, 4095])
+def test_one_crowded_leaf_of_many(ctx, bt, crowded):
+    # found wherever it is among 4,096 leaves of 40 rows; repeated keys make it
+    keys = G.gen_keys(0, 400_000, 731, 732)
+    leaf = O.leaf_ids(keys, 12)
+    bk = np.concatenate([keys[:160_000], np.repeat(keys[leaf == crowded][:1], 700)])
+    b = P.BlockStream(bt, bk, G.payload_columns(733, bt, len(bk)))
+    pk = np.concatenate([keys[::40], keys[leaf == crowded][:3]])
+    p = P.BlockStream([P.U32], pk, G.payload_columns(734, [P.U32], len(pk)))
+    r = P.runPHJ(b, p, [6, 6], ctx=ctx)
+    assert "build_leaf_tables" in {k["name"] for k in ctx.kernel_times()}
+    assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
