@@ -497,12 +497,12 @@ def main():
     per_name, alone = {}, {}
     for run in kernel_runs:
         for i, k in enumerate(run):
-            d = per_name.setdefault(k["name"], {"ms": 0.0, "launches": 0, "bytes": 0})
+            d = per_name.setdefault(k["form"], {"ms": 0.0, "launches": 0, "bytes": 0})
             d["ms"] += k["ms"]
             d["launches"] += 1
             d["bytes"] += k["bytes"]
             if not launch_overlaps(run, i):
-                e = alone.setdefault(k["name"], {"ms": 0.0, "launches": 0, "bytes": 0})
+                e = alone.setdefault(k["form"], {"ms": 0.0, "launches": 0, "bytes": 0})
                 e["ms"] += k["ms"]
                 e["launches"] += 1
                 e["bytes"] += k["bytes"]

@@ -471,6 +471,13 @@ typedef struct phj_kernel_time {
     double start_ms; /* start of the launch after the run's earliest timed launch */
 } phj_kernel_time;
 uint32_t phj_last_kernel_times(const phj_ctx *ctx, phj_kernel_time *out, uint32_t cap);
+/* Which kernel each of these records is of, in the same order.  A record's
+ * name is its step; where a step has kernels of several forms this is the one
+ * that ran: "probe_fused", the lookup and projection in one pass, is
+ * "probe_fused", "probe_inline" (tables that hold the payloads) or
+ * "small_join" (build and probe in one launch); "noalloc_probe" is itself or
+ * "small_join".  Otherwise it is the record's name. */
+uint32_t phj_last_kernel_forms(const phj_ctx *ctx, char (*out)[32], uint32_t cap);
 /* Number of this library's kernel launches issued since the context was
  * created. */
 uint64_t phj_launch_count(const phj_ctx *ctx);

@@ -53,13 +53,14 @@ void begin_run(phj_ctx * ctx)
     reset_accounting(ctx);
 }
 
-KTimer::KTimer(phj_ctx * c, const char * name, uint64_t rows, uint64_t bytes)
+KTimer::KTimer(phj_ctx * c, const char * name, uint64_t rows, uint64_t bytes, const char * form)
     : ctx(c)
 {
     if (!ctx->time_kernels || !name)
         return;
     KernelRecord r;
     r.name = name;
+    r.form = form ? form : "";
     r.rows = rows;
     r.bytes = bytes;
     r.start = take_event(ctx);
@@ -2598,6 +2599,21 @@ void phj_output_free(phj_ctx * ctx, phj_output * out)
     DeviceScope dev(ctx);
     if (ctx)
         free_output(ctx, out);
+}
+
+uint32_t phj_last_kernel_forms(const phj_ctx * ctx, char (*out)[32], uint32_t cap)
+{
+    if (!ctx || !out)
+        return 0;
+    uint32_t n = 0;
+    for (const auto & r : ctx->records)
+    {
+        if (n >= cap)
+            break;
+        std::memset(out[n], 0, sizeof(out[n]));
+        std::strncpy(out[n++], (r.form.empty() ? r.name : r.form).c_str(), sizeof(out[0]) - 1);
+    }
+    return n;
 }
 
 uint32_t phj_last_kernel_times(const phj_ctx * ctx, phj_kernel_time * out, uint32_t cap)

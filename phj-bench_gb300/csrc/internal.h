@@ -37,7 +37,8 @@ void cuda_check(cudaError_t e, const char * what, const char * file, int line);
 
 struct KernelRecord
 {
-    std::string name;
+    std::string name; // the step
+    std::string form; // the kernel that did it, where the step has several
     cudaEvent_t start = nullptr, stop = nullptr;
     uint64_t rows = 0, bytes = 0;
 };
@@ -306,12 +307,12 @@ struct Scratch
 cudaEvent_t take_event(phj_ctx * ctx);
 void begin_run(phj_ctx * ctx);
 // Records an event pair around the next launch(es) when kernel timing is on
-// (and `name` is not null).
+// (and `name` is not null).  `form`: which of the step's kernels, if it has several.
 struct KTimer
 {
     phj_ctx * ctx;
     int idx = -1;
-    KTimer(phj_ctx * c, const char * name, uint64_t rows, uint64_t bytes);
+    KTimer(phj_ctx * c, const char * name, uint64_t rows, uint64_t bytes, const char * form = nullptr);
     ~KTimer();
 };
 void after_launch(phj_ctx * ctx, const char * name, const char * file, int line);

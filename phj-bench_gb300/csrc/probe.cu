@@ -1551,7 +1551,7 @@ phj_output * probe_inline(phj_ctx * ctx, Scratch & s, const Cols & probe, uint64
         int rec = -1;
         {
             // (a single 1- or 2-byte column is nothing k_probe_fused takes)
-            KTimer kt(ctx, one_pass_schemas(left, right) ? "probe_fused" : "probe_inline", probe_rows, 0);
+            KTimer kt(ctx, one_pass_schemas(left, right) ? "probe_fused" : "probe_inline", probe_rows, 0, "probe_inline");
             rec = kt.idx;
             k_probe_inline<<<grid, kPNT, 0, ctx->stream>>>(probe.keys, probe_rows, t, pc, bc, out->keys, counter, counter + 1, probe_rows, flags);
             PHJ_LAUNCHED(ctx, "probe_inline");

@@ -139,6 +139,7 @@ uint64_t small_join(phj_ctx * ctx, const Cols & build, uint64_t build_rows, cons
     {
         KernelRecord r;
         r.name = name;
+        r.form = "small_join";
         r.rows = probe_rows;
         r.start = start;
         r.stop = stop;

@@ -171,6 +171,7 @@ def load() -> C.CDLL:
         "phj_output_fingerprint": (C.c_int, [P, P, C.POINTER(C.c_uint64)]),
         "phj_output_free": (None, [P, P]),
         "phj_last_kernel_times": (C.c_uint32, [P, C.POINTER(KernelTime), C.c_uint32]),
+        "phj_last_kernel_forms": (C.c_uint32, [P, C.POINTER(C.c_char * 32), C.c_uint32]),
         "phj_launch_count": (C.c_uint64, [P]),
         "phj_host_alloc": (C.c_int, [P, C.c_size_t, C.POINTER(P)]),
         "phj_host_free": (None, [P, P]),
@@ -563,7 +564,9 @@ class Context:
     def kernel_times(self) -> List[dict]:
         arr = (KernelTime * 256)()
         n = self.lib.phj_last_kernel_times(self.ptr, arr, 256)
-        return [{"name": arr[i].name.decode(), "ms": arr[i].ms, "rows": arr[i].rows, "bytes": arr[i].bytes, "start_ms": arr[i].start_ms}
+        forms = (C.c_char * 32 * 256)()
+        self.lib.phj_last_kernel_forms(self.ptr, forms, 256)
+        return [{"name": arr[i].name.decode(), "form": forms[i].value.decode(), "ms": arr[i].ms, "rows": arr[i].rows, "bytes": arr[i].bytes, "start_ms": arr[i].start_ms}
                 for i in range(n)]
 
     def launch_count(self) -> int:
