@@ -220,7 +220,11 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *        their uploads still queued;
  *   "test_memory_limit_mib": test hook, 0 (default) off; an allocation that
  *        takes the device memory this context holds (tables, outputs,
- *        scratch) past so many MiB fails as out of memory. */
+ *        scratch) past so many MiB fails as out of memory.
+ * PHJ-PURE and CHJ join a small build side in one launch (see
+ * phj_run_phj_pure) unless one of "probe_materialize", "table_cap_pct",
+ * "p1_tile_rows", "p1_stages", "pack_build", "chj_windows", "probe_fused" and
+ * "probe_pass_bits" asks for a form of the general path. */
 phj_status phj_ctx_set_int(phj_ctx *ctx, const char *name, int64_t value);
 /* Reads an option above, a device property ("device", "num_sms",
  * "l2_bytes"), or "scratch_bytes": the block of device memory the context

@@ -113,7 +113,12 @@ def tune(ctx: "P.Context", build: "P.Table", probe: "P.Table", scheme: str = "ph
             "probe_materialize": -1, "probe_pass_bits": 0}
     best_ms, ref_fp = _time(ctx, scheme, build, probe, best, reps, budget_mib)
     trials = 1
+    # a small build side is joined in one launch, which the radix bits do not
+    # reach: their times would be noise (the other knobs keep the general path)
+    one_launch = scheme != "phj" and any(k["form"] == "small_join" for k in ctx.kernel_times())
     for knob in KNOBS:
+        if one_launch and knob == "pass_bits":
+            continue
         for v in values[knob]:
             if v == best[knob]:
                 continue

@@ -779,8 +779,8 @@ static void run_chj_form(phj_ctx * ctx, const phj_table & B, const phj_table & P
 // the form does not apply).
 static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj_table & P, const char * name, cudaEvent_t (&ev)[3])
 {
-    if (ctx->probe_materialize >= 0 || ctx->probe_pass_bits || ctx->chj_windows > 1 || !ctx->probe_fused || !ctx->pack_build ||
-        ctx->table_cap_pct != 200 || !small_join_eligible(ctx, B.rows, P.rows, false))
+    if (ctx->probe_materialize >= 0 || ctx->probe_pass_bits || ctx->p1_tile_rows || ctx->p1_stages || ctx->chj_windows > 1 || !ctx->probe_fused ||
+        !ctx->pack_build || ctx->table_cap_pct != 200 || !small_join_eligible(ctx, B.rows, P.rows, false))
         return nullptr;
     begin_run(ctx);
     ev[0] = take_event(ctx);

@@ -49,3 +49,46 @@ def test_tuned_join_is_bit_exact_and_cached(ctx, tmp_path, scheme):
     finally:
         A.reset(ctx)
         tb.free(), tp.free()
+
+
+class OneLaunchContext:
+    """A context whose PHJ-PURE joins run in one launch at default options."""
+
+    def __init__(self):
+        self.options, self.runs = {}, []
+
+    def set_int(self, name, value):
+        self.options[name] = value
+
+    def flush_l2(self):
+        pass
+
+    def run_phj_pure(self, b, p, bits):
+        class Out:
+            def fingerprint(self):
+                return (1, 2, 3)
+
+            def free(self):
+                pass
+
+        class Res:
+            e2e_wall_ms = 1.0 - 0.001 * len(self.runs)  # each a little faster than the last, as noise may have it
+        general = any(self.options.get(k, d) != d for k, d in (("table_cap_pct", 200), ("p1_tile_rows", 0), ("p1_stages", 0),
+                                                                ("probe_materialize", -1), ("probe_pass_bits", 0)))
+        self.last = "probe_fused" if general else "small_join"
+        self.runs.append((tuple(bits), self.last))
+        return Out(), Res()
+
+    def kernel_times(self):
+        return [{"name": self.last, "form": self.last}]
+
+
+def test_radix_bits_are_not_tuned_where_one_launch_joins():
+    class Table:
+        rows, types = 5000, [P.U64]
+
+    ctx = OneLaunchContext()
+    cfg = A.tune(ctx, Table(), Table(), cache_path=None)
+    assert cfg["pass_bits"] == P.autotune_radix(5000)
+    assert {bits for bits, _ in ctx.runs} == {tuple(cfg["pass_bits"])}
+    assert any(form == "probe_fused" for _, form in ctx.runs)

@@ -129,3 +129,17 @@ def test_chains_past_the_capacity(ctx, cap):
         of.setdefault(k, set()).add(v)
     assert all(v % 2**64 in of[k % 2**64] for k, v in zip(keys[:cap].tolist(), left[:cap].tolist()))
     t.free(), u.free()
+
+
+@pytest.mark.parametrize("option,value,default", [("p1_tile_rows", 2048, 0), ("p1_stages", 2, 0), ("probe_pass_bits", 5, 0), ("table_cap_pct", 150, 200),
+                                                  ("pack_build", 0, 1), ("probe_fused", 0, 1), ("probe_materialize", 1, -1)])
+def test_an_option_of_the_general_path_keeps_it(ctx, option, value, default):
+    b, p = sides(3000, 9000, [P.U64], [P.U32], 1, 700)
+    for v, small in ((default, True), (value, False)):
+        ctx.set_int(option, v)
+        try:
+            r = P.runPHJ(b, p, [6], ctx=ctx)
+        finally:
+            ctx.set_int(option, default)
+        assert ("small_join" in {k["form"] for k in ctx.kernel_times()}) == small
+        assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
