@@ -296,13 +296,19 @@ phj_status phj_radix_shuffle(phj_ctx *ctx, const phj_table *input, const uint8_t
 /* runCHJ (src/CHJ.h:31, src/CHJ.cpp:49-152): one global device table of
  * 16-byte cells namespaced by the top 8 hash bits, 128-bit CAS inserts, then
  * an unpartitioned probe (past L2, of the probe side in sub-table order:
- * option "probe_materialize").  `threads` of the reference has no device meaning. */
+ * option "probe_materialize").  `threads` of the reference has no device meaning.
+ * Small build sides (payloads the one-pass probe takes: option "probe_fused")
+ * are joined in one launch, as in phj_run_phj_pure. */
 phj_status phj_run_chj(phj_ctx *ctx, const phj_table *build, const phj_table *probe, phj_output **out,
                        phj_chj_result *result);
 
 /* runPHJ (src/PHJ.h:31, src/PHJ.cpp:19-150): radix shuffle of both sides
  * over `pass_bits` (n_passes passes, total bits in [1, 24] on the device),
- * per-leaf tables, probe with output projection. */
+ * per-leaf tables, probe with output projection.
+ * A build side of at most 8,192 rows, or of 65,536 with a short probe side, is
+ * joined in one launch without partitioning: `pass_bits` is then checked and
+ * has no effect, and the result's time is all the probe's (the other phases
+ * are 0 ms). */
 phj_status phj_run_phj_pure(phj_ctx *ctx, const phj_table *build, const phj_table *probe, const uint8_t *pass_bits,
                             uint32_t n_passes, phj_output **out, phj_phj_result *result);
 

@@ -143,3 +143,18 @@ def test_an_option_of_the_general_path_keeps_it(ctx, option, value, default):
             ctx.set_int(option, default)
         assert ("small_join" in {k["form"] for k in ctx.kernel_times()}) == small
         assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
+
+
+def test_one_launch_counts_as_the_probe(ctx):
+    b, p = sides(3000, 9000, [P.U64], [P.U32], 1, 700)
+    t, u = ctx.upload(b), ctx.upload(p)
+    with pytest.raises(P.PhjError):
+        ctx.run_phj_pure(t, u, [16, 9])  # the bits are checked all the same
+    out, r = ctx.run_phj_pure(t, u, [6])
+    assert r.build_shuffle.wall_ms == r.build.wall_ms == r.probe_shuffle.wall_ms == 0
+    assert r.probe.wall_ms == pytest.approx(r.e2e_wall_ms) and r.e2e_wall_ms > 0
+    out.free()
+    out, r = ctx.run_chj(t, u)
+    assert r.build.wall_ms == 0 and r.probe.wall_ms == pytest.approx(r.e2e_wall_ms)
+    for o in (out, t, u):
+        o.free()
