@@ -384,7 +384,9 @@ phj_status phj_batch_run(phj_ctx *ctx, uint32_t n, const phj_table *const *build
  * to `batch_max_joins`, run through phj_batch_run.  Each request's inputs
  * are generated on the device when it starts (phj_gen_spec); its output is
  * fingerprinted on the device and freed.  workers = 1 with batching off is
- * the plain one-join-per-call form. */
+ * the plain one-join-per-call form.  A slot's context keeps the memory of its
+ * largest job between jobs (see phj_ctx_create); the budget counts requests in
+ * flight. */
 typedef struct phj_serve_config {
     int device;
     uint32_t workers;              /* execution slots, 1..64 */

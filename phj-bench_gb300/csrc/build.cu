@@ -23,6 +23,7 @@ namespace
 constexpr int kBuildNT = 256;
 constexpr uint32_t kSmemCellsMax = 8192; // 128 KiB of cells per CTA
 constexpr uint32_t kLookers = 1024;
+constexpr uint32_t kInlineLeafRows = 32; // the fewest rows a leaf, in the mean, of inline tables
 
 // Cells of a table for r rows: the power of two at or above r * pct / 100
 // (pct 200: load <= 1/2, the reference's JoinHashTable::reserve), and above r.
@@ -537,6 +538,35 @@ static uint64_t leaf_rows_estimate(uint64_t rows, uint64_t n_leaves)
     return (uint64_t)(m + 6.0 * std::sqrt(m) + 8.0);
 }
 
+// Cells a leaf of an inline table that holds `est` rows at the load.
+static uint64_t inline_cells(uint64_t est, uint32_t pct)
+{
+    return (std::max(est * pct / 100, est + 1) + 1) & ~1ull;
+}
+
+// Whether general tables of `est` rows a leaf are sized by that estimate: up
+// to 9 cells a row at the default load.  Leaves of 390 rows have 5.2 then, and
+// 2.6 by their count: 100K x 800K rows of 12 payload bytes 104 us against 150,
+// 900K x 7.2M 231 and 292, 7M x 56M 1,322 and 1,466, 14M x 64M 1,825 and 1,957;
+// 28M x 64M 2,713 and 2,581.
+static bool estimate_fits(uint64_t rows, uint64_t n_leaves, uint64_t est, uint32_t pct)
+{
+    return n_leaves * table_cells(est, pct) * 200 <= 9 * rows * pct;
+}
+
+uint64_t estimated_table_bytes(uint64_t rows, uint32_t total_bits, uint64_t payload_bytes, bool unique)
+{
+    constexpr uint32_t kPct = 200;
+    const uint64_t n_leaves = 1ull << total_bits, est = leaf_rows_estimate(rows, n_leaves);
+    uint64_t bytes = 0;
+    const bool in_cells = payload_bytes <= 8 && rows >> total_bits >= kInlineLeafRows;
+    if (in_cells)
+        bytes = n_leaves * inline_cells(est, kPct) * sizeof(Cell);
+    if (!(in_cells && unique) && estimate_fits(rows, n_leaves, est, kPct))
+        bytes = std::max(bytes, n_leaves * table_cells(est, kPct) * sizeof(Cell) + rows * 8);
+    return bytes;
+}
+
 // Rows that a table of `cells` may hold at the load the option allows.
 static uint32_t rows_at_load(uint64_t cells, uint32_t pct)
 {
@@ -547,11 +577,11 @@ bool build_inline_tables(phj_ctx * ctx, Scratch & s, const Cols & part, uint64_t
                          const PackSpec & pk, InlineTables & t, int * bad)
 {
     const uint64_t n_leaves = 1ull << total_bits;
-    // fewer than 32 rows a leaf: the margin would make the tables sparse
-    if (rows >> total_bits < 32)
+    // fewer rows a leaf: the margin would make the tables sparse
+    if (rows >> total_bits < kInlineLeafRows)
         return false;
     const uint64_t est = leaf_rows_estimate(rows, n_leaves);
-    t.cap = (uint32_t)std::min<uint64_t>((std::max(est * ctx->table_cap_pct / 100, est + 1) + 1) & ~1ull, 1u << 30);
+    t.cap = (uint32_t)std::min<uint64_t>(inline_cells(est, ctx->table_cap_pct), 1u << 30);
     const size_t smem = (size_t)t.cap * 16;
     if (smem + 2048 > ctx->smem_optin || ctx->table_cap_pct < 125)
         return false;
@@ -636,11 +666,11 @@ void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, cons
     lt.flags = reinterpret_cast<int *>(small + 1);
     uint64_t max_cap;
     const uint64_t est = estimate_rows ? leaf_rows_estimate(estimate_rows, n_leaves) : 0;
-    lt.estimated = est && (uint64_t)n_leaves * table_cells(est, ctx->table_cap_pct) * 200 <= 9 * estimate_rows * ctx->table_cap_pct;
+    lt.estimated = est && estimate_fits(estimate_rows, n_leaves, est, ctx->table_cap_pct);
     if (lt.estimated)
     {
-        // uniform tables at the estimated size, up to 4.5 cells a row at
-        // the default load: no size is read back before the build
+        // uniform tables at the estimated size: no size is read back before
+        // the build
         lt.max_rows = (uint32_t)est;
         max_cap = table_cells(est, ctx->table_cap_pct);
         lt.uniform_log2cap = (int)(63 - __builtin_clzll(max_cap));

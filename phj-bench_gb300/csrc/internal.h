@@ -397,6 +397,9 @@ struct InlineTables
 // (lt.groups): they are then followed through group_leaf_duplicates only.
 void build_leaf_tables(phj_ctx * ctx, Scratch & s, const Cols & build_part, const uint32_t * leaf_off, uint32_t n_leaves,
                        LeafTables & lt, bool lazy = false, uint64_t estimate_rows = 0, const Cols * group_dst = nullptr);
+// The most device bytes PHJ-PURE's tables sized by estimate take at default
+// options (0: the sizes are counted); `unique`: no build key repeats.
+uint64_t estimated_table_bytes(uint64_t rows, uint32_t total_bits, uint64_t payload_bytes, bool unique);
 // Inline tables over leaf-partitioned build rows, sized by estimate: false
 // (nothing done) when the leaves are too small or too large for them.
 // *bad (device, zero before) receives what the build found.

@@ -69,19 +69,36 @@ uint64_t side_row_bytes(const phj_schema & s)
 }
 
 // Estimated device bytes a request holds while it runs: its inputs, the
-// table (cells at load <= 1/2 plus the next-chain), the partition buffers of
-// a join run alone (both sides' shuffles) or the partitioned copies of a
+// table (cells at load <= 1/2 plus the next-chain, or the tables sized by
+// estimate that a join run alone may take), the partition buffers of a join
+// run alone (both sides' shuffles) or the partitioned copies of a
 // batched one, and an output of one row per probe row.
-uint64_t estimate_footprint(const phj_serve_request & r, bool batched)
+uint64_t estimate_footprint(const phj_serve_request & r, bool batched, uint32_t total_bits)
 {
     const uint64_t B = r.build.rows, P = r.probe.rows;
     const uint64_t rb = side_row_bytes(r.build.schema), rp = side_row_bytes(r.probe.schema);
     const uint64_t cells = B ? bit_ceil64(2 * B) : 1;
     const uint64_t in = B * rb + P * rp;
-    const uint64_t table = cells * 16 + B * 8;
+    const uint64_t counted = cells * 16 + B * 8;
+    const uint64_t table = batched || !B ? counted : std::max(counted, estimated_table_bytes(B, total_bits, rb - 8, r.build.kind <= 1));
     const uint64_t buffers = batched ? B * rb + P * rp : 2 * B * rb + P * rp + P * 4;
     const uint64_t out = P * (rb + rp - 8);
     return in + table + buffers + out;
+}
+
+// Radix bits of a request run alone: the configured ones, or the size's.
+uint32_t radix_bits(const phj_serve_request & r, const uint8_t * pass_bits, uint32_t n_passes)
+{
+    uint8_t own[32];
+    if (n_passes == 0)
+    {
+        phj_autotune_radix(r.build.rows, r.probe.rows, own, &n_passes);
+        pass_bits = own;
+    }
+    uint32_t total = 0;
+    for (uint32_t i = 0; i < n_passes; ++i)
+        total += pass_bits[i];
+    return std::min<uint32_t>(total, 24);
 }
 
 bool is_small(const phj_server & s, uint64_t id)
@@ -322,7 +339,7 @@ phj_status phj_serve_submit(phj_server * S, const phj_serve_request * r, uint64_
     rec.status = -1;
     S->recs.push_back(rec);
     const bool small = S->cfg.batch_max_build_rows > 0 && S->cfg.batch_max_joins > 1 && r->build.rows <= S->cfg.batch_max_build_rows;
-    S->footprint.push_back(estimate_footprint(*r, small));
+    S->footprint.push_back(estimate_footprint(*r, small, radix_bits(*r, S->cfg.pass_bits, S->cfg.n_passes)));
     S->recs.back().footprint_bytes = S->footprint.back();
     if (id)
         *id = k;
@@ -397,7 +414,7 @@ void phj_serve_destroy(phj_server * S)
 
 uint64_t phj_serve_footprint(const phj_serve_request * r, int batched)
 {
-    return r ? estimate_footprint(*r, batched != 0) : 0;
+    return r ? estimate_footprint(*r, batched != 0, radix_bits(*r, nullptr, 0)) : 0;
 }
 
 } // extern "C"

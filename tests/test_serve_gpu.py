@@ -199,3 +199,22 @@ def test_admission_budget_serialises_large_requests():
     spans = sorted((r["start_s"], r["done_s"]) for r in recs)
     for (s0, d0), (s1, d1) in zip(spans, spans[1:]):
         assert s1 >= d0 - 1e-6
+
+
+@pytest.mark.parametrize("bits,tb,kind", [
+    ((8, 8), [P.U64], 0),       # about 32 rows a leaf: 4.6 cells a row in inline tables
+    ((8, 8), [P.U64], 2),       # ... and repeated keys, for which they are given up
+    ((6, 6), [P.U64, P.U32], 0),
+    ((), [P.U64], 2),
+])
+def test_admission_estimate_covers_tables_sized_by_estimate(bits, tb, kind):
+    B, Pn = 1 << 21, 2_000_000
+    srv = P.Server(workers=1, pass_bits=bits)
+    for i in range(2):  # the second time with the block of the first
+        b = P.gen_spec(kind, B, 31 + i, 41, tb)
+        srv.submit(b, P.gen_spec(4, Pn, 51 + i, 41, [P.U32], domain=B, match_permille=150), 0.0)
+    recs = srv.run(timeout_s=120)
+    srv.close()
+    for r in recs:
+        assert r["status"] == 0
+        assert 0 < r["job_peak_bytes"] <= r["footprint_bytes"] * 1.05 + (8 << 20), r
