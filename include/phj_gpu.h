@@ -149,8 +149,9 @@ typedef struct phj_output phj_output; /* a device-resident JoinOutput (src/JoinO
  * memory, and one block for the calls' scratch, sized by the most that a call
  * held of it and an eighth more, at most a quarter of the device's memory.
  * The block grows at the start of the call after the one that needed more,
- * which then waits for this context's stream; a call that runs out of memory
- * beside the block runs again without it. */
+ * which then waits for this context's stream.  A call that runs out of memory
+ * runs again, and it and the next 64 calls do without the block and take the
+ * forms that need the least (tables of counted sizes, no copies for speed). */
 phj_status phj_ctx_create(int device, phj_ctx **out);
 void phj_ctx_destroy(phj_ctx *ctx);
 /* Waits for the context's stream and gives that memory back to the device

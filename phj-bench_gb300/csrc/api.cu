@@ -193,15 +193,6 @@ void arena_release(phj_ctx * ctx) noexcept
     a.size = a.used = 0;
 }
 
-void arena_retreat(phj_ctx * ctx) noexcept
-{
-    ScratchArena & a = ctx->arena;
-    a.most = std::max(a.size, a.want) / 2;
-    a.calls = 0;
-    arena_release(ctx);
-    a.want = 0;
-}
-
 // What both pools hold free, back to the device.
 static void pools_trim(phj_ctx * ctx)
 {
@@ -210,11 +201,19 @@ static void pools_trim(phj_ctx * ctx)
     cudaMemPoolTrimTo(ctx->scratch_pool, 0);
 }
 
+void arena_retreat(phj_ctx * ctx) noexcept
+{
+    arena_release(ctx);
+    pools_trim(ctx); // (the other pool cannot take from the block's)
+    ctx->arena.want = 0;
+    ctx->lean = kLeanCalls;
+}
+
 void arena_begin(phj_ctx * ctx)
 {
     ScratchArena & a = ctx->arena;
     a.used = a.held = a.asked = 0;
-    if (a.off || a.want <= a.size)
+    if (ctx->lean || a.want <= a.size)
         return;
     // grown to what the last call held; what the pool kept for that call goes
     // back first.  Only this context's streams are waited for.
@@ -229,8 +228,7 @@ void arena_begin(phj_ctx * ctx)
     }
     else
     {
-        // no room: this call's scratch comes from the pool, and a next
-        // attempt asks for less
+        // no room: this call's scratch comes from the pool
         cudaGetLastError();
         arena_retreat(ctx);
     }
@@ -240,16 +238,9 @@ void arena_begin(phj_ctx * ctx)
 void arena_end(phj_ctx * ctx) noexcept
 {
     ScratchArena & a = ctx->arena;
-    if (a.off)
-        return;
-    if (a.most < a.bound && ++a.calls >= 64)
-    {
-        a.most = std::min(a.bound, std::max<size_t>(a.most, 1 << 20) * 2);
-        a.calls = 0;
-    }
     // an eighth and 2 MiB more than was held, so that a little more the
     // next time is no new growth
-    if (a.asked > a.size)
+    if (!ctx->lean && a.asked > a.size)
         a.want = std::min<size_t>(a.asked + a.asked / 8 + (2 << 20), a.most) & ~size_t(255);
 }
 
@@ -864,7 +855,7 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
     const uint64_t payload = schema_bytes(B.schema);
     const uint64_t gathered = B.schema.n_payloads >= 2 && payload <= 16 ? 16 : payload;
     const bool past_l2 = B.rows * (48 + gathered) > ctx->l2_bytes / 5 * 6;
-    if (ctx->chj_windows <= 1 && P.rows > 0 && (ctx->probe_materialize < 0 ? past_l2 : ctx->probe_materialize == 1))
+    if (ctx->chj_windows <= 1 && P.rows > 0 && (ctx->probe_materialize < 0 ? past_l2 && !ctx->lean : ctx->probe_materialize == 1))
     {
         try
         {
@@ -875,6 +866,7 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
             // no room for the clustered copy of the probe side: without it
             if (e.status != PHJ_ERR_OUT_OF_MEMORY)
                 throw;
+            ctx->lean = kLeanCalls; // (nor in the next calls)
         }
     }
     run_chj_form(ctx, B, P, out, res, false);
@@ -1052,7 +1044,7 @@ static void run_phj_pure(phj_ctx * ctx, const phj_table & B, const phj_table & P
         lt.next = st->get<uint64_t>(B.rows);
         // (grouping needs a place for the payloads: the partition's temporary)
         const Cols * group_dst = btmp.keys != bpart.keys ? &btmp : nullptr;
-        build_leaf_tables(ctx, *st, bpart, leaf_off, n_leaves, lt, false, inline_found & kLeafOverflow ? 0 : B.rows, group_dst);
+        build_leaf_tables(ctx, *st, bpart, leaf_off, n_leaves, lt, false, (inline_found & kLeafOverflow) || ctx->lean ? 0 : B.rows, group_dst);
         if (lt.estimated)
         {
             // the one-pass probe goes ahead; when the tables turn out not
@@ -1997,7 +1989,7 @@ phj_status phj_ctx_create(int device, phj_ctx ** out)
         ctx->num_sms = prop.multiProcessorCount;
         ctx->smem_optin = prop.sharedMemPerBlockOptin;
         ctx->l2_bytes = prop.l2CacheSize;
-        ctx->arena.most = ctx->arena.bound = prop.totalGlobalMem / 4;
+        ctx->arena.most = prop.totalGlobalMem / 4;
         // the main stream goes first: its kernels take the SMs as the side
         // stream's short CTAs end (probe side's first pass, see k_scatter)
         int prio_least = 0, prio_greatest = 0;

@@ -751,7 +751,7 @@ void build_global_table(phj_ctx * ctx, Scratch & s, const phj_table & build, uin
     // plans: the tables' fill starts 12 us after the count did instead of 47
     // (342K x 3.6M rows: 208 -> 170 us a join, 669K x 2.7M 213 -> 177).  More
     // rows are counted first: the exact size is then worth the round trip.
-    const bool plan = n <= (16u << 20) && n_slots <= 1024;
+    const bool plan = n <= (16u << 20) && n_slots <= 1024 && !ctx->lean;
     if (plan)
     {
         lt.total_cells = std::max<uint64_t>(4 * n, 2);

@@ -104,14 +104,12 @@ struct ScratchArena
     size_t held = 0;   // scratch bytes held now, with those from the pool
     size_t asked = 0;  // the most held at a time in this call
     size_t want = 0;   // size for the next call
-    size_t most = 0;   // bound of `size`: `bound`, less after a call ran out of memory
-    size_t bound = 0;
-    uint32_t calls = 0; // since `most` was lowered
+    size_t most = 0;   // bound of `size`
     phjg::Scratch * top = nullptr; // innermost Scratch alive
-    bool off = false;  // this call runs from the pool alone
 };
 
 constexpr int64_t kHostChunkRows = 16ll << 20; // default of "host_chunk_rows"
+constexpr uint32_t kLeanCalls = 64; // calls that spare memory after one ran out of it
 
 struct phj_ctx
 {
@@ -130,6 +128,7 @@ struct phj_ctx
     // Allocation accounting of the current run (peak_mem_bytes).
     uint64_t cur_bytes = 0, peak_bytes = 0;
     uint64_t device_bytes = 0; // held now, the arena's whole block included
+    uint32_t lean = 0; // calls that spare memory yet: no arena, tables of counted sizes, no copies for speed
     std::vector<std::pair<void *, uint64_t>> live; // small: a run holds tens of buffers
     ScratchArena arena;
     // Per-kernel timing of the last run.
@@ -224,8 +223,8 @@ void arena_begin(phj_ctx * ctx);
 void arena_end(phj_ctx * ctx) noexcept;
 // Gives the arena's memory back (no call may be using it).
 void arena_release(phj_ctx * ctx) noexcept;
-// The same after a call ran out of memory beside it: the next calls keep at
-// most half as much, twice that again after each 64 that did not.
+// The same after a call ran out of memory: the next kLeanCalls calls do
+// without it and take the forms that need the least.
 void arena_retreat(phj_ctx * ctx) noexcept;
 
 // RAII holder for run-scoped scratch: cut from the context's arena while it
@@ -278,7 +277,7 @@ struct Scratch
         const size_t bytes = ((size_t)(n ? n : 1) * sizeof(T) + 255) & ~size_t(255);
         ScratchArena & a = ctx->arena;
         T * p;
-        if (!a.off && bytes <= a.size - a.used)
+        if (bytes <= a.size - a.used)
         {
             for (Scratch * t = a.top; t != this; t = t->outer)
                 t->covered = true;
@@ -628,19 +627,15 @@ inline phj_status guard(phj_ctx * ctx, F && f)
         try
         {
             f();
+            if (ctx && ctx->lean)
+                --ctx->lean;
         }
         catch (const Error & e)
         {
-            // out of memory while the arena holds some: once more without it
-            if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || !ctx->arena.base)
+            // out of memory: once more with less
+            if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || (!ctx->arena.base && ctx->lean))
                 throw;
             arena_retreat(ctx);
-            struct Off
-            {
-                phj_ctx * c;
-                ~Off() { c->arena.off = false; }
-            } off{ctx};
-            ctx->arena.off = true;
             f();
         }
         if (ctx)

@@ -124,3 +124,25 @@ def test_trim_gives_the_kept_memory_back():
         assert tuple(out.fingerprint()) == fp
         for o in (out, t, u):
             o.free()
+
+
+@pytest.mark.parametrize("scheme,limit", [("pure", 64), ("chj", 52)])
+def test_tables_of_counted_sizes_where_the_estimated_ones_do_not_fit(scheme, limit):
+    # 400K rows of 12 payload bytes on 400K: 12.8 MB of inputs, 8 partitioned
+    # (PHJ-PURE), 3.2 of chains, 6.4 packed, 9.6 of output, and 33.6 MB of
+    # tables by estimate (25.6 planned in CHJ) against 16.8 counted
+    with P.Context(0) as c:
+        c.set_int("probe_materialize", 0)
+        b, p, t, u = sides(c, 400_000, 400_000, types=(P.U64, P.U32))
+        fp = tuple(O.join_fingerprint(b, p))
+        c.set_int("test_memory_limit_mib", limit)
+        launches = []
+        for _ in range(4):
+            n0 = c.launch_count()
+            o, _ = c.run_phj_pure(t, u, [10]) if scheme == "pure" else c.run_chj(t, u)
+            launches.append(c.launch_count() - n0)
+            assert tuple(o.fingerprint()) == fp
+            o.free()
+        assert launches[0] > launches[1] == launches[2] == launches[3], launches
+        c.set_int("test_memory_limit_mib", 0)
+        t.free(), u.free()
