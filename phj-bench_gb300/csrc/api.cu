@@ -831,8 +831,9 @@ static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj
 
 static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj_output ** out, phj_chj_result * res)
 {
-    // (payloads the one-pass probe takes: both forms look up and project in
-    // one kernel and are recorded under its name)
+    // Payloads the one-pass probe takes: the record's name is the step's,
+    // "probe_fused" (its form tells the two kernels apart).  Other payloads keep
+    // the general path, which CHJ has always taken for them.
     cudaEvent_t ev[3];
     if (phj_output * o = one_pass_schemas(B.schema, P.schema) ? try_small_join(ctx, B, P, "probe_fused", ev) : nullptr)
     {
@@ -1322,11 +1323,12 @@ static void run_phj_bep(phj_ctx * ctx, const phj_table & B, const phj_table & P,
 
 // PHJ (BEP) with the byte budget on the device (bep_engine.cu): the build
 // side is partitioned to full leaf depth (src/PHJBep.cpp:128-141) and its
-// tables only planned; one persistent grid then streams the probe side
-// through per-group unrefined chains, refines, evicts and builds leaves
-// lazily, and projects into the output.  The output is sized for one row
-// per probe row; a join with more output rows (repeated build keys) runs
-// the grid again into an output of the exact size the first run counted.
+// tables only planned; scatter launches, which stream the probe side through
+// per-group unrefined chains and refine, and evictions, which build leaves
+// lazily, probe and project into the output, then take turns.  The output is
+// sized for one row per probe row; a join with more output rows (repeated
+// build keys) runs again into an output of the exact size the first run
+// counted.
 static void run_phj_bep_engine(phj_ctx * ctx, const phj_table & B, const phj_table & P, const std::vector<uint32_t> & bits, uint64_t budget_mib,
                                phj_output ** out, phj_bep_result * res)
 {

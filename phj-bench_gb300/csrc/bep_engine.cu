@@ -602,7 +602,9 @@ __device__ __forceinline__ uint32_t allocate_step(const EngineArgs & a, const Sm
 // fills them: 5.4 us a step of 4096 rows of 12 bytes, against 8.6 us for
 // steps of all 1024 threads, whose first warp scanned the buckets alone.
 // What bounds it now is the instructions of a row (issue slots 40% busy, DRAM
-// 21%, 8 to 9 warps of 32 at a barrier).  hf.bins is zero on entry and on a kTileDone return.
+// 21%, 8 to 9 warps of 32 at a barrier).  The kernel is held to 64 registers,
+// which the step, the refines and the arguments share: 182 bytes of spill
+// stores and 432 of loads a thread; what they cost has not been measured.  hf.bins is zero on entry and on a kTileDone return.
 __device__ uint32_t scatter_step(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t half, uint32_t k, uint32_t n, bool ok)
 {
     const Half & hf = sm.hf;
@@ -769,9 +771,6 @@ __device__ void refine_bucket(const EngineArgs & a, const Smem & sm, uint32_t g,
     __syncthreads();
 }
 
-// Refines the group's largest bucket (src/PHJBep.cpp:376-395) until its
-// unrefined bytes are below `low` (every bucket that holds rows when low
-// is 0).
 // A warp's refine of a bucket of few rows: as refine_bucket, counted without
 // shared memory (rows of one leaf in a step of 32 rows together).
 __device__ __forceinline__ void refine_small(const EngineArgs & a, const Smem & sm, uint32_t g, uint32_t p, unsigned long long c0)
@@ -818,8 +817,10 @@ __device__ __forceinline__ void refine_small(const EngineArgs & a, const Smem & 
     }
 }
 
-// (Of equal buckets the first.)  The buckets so refined are the first ones
-// in that order, so they are found at once -- by a binary search of the
+// Refines the group's largest bucket, of equal ones the first
+// (src/PHJBep.cpp:376-395), until its unrefined bytes are below `low` (every
+// bucket that holds rows when low is 0).  The buckets so refined are the first
+// ones in that order, so they are found at once -- by a binary search of the
 // order's last key -- and refined side by side: those of few rows a warp
 // each, the others by the whole CTA.  One after the other they took 2 to 5
 // us each, most of it barriers and the search for the largest (2M x 10M Zipf
@@ -1046,7 +1047,7 @@ __device__ __forceinline__ uint64_t block_len(const EngineArgs & a, unsigned lon
 
 // A lookup in two halves, so that several rows' first loads are in flight
 // at once: probe_issue loads the aligned pair of cells the key's probe
-// starts at (through L2: the leaf's table was built during this launch);
+// starts at (through L2);
 // probe_finish compares, follows the table past the pair when needed, and
 // returns the match count (the next-chain's length when some leaf table has
 // a repeated key) and the head build row.
@@ -1488,7 +1489,8 @@ __global__ void __launch_bounds__(kBPNT, 3) k_bep_probe(const __grid_constant__ 
 }
 
 // E's probes in every other case: chains are followed, columns of any width
-// are copied row by row.  `only_dup`: k_bep_probe has done the work unless a
+// are copied row by row.  (64 registers, 180 and 176 bytes spilled; k_bep_probe
+// spills 60 and 80 against tables of unequal size, 8 and 8 of one.)  `only_dup`: k_bep_probe has done the work unless a
 // key repeats.
 __global__ void __launch_bounds__(kBPNT, 4) k_bep_probe_chains(const __grid_constant__ EngineArgs a, int only_dup)
 {

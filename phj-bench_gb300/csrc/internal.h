@@ -482,9 +482,11 @@ uint32_t bep_smem_cells(const LeafTables & lt);
 void set_bep_smem_limits(int smem_optin);
 
 // ----- bep_engine.cu ------------------------------------------------------------------
-// PHJ/BEP with the probe-side byte budget kept on the device: one
-// persistent grid of CTA groups with per-group unrefined chains, water
-// marks, refinement, round-robin eviction and lazy leaf builds.
+// PHJ/BEP with the probe-side byte budget kept on the device: CTA groups with
+// their own unrefined chains scatter and refine at the water marks in a
+// cooperative launch; each round-robin eviction, with the lazy leaf builds and
+// the probes, is a sequence of launches after it; the host reads the state back
+// between.
 struct BepEngineInput
 {
     Cols probe; // probe side in input order
@@ -550,10 +552,10 @@ phj_output * probe_join(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, const p
 // Sets a.packed (and packed_off) when the plain projection can use packed
 // build payloads (a.any_dup known, build_rows rows in a.build).
 void pack_build_payloads(phj_ctx * ctx, Scratch & s, ProbeArgs & a, uint64_t build_rows);
-// The two halves: lookups + chunk-offset scan (returns the output rows), and
-// the projection into `out` from row `out_base` on.
 // Whether the one-pass probe takes these payload columns (unique keys).
 bool one_pass_schemas(const phj_schema & build, const phj_schema & probe);
+// The two halves: lookups + chunk-offset scan (returns the output rows), and
+// the projection into `out` from row `out_base` on.
 uint64_t probe_chunks(uint64_t probe_rows);
 uint64_t probe_lookup(phj_ctx * ctx, Scratch & s, const ProbeArgs & a, uint32_t * heads, uint32_t * counts);
 void probe_project(phj_ctx * ctx, const ProbeArgs & a, phj_output * out, uint64_t out_base, const uint32_t * heads, const uint32_t * offs,
