@@ -777,11 +777,13 @@ static phj_output * try_small_join(phj_ctx * ctx, const phj_table & B, const phj
     ev[0] = take_event(ctx);
     ev[1] = ev[2] = take_event(ctx);
     // Sized for one output row a probe row, exact for unique build keys; a
-    // join with more runs again into an output of the size it counted.  Its
-    // chains are written a row at a time, so past 400K probe rows a repeated
-    // key leaves the join to the general path before anything is probed
-    // (8K x 128K, four rows a key: 103 us in two launches against 180; 8K x
-    // 512K: 190 against 182).
+    // join with more runs again into an output of the size it counted.  Two
+    // launches win up to 400K probe rows (8K x 128K, four rows a key: 71 us
+    // against 187 in the general path; 8K x 400K 87 against 186, of 64 rows a key
+    // 210 against 312, and with 20 payload bytes 306 against 314; 64K x 400K 131
+    // against 190).  Past them a repeated key leaves the join to the general
+    // path before anything is probed: with chains written a row at a time 8K x
+    // 512K took 190 us against 182, and the line has not been measured again.
     const bool repeats_ok = P.rows <= 400000;
     // (the general path sizes its output exactly where keys repeat or the
     // payloads do not suit the one-pass probe: few matches may fit there)
