@@ -854,10 +854,14 @@ static void run_chj(phj_ctx * ctx, const phj_table & B, const phj_table & P, phj
     // 12 payload bytes: 1.3M x 5M 300 -> 334 us clustered, 2M x 32M 957 ->
     // 928, 2.5M x 20M 760 -> 684, 4M x 32M 1,301 -> 1,088; of 4 bytes: 2M x
     // 32M 819 -> 889, 4M x 16M 717 -> 673; repeated keys 2.5M x 20M 2,293 ->
-    // 2,302, 4M x 32M 3,752 -> 3,598.  "probe_materialize" forces either.
+    // 2,302, 4M x 32M 3,752 -> 3,598.  Where lookup and projection are two
+    // kernels the pass pays later: the line is twice L2 (x 40M rows, 24 payload
+    // bytes in three columns: 3M 1,260 -> 1,303, 6M 2,276 -> 1,723; 12 not packed: 3M
+    // 1,015 -> 1,123, 6M 1,565 -> 1,334).  "probe_materialize" forces either.
     const uint64_t payload = schema_bytes(B.schema);
-    const uint64_t gathered = B.schema.n_payloads >= 2 && payload <= 16 ? 16 : payload;
-    const bool past_l2 = B.rows * (48 + gathered) > ctx->l2_bytes / 5 * 6;
+    const bool one_kernel = ctx->probe_fused && one_pass_schemas(B.schema, P.schema) && (ctx->pack_build || B.schema.n_payloads < 2);
+    const uint64_t gathered = one_kernel && B.schema.n_payloads >= 2 ? 16 : payload;
+    const bool past_l2 = B.rows * (48 + gathered) > (one_kernel ? ctx->l2_bytes / 5 * 6 : ctx->l2_bytes * 2);
     if (ctx->chj_windows <= 1 && P.rows > 0 && (ctx->probe_materialize < 0 ? past_l2 && !ctx->lean : ctx->probe_materialize == 1))
     {
         try

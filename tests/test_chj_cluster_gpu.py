@@ -31,3 +31,28 @@ def test_clustered_rows_equal_the_oracle(ctx, name):
         finally:
             ctx.set_int("probe_materialize", -1)
         assert O.compare_outputs(expected, O.serialize_output(r.output)) == ""
+
+
+@pytest.mark.parametrize("build,types,pack,clustered", [
+    (3_000_000, [P.U64, P.U32], 1, True),     # one kernel looks up and projects: the line is 1.2 x L2
+    (3_000_000, [P.U64, P.U32], 0, False),    # two kernels: twice L2
+    (3_000_000, [P.U64] * 3, 1, False),
+    (6_000_000, [P.U64] * 3, 1, True),
+])
+def test_when_the_probe_side_is_put_in_order(ctx, build, types, pack, clustered):
+    b = ctx.generate(0, build, 751, 752, types)
+    p = ctx.generate(4, 4_000_000, 753, 752, [P.U64], domain=build, match_permille=700)
+    fps = []
+    for m in (-1, 0):
+        ctx.set_int("pack_build", pack)
+        ctx.set_int("probe_materialize", m)
+        try:
+            out, _ = ctx.run_chj(b, p)
+        finally:
+            ctx.set_int("pack_build", 1)
+            ctx.set_int("probe_materialize", -1)
+        assert ("probe_scatter" in {k["name"] for k in ctx.kernel_times()}) == (clustered and m < 0)
+        fps.append(out.fingerprint())
+        out.free()
+    assert fps[0] == fps[1]
+    b.free(), p.free()
