@@ -99,3 +99,22 @@ def test_one_crowded_leaf_of_many(ctx, bt, crowded):
     r = P.runPHJ(b, p, [6, 6], ctx=ctx)
     assert "build_leaf_tables" in {k["name"] for k in ctx.kernel_times()}
     assert O.compare_outputs(O.join_rows(b, p), O.serialize_output(r.output)) == ""
+
+
+@pytest.mark.parametrize("mat,builds", [(0, 1), (1, 1)])
+def test_large_tables_in_input_order_are_counted(ctx, mat, builds):
+    # 3M rows of 12 payload bytes in 16,384 leaves: 268 MB of tables by
+    # estimate, past L2; probed in input order their sizes are counted
+    b = ctx.generate(0, 3_000_000, 761, 762, [P.U64, P.U32])
+    p = ctx.generate(4, 3_000_000, 763, 762, [P.U32], domain=3_000_000, match_permille=700)
+    ctx.set_int("probe_materialize", mat)
+    try:
+        out, r = ctx.run_phj_pure(b, p, [7, 7])
+    finally:
+        ctx.set_int("probe_materialize", -1)
+    assert [k["name"] for k in ctx.kernel_times()].count("build_leaf_tables") == builds
+    tables = (268 if mat else 134) * 10**6
+    inputs, copies, out_bytes = 3_000_000 * 32, 3_000_000 * (2 * 20 + 8 + 16 + 12 * mat), 3_000_000 * 24
+    assert abs(r.peak_mem_bytes - (inputs + copies + out_bytes + tables)) < 30 * 10**6, r.peak_mem_bytes
+    for o in (out, b, p):
+        o.free()
