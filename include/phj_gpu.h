@@ -173,7 +173,7 @@ void *phj_ctx_stream(phj_ctx *ctx);
  *        (PHJ/BEP leaf builds), 1..60000, default 1000;
  *   "host_chunk_rows": probe rows per chunk of phj_run_phj_pure_host (>= 4096;
  *        at the default of 16M it is the most: short probe sides go in
- *        smaller chunks);
+ *        smaller chunks between pinned columns);
  *   "table_cap_pct": leaf table cells >= rows * pct / 100, rounded up to a
  *        power of two (110..800, default 200: the reference's bit_ceil(2 rows));
  *   "p1_tile_rows", "p1_stages": tile rows (1024/2048/4096) and bulk-copy

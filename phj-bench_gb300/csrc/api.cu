@@ -1473,13 +1473,42 @@ struct CopyDrain
 // copies (0.45 ms of uploads) have to cover.  2M x 24M rows of 16 bytes: 5.37
 // ms in chunks of 16M rows, 4.66 of 6M, 4.77 of 2M, 5.94 of 1M; 4M x 64M 11.6,
 // 11.0, 11.6 and 15.0; 1M x 12M of 12 bytes, a fifth matching: 1.30 of 16M,
-// 1.28 of 8M, 1.39 of 4M; 16M x 256M 41.7 of 16M or 8M, 42.2 of 6M.
-static uint64_t host_chunk_rows(const phj_ctx * ctx, const phj_block_stream & probe)
+// 1.28 of 8M, 1.39 of 4M; 16M x 256M 41.7 of 16M or 8M, 42.2 of 6M.  Downloads
+// into pageable memory go through the host and overlap nothing, so they want
+// large chunks: 1M x 24M rows of 40 bytes 15.5 ms in chunks of 16M rows, 17.1 of
+// 2.5M, 500K x 6M 3.0 and 3.4.  Uploads from pageable memory cost more a copy,
+// which up to 256 MiB of them is more than the overlap saves (500K x 6M rows of
+// 40 bytes in nine columns, a side: 3.25 ms of 6M and 3.63 of 2.5M; 1M x 24M 18.6
+// and 17.6).
+static bool pageable(const void * p)
+{
+    cudaPointerAttributes at{};
+    if (p && cudaPointerGetAttributes(&at, p) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return true;
+    }
+    return p && at.type == cudaMemoryTypeUnregistered;
+}
+
+static uint64_t host_chunk_rows(const phj_ctx * ctx, const phj_block_stream & build, const phj_block_stream & probe, const uint64_t * out_keys,
+                                void * const * out_left, void * const * out_right)
 {
     const uint64_t most = (uint64_t)ctx->host_chunk_rows;
     if (ctx->host_chunk_rows != kHostChunkRows)
-        return most; // pinned
-    return std::min<uint64_t>(most, std::max<uint64_t>((96ull << 20) / (8 + schema_bytes(probe.schema)), probe.total_rows / 16));
+        return most; // pinned by the option
+    bool through_host = pageable(out_keys);
+    for (uint32_t c = 0; c < build.schema.n_payloads && out_left; ++c)
+        through_host = through_host || pageable(out_left[c]);
+    for (uint32_t c = 0; c < probe.schema.n_payloads && out_right; ++c)
+        through_host = through_host || pageable(out_right[c]);
+    bool from_host = pageable(probe.keys);
+    for (uint32_t c = 0; c < probe.schema.n_payloads; ++c)
+        from_host = from_host || pageable(probe.payloads[c]);
+    const uint64_t row = 8 + schema_bytes(probe.schema);
+    if (through_host || (from_host && probe.total_rows * row <= (256ull << 20)))
+        return most;
+    return std::min<uint64_t>(most, std::max<uint64_t>((96ull << 20) / row, probe.total_rows / 16));
 }
 
 // PHJ-PURE with the inputs and the output in host memory.  The build side
@@ -2509,7 +2538,8 @@ phj_status phj_run_phj_pure_host(phj_ctx * ctx, const phj_block_stream * build, 
         for (uint32_t c = 0; c < probe->schema.n_payloads; ++c)
             if ((probe->total_rows && !probe->payloads[c]) || (out_capacity && (!out_right || !out_right[c])))
                 throw Error(PHJ_ERR_INVALID_ARGUMENT, "null probe payload column");
-        run_phj_pure_host(ctx, *build, *probe, bits, out_capacity, out_keys, out_left, out_right, out_rows, result, host_chunk_rows(ctx, *probe));
+        run_phj_pure_host(ctx, *build, *probe, bits, out_capacity, out_keys, out_left, out_right, out_rows, result,
+                          host_chunk_rows(ctx, *build, *probe, out_keys, out_left, out_right));
     });
 }
 

@@ -28,3 +28,27 @@ def test_host_chunks_equal_the_oracle(ctx, rows, chunk):
         ctx.set_int("host_chunk_rows", 16 << 20)
     assert got == n
     assert O.compare_outputs(expected, O.serialize_output(P.JoinOutput(bt, pt, keys, left, right))) == ""
+
+
+@pytest.mark.parametrize("pinned,chunks", [((True, True, True, True), 4), ((True, True, False, True), 2), ((True, True, True, False), 2),
+                                           ((True, False, True, True), 2), ((False, True, True, True), 2)])
+def test_pageable_columns_take_large_chunks(pinned, chunks):
+    # 5.9M rows of 40 bytes (225 MiB): a quarter of a chunk, then chunks of
+    # 2.5M between pinned columns; a quarter and the rest where a probe or an
+    # output column is pageable
+    bt, pt = [P.U64], [P.U64] * 4
+    rows = 5_900_000
+    b = P.BlockStream(bt, G.gen_keys(0, 50_000, 911, 912), G.payload_columns(913, bt, 50_000))
+    pk, cols = G.gen_keys(4, rows, 914, 912, domain=50_000, match_permille=60), G.payload_columns(915, pt, rows)
+    fp = O.join_fingerprint(b, P.BlockStream(pt, pk, cols))
+    with P.Context(0) as c:
+        new = [c.pinned if x else (lambda shape, dtype: np.zeros(shape, dtype)) for x in pinned]
+        hk, hc = new[0]((rows,), np.uint64), [new[1]((rows,), np.uint64) for _ in pt]
+        for to, a in zip([hk] + hc, [pk] + cols):
+            to[...] = a
+        keys, left, right = c.pinned((fp[0],), np.uint64), [new[2]((fp[0],), np.uint64)], [new[3]((fp[0],), np.uint64) for _ in pt]
+        got, _ = c.run_phj_pure_host(b, P.BlockStream(pt, hk, hc), [4, 4], keys, left, right)
+        assert got == fp[0]
+        assert [k["name"] for k in c.kernel_times()].count("probe_lookup") == chunks
+        out = P.JoinOutput(bt, pt, keys, left, right)
+        assert O.rows_fingerprint(O.serialize_output(out), bt, pt) == tuple(fp)
