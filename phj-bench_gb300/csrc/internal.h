@@ -634,8 +634,8 @@ inline phj_status guard(phj_ctx * ctx, F && f)
         }
         catch (const Error & e)
         {
-            // out of memory: once more with less
-            if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || (!ctx->arena.base && ctx->lean))
+            // out of memory: once more with less (not while the context is made)
+            if (e.status != PHJ_ERR_OUT_OF_MEMORY || !ctx || !ctx->host_small || (!ctx->arena.base && ctx->lean))
                 throw;
             arena_retreat(ctx);
             f();
